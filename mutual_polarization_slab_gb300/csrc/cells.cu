@@ -10,6 +10,7 @@
 #include <string.h>
 
 #include "cells.cuh"
+#include "cellwalk.cuh"
 
 namespace mps {
 
@@ -70,62 +71,72 @@ __global__ void k_cell_rank(const int32_t *__restrict__ unsorted, const int32_t 
     }
 }
 
-// Neighbour cell o (0..26) of cell c: offsets (o / 9 - 1, o / 3 % 3 - 1, o % 3 - 1), the x offset
-// outermost as in the reference's loop.  Computed, not read from a __constant__ table, so the kernels
-// need no per-device upload and give the same offsets on every GPU of the process.
-__device__ __forceinline__ int32_t nb_cell(int32_t c, int o, int64_t ncx, int64_t ncy, int64_t ncz) {
-    int64_t cx = c % ncx, cy = (c / ncx) % ncy, cz = c / (ncx * ncy);
-    cx = wrap_index(cx + (o / 9 - 1), ncx);
-    cy = wrap_index(cy + ((o / 3) % 3 - 1), ncy);
-    cz = wrap_index(cz + (o % 3 - 1), ncz);
-    return (int32_t)(cx + ncx * (cy + ncy * cz));
+// Screen positions (near_position) of the points in sorted order (null: as they come): a walk's candidates are consecutive 16-byte loads.
+__global__ void k_near_positions(const double *__restrict__ x, const int32_t *__restrict__ sorted, int64_t n, Box3 box,
+                                 NearBox nb, float4 *__restrict__ xs) {
+    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x)
+        xs[s] = near_position(x, sorted ? sorted[s] : s, box, nb);
 }
 
-// Warp-per-particle walk over the candidates of the 27 neighbour cells in (cell
-// offset, position in the cell) order.  Lane o < 27 holds neighbour cell o's first
-// sorted position and the exclusive prefix of the cell counts; candidate j is
-// located by a binary search over those lanes.  One warp per particle keeps the
-// dependent loads (particle, cells, candidates) to a few per particle instead of a
-// few per (particle, cell).
-struct CellWalk {
-    int64_t cstart;   // lane o < 27: sorted position of neighbour cell o's first particle
-    int pre;          // lane o < 27: candidates in cells 0..o-1
-    int total;        // candidates of all 27 cells (warp-uniform)
-};
-
-__device__ __forceinline__ CellWalk cell_walk(int32_t c, int lane, const int32_t *__restrict__ counts,
-                                              const int64_t *__restrict__ starts, int64_t ncx, int64_t ncy,
-                                              int64_t ncz) {
-    CellWalk cw;
-    cw.cstart = 0;
-    int cnt = 0;
-    if (lane < 27) {
-        const int32_t nb = nb_cell(c, lane, ncx, ncy, ncz);
-        cw.cstart = starts[nb];
-        cnt = counts[nb];
+// Row of the first table separation >= d, at least 1 (the callers have checked d <= rv[ntab - 1]), from the
+// uniform-spacing guess (d - r0) inv_dr; a table that is far from uniform takes the binary search.
+__device__ __forceinline__ int64_t probe_row(const double *__restrict__ rv, int64_t ntab, double d, double inv_dr,
+                                             double r0 = 0.0) {
+    int64_t lo = 1, hi = ntab - 1;
+    const double gf = (d - r0) * inv_dr;
+    int64_t g = gf > 1.0 ? (gf < (double)hi ? (int64_t)gf : hi) : 1;
+    for (int it = 0; it < 4; ++it) {
+        if (rv[g] < d) {
+            lo = ++g;   // g <= hi: rv[hi] >= d
+        } else if (g > 1 && rv[g - 1] >= d) {
+            hi = --g;
+        } else {
+            return g;
+        }
     }
-    int v = cnt;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, v, d);
-        if (lane >= d) v += u;
+    while (lo < hi) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (rv[mid] >= d) hi = mid; else lo = mid + 1;
     }
-    cw.pre = v - cnt;
-    cw.total = __shfl_sync(0xffffffffu, v, 31);
-    return cw;
+    return lo;
 }
 
-// Cell offset o and sorted position of candidate j (0 <= j < total); all lanes call it.
-__device__ __forceinline__ void walk_at(const CellWalk &cw, int j, int &o, int64_t &pos) {
-    int lo = 0;
+// 1/v by Newton's method y <- y (2 - v y) from a float32 seed (two steps).
+__device__ __forceinline__ double rcp_newton(double v) {
+    double y = (double)(1.0f / (float)v);
+    y = y * (2.0 - v * y);
+    y = y * (2.0 - v * y);
+    return y;
+}
+
+// sqrt(d2) and its reciprocal without a float64 division: the square root of a zero separation is 0.
+__device__ __forceinline__ double probe_distance(double d2, double *inv) {
+    const double y = rsqrt(d2), d = d2 * y;
+    *inv = y;
+    return d2 > 0.0 ? fma(0.5 * y, fma(-d, d, d2), d) : d2;
+}
+
+// Minimum-image vector r - L trunc(2 r / L) of a probe/source pair and its squared length; the comparisons give the
+// same value for |r| < L and cost no division.
+__device__ __forceinline__ double probe_diff2(const double *__restrict__ xe, int64_t e, const double *__restrict__ xp,
+                                              int64_t b, const Box3 &box, double r[3]) {
+    double d2 = 0.0;
 #pragma unroll
-    for (int step = 16; step > 0; step >>= 1) {
-        const int mid = lo + step;
-        const int p = __shfl_sync(0xffffffffu, cw.pre, mid < 27 ? mid : 26);
-        if (mid < 27 && p <= j) lo = mid;
+    for (int k = 0; k < 3; ++k) {
+        double v = xe[3 * e + k] - xp[3 * b + k];
+        const double L = box.L[k];
+        if (fabs(v) < L) {
+            if (v >= 0.5 * L)
+                v -= L;
+            else if (v <= -0.5 * L)
+                v += L;
+        } else {
+            v -= L * trunc(2.0 * v / L);
+        }
+        r[k] = v;
+        d2 += v * v;
     }
-    o = lo;
-    pos = __shfl_sync(0xffffffffu, cw.cstart, lo) + (j - __shfl_sync(0xffffffffu, cw.pre, lo));
+    return d2;
 }
 
 // Field at probe points from the dipoles of sources within rc (Compute_Field/RealSpace.m:1-60
@@ -133,66 +144,49 @@ __device__ __forceinline__ void walk_at(const CellWalk &cw, int j, int &o, int64
 // the sources of the 27 cells around the probe's cell.  Minimum image r - L trunc(2 r / L); pairs
 // with d >= rc or d = 0 are skipped; A, B interpolated between the bracketing table rows (first
 // row with rvals >= d); out[e] = sum A m + (B - A) (m . r^) r^ in a fixed order per probe.
-struct Box3 {
-    double L[3];
-};
-
-__global__ void __launch_bounds__(256) k_probe_real(const double *__restrict__ xe, int64_t ne,
+// One candidate in seven lies within rc: the walk screens them in float32 (near_walk) and the float64 pair terms, the
+// only part that GB300's float64 rate bounds, run on 32 kept pairs at a time (90,000 probes and 10,000 spheres, 29 of
+// 203 candidates a probe: 5.62 ms with every candidate in float64, 0.57 ms; the table row comes from the uniform-spacing guess instead of 13 float64
+// comparisons).
+__global__ void __launch_bounds__(128) k_probe_real(const double *__restrict__ xe, int64_t ne,
                                                     const int64_t *__restrict__ cell_e,
-                                                    const double *__restrict__ xp, const double *__restrict__ p,
-                                                    const int32_t *__restrict__ sorted,
+                                                    const float4 *__restrict__ es,
+                                                    const double *__restrict__ xp, const float4 *__restrict__ xs,
+                                                    const double *__restrict__ p,
                                                     const int32_t *__restrict__ counts,
                                                     const int64_t *__restrict__ starts, int64_t ncx, int64_t ncy,
-                                                    int64_t ncz, Box3 box, double rc, const double *__restrict__ perp,
+                                                    int64_t ncz, Box3 box, NearBox nb, double rc,
+                                                    const double *__restrict__ perp,
                                                     const double *__restrict__ para, const double *__restrict__ rv,
                                                     int64_t ntab, double *__restrict__ out, int *__restrict__ err) {
-    const int lane = threadIdx.x & 31;
+    __shared__ int32_t q[4][kNearQueue];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const double rv_last = rv[ntab - 1], inv_dr = rv_last > 0 ? (double)(ntab - 1) / rv_last : 0.0;
     for (int64_t e = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; e < ne; e += nw) {
         const int32_t c = (int32_t)(cell_e[3 * e] + ncx * (cell_e[3 * e + 1] + ncy * cell_e[3 * e + 2]));
         const CellWalk cw = cell_walk(c, lane, counts, starts, ncx, ncy, ncz);
         double acc[3] = {0.0, 0.0, 0.0};
-        for (int j0 = 0; j0 < cw.total; j0 += 32) {
-            const int j = j0 + lane;
-            int o;
-            int64_t pos;
-            walk_at(cw, j < cw.total ? j : cw.total - 1, o, pos);
-            if (j >= cw.total) continue;
-            const int32_t b = sorted[pos];
-            double r[3], d2 = 0.0;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                double v = xe[3 * e + k] - xp[3 * (int64_t)b + k];
-                v -= box.L[k] * trunc(2.0 * v / box.L[k]);
-                r[k] = v;
-                d2 += v * v;
-            }
-            const double d = sqrt(d2);
-            if (!(d < rc) || !(d > 0.0)) continue;
-            int64_t lo = 1, hi = ntab - 1;   // first row with rv >= d, searched in [1, ntab - 1]
-            if (!(rv[hi] >= d)) {
+        near_walk(cw, lane, xs, es[e], -1, nb, q[wid], [&](int32_t b) {
+            double r[3];
+            double y;
+            const double d = probe_distance(probe_diff2(xe, e, xp, b, box, r), &y);
+            if (!(d < rc) || !(d > 0.0)) return;
+            if (!(rv_last >= d)) {
                 atomicExch(err, 1);
-                continue;
+                return;
             }
-            while (lo < hi) {
-                const int64_t mid = (lo + hi) >> 1;
-                if (rv[mid] >= d) hi = mid; else lo = mid + 1;
-            }
-            const double rh = rv[lo], rl = rv[lo - 1], span = rh - rl;
-            const double A = perp[lo - 1] * (rh - d) / span + perp[lo] * (d - rl) / span;
-            const double B = para[lo - 1] * (rh - d) / span + para[lo] * (d - rl) / span;
+            const int64_t lo = probe_row(rv, ntab, d, inv_dr);
+            const double rh = rv[lo], rl = rv[lo - 1], inv = rcp_newton(rh - rl), wl = (rh - d) * inv, wh = (d - rl) * inv;
+            const double A = perp[lo - 1] * wl + perp[lo] * wh;
+            const double B = para[lo - 1] * wl + para[lo] * wh;
             const double *m = p + 3 * (int64_t)b;
-            const double mr = (m[0] * r[0] + m[1] * r[1] + m[2] * r[2]) / d;
+            const double ba = (B - A) * ((m[0] * r[0] + m[1] * r[1] + m[2] * r[2]) * y) * y;
 #pragma unroll
-            for (int k = 0; k < 3; ++k) acc[k] += A * (m[k] - mr * r[k] / d) + B * mr * r[k] / d;
-        }
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
-        if (lane == 0)
-#pragma unroll
-            for (int k = 0; k < 3; ++k) out[3 * e + k] = acc[k];
+            for (int k = 0; k < 3; ++k) acc[k] += A * m[k] + ba * r[k];
+        });
+        const double v = warp_sum4(acc[0], acc[1], acc[2], 0.0, lane);
+        if ((lane & 7) == 0 && lane < 24) out[3 * e + lane / 8] = v;
     }
 }
 
@@ -201,56 +195,42 @@ __global__ void __launch_bounds__(256) k_probe_real(const double *__restrict__ x
 // the couplings A..I of each pair interpolated from the 9 tables (field_dip_1/2, field_quad_1..3,
 // grad_quad_1..4; first row with rvals >= d), out[e] = (E (3), G (5)).  A source at the probe
 // itself (d = 0) is skipped (the reference divides by d there).
-__global__ void __launch_bounds__(256) k_probe_real_quad(const double *__restrict__ xe, int64_t ne,
+__global__ void __launch_bounds__(128) k_probe_real_quad(const double *__restrict__ xe, int64_t ne,
                                                          const int64_t *__restrict__ cell_e,
+                                                         const float4 *__restrict__ es,
                                                          const double *__restrict__ xp,
+                                                         const float4 *__restrict__ xs,
                                                          const double *__restrict__ sq,
-                                                         const int32_t *__restrict__ sorted,
                                                          const int32_t *__restrict__ counts,
                                                          const int64_t *__restrict__ starts, int64_t ncx,
-                                                         int64_t ncy, int64_t ncz, Box3 box, double rc,
+                                                         int64_t ncy, int64_t ncz, Box3 box, NearBox nb, double rc,
                                                          const double *__restrict__ tab, const double *__restrict__ rv,
                                                          int64_t ntab, double *__restrict__ out, int *__restrict__ err) {
-    const int lane = threadIdx.x & 31;
+    __shared__ int32_t q[4][kNearQueue];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const double rv_last = rv[ntab - 1], inv_dr = rv_last > 0 ? (double)(ntab - 1) / rv_last : 0.0;
     for (int64_t e = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; e < ne; e += nw) {
         const int32_t c = (int32_t)(cell_e[3 * e] + ncx * (cell_e[3 * e + 1] + ncy * cell_e[3 * e + 2]));
         const CellWalk cw = cell_walk(c, lane, counts, starts, ncx, ncy, ncz);
         double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int j0 = 0; j0 < cw.total; j0 += 32) {
-            const int j = j0 + lane;
-            int o;
-            int64_t pos;
-            walk_at(cw, j < cw.total ? j : cw.total - 1, o, pos);
-            if (j >= cw.total) continue;
-            const int32_t b = sorted[pos];
-            double r[3], d2 = 0.0;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                double v = xe[3 * e + k] - xp[3 * (int64_t)b + k];
-                v -= box.L[k] * trunc(2.0 * v / box.L[k]);
-                r[k] = v;
-                d2 += v * v;
-            }
-            const double d = sqrt(d2);
-            if (!(d < rc) || !(d > 0.0)) continue;
-            int64_t lo = 1, hi = ntab - 1;
-            if (!(rv[hi] >= d)) {
+        near_walk(cw, lane, xs, es[e], -1, nb, q[wid], [&](int32_t b) {
+            double r[3];
+            double y;
+            const double d = probe_distance(probe_diff2(xe, e, xp, b, box, r), &y);
+            if (!(d < rc) || !(d > 0.0)) return;
+            if (!(rv_last >= d)) {
                 atomicExch(err, 1);
-                continue;
+                return;
             }
-            while (lo < hi) {
-                const int64_t mid = (lo + hi) >> 1;
-                if (rv[mid] >= d) hi = mid; else lo = mid + 1;
-            }
-            const double rh = rv[lo], rl = rv[lo - 1], span = rh - rl;
+            const int64_t lo = probe_row(rv, ntab, d, inv_dr);
+            const double rh = rv[lo], rl = rv[lo - 1], inv = rcp_newton(rh - rl), wl = (rh - d) * inv, wh = (d - rl) * inv;
             double cf[9];
 #pragma unroll
-            for (int q = 0; q < 9; ++q)
-                cf[q] = tab[q * ntab + lo - 1] * (rh - d) / span + tab[q * ntab + lo] * (d - rl) / span;
+            for (int t = 0; t < 9; ++t) cf[t] = tab[t * ntab + lo - 1] * wl + tab[t * ntab + lo] * wh;
             const double A = cf[0], B = cf[1], Cc = cf[2], D = cf[3], E = cf[4], F = cf[5], Gg = cf[6], H = cf[7],
                          I = cf[8];
-            const double rx = r[0] / d, ry = r[1] / d, rz = r[2] / d;
+            const double rx = r[0] * y, ry = r[1] * y, rz = r[2] * y;
             const double *m = sq + 8 * (int64_t)b;
             const double Sx = m[0], Sy = m[1], Sz = m[2], Q0 = m[3], Q1 = m[4], Q2 = m[5], Q3 = m[6], Q4 = m[7];
             const double sr = Sx * rx + Sy * ry + Sz * rz;
@@ -276,14 +256,12 @@ __global__ void __launch_bounds__(256) k_probe_real_quad(const double *__restric
                 if (k == 0 || k == 3) v += di;
                 acc[3 + k] += v;
             }
+        });
+        const double v = warp_sum4(acc[0], acc[1], acc[2], acc[3], lane), w = warp_sum4(acc[4], acc[5], acc[6], acc[7], lane);
+        if ((lane & 7) == 0) {
+            out[8 * e + lane / 8] = v;
+            out[8 * e + 4 + lane / 8] = w;
         }
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
-        if (lane == 0)
-#pragma unroll
-            for (int k = 0; k < 8; ++k) out[8 * e + k] = acc[k];
     }
 }
 
@@ -291,68 +269,52 @@ __global__ void __launch_bounds__(256) k_probe_real_quad(const double *__restric
 // smallest radius (class cmin), so the couplings of a probe/source pair come from the table column
 // of the classes (cmin, cls[b]) (column order of CS/RealSpaceTable.m: i <= j, row-major over i);
 // rvals need not start at 0: a separation below rvals[0] or above rvals[ntab-1] is out of the table.
-__global__ void __launch_bounds__(256) k_probe_real_cs(const double *__restrict__ xe, int64_t ne,
+__global__ void __launch_bounds__(128) k_probe_real_cs(const double *__restrict__ xe, int64_t ne,
                                                        const int64_t *__restrict__ cell_e,
-                                                       const double *__restrict__ xp, const double *__restrict__ p,
+                                                       const float4 *__restrict__ es,
+                                                       const double *__restrict__ xp, const float4 *__restrict__ xs,
+                                                       const double *__restrict__ p,
                                                        const int32_t *__restrict__ cls, int32_t cmin, int32_t M,
-                                                       const int32_t *__restrict__ sorted,
                                                        const int32_t *__restrict__ counts,
                                                        const int64_t *__restrict__ starts, int64_t ncx, int64_t ncy,
-                                                       int64_t ncz, Box3 box, double rc,
+                                                       int64_t ncz, Box3 box, NearBox nb, double rc,
                                                        const double *__restrict__ perp,
                                                        const double *__restrict__ para,
                                                        const double *__restrict__ rv, int64_t ntab,
                                                        double *__restrict__ out, int *__restrict__ err) {
-    const int lane = threadIdx.x & 31;
+    __shared__ int32_t q[4][kNearQueue];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const double rv_first = rv[0], rv_last = rv[ntab - 1];
+    // rows start at rv_first, not at zero: the guess is the offset from it
+    const double inv_dr = rv_last > rv_first ? (double)(ntab - 1) / (rv_last - rv_first) : 0.0;
     for (int64_t e = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; e < ne; e += nw) {
         const int32_t c = (int32_t)(cell_e[3 * e] + ncx * (cell_e[3 * e + 1] + ncy * cell_e[3 * e + 2]));
         const CellWalk cw = cell_walk(c, lane, counts, starts, ncx, ncy, ncz);
         double acc[3] = {0.0, 0.0, 0.0};
-        for (int j0 = 0; j0 < cw.total; j0 += 32) {
-            const int j = j0 + lane;
-            int o;
-            int64_t pos;
-            walk_at(cw, j < cw.total ? j : cw.total - 1, o, pos);
-            if (j >= cw.total) continue;
-            const int32_t b = sorted[pos];
-            double r[3], d2 = 0.0;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                double v = xe[3 * e + k] - xp[3 * (int64_t)b + k];
-                v -= box.L[k] * trunc(2.0 * v / box.L[k]);
-                r[k] = v;
-                d2 += v * v;
-            }
-            const double d = sqrt(d2);
-            if (!(d < rc)) continue;
-            if (!(d > rv[0]) || !(rv[ntab - 1] >= d)) {
+        near_walk(cw, lane, xs, es[e], -1, nb, q[wid], [&](int32_t b) {
+            double r[3];
+            double y;
+            const double d = probe_distance(probe_diff2(xe, e, xp, b, box, r), &y);
+            if (!(d < rc)) return;
+            if (!(d > rv_first) || !(rv_last >= d)) {
                 atomicExch(err, 1);
-                continue;
+                return;
             }
-            int64_t lo = 1, hi = ntab - 1;
-            while (lo < hi) {
-                const int64_t mid = (lo + hi) >> 1;
-                if (rv[mid] >= d) hi = mid; else lo = mid + 1;
-            }
+            const int64_t lo = probe_row(rv, ntab, d, inv_dr, rv_first);
             const int32_t ci = cmin < cls[b] ? cmin : cls[b], cj = cmin < cls[b] ? cls[b] : cmin;
             const int64_t col = (int64_t)ci * M - (int64_t)ci * (ci - 1) / 2 + (cj - ci);
             const double *tp = perp + col * ntab, *ta = para + col * ntab;
-            const double rh = rv[lo], rl = rv[lo - 1], span = rh - rl;
-            const double A = tp[lo - 1] * (rh - d) / span + tp[lo] * (d - rl) / span;
-            const double B = ta[lo - 1] * (rh - d) / span + ta[lo] * (d - rl) / span;
+            const double rh = rv[lo], rl = rv[lo - 1], inv = rcp_newton(rh - rl), wl = (rh - d) * inv, wh = (d - rl) * inv;
+            const double A = tp[lo - 1] * wl + tp[lo] * wh;
+            const double B = ta[lo - 1] * wl + ta[lo] * wh;
             const double *m = p + 3 * (int64_t)b;
-            const double mr = (m[0] * r[0] + m[1] * r[1] + m[2] * r[2]) / d;
+            const double ba = (B - A) * ((m[0] * r[0] + m[1] * r[1] + m[2] * r[2]) * y) * y;
 #pragma unroll
-            for (int k = 0; k < 3; ++k) acc[k] += A * (m[k] - mr * r[k] / d) + B * mr * r[k] / d;
-        }
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
-        if (lane == 0)
-#pragma unroll
-            for (int k = 0; k < 3; ++k) out[3 * e + k] = acc[k];
+            for (int k = 0; k < 3; ++k) acc[k] += A * m[k] + ba * r[k];
+        });
+        const double v = warp_sum4(acc[0], acc[1], acc[2], 0.0, lane);
+        if ((lane & 7) == 0 && lane < 24) out[3 * e + lane / 8] = v;
     }
 }
 
@@ -464,14 +426,6 @@ __device__ __forceinline__ double rsqrt_newton(double s) {
     double y = (double)rsqrtf((float)s);
     y = y * (1.5 - 0.5 * s * y * y);
     y = y * (1.5 - 0.5 * s * y * y);
-    return y;
-}
-
-// 1/v by Newton's method y <- y (2 - v y) from a float32 seed (two steps).
-__device__ __forceinline__ double rcp_newton(double v) {
-    double y = (double)(1.0f / (float)v);
-    y = y * (2.0 - v * y);
-    y = y * (2.0 - v * y);
     return y;
 }
 
@@ -1160,6 +1114,14 @@ int pairs_df_to_f64(const PairData<dfv> &pdf, int64_t np, PairData<double> p64, 
 }
 
 
+int near_positions(const double *x, const int32_t *sorted, int64_t n, const Box3 &box, const NearBox &nb, float4 *xs,
+                   cudaStream_t s) {
+    if (n == 0) return MPS_OK;
+    k_near_positions<<<grid_for(n, 256), 256, 0, s>>>(x, sorted, n, box, nb, xs);
+    MPS_LAUNCH_CHECK();
+    return MPS_OK;
+}
+
 int probe_real_space(const double *xe, int64_t ne, const double *xp, const double *p, int64_t np, const double *box,
                      double rc, const double *perp, const double *para, const double *rv, int64_t ntab, double *out,
                      cudaStream_t s) {
@@ -1171,7 +1133,10 @@ int probe_real_space(const double *xe, int64_t ne, const double *xp, const doubl
     int64_t *cell_p = nullptr, *cell_e = nullptr;
     void *bins = nullptr;
     int *err = nullptr;
+    float4 *xs = nullptr, *es = nullptr;
     auto cleanup = [&]() {
+        if (xs) cudaFreeAsync(xs, s);
+        if (es) cudaFreeAsync(es, s);
         if (cell_p) cudaFreeAsync(cell_p, s);
         if (cell_e) cudaFreeAsync(cell_e, s);
         if (bins) cudaFreeAsync(bins, s);
@@ -1180,6 +1145,8 @@ int probe_real_space(const double *xe, int64_t ne, const double *xp, const doubl
     if (cudaMallocAsync((void **)&cell_p, sizeof(int64_t) * 3 * (np > 0 ? np : 1), s) != cudaSuccess ||
         cudaMallocAsync((void **)&cell_e, sizeof(int64_t) * 3 * ne, s) != cudaSuccess ||
         cudaMallocAsync(&bins, cell_bins_bytes(np, ncells), s) != cudaSuccess ||
+        cudaMallocAsync((void **)&xs, sizeof(float4) * (np > 0 ? np : 1), s) != cudaSuccess ||
+        cudaMallocAsync((void **)&es, sizeof(float4) * ne, s) != cudaSuccess ||
         cudaMallocAsync((void **)&err, sizeof(int), s) != cudaSuccess) {
         cleanup();
         return MPS_NO_MEMORY;
@@ -1189,11 +1156,15 @@ int probe_real_space(const double *xe, int64_t ne, const double *xp, const doubl
     if (!rcode) rcode = cell_assign(xp, np, box, ncell, cell_p, s);
     if (!rcode) rcode = cell_bins_build(cell_p, np, ncell, bins, cb, s);
     if (!rcode) rcode = cell_assign(xe, ne, box, ncell, cell_e, s);
+    const bool per[3] = {true, true, true};
+    const Box3 b3{{box[0], box[1], box[2]}};
+    const NearBox nb = make_near_box(box, rc, per);
+    if (!rcode) rcode = near_positions(xp, cb.sorted, np, b3, nb, xs, s);
+    if (!rcode) rcode = near_positions(xe, nullptr, ne, b3, nb, es, s);
     if (!rcode) {
-        Box3 b3{{box[0], box[1], box[2]}};
-        k_probe_real<<<grid_for(ne * 32, 256, 152 * 64), 256, 0, s>>>(
-            xe, ne, cell_e, xp, p, cb.sorted, cb.counts, cb.starts, ncell[0], ncell[1], ncell[2], b3, rc, perp, para,
-            rv, ntab, out, err);
+        k_probe_real<<<grid_for(ne * 32, 128, 152 * 128), 128, 0, s>>>(
+            xe, ne, cell_e, es, xp, xs, p, cb.counts, cb.starts, ncell[0], ncell[1], ncell[2], b3, nb, rc, perp, para, rv, ntab,
+            out, err);
         if (cudaGetLastError() != cudaSuccess) rcode = MPS_CUDA_ERR;
     }
     int herr = 0;
@@ -1217,7 +1188,10 @@ int probe_real_space_quad(const double *xe, int64_t ne, const double *xp, const 
     int64_t *cell_p = nullptr, *cell_e = nullptr;
     void *bins = nullptr;
     int *err = nullptr;
+    float4 *xs = nullptr, *es = nullptr;
     auto cleanup = [&]() {
+        if (xs) cudaFreeAsync(xs, s);
+        if (es) cudaFreeAsync(es, s);
         if (cell_p) cudaFreeAsync(cell_p, s);
         if (cell_e) cudaFreeAsync(cell_e, s);
         if (bins) cudaFreeAsync(bins, s);
@@ -1226,6 +1200,8 @@ int probe_real_space_quad(const double *xe, int64_t ne, const double *xp, const 
     if (cudaMallocAsync((void **)&cell_p, sizeof(int64_t) * 3 * (np > 0 ? np : 1), s) != cudaSuccess ||
         cudaMallocAsync((void **)&cell_e, sizeof(int64_t) * 3 * ne, s) != cudaSuccess ||
         cudaMallocAsync(&bins, cell_bins_bytes(np, ncells), s) != cudaSuccess ||
+        cudaMallocAsync((void **)&xs, sizeof(float4) * (np > 0 ? np : 1), s) != cudaSuccess ||
+        cudaMallocAsync((void **)&es, sizeof(float4) * ne, s) != cudaSuccess ||
         cudaMallocAsync((void **)&err, sizeof(int), s) != cudaSuccess) {
         cleanup();
         return MPS_NO_MEMORY;
@@ -1235,11 +1211,15 @@ int probe_real_space_quad(const double *xe, int64_t ne, const double *xp, const 
     if (!rcode) rcode = cell_assign(xp, np, box, ncell, cell_p, s);
     if (!rcode) rcode = cell_bins_build(cell_p, np, ncell, bins, cb, s);
     if (!rcode) rcode = cell_assign(xe, ne, box, ncell, cell_e, s);
+    const bool per[3] = {true, true, true};
+    const Box3 b3{{box[0], box[1], box[2]}};
+    const NearBox nb = make_near_box(box, rc, per);
+    if (!rcode) rcode = near_positions(xp, cb.sorted, np, b3, nb, xs, s);
+    if (!rcode) rcode = near_positions(xe, nullptr, ne, b3, nb, es, s);
     if (!rcode) {
-        Box3 b3{{box[0], box[1], box[2]}};
-        k_probe_real_quad<<<grid_for(ne * 32, 256, 152 * 64), 256, 0, s>>>(
-            xe, ne, cell_e, xp, sq, cb.sorted, cb.counts, cb.starts, ncell[0], ncell[1], ncell[2], b3, rc, tab9, rv,
-            ntab, out, err);
+        k_probe_real_quad<<<grid_for(ne * 32, 128, 152 * 128), 128, 0, s>>>(
+            xe, ne, cell_e, es, xp, xs, sq, cb.counts, cb.starts, ncell[0], ncell[1], ncell[2], b3, nb, rc, tab9, rv, ntab, out,
+            err);
         if (cudaGetLastError() != cudaSuccess) rcode = MPS_CUDA_ERR;
     }
     int herr = 0;
@@ -1263,7 +1243,10 @@ int probe_real_space_cs(const double *xe, int64_t ne, const double *xp, const do
     int64_t *cell_p = nullptr, *cell_e = nullptr;
     void *bins = nullptr;
     int *err = nullptr;
+    float4 *xs = nullptr, *es = nullptr;
     auto cleanup = [&]() {
+        if (xs) cudaFreeAsync(xs, s);
+        if (es) cudaFreeAsync(es, s);
         if (cell_p) cudaFreeAsync(cell_p, s);
         if (cell_e) cudaFreeAsync(cell_e, s);
         if (bins) cudaFreeAsync(bins, s);
@@ -1272,6 +1255,8 @@ int probe_real_space_cs(const double *xe, int64_t ne, const double *xp, const do
     if (cudaMallocAsync((void **)&cell_p, sizeof(int64_t) * 3 * (np > 0 ? np : 1), s) != cudaSuccess ||
         cudaMallocAsync((void **)&cell_e, sizeof(int64_t) * 3 * ne, s) != cudaSuccess ||
         cudaMallocAsync(&bins, cell_bins_bytes(np, ncells), s) != cudaSuccess ||
+        cudaMallocAsync((void **)&xs, sizeof(float4) * (np > 0 ? np : 1), s) != cudaSuccess ||
+        cudaMallocAsync((void **)&es, sizeof(float4) * ne, s) != cudaSuccess ||
         cudaMallocAsync((void **)&err, sizeof(int), s) != cudaSuccess) {
         cleanup();
         return MPS_NO_MEMORY;
@@ -1281,11 +1266,15 @@ int probe_real_space_cs(const double *xe, int64_t ne, const double *xp, const do
     if (!rcode) rcode = cell_assign(xp, np, box, ncell, cell_p, s);
     if (!rcode) rcode = cell_bins_build(cell_p, np, ncell, bins, cb, s);
     if (!rcode) rcode = cell_assign(xe, ne, box, ncell, cell_e, s);
+    const bool per[3] = {true, true, true};
+    const Box3 b3{{box[0], box[1], box[2]}};
+    const NearBox nb = make_near_box(box, rc, per);
+    if (!rcode) rcode = near_positions(xp, cb.sorted, np, b3, nb, xs, s);
+    if (!rcode) rcode = near_positions(xe, nullptr, ne, b3, nb, es, s);
     if (!rcode) {
-        Box3 b3{{box[0], box[1], box[2]}};
-        k_probe_real_cs<<<grid_for(ne * 32, 256, 152 * 64), 256, 0, s>>>(
-            xe, ne, cell_e, xp, p, cls, cmin, M, cb.sorted, cb.counts, cb.starts, ncell[0], ncell[1], ncell[2], b3,
-            rc, perp, para, rv, ntab, out, err);
+        k_probe_real_cs<<<grid_for(ne * 32, 128, 152 * 128), 128, 0, s>>>(
+            xe, ne, cell_e, es, xp, xs, p, cls, cmin, M, cb.counts, cb.starts, ncell[0], ncell[1], ncell[2], b3, nb, rc, perp,
+            para, rv, ntab, out, err);
         if (cudaGetLastError() != cudaSuccess) rcode = MPS_CUDA_ERR;
     }
     int herr = 0;

@@ -29,6 +29,10 @@ struct PairData {
     T *dist;          // separation (only kept when an operator interpolates more tables)
 };
 
+struct Box3 {
+    double L[3];
+};
+
 void compute_ncell(const double *box, double rmax, int64_t *ncell);
 size_t cell_bins_bytes(int64_t n, int64_t ncells);
 int cell_assign(const double *x, int64_t n, const double *box, const int64_t *ncell, int64_t *cell3, cudaStream_t s);
