@@ -20,6 +20,7 @@
 #include "sizes.cuh"
 #include <algorithm>
 #include "dffft.cuh"
+#include "fft64.cuh"
 #include "adjoint.cuh"
 #include "gradop.cuh"
 
@@ -75,15 +76,18 @@ struct GreenCoef {
     float *h32 = nullptr;
     float *hs32 = nullptr;   // H / |k|^2 of the gradient-form float32 operator (built on first use)
     float2 *tm6 = nullptr;   // double-float scale tensor H q q^T, 6 x Gc (built on first use)
-    cudaEvent_t ev_h = nullptr, ev_hs32 = nullptr, ev_tm6 = nullptr;   // recorded after each fill
+    double *hs64 = nullptr;  // 0.5 H / |k|^2 of the float64 transforms (built on first use)
+    cudaEvent_t ev_h = nullptr, ev_hs32 = nullptr, ev_tm6 = nullptr, ev_hs64 = nullptr;   // recorded after each fill
     ~GreenCoef() {
         if (h64) cudaFree(h64);
         if (h32) cudaFree(h32);
         if (hs32) cudaFree(hs32);
         if (tm6) cudaFree(tm6);
+        if (hs64) cudaFree(hs64);
         if (ev_h) cudaEventDestroy(ev_h);
         if (ev_hs32) cudaEventDestroy(ev_hs32);
         if (ev_tm6) cudaEventDestroy(ev_tm6);
+        if (ev_hs64) cudaEventDestroy(ev_hs64);
     }
 };
 
@@ -222,11 +226,13 @@ struct mps_system {
     int64_t stage_count[3] = {0, 0, 0};
     DfPlan3 dfp;                 // double-float FFT plans of the grid
     int df_state = 0;            // 0 not built yet, 1 usable, -1 unsupported grid
+    F64Plan3 f64p;               // float64 FFT plans of the grid
+    int f64_state = 0;           // as df_state
     int resid_prec = MPS_FP64;   // operator of the refinement residuals
     float *g32 = nullptr;        // gradient factors dw_d/dr of the gradient-form operator, n x 3 x P
     int inner_prec = MPS_FP32;   // operator of the mixed solve's inner GMRES
     // this system's stream has waited for the shared lazily built Green's buffers (hs32, tm6)
-    bool hs32_ready = false, tm6_ready = false;
+    bool hs32_ready = false, tm6_ready = false, hs64_ready = false;
     InnerGrid *inner = nullptr;      // coarser inner discretisation of the gradient-form operator, or null
     // Arnoldi-step graphs (captured on their own stream once every lazily built buffer of the matvec exists:
     // after the first matvec of that precision and batch width outside a capture)
@@ -709,6 +715,37 @@ static int ensure_tiles(mps_system *s, int use, cudaStream_t st, bool *used) {
 
 static bool df_usable(mps_system *s);
 
+// The float64 transforms of fft64.cu take every axis up to 1024 whose prime factors are at most 127 (measured faster
+// than cuFFT at every length tried, see there); other grids keep cuFFT.
+static bool f64_usable(mps_system *s) {
+    if (s->f64_state == 0) {
+        if (f64_plan(s->gp, &s->f64p) != MPS_OK) return false;
+        s->f64_state = s->f64p.ok ? 1 : -1;
+    }
+    return s->f64_state == 1;
+}
+
+// The scale coefficient of the float64 transforms, from the process cache or computed on stream st.
+static int f64_prepare(mps_system *s, cudaStream_t st) {
+    if (s->hs64_ready) return MPS_OK;
+    std::lock_guard<std::mutex> lk(g_green_mu);
+    if (!s->green->hs64) {
+        double *hs = nullptr;
+        MPS_TRY(dalloc_persistent(&hs, sizeof(double) * s->Gc));
+        int rc = f64_scale_coef(s->gp, s->green->h64, hs, st);
+        if (!rc) rc = green_mark_filled(&s->green->ev_hs64, st);
+        if (rc) {
+            cudaFree(hs);
+            return rc;
+        }
+        s->green->hs64 = hs;
+    } else {
+        MPS_CUDA_TRY(cudaStreamWaitEvent(st, s->green->ev_hs64, 0));   // filled by another system
+    }
+    s->hs64_ready = true;
+    return MPS_OK;
+}
+
 // Float32 pair sum (accumulates into out) on the system's float copy of the moments.
 static int real_space_f32(mps_system *s, const double *m, double *out, int nrhs, cudaStream_t st) {
     if (!s->m32) MPS_TRY(dalloc(&s->m32, sizeof(float) * m32_floats(s->n, s->max_rhs), st));
@@ -742,6 +779,8 @@ template <typename T>
 static int matvec_impl(mps_system *s, const double *m, double *out, int nrhs, cudaStream_t st) {
     const bool dbl = sizeof(T) == 8;
     const bool own_fft = !dbl && own_fft32() && df_usable(s);
+    const bool f64_fft = dbl && f64_usable(s);
+    if (f64_fft) MPS_TRY(f64_prepare(s, st));
     bool use_tiles = false;
     MPS_TRY(ensure_tiles(s, dbl ? kTileF64 : kTileRef32, st, &use_tiles));
     const TileBins &tb = dbl ? s->tb64 : s->tb32;
@@ -767,6 +806,13 @@ static int matvec_impl(mps_system *s, const double *m, double *out, int nrhs, cu
         MPS_TRY(f32_z_scale_dipole((float2 *)spec, nrhs, s->gp, s->dfp, (const float *)hh, st));
         STAGE_MARK(4);
         MPS_TRY(f32_inverse_yx((float2 *)spec, (float *)grid, 3 * nrhs, s->gp, s->dfp, st));
+        STAGE_MARK(5);
+    } else if (f64_fft) {
+        MPS_TRY(f64_forward_xy((const double *)grid, spec, 3 * nrhs, s->gp, s->f64p, st));
+        STAGE_MARK(3);
+        MPS_TRY(f64_z_scale_dipole(spec, nrhs, s->gp, s->f64p, s->green->hs64, st));
+        STAGE_MARK(4);
+        MPS_TRY(f64_inverse_yx(spec, (double *)grid, 3 * nrhs, s->gp, s->f64p, st));
         STAGE_MARK(5);
     } else {
         MPS_TRY(exec_plan(s, dbl ? CUFFT_D2Z : CUFFT_R2C, 3 * nrhs, grid, spec, 0, st));
