@@ -213,6 +213,7 @@ struct mps_system {
     size_t fft_work_bytes = 0;
     TileBins tb64, tb32;        // tile binning for the tiled spread/contract (per precision tile depth)
     TileBins tbg;               // tiles of the gradient-form spread (depth 12 where the grid allows it)
+    TileBins tbn;               // tiles of the float64 node spread
     double *partial64 = nullptr;
     int tb_use[2] = {-1, -1};         // tuner consumer that built tb64 / tb32
     float *partial32 = nullptr;
@@ -333,6 +334,7 @@ static void free_system(mps_system *s) {
     tile_bins_free(s->tb64, s->stream);
     tile_bins_free(s->tb32, s->stream);
     tile_bins_free(s->tbg, s->stream);
+    tile_bins_free(s->tbn, s->stream);
     if (s->partial64) cudaFreeAsync(s->partial64, s->stream);
     if (s->partial32) cudaFreeAsync(s->partial32, s->stream);
     if (s->partialg) cudaFreeAsync(s->partialg, s->stream);
@@ -529,10 +531,10 @@ static int stage_begin(mps_system *s, int precision, StageEvents **ev, cudaStrea
 // consumer runs, and the fastest is kept for the rest of the process.  The
 // consumers: the float32 reference operator (tiled spread + contract), the
 // float32 gradient operator (its spread; depth 12 without timing where the grid
-// allows it, see tuned_depth), the float64 operator (spread) and the double-float
-// operator (spread).  The reference-form float32 kernels use tb32, the gradient
-// form tbg, the float64-width kernels tb64.
-enum TileUse { kTileRef32 = 0, kTileGrad32 = 1, kTileF64 = 2, kTileDF = 3 };
+// allows it, see tuned_depth) and the double-float operator (spread).  The
+// reference-form float32 kernels use tb32, the gradient form tbg, the double-float
+// kernels tb64 (the float64 spread has tiles of its own, tbn, and no choice to time).
+enum TileUse { kTileRef32 = 0, kTileGrad32 = 1, kTileDF = 2 };
 struct TuneKey {
     int dev;
     int N[3];
@@ -573,9 +575,6 @@ static int time_tiles(mps_system *s, int use, int tz, int nrhs, const double *m,
                 break;
             case kTileGrad32:
                 rc = spread_grad_tiled(m, s->n, nrhs, s->start, s->w32, s->g32, s->gp, tb, s->grid32, st);
-                break;
-            case kTileF64:
-                rc = spread_tiled<double>(m, s->n, nrhs, s->start, s->w64, s->gp, tb, s->grid64, st);
                 break;
             default:
                 rc = spread_tiled_df(m, s->n, nrhs, s->start, s->wdf, s->gp, tb, (dfv *)s->grid64, st);
@@ -693,7 +692,7 @@ static int ensure_tiles(mps_system *s, int use, cudaStream_t st, bool *used) {
     *used = false;
     // the tiled kernels use the separable Gaussian weights of the dipole operator
     if (!s->tiled || s->kind != MPS_DIPOLE || !s->w32 || !s->w64) return MPS_OK;
-    const bool dbl = use == kTileF64 || use == kTileDF;
+    const bool dbl = use == kTileDF;
     const bool grad = use == kTileGrad32;
     TileBins &tb = dbl ? s->tb64 : (grad ? s->tbg : s->tb32);
     if (!tb.mem) {
@@ -782,9 +781,12 @@ static int matvec_impl(mps_system *s, const double *m, double *out, int nrhs, cu
     const bool f64_fft = dbl && f64_usable(s);
     if (f64_fft) MPS_TRY(f64_prepare(s, st));
     bool use_tiles = false;
-    MPS_TRY(ensure_tiles(s, dbl ? kTileF64 : kTileRef32, st, &use_tiles));
-    const TileBins &tb = dbl ? s->tb64 : s->tb32;
-    T *partial = dbl ? (T *)s->partial64 : (T *)s->partial32;
+    if (dbl) {
+        use_tiles = s->tiled && nodes_supported(s->gp);
+        if (use_tiles && !s->tbn.mem) MPS_TRY(node_bins_build(s->start, s->n, s->gp, s->max_rhs, s->tbn, st));
+    } else {
+        MPS_TRY(ensure_tiles(s, kTileRef32, st, &use_tiles));
+    }
     MPS_TRY(ensure_grids(s, dbl ? MPS_FP64 : MPS_FP32, st));
     T *grid = dbl ? (T *)s->grid64 : (T *)s->grid32;
     void *spec = dbl ? s->spec64 : s->spec32;
@@ -795,10 +797,14 @@ static int matvec_impl(mps_system *s, const double *m, double *out, int nrhs, cu
     MPS_TRY(stage_begin(s, dbl ? MPS_FP64 : MPS_FP32, &ev, st));
     if (s->slab_factor != 0.0) MPS_TRY(slab_terms(m, s->n, nrhs, s->slab_factor / vol, s->slab, st));
     STAGE_MARK(1);
-    if (use_tiles)
-        MPS_TRY(spread_tiled<T>(m, s->n, nrhs, s->start, w, s->gp, tb, grid, st));
-    else
+    if (use_tiles) {
+        if constexpr (sizeof(T) == 8)
+            MPS_TRY(spread_nodes(m, s->n, nrhs, s->start, s->w64, s->gp, s->tbn, s->grid64, st));
+        else
+            MPS_TRY(spread_tiled<float>(m, s->n, nrhs, s->start, s->w32, s->gp, s->tb32, s->grid32, st));
+    } else {
         MPS_TRY(spread<T>(m, s->n, nrhs, s->start, w, s->gp, grid, st));
+    }
     STAGE_MARK(2);
     if (own_fft) {
         MPS_TRY(f32_forward_xy((const float *)grid, (float2 *)spec, 3 * nrhs, s->gp, s->dfp, st));
@@ -822,14 +828,16 @@ static int matvec_impl(mps_system *s, const double *m, double *out, int nrhs, cu
         MPS_TRY(exec_plan(s, dbl ? CUFFT_Z2D : CUFFT_C2R, 3 * nrhs, spec, grid, 0, st));
         STAGE_MARK(5);
     }
-    // float64: the warp-per-particle gather keeps more lanes busy, which is what
-    // matters at GB300's float64 issue rate; float32: the shared-memory tile.
-    if (use_tiles && !dbl) {
-        MPS_TRY(tile_bins_pentry(s->start, s->gp, s->tb32, st));
-        MPS_TRY(contract_tiled<T>(grid, s->n, nrhs, s->start, w, s->gp, tb, partial, out, st));
+    // float64: the warp-per-particle gather, whose lanes stay busy; float32: the shared-memory tile
+    bool contracted = false;
+    if constexpr (sizeof(T) == 4) {
+        if (use_tiles) {
+            MPS_TRY(tile_bins_pentry(s->start, s->gp, s->tb32, st));
+            MPS_TRY(contract_tiled<float>(s->grid32, s->n, nrhs, s->start, s->w32, s->gp, s->tb32, s->partial32, out, st));
+            contracted = true;
+        }
     }
-    else
-        MPS_TRY(contract<T>(grid, s->n, nrhs, s->start, w, s->gp, out, st));
+    if (!contracted) MPS_TRY(contract<T>(grid, s->n, nrhs, s->start, w, s->gp, out, st));
     STAGE_MARK(6);
     if (dbl) {
         MPS_TRY(ensure_p64(s, st));
@@ -3103,7 +3111,7 @@ extern "C" int mps_system_graphs(const mps_system *sys, int32_t *built, int32_t 
 
 extern "C" int mps_system_tuning(const mps_system *sys, int32_t *tile_depth, float *ms) {
     if (!sys || !tile_depth || !ms) return MPS_BAD_ARG;
-    tile_depth[0] = sys->tb64.tz;
+    tile_depth[0] = sys->tb64.mem ? sys->tb64.tz : sys->tbn.tz;
     tile_depth[1] = sys->inner ? sys->inner->tb.tz : (sys->tbg.mem ? sys->tbg.tz : sys->tb32.tz);
     for (int p = 0; p < 2; ++p) {
         TuneKey key;

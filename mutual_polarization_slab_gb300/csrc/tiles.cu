@@ -171,13 +171,13 @@ static int64_t axis_tile_bound(int N, int T, int P) {
 
 // Tile lists without a host round trip: the entry arrays are sized by the per-particle bound (nentries holds that
 // capacity), the offsets and totals stay on the device.
-int tile_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tz, TileBins &tb, cudaStream_t s) {
+static int bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tx, int ty, int tz, TileBins &tb,
+                      cudaStream_t s) {
     tile_bins_free(tb, s);
-    if (!tiles_supported(gp, tz) || n < 1) return MPS_BAD_ARG;
     TileGeom tg;
     tg.P = gp.P;
-    tg.T[0] = kTileX;
-    tg.T[1] = kTileY;
+    tg.T[0] = tx;
+    tg.T[1] = ty;
     tg.T[2] = tz;
     int64_t per = 1;
     for (int d = 0; d < 3; ++d) {
@@ -185,6 +185,8 @@ int tile_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int t
         tg.nt[d] = (gp.N[d] + tg.T[d] - 1) / tg.T[d];
         per *= axis_tile_bound(gp.N[d], tg.T[d], gp.P);
     }
+    tb.tx = tx;
+    tb.ty = ty;
     tb.tz = tz;
     tb.ntx = tg.nt[0];
     tb.nty = tg.nt[1];
@@ -237,6 +239,11 @@ int tile_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int t
     return MPS_OK;
 }
 
+int tile_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tz, TileBins &tb, cudaStream_t s) {
+    if (!tiles_supported(gp, tz) || n < 1) return MPS_BAD_ARG;
+    return bins_build(start, n, gp, kTileX, kTileY, tz, tb, s);
+}
+
 // A warp per tile: for each of its (sorted) entries, where it sits in the particle's own list.
 __global__ void k_tile_pentry(const int64_t *__restrict__ tstart, int64_t ntiles, const int32_t *__restrict__ entries,
                               const int32_t *__restrict__ start, TileGeom tg, const int64_t *__restrict__ pstart,
@@ -255,8 +262,8 @@ int tile_bins_pentry(const int32_t *start, const GridParams &gp, TileBins &tb, c
     if (tb.has_pentry || !tb.mem) return MPS_OK;
     TileGeom tg;
     tg.P = gp.P;
-    tg.T[0] = kTileX;
-    tg.T[1] = kTileY;
+    tg.T[0] = tb.tx;
+    tg.T[1] = tb.ty;
     tg.T[2] = tb.tz;
     for (int d = 0; d < 3; ++d) {
         tg.N[d] = gp.N[d];
@@ -423,6 +430,192 @@ __global__ void __launch_bounds__(256) k_spread_tiled(const double *__restrict__
             }
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// Float64 spread, node by node
+// ---------------------------------------------------------------------------
+// A float64 warp instruction costs GB300 the same whether one lane is active or thirty-two, so the tiled spread above,
+// whose lanes sit idle wherever a particle misses their column (about 60 % of them at P = 10), loses on every one.
+// Here a lane owns single nodes and walks the particles that cover each: the particles of an 8 x 8 x TZ tile are staged
+// up to kNodeChunk at a time with their factors aligned to the tile and, per tile column, row and plane, the bit mask of
+// the particles that reach it; the AND of a node's three masks lists its particles.  The lanes of a warp (a 4 x 4 x 2
+// patch) walk different particles at the same time, and what is lost is the difference between the patch's largest list
+// and its mean (14 particles a node and 18 in the largest list at P = 10 and one particle in 71 nodes).  The products
+// m wx are formed once per particle and column while staging, so a node's particle costs one product wy wz and one
+// multiply-add per component.  Lists run in the order of the particles' ids: the sums are deterministic, every node is
+// written once.  Measured against the tiled spread: three vectors, N = 100,000, 192^3, P = 10 3.82 -> 2.31 ms; one vector,
+// N = 20,000, 86^3, P = 8 277 -> 142 us; one vector, N = 500, 25^3 62 -> 12 us; 36 vectors, N = 2000, 31^3, P = 5 twelve
+// launches of 110 us -> one of 142 us.
+constexpr int kNodeTile = 8;
+constexpr int kNodeChunk = 96;      // 3 mask words
+constexpr int kNodeWords = kNodeChunk / 32;
+
+// Depth 8 (two nodes a thread) unless that leaves fewer than two blocks for every SM, then 4 (one node a thread: there
+// the length of a lane's list is the time a block takes).
+static int node_tile_depth(const GridParams &gp, int nrhs) {
+    const int64_t nxy = (int64_t)((gp.N[0] + kNodeTile - 1) / kNodeTile) * ((gp.N[1] + kNodeTile - 1) / kNodeTile);
+    return nxy * ((gp.N[2] + 7) / 8) * ((nrhs + 2) / 3) >= 304 ? 8 : 4;
+}
+
+bool nodes_supported(const GridParams &gp) {
+    return gp.P >= 1 && gp.P <= kMaxP && gp.N[0] >= kNodeTile && gp.N[1] >= kNodeTile && gp.N[2] >= kNodeTile;
+}
+
+int node_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int nrhs, TileBins &tb, cudaStream_t s) {
+    if (!nodes_supported(gp) || n < 1) return MPS_BAD_ARG;
+    return bins_build(start, n, gp, kNodeTile, kNodeTile, node_tile_depth(gp, nrhs), tb, s);
+}
+
+template <int NR, int TZ>
+struct NodeStage {
+    static constexpr int C = 3 * NR;
+    double mwx[kNodeChunk][kNodeTile * C + 1];      // m_c wx at the tile's columns (odd stride: no bank conflicts)
+    double wyz[kNodeChunk][kNodeTile + TZ + 1];     // wy at its rows, wz at its planes
+    unsigned mask[kNodeWords][2 * kNodeTile + TZ];  // particles that reach a column, row, plane
+};
+
+constexpr int kNodeThreads = 256;
+
+template <int NR, int TZ>
+__global__ void __launch_bounds__(kNodeThreads) k_spread_nodes(const double *__restrict__ m, int64_t n, int rfirst,
+                                                          const int32_t *__restrict__ start,
+                                                          const double *__restrict__ w, GridParams gp,
+                                                          const int64_t *__restrict__ tstart,
+                                                          const int32_t *__restrict__ entries, int ntx, int nty,
+                                                          double *__restrict__ grid) {
+    constexpr int C = 3 * NR, NQ = TZ / 4;
+    extern __shared__ __align__(16) unsigned char smem_nodes[];
+    NodeStage<NR, TZ> &st = *reinterpret_cast<NodeStage<NR, TZ> *>(smem_nodes);
+    const int r0 = rfirst + NR * (int)blockIdx.y;
+    const int64_t t = blockIdx.x;
+    const int X0 = (int)(t % ntx) * kNodeTile, Y0 = (int)((t / ntx) % nty) * kNodeTile,
+              Z0 = (int)(t / ((int64_t)ntx * nty)) * TZ;
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int P = gp.P, Nx = gp.N[0], Ny = gp.N[1], Nz = gp.N[2];
+    // warp: patch of 4 x 4 columns and 2 planes, for its node q planes TZ / 2 (wid >> 2) + 2 q + {0, 1}
+    const int x = 4 * (wid & 1) + (lane & 3), y = 4 * ((wid >> 1) & 1) + ((lane >> 2) & 3);
+    const int zb = TZ / 2 * (wid >> 2) + (lane >> 4);
+    double acc[NQ][C];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+#pragma unroll
+        for (int c = 0; c < C; ++c) acc[q][c] = 0.0;
+    const int64_t e0 = tstart[t], e1 = tstart[t + 1];
+    for (int64_t cb = e0; cb < e1; cb += kNodeChunk) {
+        const int cnt = (int)min((int64_t)kNodeChunk, e1 - cb);
+        // staging: a warp takes 32 particles (one per lane) and one axis of the tile; the factors' loads come first
+        for (int task = wid; task < 3 * kNodeWords; task += kNodeThreads / 32) {
+            const int word = task / 3, d = task - 3 * word, pp = 32 * word + lane;
+            const int origin = d == 0 ? X0 : (d == 1 ? Y0 : Z0), Nd = d == 0 ? Nx : (d == 1 ? Ny : Nz);
+            const int len = d == 2 ? TZ : kNodeTile;
+            const bool in = pp < cnt;
+            const int32_t a = in ? entries[cb + pp] : 0;
+            int j = in ? origin - start[3 * (int64_t)a + d] : 0;   // stencil index of the tile's first node
+            if (j < 0) j += Nd;
+            const double *wa = w + ((int64_t)a * 3 + d) * P;
+            double v[kNodeTile], mv[C];
+            unsigned hits = 0u;
+#pragma unroll
+            for (int k = 0; k < kNodeTile; ++k) {
+                const bool hit = in && k < len && j < P && origin + k < Nd;
+                v[k] = hit ? wa[j] : 0.0;
+                hits |= hit ? 1u << k : 0u;
+                if (++j >= Nd) j = 0;
+            }
+            if (d == 0) {
+#pragma unroll
+                for (int r = 0; r < NR; ++r)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) mv[3 * r + c] = in ? m[((int64_t)(r0 + r) * n + a) * 3 + c] : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < kNodeTile; ++k) {
+                if (k >= len) break;
+                const unsigned mk = __ballot_sync(0xffffffffu, (hits >> k) & 1u);
+                if (lane == 0) st.mask[word][d * kNodeTile + k] = mk;
+                if (d == 0) {
+#pragma unroll
+                    for (int c = 0; c < C; ++c) st.mwx[pp][k * C + c] = v[k] * mv[c];
+                } else {
+                    st.wyz[pp][(d - 1) * kNodeTile + k] = v[k];
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const int z = zb + 2 * q;
+            unsigned b[kNodeWords];
+#pragma unroll
+            for (int k = 0; k < kNodeWords; ++k)
+                b[k] = st.mask[k][x] & st.mask[k][kNodeTile + y] & st.mask[k][2 * kNodeTile + z];
+            while (true) {
+                // the next particle of this lane's list
+                int p;
+                if (b[0]) {
+                    p = __ffs(b[0]) - 1;
+                    b[0] &= b[0] - 1;
+                } else if (b[1]) {
+                    p = 31 + __ffs(b[1]);
+                    b[1] &= b[1] - 1;
+                } else if (b[2]) {
+                    p = 63 + __ffs(b[2]);
+                    b[2] &= b[2] - 1;
+                } else {
+                    break;
+                }
+                const double wv = st.wyz[p][y] * st.wyz[p][kNodeTile + z];
+                const double *mw = &st.mwx[p][x * C];
+#pragma unroll
+                for (int c = 0; c < C; ++c) acc[q][c] += wv * mw[c];
+            }
+        }
+        __syncthreads();
+    }
+    if (X0 + x < Nx && Y0 + y < Ny) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const int gz = Z0 + zb + 2 * q;
+            if (gz < Nz) {
+                double *g = grid + (int64_t)3 * r0 * gp.G + ((int64_t)gz * Ny + Y0 + y) * Nx + X0 + x;
+#pragma unroll
+                for (int c = 0; c < C; ++c) g[c * gp.G] = acc[q][c];
+            }
+        }
+    }
+}
+
+template <int NR, int TZ>
+static int nodes_launch(const double *m, int64_t n, int r0, int groups, const int32_t *start, const double *w,
+                        const GridParams &gp, const TileBins &tb, double *grid, cudaStream_t s) {
+    const size_t smem = sizeof(NodeStage<NR, TZ>);
+    if (smem > 48 * 1024)
+        MPS_CUDA_TRY(cudaFuncSetAttribute(k_spread_nodes<NR, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)smem));
+    k_spread_nodes<NR, TZ><<<dim3((unsigned)tb.ntiles, groups), kNodeThreads, smem, s>>>(
+        m, n, r0, start, w, gp, tb.tile_start, tb.entries, tb.ntx, tb.nty, grid);
+    MPS_LAUNCH_CHECK();
+    return MPS_OK;
+}
+
+// Three vectors to a block; all their groups in one launch (small grids have too few tiles to fill the GPU).
+template <int TZ>
+static int nodes_dispatch(const double *m, int64_t n, int nrhs, const int32_t *start, const double *w,
+                          const GridParams &gp, const TileBins &tb, double *grid, cudaStream_t s) {
+    const int full = nrhs / 3, rest = nrhs - 3 * full;
+    int rc = full ? nodes_launch<3, TZ>(m, n, 0, full, start, w, gp, tb, grid, s) : MPS_OK;
+    if (!rc && rest == 2) rc = nodes_launch<2, TZ>(m, n, 3 * full, 1, start, w, gp, tb, grid, s);
+    if (!rc && rest == 1) rc = nodes_launch<1, TZ>(m, n, 3 * full, 1, start, w, gp, tb, grid, s);
+    return rc;
+}
+
+int spread_nodes(const double *m, int64_t n, int nrhs, const int32_t *start, const double *w, const GridParams &gp,
+                 const TileBins &tb, double *grid, cudaStream_t s) {
+    if (tb.tx != kNodeTile || tb.ty != kNodeTile) return MPS_BAD_ARG;
+    if (tb.tz == 8) return nodes_dispatch<8>(m, n, nrhs, start, w, gp, tb, grid, s);
+    if (tb.tz == 4) return nodes_dispatch<4>(m, n, nrhs, start, w, gp, tb, grid, s);
+    return MPS_BAD_ARG;
 }
 
 // ---------------------------------------------------------------------------
@@ -752,11 +945,7 @@ int dfv_to_f64_inplace(double *g, int64_t total, cudaStream_t s) {
 
 template int spread_tiled<float>(const double *, int64_t, int, const int32_t *, const float *, const GridParams &,
                                  const TileBins &, float *, cudaStream_t);
-template int spread_tiled<double>(const double *, int64_t, int, const int32_t *, const double *, const GridParams &,
-                                  const TileBins &, double *, cudaStream_t);
 template int contract_tiled<float>(const float *, int64_t, int, const int32_t *, const float *, const GridParams &,
                                    const TileBins &, float *, double *, cudaStream_t);
-template int contract_tiled<double>(const double *, int64_t, int, const int32_t *, const double *,
-                                    const GridParams &, const TileBins &, double *, double *, cudaStream_t);
 
 }  // namespace mps

@@ -13,7 +13,8 @@ constexpr int kMaxTilesPerDim = 4;
 
 // Particles binned into every grid tile their P^3 stencil touches.
 struct TileBins {
-    int tz = 0;                 // tile depth (z)
+    int tx = kTileX, ty = kTileY;   // tile width (x) and height (y)
+    int tz = 0;                     // tile depth (z)
     int ntx = 0, nty = 0, ntz = 0;
     int64_t ntiles = 0;
     int64_t nentries = 0;
@@ -37,6 +38,9 @@ constexpr int kHomeBlock = 8;
 
 bool tiles_supported(const GridParams &gp, int tz);
 int tile_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tz, TileBins &tb, cudaStream_t s);
+// Bins for spread_nodes: 8 x 8 tiles of the depth that node_tile_depth gives.
+int node_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int nrhs, TileBins &tb, cudaStream_t s);
+bool nodes_supported(const GridParams &gp);
 // Fills tb.pentry (once) for the gathers of the tiled contractions.
 int tile_bins_pentry(const int32_t *start, const GridParams &gp, TileBins &tb, cudaStream_t s);
 // Fills the home bins (once) for the staged contractions.
@@ -47,6 +51,10 @@ void tile_bins_free(TileBins &tb, cudaStream_t s);
 template <typename T>
 int spread_tiled(const double *m, int64_t n, int nrhs, const int32_t *start, const T *w, const GridParams &gp,
                  const TileBins &tb, T *grid, cudaStream_t s);
+
+// The float64 spread (same result, node by node from the particles that cover it); tb from node_bins_build.
+int spread_nodes(const double *m, int64_t n, int nrhs, const int32_t *start, const double *w, const GridParams &gp,
+                 const TileBins &tb, double *grid, cudaStream_t s);
 
 // out[r][a][c] = hprod * sum over the stencil (overwrites); partial: nentries * 3 * min(nrhs,3) of T.
 template <typename T>
