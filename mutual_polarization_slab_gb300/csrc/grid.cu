@@ -94,53 +94,55 @@ __global__ void __launch_bounds__(256) k_spread(const double *__restrict__ m, in
     }
 }
 
-// Contract: one warp per particle, gather + warp reduction; out = Hk (overwrites).
+// Contract: one warp per particle in the visiting order, gather + warp reduction; out = Hk (overwrites).  Lanes take the
+// stencil's (x, y) columns; a column's z sums are weighted by wx wy once, so a node costs one multiply-add per component
+// (in float64 the arithmetic bounds this kernel: three vectors, N = 100,000, P = 10 2.55 -> 1.92 ms, where 3.3
+// multiply-adds a node take 1.98 at the measured rate; one vector, N = 20,000, P = 8 100 -> 70 us; 36 vectors,
+// N = 2000, P = 5 202 -> 109 us).
+// Blocks of 4 warps and one warp per particle and vector (grid y): a few hundred particles still reach every SM.
 template <typename T>
-__global__ void __launch_bounds__(256) k_contract(const T *__restrict__ grid, int64_t n, int nrhs,
+__global__ void __launch_bounds__(128) k_contract(const T *__restrict__ grid, int64_t n,
                                                   const int32_t *__restrict__ start, const T *__restrict__ w,
                                                   GridParams gp, double *__restrict__ out) {
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, r = blockIdx.y;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int P = gp.P;
     const int Nx = gp.N[0], Ny = gp.N[1], Nz = gp.N[2];
-    const int64_t G = gp.G;
-    for (int64_t a = warp; a < n; a += nw) {
+    const int64_t G = gp.G, plane = (int64_t)Nx * Ny;
+    const T *g0 = grid + (int64_t)(3 * r) * G;
+    for (int64_t i = warp; i < n; i += nw) {
+        const int64_t a = gp.order ? gp.order[i] : i;
         const int sx = start[3 * a], sy = start[3 * a + 1], sz = start[3 * a + 2];
         const T *wa = w + a * 3 * P;
-        for (int r = 0; r < nrhs; ++r) {
-            const T *g0 = grid + (int64_t)(3 * r) * G;
-            T a0 = 0, a1 = 0, a2 = 0;
-            for (int row0 = 0; row0 < P * P; row0 += 32) {
-                int idx, sub, lpp;
-                if (!stencil_row(row0, P, lane, &idx, &sub, &lpp)) continue;
-                const int jx = idx % P, jy = idx / P;
-                int ix = sx + jx;
-                if (ix >= Nx) ix -= Nx;
-                int iy = sy + jy;
-                if (iy >= Ny) iy -= Ny;
-                const T wxy = wa[jx] * wa[P + jy];
-                const int64_t rowb = (int64_t)ix + (int64_t)Nx * iy;
-                for (int jz = sub; jz < P; jz += lpp) {
-                    int iz = sz + jz;
-                    if (iz >= Nz) iz -= Nz;
-                    const T wv = wxy * wa[2 * P + jz];
-                    const int64_t node = rowb + (int64_t)Nx * Ny * iz;
-                    a0 += wv * g0[node];
-                    a1 += wv * g0[G + node];
-                    a2 += wv * g0[2 * G + node];
-                }
+        T a0 = 0, a1 = 0, a2 = 0;
+        for (int row0 = 0; row0 < P * P; row0 += 32) {
+            int idx, sub, lpp;
+            if (!stencil_row(row0, P, lane, &idx, &sub, &lpp)) continue;
+            const int jx = idx % P, jy = idx / P;
+            int ix = sx + jx;
+            if (ix >= Nx) ix -= Nx;
+            int iy = sy + jy;
+            if (iy >= Ny) iy -= Ny;
+            const T *gr = g0 + ix + (int64_t)Nx * iy;
+            const T wxy = wa[jx] * wa[P + jy];
+            T c0 = 0, c1 = 0, c2 = 0;
+#pragma unroll 4
+            for (int jz = sub; jz < P; jz += lpp) {
+                int iz = sz + jz;
+                if (iz >= Nz) iz -= Nz;
+                const T wz = wa[2 * P + jz];
+                const T *g = gr + plane * iz;
+                c0 += wz * g[0];
+                c1 += wz * g[G];
+                c2 += wz * g[2 * G];
             }
-            a0 = warp_sum(a0);
-            a1 = warp_sum(a1);
-            a2 = warp_sum(a2);
-            if (lane == 0) {
-                double *o = out + ((int64_t)r * n + a) * 3;
-                o[0] = (double)a0 * gp.hprod;
-                o[1] = (double)a1 * gp.hprod;
-                o[2] = (double)a2 * gp.hprod;
-            }
+            a0 += wxy * c0;
+            a1 += wxy * c1;
+            a2 += wxy * c2;
         }
+        const T v = warp_sum4(a0, a1, a2, (T)0, lane);
+        if ((lane & 7) == 0 && lane < 24) out[((int64_t)r * n + a) * 3 + lane / 8] = (double)v * gp.hprod;
     }
 }
 
@@ -489,8 +491,12 @@ template <typename T>
 int contract(const T *grid, int64_t n, int nrhs, const int32_t *start, const T *w, const GridParams &gp, double *out,
              cudaStream_t s) {
     if (n == 0) return MPS_OK;
-    k_contract<T><<<grid_for(n * 32, 256, 152 * 64), 256, 0, s>>>(grid, n, nrhs, start, w, gp, out);
-    MPS_LAUNCH_CHECK();
+    for (int r0 = 0; r0 < nrhs; r0 += 32768) {   // grid y stays below its limit of 65535
+        const int nr = nrhs - r0 < 32768 ? nrhs - r0 : 32768;
+        k_contract<T><<<dim3(grid_for(n * 32, 128, 152 * 128), nr), 128, 0, s>>>(grid + (int64_t)3 * r0 * gp.G, n, start,
+                                                                                w, gp, out + (int64_t)3 * r0 * n);
+        MPS_LAUNCH_CHECK();
+    }
     return MPS_OK;
 }
 
