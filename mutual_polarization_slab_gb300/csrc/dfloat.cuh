@@ -8,15 +8,23 @@
 
 namespace mps {
 
+// (double)f by integer instructions: the conversion instruction runs on GB300's narrow float64 pipe.  Zeros, denormals,
+// infinities and NaNs take it all the same.
+__device__ __forceinline__ double float_to_double(float f) {
+    const unsigned u = __float_as_uint(f), a = u & 0x7fffffffu;
+    if (a - 0x00800000u >= 0x7f000000u) return a == 0u ? __hiloint2double((int)u, 0) : (double)f;
+    return __hiloint2double((int)((u & 0x80000000u) | ((a >> 3) + 0x38000000u)), (int)(u << 29));
+}
+
 struct __align__(8) dfv {
     float hi, lo;
     dfv() = default;
     __device__ __forceinline__ dfv(float h, float l) : hi(h), lo(l) {}
     __device__ __forceinline__ explicit dfv(double v) {
         hi = __double2float_rn(v);
-        lo = __double2float_rn(v - (double)hi);
+        lo = __double2float_rn(v - float_to_double(hi));
     }
-    __device__ __forceinline__ explicit operator double() const { return (double)hi + (double)lo; }
+    __device__ __forceinline__ explicit operator double() const { return float_to_double(hi) + float_to_double(lo); }
 };
 
 __device__ __forceinline__ dfv dfv_fast_two_sum(float a, float b) {

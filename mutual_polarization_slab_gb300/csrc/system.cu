@@ -774,77 +774,90 @@ static bool own_fft32() {
     return e && strcmp(e, "own") == 0;
 }
 
-template <typename T>
-static int matvec_impl(mps_system *s, const double *m, double *out, int nrhs, cudaStream_t st) {
-    const bool dbl = sizeof(T) == 8;
-    const bool own_fft = !dbl && own_fft32() && df_usable(s);
-    const bool f64_fft = dbl && f64_usable(s);
-    if (f64_fft) MPS_TRY(f64_prepare(s, st));
-    bool use_tiles = false;
-    if (dbl) {
-        use_tiles = s->tiled && nodes_supported(s->gp);
-        if (use_tiles && !s->tbn.mem) MPS_TRY(node_bins_build(s->start, s->n, s->gp, s->max_rhs, s->tbn, st));
+// Wave-space field grids of nrhs moment vectors in float64 (spread, transforms, dipole scale), left in s->grid64.  Stage
+// marks 2..5 of the calling matvec (ev may be null).
+static int f64_field_grids(mps_system *s, const double *m, int nrhs, StageEvents *ev, cudaStream_t st) {
+    const bool own = f64_usable(s), nodes = s->tiled && nodes_supported(s->gp);
+    if (own) MPS_TRY(f64_prepare(s, st));
+    if (nodes && !s->tbn.mem) MPS_TRY(node_bins_build(s->start, s->n, s->gp, s->max_rhs, s->tbn, st));
+    MPS_TRY(ensure_grids(s, MPS_FP64, st));
+    if (nodes)
+        MPS_TRY(spread_nodes(m, s->n, nrhs, s->start, s->w64, s->gp, s->tbn, s->grid64, st));
+    else
+        MPS_TRY(spread<double>(m, s->n, nrhs, s->start, s->w64, s->gp, s->grid64, st));
+    STAGE_MARK(2);
+    if (own) {
+        MPS_TRY(f64_forward_xy(s->grid64, s->spec64, 3 * nrhs, s->gp, s->f64p, st));
+        STAGE_MARK(3);
+        MPS_TRY(f64_z_scale_dipole(s->spec64, nrhs, s->gp, s->f64p, s->green->hs64, st));
+        STAGE_MARK(4);
+        MPS_TRY(f64_inverse_yx(s->spec64, s->grid64, 3 * nrhs, s->gp, s->f64p, st));
     } else {
-        MPS_TRY(ensure_tiles(s, kTileRef32, st, &use_tiles));
+        MPS_TRY(exec_plan(s, CUFFT_D2Z, 3 * nrhs, s->grid64, s->spec64, 0, st));
+        STAGE_MARK(3);
+        MPS_TRY(scale_half<double>(s->spec64, nrhs, s->gp, s->h64, st));
+        STAGE_MARK(4);
+        MPS_TRY(exec_plan(s, CUFFT_Z2D, 3 * nrhs, s->spec64, s->grid64, 0, st));
     }
-    MPS_TRY(ensure_grids(s, dbl ? MPS_FP64 : MPS_FP32, st));
-    T *grid = dbl ? (T *)s->grid64 : (T *)s->grid32;
-    void *spec = dbl ? s->spec64 : s->spec32;
-    const T *w = dbl ? (const T *)s->w64 : (const T *)s->w32;
-    const T *hh = dbl ? (const T *)s->h64 : (const T *)s->h32;
+    STAGE_MARK(5);
+    return MPS_OK;
+}
+
+static int matvec_f64(mps_system *s, const double *m, double *out, int nrhs, cudaStream_t st) {
     const double vol = s->box[0] * s->box[1] * s->box[2];
     StageEvents *ev = nullptr;
-    MPS_TRY(stage_begin(s, dbl ? MPS_FP64 : MPS_FP32, &ev, st));
+    MPS_TRY(stage_begin(s, MPS_FP64, &ev, st));
     if (s->slab_factor != 0.0) MPS_TRY(slab_terms(m, s->n, nrhs, s->slab_factor / vol, s->slab, st));
     STAGE_MARK(1);
-    if (use_tiles) {
-        if constexpr (sizeof(T) == 8)
-            MPS_TRY(spread_nodes(m, s->n, nrhs, s->start, s->w64, s->gp, s->tbn, s->grid64, st));
-        else
-            MPS_TRY(spread_tiled<float>(m, s->n, nrhs, s->start, s->w32, s->gp, s->tb32, s->grid32, st));
-    } else {
-        MPS_TRY(spread<T>(m, s->n, nrhs, s->start, w, s->gp, grid, st));
-    }
+    MPS_TRY(f64_field_grids(s, m, nrhs, ev, st));
+    MPS_TRY(contract<double>(s->grid64, s->n, nrhs, s->start, s->w64, s->gp, out, st));
+    STAGE_MARK(6);
+    MPS_TRY(ensure_p64(s, st));
+    MPS_TRY(real_space_csr<double>(m, out, s->n, nrhs, s->row_ptr, s->p64, s->diag, s->diag_idx, s->slab, true, st));
+    STAGE_MARK(7);
+    return MPS_OK;
+}
+
+// The reference discretisation in float32.
+static int matvec_f32(mps_system *s, const double *m, double *out, int nrhs, cudaStream_t st) {
+    const bool own_fft = own_fft32() && df_usable(s);
+    bool use_tiles = false;
+    MPS_TRY(ensure_tiles(s, kTileRef32, st, &use_tiles));
+    MPS_TRY(ensure_grids(s, MPS_FP32, st));
+    float *grid = s->grid32;
+    const double vol = s->box[0] * s->box[1] * s->box[2];
+    StageEvents *ev = nullptr;
+    MPS_TRY(stage_begin(s, MPS_FP32, &ev, st));
+    if (s->slab_factor != 0.0) MPS_TRY(slab_terms(m, s->n, nrhs, s->slab_factor / vol, s->slab, st));
+    STAGE_MARK(1);
+    if (use_tiles)
+        MPS_TRY(spread_tiled<float>(m, s->n, nrhs, s->start, s->w32, s->gp, s->tb32, grid, st));
+    else
+        MPS_TRY(spread<float>(m, s->n, nrhs, s->start, s->w32, s->gp, grid, st));
     STAGE_MARK(2);
     if (own_fft) {
-        MPS_TRY(f32_forward_xy((const float *)grid, (float2 *)spec, 3 * nrhs, s->gp, s->dfp, st));
+        MPS_TRY(f32_forward_xy(grid, (float2 *)s->spec32, 3 * nrhs, s->gp, s->dfp, st));
         STAGE_MARK(3);
-        MPS_TRY(f32_z_scale_dipole((float2 *)spec, nrhs, s->gp, s->dfp, (const float *)hh, st));
+        MPS_TRY(f32_z_scale_dipole((float2 *)s->spec32, nrhs, s->gp, s->dfp, s->h32, st));
         STAGE_MARK(4);
-        MPS_TRY(f32_inverse_yx((float2 *)spec, (float *)grid, 3 * nrhs, s->gp, s->dfp, st));
-        STAGE_MARK(5);
-    } else if (f64_fft) {
-        MPS_TRY(f64_forward_xy((const double *)grid, spec, 3 * nrhs, s->gp, s->f64p, st));
-        STAGE_MARK(3);
-        MPS_TRY(f64_z_scale_dipole(spec, nrhs, s->gp, s->f64p, s->green->hs64, st));
-        STAGE_MARK(4);
-        MPS_TRY(f64_inverse_yx(spec, (double *)grid, 3 * nrhs, s->gp, s->f64p, st));
+        MPS_TRY(f32_inverse_yx((float2 *)s->spec32, grid, 3 * nrhs, s->gp, s->dfp, st));
         STAGE_MARK(5);
     } else {
-        MPS_TRY(exec_plan(s, dbl ? CUFFT_D2Z : CUFFT_R2C, 3 * nrhs, grid, spec, 0, st));
+        MPS_TRY(exec_plan(s, CUFFT_R2C, 3 * nrhs, grid, s->spec32, 0, st));
         STAGE_MARK(3);
-        MPS_TRY(scale_half<T>(spec, nrhs, s->gp, hh, st));
+        MPS_TRY(scale_half<float>(s->spec32, nrhs, s->gp, s->h32, st));
         STAGE_MARK(4);
-        MPS_TRY(exec_plan(s, dbl ? CUFFT_Z2D : CUFFT_C2R, 3 * nrhs, spec, grid, 0, st));
+        MPS_TRY(exec_plan(s, CUFFT_C2R, 3 * nrhs, s->spec32, grid, 0, st));
         STAGE_MARK(5);
     }
-    // float64: the warp-per-particle gather, whose lanes stay busy; float32: the shared-memory tile
-    bool contracted = false;
-    if constexpr (sizeof(T) == 4) {
-        if (use_tiles) {
-            MPS_TRY(tile_bins_pentry(s->start, s->gp, s->tb32, st));
-            MPS_TRY(contract_tiled<float>(s->grid32, s->n, nrhs, s->start, s->w32, s->gp, s->tb32, s->partial32, out, st));
-            contracted = true;
-        }
+    if (use_tiles) {   // the shared-memory tile
+        MPS_TRY(tile_bins_pentry(s->start, s->gp, s->tb32, st));
+        MPS_TRY(contract_tiled<float>(grid, s->n, nrhs, s->start, s->w32, s->gp, s->tb32, s->partial32, out, st));
+    } else {
+        MPS_TRY(contract<float>(grid, s->n, nrhs, s->start, s->w32, s->gp, out, st));
     }
-    if (!contracted) MPS_TRY(contract<T>(grid, s->n, nrhs, s->start, w, s->gp, out, st));
     STAGE_MARK(6);
-    if (dbl) {
-        MPS_TRY(ensure_p64(s, st));
-        MPS_TRY(real_space_csr<double>(m, out, s->n, nrhs, s->row_ptr, s->p64, s->diag, s->diag_idx, s->slab, true, st));
-    } else {
-        MPS_TRY(real_space_f32(s, m, out, nrhs, st));
-    }
+    MPS_TRY(real_space_f32(s, m, out, nrhs, st));
     STAGE_MARK(7);
     return MPS_OK;
 }
@@ -1121,7 +1134,7 @@ static int matvec_grad(mps_system *s, const double *m, double *out, int nrhs, cu
     }
     bool use_tiles = false;
     MPS_TRY(ensure_tiles(s, kTileGrad32, st, &use_tiles));
-    if (!use_tiles) return matvec_impl<float>(s, m, out, nrhs, st);
+    if (!use_tiles) return matvec_f32(s, m, out, nrhs, st);
     MPS_TRY(ensure_grids(s, MPS_FP32, st));
     if (!s->hs32_ready) {
         std::lock_guard<std::mutex> lk(g_green_mu);
@@ -1223,7 +1236,7 @@ static int matvec_real(mps_system *s, const double *m, double *out, int nrhs, in
     if (s->kind == MPS_DIPOLE_QUADRUPOLE)
         return precision == MPS_FP64 ? matvec_quad<double>(s, m, out, nrhs, st)
                                      : matvec_quad<float>(s, m, out, nrhs, st);
-    return precision == MPS_FP64 ? matvec_impl<double>(s, m, out, nrhs, st) : matvec_impl<float>(s, m, out, nrhs, st);
+    return precision == MPS_FP64 ? matvec_f64(s, m, out, nrhs, st) : matvec_f32(s, m, out, nrhs, st);
 }
 
 // (Re m, Im m) per particle -> the 2 nc real vectors, and back with the imaginary
@@ -3137,28 +3150,33 @@ extern "C" int mps_adjoint_forces(mps_system *sys, const double *m, const double
     if (diag_index < 0 || diag_index >= sys->n_diag) return MPS_BAD_ARG;
     MPS_TRY(build_status(sys));
     cudaStream_t st = (cudaStream_t)stream;
-    MPS_TRY(ensure_p64(sys, st));
     const int64_t n = sys->n;
     int *err = nullptr;
+    double2 *slopes = nullptr;
+    double *g = nullptr;
     MPS_TRY(dalloc(&err, sizeof(int), st));
-    int rc = MPS_OK;
-    if (cudaMemsetAsync(err, 0, sizeof(int), st) != cudaSuccess) rc = MPS_CUDA_ERR;
-    if (!rc) rc = rs_force(m, n, sys->row_ptr, sys->p64, perp, para, rvals, n_tab, forces, err, st);
+    int rc = dalloc(&slopes, sizeof(double2) * (size_t)n_tab, st);
+    if (!rc) rc = dalloc(&g, sizeof(double) * 3 * (size_t)n * sys->gp.P, st);
+    if (!rc && cudaMemsetAsync(err, 0, sizeof(int), st) != cudaSuccess) rc = MPS_CUDA_ERR;
+    // the double-float pair list serves as it is where no float64 copy exists
+    if (!rc)
+        rc = sys->p64.A ? rs_force<double>(m, n, sys->row_ptr, sys->p64, perp, para, rvals, n_tab, slopes, sys->order,
+                                           forces, err, st)
+                        : rs_force<dfv>(m, n, sys->row_ptr, sys->pdf, perp, para, rvals, n_tab, slopes, sys->order,
+                                        forces, err, st);
     // wave space: phi = IFFT(scale(FFT(spread(m)))), float64-accurate, then the weight-gradient contraction.
     // Grids the double-float FFTs support take the double-float pipeline (float64 issue is slow on GB300) and
-    // convert phi to float64 in place; the others use the float64 spread and cuFFT.
+    // convert phi to float64 in place; the others use the float64 stages.
     if (!rc && df_usable(sys)) {
         bool tiles_used = false;
         rc = df_field_grids(sys, m, 1, nullptr, st, &tiles_used);
         if (!rc) rc = dfv_to_f64_inplace(sys->grid64, 3 * sys->gp.G, st);
     } else if (!rc) {
-        rc = ensure_grids(sys, MPS_FP64, st);
-        if (!rc) rc = spread<double>(m, n, 1, sys->start, sys->w64, sys->gp, sys->grid64, st);
-        if (!rc) rc = exec_plan(sys, CUFFT_D2Z, 3, sys->grid64, sys->spec64, 0, st);
-        if (!rc) rc = scale_half<double>(sys->spec64, 1, sys->gp, sys->h64, st);
-        if (!rc) rc = exec_plan(sys, CUFFT_Z2D, 3, sys->spec64, sys->grid64, 0, st);
+        rc = f64_field_grids(sys, m, 1, nullptr, st);
     }
-    if (!rc) rc = wave_force(sys->grid64, sys->x, m, n, sys->start, sys->w64, sys->gp, forces, st);
+    if (!rc) rc = wave_force(sys->grid64, sys->x, m, n, sys->start, sys->w64, g, sys->gp, forces, st);
+    if (slopes) cudaFreeAsync(slopes, st);
+    if (g) cudaFreeAsync(g, st);
     if (!rc && dE_deps) {
         double self = 0.0;
         if (cudaMemcpyAsync(&self, perp, sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
