@@ -211,11 +211,11 @@ struct mps_system {
     double *host_scr = nullptr;
     void *fft_work = nullptr;
     size_t fft_work_bytes = 0;
-    TileBins tb64, tb32;        // tile binning for the tiled spread/contract (per precision tile depth)
+    TileBins tb32;              // tiles of the float32 reference form's spread and contraction (tuned depth)
     TileBins tbg;               // tiles of the gradient-form spread (depth 12 where the grid allows it)
-    TileBins tbn;               // tiles of the float64 node spread
+    TileBins tbn;               // tiles of the float64 and double-float node spread
+    TileBins tb64;              // tiles of the tiled double-float contraction (A/B form)
     double *partial64 = nullptr;
-    int tb_use[2] = {-1, -1};         // tuner consumer that built tb64 / tb32
     float *partial32 = nullptr;
     float *partialg = nullptr;        // partial sums of the tiled gradient-form contraction (A/B form) ...
     int64_t partialg_n = 0;           // ... and its capacity in floats
@@ -529,12 +529,11 @@ static int stage_begin(mps_system *s, int precision, StageEvents **ev, cudaStrea
 // Autotuner for the tiled kernels: the tile depth (z) is timed on the first
 // system of each (grid, support, consumer, batch width) with the kernels that
 // consumer runs, and the fastest is kept for the rest of the process.  The
-// consumers: the float32 reference operator (tiled spread + contract), the
+// consumers: the float32 reference operator (tiled spread + contract) and the
 // float32 gradient operator (its spread; depth 12 without timing where the grid
-// allows it, see tuned_depth) and the double-float operator (spread).  The
-// reference-form float32 kernels use tb32, the gradient form tbg, the double-float
-// kernels tb64 (the float64 spread has tiles of its own, tbn, and no choice to time).
-enum TileUse { kTileRef32 = 0, kTileGrad32 = 1, kTileDF = 2 };
+// allows it, see tuned_depth).  The reference-form kernels use tb32, the gradient
+// form tbg (the node spread of the other precisions has no depth to time).
+enum TileUse { kTileRef32 = 0, kTileGrad32 = 1 };
 struct TuneKey {
     int dev;
     int N[3];
@@ -576,9 +575,6 @@ static int time_tiles(mps_system *s, int use, int tz, int nrhs, const double *m,
             case kTileGrad32:
                 rc = spread_grad_tiled(m, s->n, nrhs, s->start, s->w32, s->g32, s->gp, tb, s->grid32, st);
                 break;
-            default:
-                rc = spread_tiled_df(m, s->n, nrhs, s->start, s->wdf, s->gp, tb, (dfv *)s->grid64, st);
-                break;
         }
         cudaEventRecord(e1, st);
         cudaEventSynchronize(e1);
@@ -593,8 +589,6 @@ static int time_tiles(mps_system *s, int use, int tz, int nrhs, const double *m,
     *ms = best;
     return rc;
 }
-
-static bool tile_depth_known(const mps_system *s, int use);
 
 static int tuned_depth(mps_system *s, int use, cudaStream_t st, int *tz) {
     // MPS_TILE_DEPTH=4 or 8 fixes the depth instead of timing (A/B comparisons and tests); not cached
@@ -667,36 +661,16 @@ static int tuned_depth(mps_system *s, int use, cudaStream_t st, int *tz) {
     return MPS_OK;
 }
 
-// The tile depth of a consumer is settled without timing: fixed by MPS_TILE_DEPTH, the gradient form's fixed
-// depth, or already timed in this process for this (device, grid, support, consumer, batch width).
-static bool tile_depth_known(const mps_system *s, int use) {
-    if (const char *fd = getenv("MPS_TILE_DEPTH")) {
-        const int d = atoi(fd);
-        if (d == 4 || d == 8 || ((d == 12 || d == 16) && use == kTileGrad32)) return true;
-    }
-    if (use == kTileGrad32) return true;
-    TuneKey key;
-    memset(&key, 0, sizeof(key));
-    key.dev = current_device();
-    for (int k = 0; k < 3; ++k) key.N[k] = s->gp.N[k];
-    key.P = s->gp.P;
-    key.use = use;
-    key.nrhs = s->max_rhs < 3 ? s->max_rhs : 3;
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    return g_tune.find(key) != g_tune.end();
-}
-
 // Lazily bins the particles for the tiled kernels of one precision (tile depth
 // from the autotuner, timed for the consumer that asks first).
 static int ensure_tiles(mps_system *s, int use, cudaStream_t st, bool *used) {
     *used = false;
     // the tiled kernels use the separable Gaussian weights of the dipole operator
     if (!s->tiled || s->kind != MPS_DIPOLE || !s->w32 || !s->w64) return MPS_OK;
-    const bool dbl = use == kTileDF;
     const bool grad = use == kTileGrad32;
-    TileBins &tb = dbl ? s->tb64 : (grad ? s->tbg : s->tb32);
+    TileBins &tb = grad ? s->tbg : s->tb32;
     if (!tb.mem) {
-        MPS_TRY(ensure_grids(s, dbl ? MPS_FP64 : MPS_FP32, st));
+        MPS_TRY(ensure_grids(s, MPS_FP32, st));
         int tz = 0;
         MPS_TRY(tuned_depth(s, use, st, &tz));
         if (tz == 0 || !tiles_supported(s->gp, tz)) {
@@ -704,11 +678,17 @@ static int ensure_tiles(mps_system *s, int use, cudaStream_t st, bool *used) {
             return MPS_OK;
         }
         MPS_TRY(tile_bins_build(s->start, s->n, s->gp, tz, tb, st));
-        if (!grad) s->tb_use[dbl ? 0 : 1] = use;
     }
-    if (!dbl && !s->partial32 && use == kTileRef32)
+    if (!s->partial32 && use == kTileRef32)
         MPS_TRY(dalloc(&s->partial32, (size_t)tb.nentries * 9 * sizeof(float), st));
     *used = true;
+    return MPS_OK;
+}
+
+// Tiles of the node spread, built once where the grid and the support allow it.
+static int ensure_nodes(mps_system *s, cudaStream_t st, bool *used) {
+    *used = nodes_supported(s->gp);
+    if (*used && !s->tbn.mem) MPS_TRY(node_bins_build(s->start, s->n, s->gp, s->max_rhs, s->tbn, st));
     return MPS_OK;
 }
 
@@ -777,12 +757,13 @@ static bool own_fft32() {
 // Wave-space field grids of nrhs moment vectors in float64 (spread, transforms, dipole scale), left in s->grid64.  Stage
 // marks 2..5 of the calling matvec (ev may be null).
 static int f64_field_grids(mps_system *s, const double *m, int nrhs, StageEvents *ev, cudaStream_t st) {
-    const bool own = f64_usable(s), nodes = s->tiled && nodes_supported(s->gp);
+    const bool own = f64_usable(s);
+    bool nodes = false;
     if (own) MPS_TRY(f64_prepare(s, st));
-    if (nodes && !s->tbn.mem) MPS_TRY(node_bins_build(s->start, s->n, s->gp, s->max_rhs, s->tbn, st));
+    MPS_TRY(ensure_nodes(s, st, &nodes));
     MPS_TRY(ensure_grids(s, MPS_FP64, st));
     if (nodes)
-        MPS_TRY(spread_nodes(m, s->n, nrhs, s->start, s->w64, s->gp, s->tbn, s->grid64, st));
+        MPS_TRY(spread_nodes<double>(m, s->n, nrhs, s->start, s->w64, s->gp, s->tbn, s->grid64, st));
     else
         MPS_TRY(spread<double>(m, s->n, nrhs, s->start, s->w64, s->gp, s->grid64, st));
     STAGE_MARK(2);
@@ -867,14 +848,13 @@ static int matvec_f32(mps_system *s, const double *m, double *out, int nrhs, cud
 // weights and grids), the FFTs and Green's scale are the double-float transforms
 // of dffft.cu; the pair sum is the float64 kernel.
 // First-use setup of the double-float operator: weights, tile bins (autotuned depth), grids, scale tensor.
-static int df_prepare(mps_system *s, cudaStream_t st, bool *use_tiles_out) {
+static int df_prepare(mps_system *s, cudaStream_t st, bool *nodes_out) {
     const int64_t nw = (int64_t)s->n * 3 * s->gp.P;
     if (!s->wdf) {
         MPS_TRY(dalloc(&s->wdf, sizeof(dfv) * (size_t)nw, st));
         MPS_TRY(weights_df(s->w64, nw, s->wdf, st));
     }
-    bool use_tiles = false;
-    MPS_TRY(ensure_tiles(s, kTileDF, st, &use_tiles));
+    MPS_TRY(ensure_nodes(s, st, nodes_out));
     MPS_TRY(ensure_grids(s, MPS_FP64, st));
     if (!s->tm6_ready) {
         std::lock_guard<std::mutex> lk(g_green_mu);
@@ -889,22 +869,20 @@ static int df_prepare(mps_system *s, cudaStream_t st, bool *use_tiles_out) {
         }
         s->tm6_ready = true;
     }
-    *use_tiles_out = use_tiles;
     return MPS_OK;
 }
 
 // Wave-space field grids of nrhs moment vectors with the float64-accurate operator: double-float spread,
 // FFTs and dipole scale; the 3 nrhs component grids are left in s->grid64 as (hi, lo) float pairs.  Stage
 // marks 2..5 of the calling matvec (ev may be null).
-static int df_field_grids(mps_system *s, const double *m, int nrhs, StageEvents *ev, cudaStream_t st,
-                          bool *use_tiles_out) {
-    bool use_tiles = false;
-    MPS_TRY(df_prepare(s, st, &use_tiles));
+static int df_field_grids(mps_system *s, const double *m, int nrhs, StageEvents *ev, cudaStream_t st) {
+    bool nodes = false;
+    MPS_TRY(df_prepare(s, st, &nodes));
     dfv *grid = (dfv *)s->grid64;           // (hi, lo) float pairs: the size of a double
     float4 *spec = (float4 *)s->spec64;     // float4 per complex value: the size of a double2
     const int64_t gvals = (int64_t)3 * nrhs * s->gp.G;
-    if (use_tiles) {
-        MPS_TRY(spread_tiled_df(m, s->n, nrhs, s->start, s->wdf, s->gp, s->tb64, grid, st));
+    if (nodes) {
+        MPS_TRY(spread_nodes<dfv>(m, s->n, nrhs, s->start, s->wdf, s->gp, s->tbn, grid, st));
     } else {
         MPS_TRY(spread<double>(m, s->n, nrhs, s->start, s->w64, s->gp, s->grid64, st));
         MPS_TRY(f64_to_dfv_inplace(s->grid64, gvals, st));
@@ -916,7 +894,6 @@ static int df_field_grids(mps_system *s, const double *m, int nrhs, StageEvents 
     STAGE_MARK(4);
     MPS_TRY(df_inverse_yx(spec, (float2 *)grid, 3 * nrhs, s->gp, s->dfp, st));
     STAGE_MARK(5);
-    *use_tiles_out = use_tiles;
     return MPS_OK;
 }
 
@@ -926,9 +903,8 @@ static int pair_sum_join(mps_system *s, double *out, int nrhs, cudaStream_t st);
 
 static int matvec_df(mps_system *s, const double *m, double *out, int nrhs, cudaStream_t st) {
     const double vol = s->box[0] * s->box[1] * s->box[2];
-    bool prepared_tiles = false;
-    MPS_TRY(df_prepare(s, st, &prepared_tiles));   // first-use setup outside the stage timing
-    (void)prepared_tiles;
+    bool prepared = false;
+    MPS_TRY(df_prepare(s, st, &prepared));   // first-use setup outside the stage timing
     StageEvents *ev = nullptr;
     MPS_TRY(stage_begin(s, MPS_DF, &ev, st));
     if (s->slab_factor != 0.0) MPS_TRY(slab_terms(m, s->n, nrhs, s->slab_factor / vol, s->slab, st));
@@ -937,15 +913,16 @@ static int matvec_df(mps_system *s, const double *m, double *out, int nrhs, cuda
     const bool beside = pair_sum_beside(ev);
     if (beside) MPS_TRY(pair_sum_fork(s, m, nrhs, st, true));
     STAGE_MARK(1);
-    bool use_tiles = false;
-    MPS_TRY(df_field_grids(s, m, nrhs, ev, st, &use_tiles));
+    MPS_TRY(df_field_grids(s, m, nrhs, ev, st));
     dfv *grid = (dfv *)s->grid64;
     const int64_t gvals = (int64_t)3 * nrhs * s->gp.G;
     const char *ce = getenv("MPS_DF_CONTRACT");   // "tiled": the tiled contraction (A/B timing)
-    const bool tiled_contract = use_tiles && ce && strcmp(ce, "tiled") == 0;
+    const int tz = tiles_supported(s->gp, 8) ? 8 : 4;
+    const bool tiled_contract = ce && strcmp(ce, "tiled") == 0 && tiles_supported(s->gp, tz);
     if (s->gp.P <= kMaxP && !tiled_contract) {
         MPS_TRY(contract_df_warp(grid, s->n, nrhs, s->order, s->start, s->wdf, s->gp, out, st));
-    } else if (use_tiles) {
+    } else if (tiled_contract) {
+        if (!s->tb64.mem) MPS_TRY(tile_bins_build(s->start, s->n, s->gp, tz, s->tb64, st));
         if (!s->partial64) MPS_TRY(dalloc(&s->partial64, (size_t)s->tb64.nentries * 9 * sizeof(double), st));
         MPS_TRY(tile_bins_pentry(s->start, s->gp, s->tb64, st));
         MPS_TRY(contract_tiled_df(grid, s->n, nrhs, s->start, s->w64, s->gp, s->tb64, s->partial64, out, st));
@@ -2127,9 +2104,9 @@ static int refine_mixed(mps_system *s, const double *b, double *x, int nrhs, con
     int step = 0;
     int e = MPS_OK;
     // The double-float residual's first-use set-up (weights, tiles, grids, scale tensor) runs on the system's
-    // prep stream beside the first inner solve, when nothing in it has to be timed (its tile depth is known).
+    // prep stream beside the first inner solve.
     cudaEvent_t ev_prep = nullptr;
-    if (s->resid_prec == MPS_DF && df_usable(s) && !s->wdf && tile_depth_known(s, kTileDF)) {
+    if (s->resid_prec == MPS_DF && df_usable(s) && !s->wdf) {
         cudaEvent_t ev_in = nullptr;
         bool ok = (s->prep || cudaStreamCreateWithFlags(&s->prep, cudaStreamNonBlocking) == cudaSuccess) &&
                   cudaEventCreateWithFlags(&ev_in, cudaEventDisableTiming) == cudaSuccess &&
@@ -3124,21 +3101,20 @@ extern "C" int mps_system_graphs(const mps_system *sys, int32_t *built, int32_t 
 
 extern "C" int mps_system_tuning(const mps_system *sys, int32_t *tile_depth, float *ms) {
     if (!sys || !tile_depth || !ms) return MPS_BAD_ARG;
-    tile_depth[0] = sys->tb64.mem ? sys->tb64.tz : sys->tbn.tz;
+    tile_depth[0] = sys->tbn.tz;
     tile_depth[1] = sys->inner ? sys->inner->tb.tz : (sys->tbg.mem ? sys->tbg.tz : sys->tb32.tz);
-    for (int p = 0; p < 2; ++p) {
-        TuneKey key;
-        memset(&key, 0, sizeof(key));
-        key.dev = current_device();
-        for (int k = 0; k < 3; ++k) key.N[k] = sys->gp.N[k];
-        key.P = sys->gp.P;
-        key.use = p == 1 && sys->tbg.mem ? (int)kTileGrad32 : sys->tb_use[p];
-        key.nrhs = sys->max_rhs < 3 ? sys->max_rhs : 3;
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        auto it = g_tune.find(key);
-        ms[2 * p] = it != g_tune.end() ? it->second.ms[0] : -1.f;
-        ms[2 * p + 1] = it != g_tune.end() ? it->second.ms[1] : -1.f;
-    }
+    ms[0] = ms[1] = -1.f;   // the node spread's depth is not timed
+    TuneKey key;
+    memset(&key, 0, sizeof(key));
+    key.dev = current_device();
+    for (int k = 0; k < 3; ++k) key.N[k] = sys->gp.N[k];
+    key.P = sys->gp.P;
+    key.use = sys->tbg.mem ? kTileGrad32 : kTileRef32;
+    key.nrhs = sys->max_rhs < 3 ? sys->max_rhs : 3;
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    auto it = g_tune.find(key);
+    ms[2] = it != g_tune.end() ? it->second.ms[0] : -1.f;
+    ms[3] = it != g_tune.end() ? it->second.ms[1] : -1.f;
     return MPS_OK;
 }
 
@@ -3168,8 +3144,7 @@ extern "C" int mps_adjoint_forces(mps_system *sys, const double *m, const double
     // Grids the double-float FFTs support take the double-float pipeline (float64 issue is slow on GB300) and
     // convert phi to float64 in place; the others use the float64 stages.
     if (!rc && df_usable(sys)) {
-        bool tiles_used = false;
-        rc = df_field_grids(sys, m, 1, nullptr, st, &tiles_used);
+        rc = df_field_grids(sys, m, 1, nullptr, st);
         if (!rc) rc = dfv_to_f64_inplace(sys->grid64, 3 * sys->gp.G, st);
     } else if (!rc) {
         rc = f64_field_grids(sys, m, 1, nullptr, st);

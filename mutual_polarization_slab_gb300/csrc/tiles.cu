@@ -19,6 +19,7 @@
 #include <algorithm>
 
 #include <atomic>
+#include <type_traits>
 #include <cstdlib>
 #include <cstring>
 #include "dfloat.cuh"
@@ -433,7 +434,7 @@ __global__ void __launch_bounds__(256) k_spread_tiled(const double *__restrict__
 }
 
 // ---------------------------------------------------------------------------
-// Float64 spread, node by node
+// Float64 and double-float spread, node by node
 // ---------------------------------------------------------------------------
 // A float64 warp instruction costs GB300 the same whether one lane is active or thirty-two, so the tiled spread above,
 // whose lanes sit idle wherever a particle misses their column (about 60 % of them at P = 10), loses on every one.
@@ -447,6 +448,10 @@ __global__ void __launch_bounds__(256) k_spread_tiled(const double *__restrict__
 // written once.  Measured against the tiled spread: three vectors, N = 100,000, 192^3, P = 10 3.82 -> 2.31 ms; one vector,
 // N = 20,000, 86^3, P = 8 277 -> 142 us; one vector, N = 500, 25^3 62 -> 12 us; 36 vectors, N = 2000, 31^3, P = 5 twelve
 // launches of 110 us -> one of 142 us.
+// In double-float a node's step is some 11 float instructions a component, and reading m wx of a lane's own particle
+// from shared memory costs as much; there a lane takes two nodes along z at once, with one list for both (11 of 10
+// planes) and one read.  Measured against the tiled double-float spread: one vector, N = 200,000, 240^3, P = 10
+// 1165 -> 646 us; one vector, N = 8228 in half of a 60 x 72 x 160 grid, P = 8 65 -> 28 us.
 constexpr int kNodeTile = 8;
 constexpr int kNodeChunk = 96;      // 3 mask words
 constexpr int kNodeWords = kNodeChunk / 32;
@@ -467,40 +472,43 @@ int node_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int n
     return bins_build(start, n, gp, kNodeTile, kNodeTile, node_tile_depth(gp, nrhs), tb, s);
 }
 
-template <int NR, int TZ>
+template <typename T, int NR, int TZ>
 struct NodeStage {
     static constexpr int C = 3 * NR;
-    double mwx[kNodeChunk][kNodeTile * C + 1];      // m_c wx at the tile's columns (odd stride: no bank conflicts)
-    double wyz[kNodeChunk][kNodeTile + TZ + 1];     // wy at its rows, wz at its planes
+    T mwx[kNodeChunk][kNodeTile * C + 1];           // m_c wx at the tile's columns (odd stride: no bank conflicts)
+    T wyz[kNodeChunk][kNodeTile + TZ + 1];          // wy at its rows, wz at its planes
     unsigned mask[kNodeWords][2 * kNodeTile + TZ];  // particles that reach a column, row, plane
 };
 
 constexpr int kNodeThreads = 256;
 
-template <int NR, int TZ>
+template <typename T, int NR, int TZ>
 __global__ void __launch_bounds__(kNodeThreads) k_spread_nodes(const double *__restrict__ m, int64_t n, int rfirst,
                                                           const int32_t *__restrict__ start,
-                                                          const double *__restrict__ w, GridParams gp,
+                                                          const T *__restrict__ w, GridParams gp,
                                                           const int64_t *__restrict__ tstart,
                                                           const int32_t *__restrict__ entries, int ntx, int nty,
-                                                          double *__restrict__ grid) {
+                                                          T *__restrict__ grid) {
     constexpr int C = 3 * NR, NQ = TZ / 4;
+    constexpr bool PAIR = std::is_same<T, dfv>::value && NQ == 2;   // a lane's two nodes share a list
     extern __shared__ __align__(16) unsigned char smem_nodes[];
-    NodeStage<NR, TZ> &st = *reinterpret_cast<NodeStage<NR, TZ> *>(smem_nodes);
+    NodeStage<T, NR, TZ> &st = *reinterpret_cast<NodeStage<T, NR, TZ> *>(smem_nodes);
     const int r0 = rfirst + NR * (int)blockIdx.y;
     const int64_t t = blockIdx.x;
     const int X0 = (int)(t % ntx) * kNodeTile, Y0 = (int)((t / ntx) % nty) * kNodeTile,
               Z0 = (int)(t / ((int64_t)ntx * nty)) * TZ;
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int P = gp.P, Nx = gp.N[0], Ny = gp.N[1], Nz = gp.N[2];
-    // warp: patch of 4 x 4 columns and 2 planes, for its node q planes TZ / 2 (wid >> 2) + 2 q + {0, 1}
+    // warp: patch of 4 x 4 columns and 2 planes, for its node q planes TZ / 2 (wid >> 2) + 2 q + {0, 1}; with pairs,
+    // planes TZ / 2 (wid >> 2) + {0, 1} and {2, 3}
     const int x = 4 * (wid & 1) + (lane & 3), y = 4 * ((wid >> 1) & 1) + ((lane >> 2) & 3);
-    const int zb = TZ / 2 * (wid >> 2) + (lane >> 4);
-    double acc[NQ][C];
+    const int zb = TZ / 2 * (wid >> 2) + (PAIR ? 2 : 1) * (lane >> 4);
+    constexpr int ZQ = PAIR ? 1 : 2;                                // plane step between a lane's nodes
+    ProdAcc<T> acc[NQ][C];
 #pragma unroll
     for (int q = 0; q < NQ; ++q)
 #pragma unroll
-        for (int c = 0; c < C; ++c) acc[q][c] = 0.0;
+        for (int c = 0; c < C; ++c) acc[q][c].zero();
     const int64_t e0 = tstart[t], e1 = tstart[t + 1];
     for (int64_t cb = e0; cb < e1; cb += kNodeChunk) {
         const int cnt = (int)min((int64_t)kNodeChunk, e1 - cb);
@@ -513,13 +521,13 @@ __global__ void __launch_bounds__(kNodeThreads) k_spread_nodes(const double *__r
             const int32_t a = in ? entries[cb + pp] : 0;
             int j = in ? origin - start[3 * (int64_t)a + d] : 0;   // stencil index of the tile's first node
             if (j < 0) j += Nd;
-            const double *wa = w + ((int64_t)a * 3 + d) * P;
-            double v[kNodeTile], mv[C];
+            const T *wa = w + ((int64_t)a * 3 + d) * P;
+            T v[kNodeTile], mv[C];
             unsigned hits = 0u;
 #pragma unroll
             for (int k = 0; k < kNodeTile; ++k) {
                 const bool hit = in && k < len && j < P && origin + k < Nd;
-                v[k] = hit ? wa[j] : 0.0;
+                v[k] = hit ? wa[j] : (T)0;
                 hits |= hit ? 1u << k : 0u;
                 if (++j >= Nd) j = 0;
             }
@@ -527,7 +535,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_spread_nodes(const double *__r
 #pragma unroll
                 for (int r = 0; r < NR; ++r)
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) mv[3 * r + c] = in ? m[((int64_t)(r0 + r) * n + a) * 3 + c] : 0.0;
+                    for (int c = 0; c < 3; ++c) mv[3 * r + c] = in ? (T)m[((int64_t)(r0 + r) * n + a) * 3 + c] : (T)0;
             }
 #pragma unroll
             for (int k = 0; k < kNodeTile; ++k) {
@@ -544,12 +552,15 @@ __global__ void __launch_bounds__(kNodeThreads) k_spread_nodes(const double *__r
         }
         __syncthreads();
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
+        for (int q = 0; q < (PAIR ? 1 : NQ); ++q) {
             const int z = zb + 2 * q;
             unsigned b[kNodeWords];
 #pragma unroll
-            for (int k = 0; k < kNodeWords; ++k)
-                b[k] = st.mask[k][x] & st.mask[k][kNodeTile + y] & st.mask[k][2 * kNodeTile + z];
+            for (int k = 0; k < kNodeWords; ++k) {
+                unsigned mz = st.mask[k][2 * kNodeTile + z];
+                if (PAIR) mz |= st.mask[k][2 * kNodeTile + z + 1];
+                b[k] = st.mask[k][x] & st.mask[k][kNodeTile + y] & mz;
+            }
             while (true) {
                 // the next particle of this lane's list
                 int p;
@@ -565,10 +576,21 @@ __global__ void __launch_bounds__(kNodeThreads) k_spread_nodes(const double *__r
                 } else {
                     break;
                 }
-                const double wv = st.wyz[p][y] * st.wyz[p][kNodeTile + z];
-                const double *mw = &st.mwx[p][x * C];
+                const T wy = st.wyz[p][y];
+                const T *mw = &st.mwx[p][x * C];
+                const T wv = wy * st.wyz[p][kNodeTile + z];
+                if (PAIR) {
+                    const T wv1 = wy * st.wyz[p][kNodeTile + z + 1];
 #pragma unroll
-                for (int c = 0; c < C; ++c) acc[q][c] += wv * mw[c];
+                    for (int c = 0; c < C; ++c) {
+                        const T v = mw[c];
+                        acc[0][c].add(wv, v);
+                        acc[NQ - 1][c].add(wv1, v);
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < C; ++c) acc[q][c].add(wv, mw[c]);
+                }
             }
         }
         __syncthreads();
@@ -576,47 +598,53 @@ __global__ void __launch_bounds__(kNodeThreads) k_spread_nodes(const double *__r
     if (X0 + x < Nx && Y0 + y < Ny) {
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
-            const int gz = Z0 + zb + 2 * q;
+            const int gz = Z0 + zb + ZQ * q;
             if (gz < Nz) {
-                double *g = grid + (int64_t)3 * r0 * gp.G + ((int64_t)gz * Ny + Y0 + y) * Nx + X0 + x;
+                T *g = grid + (int64_t)3 * r0 * gp.G + ((int64_t)gz * Ny + Y0 + y) * Nx + X0 + x;
 #pragma unroll
-                for (int c = 0; c < C; ++c) g[c * gp.G] = acc[q][c];
+                for (int c = 0; c < C; ++c) g[c * gp.G] = acc[q][c].get();
             }
         }
     }
 }
 
-template <int NR, int TZ>
-static int nodes_launch(const double *m, int64_t n, int r0, int groups, const int32_t *start, const double *w,
-                        const GridParams &gp, const TileBins &tb, double *grid, cudaStream_t s) {
-    const size_t smem = sizeof(NodeStage<NR, TZ>);
+template <typename T, int NR, int TZ>
+static int nodes_launch(const double *m, int64_t n, int r0, int groups, const int32_t *start, const T *w,
+                        const GridParams &gp, const TileBins &tb, T *grid, cudaStream_t s) {
+    const size_t smem = sizeof(NodeStage<T, NR, TZ>);
     if (smem > 48 * 1024)
-        MPS_CUDA_TRY(cudaFuncSetAttribute(k_spread_nodes<NR, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        MPS_CUDA_TRY(cudaFuncSetAttribute(k_spread_nodes<T, NR, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
-    k_spread_nodes<NR, TZ><<<dim3((unsigned)tb.ntiles, groups), kNodeThreads, smem, s>>>(
+    k_spread_nodes<T, NR, TZ><<<dim3((unsigned)tb.ntiles, groups), kNodeThreads, smem, s>>>(
         m, n, r0, start, w, gp, tb.tile_start, tb.entries, tb.ntx, tb.nty, grid);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
 }
 
 // Three vectors to a block; all their groups in one launch (small grids have too few tiles to fill the GPU).
-template <int TZ>
-static int nodes_dispatch(const double *m, int64_t n, int nrhs, const int32_t *start, const double *w,
-                          const GridParams &gp, const TileBins &tb, double *grid, cudaStream_t s) {
+template <typename T, int TZ>
+static int nodes_dispatch(const double *m, int64_t n, int nrhs, const int32_t *start, const T *w,
+                          const GridParams &gp, const TileBins &tb, T *grid, cudaStream_t s) {
     const int full = nrhs / 3, rest = nrhs - 3 * full;
-    int rc = full ? nodes_launch<3, TZ>(m, n, 0, full, start, w, gp, tb, grid, s) : MPS_OK;
-    if (!rc && rest == 2) rc = nodes_launch<2, TZ>(m, n, 3 * full, 1, start, w, gp, tb, grid, s);
-    if (!rc && rest == 1) rc = nodes_launch<1, TZ>(m, n, 3 * full, 1, start, w, gp, tb, grid, s);
+    int rc = full ? nodes_launch<T, 3, TZ>(m, n, 0, full, start, w, gp, tb, grid, s) : MPS_OK;
+    if (!rc && rest == 2) rc = nodes_launch<T, 2, TZ>(m, n, 3 * full, 1, start, w, gp, tb, grid, s);
+    if (!rc && rest == 1) rc = nodes_launch<T, 1, TZ>(m, n, 3 * full, 1, start, w, gp, tb, grid, s);
     return rc;
 }
 
-int spread_nodes(const double *m, int64_t n, int nrhs, const int32_t *start, const double *w, const GridParams &gp,
-                 const TileBins &tb, double *grid, cudaStream_t s) {
+template <typename T>
+int spread_nodes(const double *m, int64_t n, int nrhs, const int32_t *start, const T *w, const GridParams &gp,
+                 const TileBins &tb, T *grid, cudaStream_t s) {
     if (tb.tx != kNodeTile || tb.ty != kNodeTile) return MPS_BAD_ARG;
-    if (tb.tz == 8) return nodes_dispatch<8>(m, n, nrhs, start, w, gp, tb, grid, s);
-    if (tb.tz == 4) return nodes_dispatch<4>(m, n, nrhs, start, w, gp, tb, grid, s);
+    if (tb.tz == 8) return nodes_dispatch<T, 8>(m, n, nrhs, start, w, gp, tb, grid, s);
+    if (tb.tz == 4) return nodes_dispatch<T, 4>(m, n, nrhs, start, w, gp, tb, grid, s);
     return MPS_BAD_ARG;
 }
+
+template int spread_nodes<double>(const double *, int64_t, int, const int32_t *, const double *, const GridParams &,
+                                  const TileBins &, double *, cudaStream_t);
+template int spread_nodes<dfv>(const double *, int64_t, int, const int32_t *, const dfv *, const GridParams &,
+                               const TileBins &, dfv *, cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // Contract
@@ -757,15 +785,6 @@ int spread_tiled(const double *m, int64_t n, int nrhs, const int32_t *start, con
                  const TileBins &tb, T *grid, cudaStream_t s) {
     if (tb.tz == 8) return spread_dispatch<T, 8, T, T>(m, n, nrhs, start, w, gp, tb, grid, s);
     if (tb.tz == 4) return spread_dispatch<T, 4, T, T>(m, n, nrhs, start, w, gp, tb, grid, s);
-    return MPS_BAD_ARG;
-}
-
-int spread_tiled_df(const double *m, int64_t n, int nrhs, const int32_t *start, const dfv *w, const GridParams &gp,
-                    const TileBins &tb, dfv *grid, cudaStream_t s) {
-    // three vectors per launch: one vector per launch (a third of the registers) measured slower, the
-    // per-particle staging and w products then being repeated for every vector
-    if (tb.tz == 8) return spread_dispatch<dfv, 8, dfv, dfv>(m, n, nrhs, start, w, gp, tb, grid, s);
-    if (tb.tz == 4) return spread_dispatch<dfv, 4, dfv, dfv>(m, n, nrhs, start, w, gp, tb, grid, s);
     return MPS_BAD_ARG;
 }
 

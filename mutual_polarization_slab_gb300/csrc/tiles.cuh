@@ -52,20 +52,17 @@ template <typename T>
 int spread_tiled(const double *m, int64_t n, int nrhs, const int32_t *start, const T *w, const GridParams &gp,
                  const TileBins &tb, T *grid, cudaStream_t s);
 
-// The float64 spread (same result, node by node from the particles that cover it); tb from node_bins_build.
-int spread_nodes(const double *m, int64_t n, int nrhs, const int32_t *start, const double *w, const GridParams &gp,
-                 const TileBins &tb, double *grid, cudaStream_t s);
+// The same in float64 (T = double) or with double-float accumulation on double-float weights (T = dfv, the grids stored
+// as (hi, lo) float pairs), node by node from the particles that cover it; tb from node_bins_build.
+template <typename T>
+int spread_nodes(const double *m, int64_t n, int nrhs, const int32_t *start, const T *w, const GridParams &gp,
+                 const TileBins &tb, T *grid, cudaStream_t s);
 
 // out[r][a][c] = hprod * sum over the stencil (overwrites); partial: nentries * 3 * min(nrhs,3) of T.
 template <typename T>
 int contract_tiled(const T *grid, int64_t n, int nrhs, const int32_t *start, const T *w, const GridParams &gp,
                    const TileBins &tb, T *partial, double *out, cudaStream_t s);
 
-// The same kernels with double-float accumulation (float-pair arithmetic) on
-// double-float weights, the grids stored as (hi, lo) float pairs: the float64-accurate
-// matvec without float64 issue (no conversion to or from float64 between stages).
-int spread_tiled_df(const double *m, int64_t n, int nrhs, const int32_t *start, const dfv *w, const GridParams &gp,
-                    const TileBins &tb, dfv *grid, cudaStream_t s);
 // Warp-per-particle contraction of double-float grids (particles in `order`, null =
 // input order); out[r][a][c] = hprod * sum (overwrites).  w: double-float weights.
 int contract_df_warp(const dfv *grid, int64_t n, int nrhs, const int32_t *order, const int32_t *start, const dfv *w,

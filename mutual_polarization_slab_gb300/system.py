@@ -320,11 +320,11 @@ class SpectralEwaldSystem:
         return out
 
     def tuning(self):
-        """Autotuned tile depth per precision and the timings it was chosen from (ms)."""
+        """Tile per precision and, where its depth was timed, the timings it was chosen from (ms; -1 untimed)."""
         tz = (C.c_int32 * 2)()
         ms = (C.c_float * 4)()
         L.check(self._lib.mps_system_tuning(self._h, tz, ms))
-        return {"fp64": {"tile": [16, 16, int(tz[0])], "ms_depth4": ms[0], "ms_depth8": ms[1]},
+        return {"fp64": {"tile": [8, 8, int(tz[0])], "ms_depth4": ms[0], "ms_depth8": ms[1]},
                 "fp32": {"tile": [16, 16, int(tz[1])], "ms_depth4": ms[2], "ms_depth8": ms[3]}}
 
     def graphs(self):
