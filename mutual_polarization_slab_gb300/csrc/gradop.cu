@@ -75,6 +75,10 @@ __global__ void k_grad_scale_coef(GridParams gp, const double *__restrict__ H, f
 // could not skip) skips a particle with one uniform test and otherwise runs a branch-free
 // update: value(x,y,z) = (mx gx wy + my wx gy) wz + mz wx wy gz, over the groups
 // of 4 tile planes the particle reaches (a plane mask staged with the factors).
+// Staging: a lane aligns one particle's factors to half of one axis and keeps the mask of the positions covered (no
+// divisions, no shared-memory atomics); the warps then walk only the particles that reach their patch, from ballots.
+// Alone, at depth 12: 0.288 -> 0.217 ms a launch for three vectors of N = 1e5 on 144^3, 0.387 -> 0.241 for one of
+// N = 2e5 on 192^3.
 // particles staged per barrier interval: 96 measured 0.300 ms per launch at the bench workload against 0.323
 // for 32 (fewer barriers, and the warps' uneven shares of a chunk even out), 0.306 for 64 and 0.301 for 128
 constexpr int kGChunk = 96;
@@ -89,13 +93,11 @@ __global__ void __launch_bounds__(256, TZ > 12 ? 3 : (TZ > 8 ? 4 : 5)) k_spread_
                                                            GridParams gp, const int64_t *__restrict__ tstart,
                                                            const int32_t *__restrict__ entries, int ntx, int nty,
                                                            float *__restrict__ grid) {
-    constexpr int kPos = kTileX + kTileY + TZ;   // aligned positions per particle
+    constexpr int kPos = kTileX + kTileY + TZ + 1 - TZ % 2;   // aligned positions per particle (odd: no bank conflicts)
     constexpr int kMS = (3 * NR + 3) & ~3;       // moments, padded to a float4 multiple
     __shared__ float2 s_f[kGChunk][kPos];        // (w, dw/dr) at tile columns, rows, planes
     __shared__ __align__(16) float s_m[kGChunk][kMS];
-    __shared__ unsigned s_rows[kGChunk];
-    __shared__ unsigned s_cols[kGChunk];
-    __shared__ unsigned s_planes[kGChunk];
+    __shared__ unsigned s_mask[6][kGChunk];      // positions covered: halves of the columns, rows, planes
     const int64_t t = blockIdx.x;
     const int bx = (int)(t % ntx), by = (int)((t / ntx) % nty), bz = (int)(t / ((int64_t)ntx * nty));
     const int X0 = bx * kTileX, Y0 = by * kTileY, Z0 = bz * TZ;
@@ -113,7 +115,6 @@ __global__ void __launch_bounds__(256, TZ > 12 ? 3 : (TZ > 8 ? 4 : 5)) k_spread_
     const int64_t e0 = tstart[t], e1 = tstart[t + 1];
     for (int64_t cb = e0; cb < e1; cb += kGChunk) {
         const int cnt = (int)min((int64_t)kGChunk, e1 - cb);
-        if (threadIdx.x < kGChunk) s_rows[threadIdx.x] = s_cols[threadIdx.x] = s_planes[threadIdx.x] = 0u;
         if (threadIdx.x < cnt) {
             const int32_t a = entries[cb + threadIdx.x];
 #pragma unroll
@@ -124,47 +125,57 @@ __global__ void __launch_bounds__(256, TZ > 12 ? 3 : (TZ > 8 ? 4 : 5)) k_spread_
                 s_m[threadIdx.x][3 * r + 2] = (float)ma[2];
             }
         }
-        __syncthreads();
-        for (int q = threadIdx.x; q < cnt * kPos; q += blockDim.x) {
-            const int pp = q / kPos, k = q - (q / kPos) * kPos;
-            const int32_t a = entries[cb + pp];
-            const int d = k < kTileX ? 0 : (k < kTileX + kTileY ? 1 : 2);
-            const int tpos = k - (d == 0 ? 0 : (d == 1 ? kTileX : kTileX + kTileY));
-            const int origin = d == 0 ? X0 : (d == 1 ? Y0 : Z0);
-            const int Nd = d == 0 ? Nx : (d == 1 ? Ny : Nz);
-            const int node = origin + tpos;
-            int j = node - start[3 * (int64_t)a + d];   // stencil index of this tile position
+        // a warp aligns the factors of 32 particles (one per lane) to half of one of the tile's axes, and each lane
+        // keeps the mask of the positions its particle covers
+        for (int task = wid; task < 6 * (kGChunk / 32); task += 8) {
+            const int pp = 32 * (task / 6) + lane, d = (task % 6) >> 1, half = task & 1;
+            if (pp >= cnt) continue;
+            const int len = d == 2 ? TZ : kTileX, k0 = half ? len / 2 : 0, k1 = half ? len : len / 2;
+            const int origin = d == 0 ? X0 : (d == 1 ? Y0 : Z0), Nd = d == 0 ? Nx : (d == 1 ? Ny : Nz);
+            const int64_t a = entries[cb + pp];
+            int j = origin + k0 - start[3 * a + d];   // stencil index of the first position, in [-N, 2 N)
             if (j < 0) j += Nd;
-            float2 f = make_float2(0.f, 0.f);
-            if (node < Nd && j < P) {
-                const int64_t o = (int64_t)a * 3 * P + d * P + j;
-                f = make_float2(w[o], g[o]);
-                atomicOr(d == 0 ? &s_cols[pp] : (d == 1 ? &s_rows[pp] : &s_planes[pp]), 1u << tpos);
+            if (j >= Nd) j -= Nd;
+            const float *wa = w + (a * 3 + d) * P, *ga = g + (a * 3 + d) * P;
+            const int base = d * kTileX;
+            unsigned mask = 0u;
+#pragma unroll 4
+            for (int k = k0; k < k1; ++k) {
+                const bool hit = j < P && origin + k < Nd;
+                s_f[pp][base + k] = hit ? make_float2(wa[j], ga[j]) : make_float2(0.f, 0.f);
+                mask |= hit ? 1u << k : 0u;
+                if (++j >= Nd) j = 0;
             }
-            s_f[pp][k] = f;
+            s_mask[2 * d + half][pp] = mask;
         }
         __syncthreads();
-        for (int pp = 0; pp < cnt; ++pp) {
-            // the particle misses this warp's patch: none of its 4 rows or none of its 8 columns is covered
-            if (((s_rows[pp] >> (4 * py)) & 0xFu) == 0u || ((s_cols[pp] >> (8 * px)) & 0xFFu) == 0u) continue;
-            const float2 fx = s_f[pp][tx], fy = s_f[pp][kTileX + ty];
-            const float gxwy = fx.y * fy.x, wxgy = fx.x * fy.y, wxwy = fx.x * fy.x;
-            float cA[NR], cB[NR];
+        for (int word = 0; word < cnt; word += 32) {
+            // the particles that reach this warp's patch: some of its 4 rows and some of its 8 columns are covered
+            bool reach = false;
+            if (word + lane < cnt)
+                reach = ((s_mask[px][word + lane] >> (8 * px)) & 0xFFu) != 0u &&
+                        ((s_mask[2 + (py >> 1)][word + lane] >> (4 * py)) & 0xFu) != 0u;
+            for (unsigned list = __ballot_sync(0xffffffffu, reach); list; list &= list - 1) {
+                const int pp = word + __ffs(list) - 1;
+                const float2 fx = s_f[pp][tx], fy = s_f[pp][kTileX + ty];
+                const float gxwy = fx.y * fy.x, wxgy = fx.x * fy.y, wxwy = fx.x * fy.x;
+                float cA[NR], cB[NR];
 #pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                cA[r] = s_m[pp][3 * r] * gxwy + s_m[pp][3 * r + 1] * wxgy;
-                cB[r] = s_m[pp][3 * r + 2] * wxwy;
-            }
-            // planes in groups of 4; a group the particle does not reach is skipped (uniform over the CTA)
-            const unsigned planes = s_planes[pp];
+                for (int r = 0; r < NR; ++r) {
+                    cA[r] = s_m[pp][3 * r] * gxwy + s_m[pp][3 * r + 1] * wxgy;
+                    cB[r] = s_m[pp][3 * r + 2] * wxwy;
+                }
+                // planes in groups of 4; a group the particle does not reach is skipped (uniform over the CTA)
+                const unsigned planes = s_mask[4][pp] | s_mask[5][pp];
 #pragma unroll
-            for (int z0 = 0; z0 < TZ; z0 += 4) {
-                if (TZ > 4 && ((planes >> z0) & 0xFu) == 0u) continue;
+                for (int z0 = 0; z0 < TZ; z0 += 4) {
+                    if (TZ > 4 && ((planes >> z0) & 0xFu) == 0u) continue;
 #pragma unroll
-                for (int z = z0; z < z0 + 4 && z < TZ; ++z) {
-                    const float2 fz = s_f[pp][kTileX + kTileY + z];
+                    for (int z = z0; z < z0 + 4 && z < TZ; ++z) {
+                        const float2 fz = s_f[pp][kTileX + kTileY + z];
 #pragma unroll
-                    for (int r = 0; r < NR; ++r) acc[z][r] += cA[r] * fz.x + cB[r] * fz.y;
+                        for (int r = 0; r < NR; ++r) acc[z][r] += cA[r] * fz.x + cB[r] * fz.y;
+                    }
                 }
             }
         }
@@ -391,76 +402,111 @@ __global__ void __launch_bounds__(256, 3) k_contract_grad_warp(const float *__re
 // is a template parameter, so the z runs unroll completely with the z factors in
 // registers and the shared-memory offsets are immediates.  A node is staged by about
 // (R / kHomeBlock)^3 blocks (9.6 at P = 10), all from L2.
+// With one vector a CTA takes 2 x 2 home blocks (5.2 stagings a node): 0.256 -> 0.156 ms for N = 2e5 on 192^3, with the
+// region staged row by row (the wraps worked out once a row, not once a node).
 // 67 KB of shared memory at P = 10 and 3 vectors, 3 blocks per SM (80 registers): the mixed step at the bench
 // workload took 19.25 ms against 20.08 with the warp gather; float4 nodes (the 3 vectors interleaved, 87 KB,
 // 2 blocks per SM) took 20.17.
 constexpr int kHomeChunk = 32;
 
-template <int NR, int P>
-constexpr size_t home_smem_bytes() {
-    constexpr int R = kHomeBlock + P - 1;
-    return sizeof(float) * (size_t)NR * R * R * R + sizeof(float) * 2 * kHomeChunk * 3 * P +
-           sizeof(int) * 4 * kHomeChunk;
-}
+// A CTA covers BX x BY home blocks: the margin of P - 1 nodes is staged once for all of them.
+template <int NR, int P, int BX, int BY>
+struct HomeTile {
+    static constexpr int RX = BX * kHomeBlock + P - 1, RY = BY * kHomeBlock + P - 1, RZ = kHomeBlock + P - 1;
+    static constexpr int VOL = RX * RY * RZ;
+    static constexpr size_t smem =
+        sizeof(float) * ((size_t)NR * VOL + 2 * kHomeChunk * 3 * P) + sizeof(int) * 4 * kHomeChunk;
+};
 
-template <int NR, int P>
-__global__ void __launch_bounds__(256, 3) k_contract_grad_home(const float *__restrict__ grid, int64_t n, int r0,
-                                                               const int64_t *__restrict__ hstart,
-                                                               const int32_t *__restrict__ hentries, int nbx, int nby,
-                                                               const int32_t *__restrict__ start,
-                                                               const float *__restrict__ w, const float *__restrict__ g,
-                                                               GridParams gp, double *__restrict__ out) {
-    constexpr int R = kHomeBlock + P - 1;
-    constexpr int RR = R * R;
-    constexpr int VOL = RR * R;
+template <int NR, int P, int BX, int BY>
+__global__ void __launch_bounds__(256, NR == 1 ? 4 : 3) k_contract_grad_home(
+    const float *__restrict__ grid, int64_t n, int r0, const int64_t *__restrict__ hstart,
+    const int32_t *__restrict__ hentries, int nbx, int nby, const int32_t *__restrict__ start,
+    const float *__restrict__ w, const float *__restrict__ g, GridParams gp, double *__restrict__ out) {
+    using HT = HomeTile<NR, P, BX, BY>;
+    constexpr int RX = HT::RX, RY = HT::RY, RZ = HT::RZ, VOL = HT::VOL, RR = RX * RY;
     constexpr int F = 3 * P;                        // per-axis factors of one particle
+    constexpr int NB = BX * BY;
     extern __shared__ float s_reg[];                // [NR][VOL] nodes, x fastest
     float *s_w = s_reg + NR * VOL;                  // [kHomeChunk][F]
     float *s_g = s_w + kHomeChunk * F;              // [kHomeChunk][F]
     int *s_p = (int *)(s_g + kHomeChunk * F);       // [kHomeChunk][4]: offsets in the block, particle id
+    const int tbx = (nbx + BX - 1) / BX, tby = (nby + BY - 1) / BY;
     const int64_t b = blockIdx.x;
-    const int64_t e0 = hstart[b], e1 = hstart[b + 1];
-    if (e0 == e1) return;   // the whole CTA leaves: no barrier is left waiting
+    const int bx0 = (int)(b % tbx) * BX, by0 = (int)((b / tbx) % tby) * BY, bz = (int)(b / ((int64_t)tbx * tby));
+    // the home blocks' particle lists, one after the other
+    int64_t first[NB];
+    int upto[NB], total = 0;
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+        const int bx = bx0 + k % BX, by = by0 + k / BX;
+        first[k] = 0;
+        if (bx < nbx && by < nby) {
+            const int64_t hb = ((int64_t)bz * nby + by) * nbx + bx;
+            first[k] = hstart[hb] - total;
+            total += (int)(hstart[hb + 1] - hstart[hb]);
+        }
+        upto[k] = total;
+    }
+    if (total == 0) return;   // the whole CTA leaves: no barrier is left waiting
+    auto entry = [&](int q) {
+        int64_t e = first[0];
+#pragma unroll
+        for (int k = 1; k < NB; ++k) e = q >= upto[k - 1] ? first[k] : e;
+        return (int64_t)hentries[e + q];
+    };
     const int Nx = gp.N[0], Ny = gp.N[1], Nz = gp.N[2];
     const int64_t G = gp.G;
-    const int X0 = (int)(b % nbx) * kHomeBlock, Y0 = (int)((b / nbx) % nby) * kHomeBlock,
-              Z0 = (int)(b / ((int64_t)nbx * nby)) * kHomeBlock;
+    const int X0 = bx0 * kHomeBlock, Y0 = by0 * kHomeBlock, Z0 = bz * kHomeBlock;
     const float *g0 = grid + (int64_t)r0 * G;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    // origin + offset < 3 N (the host requires it): at most two wraps
+    auto wrap2 = [](int i, int N) {
+        i -= i >= N ? N : 0;
+        return i - (i >= N ? N : 0);
+    };
+    // rows of the region: LX lanes a row (a 17th column goes by itself), the x wrap worked out once
+    constexpr int LX = RX <= 17 ? 16 : 32, ROWS = 32 / LX;
+    static_assert(RX <= LX + 1, "one column at most is left over");
+    {
+        const int x = lane % LX, gx = wrap2(X0 + x, Nx);
+        if (x < RX) {
 #pragma unroll 4
-    for (int q = threadIdx.x; q < VOL; q += blockDim.x) {
-        const int row = q / R, x = q - row * R;
-        const int z = row / R, y = row - z * R;
-        // origin + offset < 3 N (the host requires N >= kHomeBlock and N >= P): at most two wraps
-        int gx = X0 + x, gy = Y0 + y, gz = Z0 + z;
-        gx -= gx >= Nx ? Nx : 0;
-        gx -= gx >= Nx ? Nx : 0;
-        gy -= gy >= Ny ? Ny : 0;
-        gy -= gy >= Ny ? Ny : 0;
-        gz -= gz >= Nz ? Nz : 0;
-        gz -= gz >= Nz ? Nz : 0;
-        const int64_t node = ((int64_t)gz * Ny + gy) * Nx + gx;
+            for (int row = wid * ROWS + lane / LX; row < RY * RZ; row += 8 * ROWS) {
+                const int z = row / RY, y = row - z * RY;
+                const float *src = g0 + ((int64_t)wrap2(Z0 + z, Nz) * Ny + wrap2(Y0 + y, Ny)) * Nx + gx;
 #pragma unroll
-        for (int r = 0; r < NR; ++r) s_reg[r * VOL + q] = __ldg(g0 + r * G + node);
+                for (int r = 0; r < NR; ++r) s_reg[r * VOL + row * RX + x] = __ldg(src + r * G);
+            }
+        }
+        if (RX > LX) {
+            const int gl = wrap2(X0 + LX, Nx);
+            for (int row = threadIdx.x; row < RY * RZ; row += 256) {
+                const int z = row / RY, y = row - z * RY;
+                const float *src = g0 + ((int64_t)wrap2(Z0 + z, Nz) * Ny + wrap2(Y0 + y, Ny)) * Nx + gl;
+#pragma unroll
+                for (int r = 0; r < NR; ++r) s_reg[r * VOL + row * RX + LX] = __ldg(src + r * G);
+            }
+        }
     }
-    const int lane = threadIdx.x & 31;
-    for (int64_t c0 = e0; c0 < e1; c0 += kHomeChunk) {
-        const int cnt = (int)min((int64_t)kHomeChunk, e1 - c0);
-        for (int q = threadIdx.x; q < cnt * F; q += blockDim.x) {
+    for (int c0 = 0; c0 < total; c0 += kHomeChunk) {
+        const int cnt = min(kHomeChunk, total - c0);
+        for (int q = threadIdx.x; q < cnt * F; q += 256) {
             const int p = q / F, k = q - p * F;
-            const int64_t a = hentries[c0 + p];
+            const int64_t a = entry(c0 + p);
             s_w[q] = w[a * F + k];
             s_g[q] = g[a * F + k];
         }
         if (threadIdx.x < cnt) {
-            const int64_t a = hentries[c0 + threadIdx.x];
-            // the home block holds the stencil's first node: offsets in [0, kHomeBlock)
+            const int64_t a = entry(c0 + threadIdx.x);
+            // a home block holds the stencil's first node: offsets in [0, BX kHomeBlock) and so on
             s_p[4 * threadIdx.x + 0] = start[3 * a] - X0;
             s_p[4 * threadIdx.x + 1] = start[3 * a + 1] - Y0;
             s_p[4 * threadIdx.x + 2] = start[3 * a + 2] - Z0;
             s_p[4 * threadIdx.x + 3] = (int)a;
         }
         __syncthreads();   // the region (first pass) and this chunk's particle data are in place
-        for (int pp = threadIdx.x >> 5; pp < cnt; pp += blockDim.x >> 5) {
+        for (int pp = wid; pp < cnt; pp += 8) {
             const int ox = s_p[4 * pp], oy = s_p[4 * pp + 1], oz = s_p[4 * pp + 2];
             const int64_t a = s_p[4 * pp + 3];
             const float *wa = s_w + pp * F, *ga = s_g + pp * F;
@@ -478,7 +524,7 @@ __global__ void __launch_bounds__(256, 3) k_contract_grad_home(const float *__re
                 int idx, sub, lpp;   // lpp is a constant of each unrolled round
                 if (!stencil_row(row0, P, lane, &idx, &sub, &lpp)) continue;
                 const int jx = idx % P, jy = idx / P;
-                const float *col = s_reg + (oz * R + oy + jy) * R + ox + jx;
+                const float *col = s_reg + (oz * RY + oy + jy) * RX + ox + jx;
                 float s0[NR], s1[NR];
 #pragma unroll
                 for (int r = 0; r < NR; ++r) s0[r] = s1[r] = 0.f;
@@ -531,27 +577,33 @@ bool contract_grad_home_supported(const GridParams &gp) {
     return true;
 }
 
-template <int NR, int P>
+template <int NR, int P, int BX, int BY>
 static int home_launch(const float *grid, int64_t n, int r0, const int32_t *start, const float *w, const float *g,
                        const GridParams &gp, const TileBins &tb, double *out, cudaStream_t s) {
-    constexpr size_t smem = home_smem_bytes<NR, P>();
+    constexpr size_t smem = HomeTile<NR, P, BX, BY>::smem;
     if (smem > 48 * 1024)
-        MPS_CUDA_TRY(cudaFuncSetAttribute(k_contract_grad_home<NR, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
-    k_contract_grad_home<NR, P><<<(unsigned)tb.nhome, 256, smem, s>>>(grid, n, r0, tb.hstart, tb.hentries, tb.nhb[0],
-                                                                       tb.nhb[1], start, w, g, gp, out);
+        MPS_CUDA_TRY(cudaFuncSetAttribute(k_contract_grad_home<NR, P, BX, BY>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const unsigned blocks = (unsigned)((tb.nhb[0] + BX - 1) / BX) * (unsigned)((tb.nhb[1] + BY - 1) / BY) *
+                            (unsigned)tb.nhb[2];
+    k_contract_grad_home<NR, P, BX, BY><<<blocks, 256, smem, s>>>(grid, n, r0, tb.hstart, tb.hentries, tb.nhb[0],
+                                                                  tb.nhb[1], start, w, g, gp, out);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
 }
 
+// One vector leaves room for four home blocks to a CTA: taken where every SM still gets four CTAs and the wider region
+// wraps at most twice.
 template <int P>
 static int home_dispatch(const float *grid, int64_t n, int nrhs, const int32_t *start, const float *w, const float *g,
                          const GridParams &gp, const TileBins &tb, double *out, cudaStream_t s) {
+    const bool wide = tb.nhome >= 4 * 4 * 152 && gp.N[0] >= 16 && gp.N[1] >= 16;
     for (int r0 = 0; r0 < nrhs; r0 += 3) {
         const int nr = min(3, nrhs - r0);
-        const int rc = nr == 3   ? home_launch<3, P>(grid, n, r0, start, w, g, gp, tb, out, s)
-                       : nr == 2 ? home_launch<2, P>(grid, n, r0, start, w, g, gp, tb, out, s)
-                                 : home_launch<1, P>(grid, n, r0, start, w, g, gp, tb, out, s);
+        const int rc = nr == 3   ? home_launch<3, P, 1, 1>(grid, n, r0, start, w, g, gp, tb, out, s)
+                       : nr == 2 ? home_launch<2, P, 1, 1>(grid, n, r0, start, w, g, gp, tb, out, s)
+                       : wide    ? home_launch<1, P, 2, 2>(grid, n, r0, start, w, g, gp, tb, out, s)
+                                 : home_launch<1, P, 1, 1>(grid, n, r0, start, w, g, gp, tb, out, s);
         if (rc) return rc;
     }
     return MPS_OK;
