@@ -4,6 +4,8 @@
 
 #include "realspace.cuh"
 
+#include <algorithm>
+
 namespace mps {
 
 // ---------------------------------------------------------------------------
@@ -297,9 +299,6 @@ int real_space_csr(const double *m, double *out, int64_t n, int nrhs, const int6
 
 template int real_space_csr<double>(const double *, double *, int64_t, int, const int64_t *, PairData<double>,
                                     const double *, const int32_t *, const double *, bool, cudaStream_t);
-template int real_space_csr<float>(const double *, double *, int64_t, int, const int64_t *, PairData<float>,
-                                   const double *, const int32_t *, const double *, bool, cudaStream_t);
-
 __global__ void k_to_dfv(const double *__restrict__ m, int64_t total, dfv *__restrict__ md) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
         md[i] = dfv(m[i]);
@@ -310,6 +309,14 @@ int real_space_csr_df(const double *m, dfv *mdf, double *out, int64_t n, int nrh
                       bool accumulate, const int32_t *order, cudaStream_t s) {
     k_to_dfv<<<grid_for((int64_t)nrhs * n * 3, 256), 256, 0, s>>>(m, (int64_t)nrhs * n * 3, mdf);
     MPS_LAUNCH_CHECK();
+    if (n * 8 < 152 * 2 * 256) {   // a warp per row and vector, as in float64
+        for (int r0 = 0; r0 < nrhs; r0 += 32768) {
+            k_rs_csr<dfv, 32, 1, dfv><<<dim3(grid_for(n * 32, 128, 152 * 64), min(32768, nrhs - r0)), 128, 0, s>>>(
+                m, out, n, nrhs, r0, row_ptr, pd, diag, diag_of_rhs, slab, accumulate, mdf, order);
+            MPS_LAUNCH_CHECK();
+        }
+        return MPS_OK;
+    }
     constexpr int G = 8;
     const unsigned grid = grid_for(n * G, 256, 152 * 64);
     for (int r0 = 0; r0 < nrhs; r0 += 3) {
@@ -328,150 +335,114 @@ int real_space_csr_df(const double *m, dfv *mdf, double *out, int64_t n, int nrh
     return MPS_OK;
 }
 
-// Float copy of the moments with each particle's nrhs x 3 components side by side (stride S floats, a multiple of
-// 4): the pair loop gathers a neighbour's block of vectors with 16-byte loads from one place instead of one
-// 4-byte load per vector and component from nrhs planes.
-__global__ void k_to_f32_rows(const double *__restrict__ m, int64_t n, int nrhs, int S, float *__restrict__ mf) {
-    const int64_t total = (int64_t)nrhs * n * 3;
+// Float copy of the moments, each particle's nrhs vectors side by side as float4 (x, y, z, 0): a pair's gather is one
+// 16-byte load a vector, from one place.  Converted once per matvec, not once per pair: float64 -> float32 conversions
+// run on GB300's narrow float64 pipe.
+__global__ void k_to_f32_rows(const double *__restrict__ m, int64_t n, int nrhs, float4 *__restrict__ mf) {
+    const int64_t total = (int64_t)nrhs * n;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = t / (n * 3), rem = t - r * n * 3;
-        const int64_t a = rem / 3;
-        const int c = (int)(rem - a * 3);
-        mf[a * S + r * 3 + c] = (float)m[t];
+        const int64_t a = t / nrhs, r = t - a * nrhs;
+        const double *v = m + (r * n + a) * 3;
+        mf[t] = make_float4((float)v[0], (float)v[1], (float)v[2], 0.f);
     }
 }
 
-size_t m32_floats(int64_t n, int nrhs) { return (size_t)n * (size_t)((3 * nrhs + 3) & ~3); }
+size_t m32_floats(int64_t n, int nrhs) { return (size_t)n * (size_t)nrhs * 4; }
 
-// The float32 pair sum of k_rs_csr (same sums, same order) on the row copy of k_to_f32_rows: a neighbour's R
-// vectors are ceil(3R / 4) float4 loads at a 16-byte aligned offset (r0 is a multiple of 4 and S of 4, so
-// 3 r0 + 4 ceil(3R / 4) <= S: a read past the block's last component stays inside the particle's row).
-template <int G, int R>
+// Float32 pair sum.  A warp takes a row and a lane one vector of one pair: RL vectors side by side, 32 / RL pairs at a
+// time.  The loads are what costs here (a warp's load takes the L1 a pass for every line it touches): 4 lanes to a row
+// and all vectors in a lane's registers touched 8 lines with each pair array and 32 with each 16 bytes of the gathered
+// moments; now a pair array's load touches one or two, and a gather one line a pair.  The row's sums end in float64 with
+// the diagonal, each component on a lane of its own.
+// Alone: one vector, N = 200,000, 60 neighbours 264 -> 122 us; 48 vectors, N = 3000 55 -> 25 us; three vectors, N = 100,000
+// 104 -> 115 us (a quarter of the lanes idle), but less in the way of the spread that runs beside it.
+template <int RL>
 __global__ void __launch_bounds__(256) k_rs_csr_f32(const double *__restrict__ m, double *__restrict__ out, int64_t n,
-                                                    int nrhs, int r0, const int64_t *__restrict__ row_ptr,
+                                                    int nrhs, int rfirst, const int64_t *__restrict__ row_ptr,
                                                     PairData<float> pd, const double *__restrict__ diag,
                                                     const int32_t *__restrict__ diag_of_rhs,
                                                     const double *__restrict__ slab, int accumulate,
-                                                    const float *__restrict__ mf, int S,
-                                                    const int32_t *__restrict__ order) {
-    constexpr int NQ = (3 * R + 3) / 4;   // float4 loads per neighbour
-    const int lane = threadIdx.x % G;
-    const int64_t grp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
-    const int64_t ngrp = ((int64_t)gridDim.x * blockDim.x) / G;
-    r0 += (int)blockIdx.y * R;
-    const int nr = min(R, nrhs - r0);
-    const float *mb0 = mf + 3 * r0;
-    for (int64_t i = grp; i < n; i += ngrp) {
+                                                    const float4 *__restrict__ mf, const int32_t *__restrict__ order) {
+    constexpr int PP = 32 / RL;   // pairs at a time
+    static_assert(PP >= 4, "three lanes of a vector take its components");
+    const int lane = threadIdx.x & 31, q = lane / RL;
+    const int r = rfirst + (int)blockIdx.y * RL + lane % RL;
+    const bool live = r < nrhs;
+    const int rc = live ? r : nrhs - 1;
+    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const double *dg = diag + (int64_t)(diag_of_rhs ? diag_of_rhs[rc] : 0) * n;
+    const double sl = q == 2 ? slab[rc] : 0.0;
+    for (int64_t i = warp; i < n; i += nw) {
+        // rows in `order` (cell order): neighbouring warps read overlapping neighbour moments
         const int64_t a = order ? (int64_t)order[i] : i;
-        float acc[R][3];
-#pragma unroll
-        for (int r = 0; r < R; ++r) acc[r][0] = acc[r][1] = acc[r][2] = 0.f;
-        const int64_t e0 = row_ptr[a], e1 = row_ptr[a + 1];
-#pragma unroll 2
-        for (int64_t e = e0 + lane; e < e1; e += G) {
+        float ax = 0.f, ay = 0.f, az = 0.f;
+        const int64_t e1 = row_ptr[a + 1];
+#pragma unroll 4
+        for (int64_t e = row_ptr[a] + q; e < e1; e += PP) {
             const int32_t b = pd.nbr[e];
             const float av = pd.A[e], ba = pd.BA[e];
             const float rx = pd.rx[e], ry = pd.ry[e], rz = pd.rz[e];
-            const float4 *q = reinterpret_cast<const float4 *>(mb0 + (int64_t)b * S);
-            float v[4 * NQ];
-#pragma unroll
-            for (int k = 0; k < NQ; ++k) {
-                const float4 t = __ldg(q + k);
-                v[4 * k] = t.x;
-                v[4 * k + 1] = t.y;
-                v[4 * k + 2] = t.z;
-                v[4 * k + 3] = t.w;
-            }
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                if (r < nr) {
-                    const float mx = v[3 * r], my = v[3 * r + 1], mz = v[3 * r + 2];
-                    const float s = ba * (mx * rx + my * ry + mz * rz);
-                    acc[r][0] += av * mx + s * rx;
-                    acc[r][1] += av * my + s * ry;
-                    acc[r][2] += av * mz + s * rz;
-                }
-            }
+            const float4 v = __ldg(mf + (int64_t)b * nrhs + rc);
+            const float s = ba * (v.x * rx + v.y * ry + v.z * rz);
+            ax += av * v.x + s * rx;
+            ay += av * v.y + s * ry;
+            az += av * v.z + s * rz;
         }
 #pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-#pragma unroll
-                for (int o = G / 2; o > 0; o >>= 1) acc[r][c] += __shfl_xor_sync(0xffffffffu, acc[r][c], o, G);
-        if (lane == 0) {
-            for (int r = 0; r < nr; ++r) {
-                const int rr = r0 + r;
-                const double dg = diag[(int64_t)(diag_of_rhs ? diag_of_rhs[rr] : 0) * n + a];
-                const double *ma = m + ((int64_t)rr * n + a) * 3;
-                double *o = out + ((int64_t)rr * n + a) * 3;
-                double v0 = dg * ma[0] + (double)acc[r][0];
-                double v1 = dg * ma[1] + (double)acc[r][1];
-                double v2 = dg * ma[2] + (double)acc[r][2] + slab[rr];
-                if (accumulate) {
-                    v0 += o[0];
-                    v1 += o[1];
-                    v2 += o[2];
-                }
-                o[0] = v0;
-                o[1] = v1;
-                o[2] = v2;
-            }
+        for (int o = RL; o < 32; o <<= 1) {
+            ax += __shfl_xor_sync(0xffffffffu, ax, o);
+            ay += __shfl_xor_sync(0xffffffffu, ay, o);
+            az += __shfl_xor_sync(0xffffffffu, az, o);
+        }
+        if (live && q < 3) {
+            const int64_t k = ((int64_t)r * n + a) * 3 + q;
+            double v = dg[a] * m[k] + float_to_double(q == 0 ? ax : (q == 1 ? ay : az)) + sl;
+            if (accumulate) v += out[k];
+            out[k] = v;
         }
     }
 }
 
-// Float32 pair sum on a float copy of the moments (converted once per matvec, not
-// once per pair: float64 -> float32 conversions run on GB300's narrow float64
-// pipe), rows in `order`, up to 8 right-hand sides per pass over the pair data.
-template <int G>
-static int rs_f32_launches(const double *m, float *m32, double *out, int64_t n, int nrhs, int S,
-                           const int64_t *row_ptr, PairData<float> pd, const double *diag, const int32_t *diag_of_rhs,
-                           const double *slab, bool accumulate, const int32_t *order, cudaStream_t s) {
-    const unsigned grid = grid_for(n * G, 256, 152 * 64);
-    // blocks of 8 vectors, then one of 4, then the last 3, 2 or 1: every block starts at a multiple of 4
-    for (int r0 = 0; r0 < nrhs;) {
-        const int nr = nrhs - r0;
-        if (nr >= 8) {
-            // every full block of 8 vectors in one launch (grid y): small systems fill the GPU with all of them
-            const int nb = nr / 8;
-            k_rs_csr_f32<G, 8><<<dim3(grid, nb), 256, 0, s>>>(m, out, n, nrhs, r0, row_ptr, pd, diag, diag_of_rhs,
-                                                              slab, accumulate, m32, S, order);
-            r0 += 8 * nb;
-        } else if (nr >= 4) {
-            k_rs_csr_f32<G, 4><<<grid, 256, 0, s>>>(m, out, n, nrhs, r0, row_ptr, pd, diag, diag_of_rhs, slab,
-                                                    accumulate, m32, S, order);
-            r0 += 4;
-        } else if (nr == 3) {
-            k_rs_csr_f32<G, 3><<<grid, 256, 0, s>>>(m, out, n, nrhs, r0, row_ptr, pd, diag, diag_of_rhs, slab,
-                                                    accumulate, m32, S, order);
-            r0 += 3;
-        } else if (nr == 2) {
-            k_rs_csr_f32<G, 2><<<grid, 256, 0, s>>>(m, out, n, nrhs, r0, row_ptr, pd, diag, diag_of_rhs, slab,
-                                                    accumulate, m32, S, order);
-            r0 += 2;
-        } else {
-            k_rs_csr_f32<G, 1><<<grid, 256, 0, s>>>(m, out, n, nrhs, r0, row_ptr, pd, diag, diag_of_rhs, slab,
-                                                    accumulate, m32, S, order);
-            r0 += 1;
-        }
-        MPS_LAUNCH_CHECK();
-    }
+template <int RL>
+static int rs_f32_launch(const double *m, const float4 *mf, double *out, int64_t n, int nrhs, int r0, int blocks,
+                         const int64_t *row_ptr, PairData<float> pd, const double *diag, const int32_t *diag_of_rhs,
+                         const double *slab, bool accumulate, const int32_t *order, cudaStream_t s) {
+    k_rs_csr_f32<RL><<<dim3(grid_for(n * 32, 256, 152 * 64), blocks), 256, 0, s>>>(
+        m, out, n, nrhs, r0, row_ptr, pd, diag, diag_of_rhs, slab, accumulate, mf, order);
+    MPS_LAUNCH_CHECK();
     return MPS_OK;
 }
 
-// Float32 pair sum on a float copy of the moments (converted once per matvec, not
-// once per pair: float64 -> float32 conversions run on GB300's narrow float64
-// pipe), rows in `order`, up to 8 right-hand sides per pass over the pair data.
+// Eight vectors side by side (all such blocks in one launch: small systems fill the GPU with them), a rest of up to four
+// as 4, 2 or 1, a larger one as a block of eight with idle lanes.
 int real_space_csr_f32(const double *m, float *m32, double *out, int64_t n, int nrhs, const int64_t *row_ptr,
                        PairData<float> pd, const double *diag, const int32_t *diag_of_rhs, const double *slab,
                        bool accumulate, const int32_t *order, cudaStream_t s) {
-    const int S = (3 * nrhs + 3) & ~3;
-    k_to_f32_rows<<<grid_for((int64_t)nrhs * n * 3, 256), 256, 0, s>>>(m, n, nrhs, S, m32);
+    float4 *mf = reinterpret_cast<float4 *>(m32);
+    k_to_f32_rows<<<grid_for((int64_t)nrhs * n, 256), 256, 0, s>>>(m, n, nrhs, mf);
     MPS_LAUNCH_CHECK();
-    // 4 lanes per particle: the polydisperse batch (48 vectors, configurations of 500..20,000 spheres) took 7.14 s
-    // against 7.27 s with 8 lanes, the headline step 18.74 against 18.75 ms; 16 lanes took 19.08 ms
-    return rs_f32_launches<4>(m, m32, out, n, nrhs, S, row_ptr, pd, diag, diag_of_rhs, slab, accumulate, order, s);
+    int r0 = 0;
+    while (r0 < nrhs) {
+        const int left = nrhs - r0;
+        int rc;
+        if (left > 4) {
+            const int blocks = std::min(32768, left / 8 + (left % 8 > 4 ? 1 : 0));
+            rc = rs_f32_launch<8>(m, mf, out, n, nrhs, r0, blocks, row_ptr, pd, diag, diag_of_rhs, slab, accumulate,
+                                  order, s);
+            r0 += 8 * blocks;
+        } else {
+            rc = left > 2    ? rs_f32_launch<4>(m, mf, out, n, nrhs, r0, 1, row_ptr, pd, diag, diag_of_rhs, slab,
+                                                accumulate, order, s)
+                 : left == 2 ? rs_f32_launch<2>(m, mf, out, n, nrhs, r0, 1, row_ptr, pd, diag, diag_of_rhs, slab,
+                                                accumulate, order, s)
+                             : rs_f32_launch<1>(m, mf, out, n, nrhs, r0, 1, row_ptr, pd, diag, diag_of_rhs, slab,
+                                                accumulate, order, s);
+            r0 = nrhs;
+        }
+        if (rc) return rc;
+    }
+    return MPS_OK;
 }
 
 // Diagonal (dielectric + self) per particle and permittivity set.
