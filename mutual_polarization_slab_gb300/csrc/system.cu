@@ -1275,11 +1275,21 @@ constexpr int kDotItems = 8;
 constexpr int kDotChunk = kDotThreads * kDotItems;
 constexpr int kMaxCols = 64;
 
+// Sum over a block's partials of one column, by a warp (all lanes return it): lane l takes blocks l, l + 32, ...
+__device__ __forceinline__ double partials_sum(const double *__restrict__ partial, int64_t r, int nblk, int c, int lane) {
+    double s = 0.0;
+    for (int b = lane; b < nblk; b += 32) s += __ldcg(partial + (r * nblk + b) * kMaxCols + c);
+    return warp_sum(s);
+}
+
 // partial[r][blk][c] = sum over the block's rows of V_r[c][i] * w_r[i]; the last
 // block of each system to finish (ticket counter, threadfence pattern) sums the
-// partials in block order and writes out[r][c]: one launch, fixed summation order.
+// partials in a fixed order and writes out[r][c]: one launch, fixed summation order.
 // With jd non-null the column count is ncols + *jd (the Arnoldi step held on the
-// device by a captured graph).
+// device by a captured graph).  The multiply-adds bound it (float64 rate), so four
+// columns share a warp's reduction (6 additions instead of 20), and the partials of
+// a column are summed by a warp: one thread's chain of a few hundred dependent
+// additions took longer than the rest of the kernel.
 __global__ void __launch_bounds__(kDotThreads) k_multidot(const double *__restrict__ V, int64_t ldv, int64_t vstride,
                                                           int ncols, const double *__restrict__ w, int64_t wstride,
                                                           int64_t n3, double *__restrict__ partial, int nblk,
@@ -1289,28 +1299,26 @@ __global__ void __launch_bounds__(kDotThreads) k_multidot(const double *__restri
     __shared__ bool last;
     const int r = blockIdx.y;
     if (jd) ncols += *jd;   // graph form: the column count follows the device step counter
-    const double *Vr = V + r * vstride;
-    const double *wr = w + r * wstride;
-    const int64_t i0 = (int64_t)blockIdx.x * kDotChunk;
+    const int64_t i0 = (int64_t)blockIdx.x * kDotChunk + threadIdx.x;
+    const double *Vr = V + r * vstride + i0;
+    const double *wr = w + r * wstride + i0;
     double wv[kDotItems];
 #pragma unroll
-    for (int k = 0; k < kDotItems; ++k) {
-        int64_t i = i0 + (int64_t)k * kDotThreads + threadIdx.x;
-        wv[k] = i < n3 ? wr[i] : 0.0;
-    }
+    for (int k = 0; k < kDotItems; ++k) wv[k] = i0 + k * kDotThreads < n3 ? wr[k * kDotThreads] : 0.0;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    // columns interleaved in fours: the loads of the next columns overlap this column's shuffle reduction
-#pragma unroll 4
-    for (int c = 0; c < ncols; ++c) {
-        const double *Vc = Vr + (int64_t)c * ldv;
-        double acc = 0.0;
+    for (int c = 0; c < ncols; c += 4) {
+        double acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-        for (int k = 0; k < kDotItems; ++k) {
-            int64_t i = i0 + (int64_t)k * kDotThreads + threadIdx.x;
-            if (i < n3) acc += Vc[i] * wv[k];
+        for (int q = 0; q < 4; ++q) {
+            if (c + q < ncols) {
+                const double *Vc = Vr + (int64_t)(c + q) * ldv;
+#pragma unroll
+                for (int k = 0; k < kDotItems; ++k)
+                    if (i0 + k * kDotThreads < n3) acc[q] += Vc[k * kDotThreads] * wv[k];
+            }
         }
-        acc = warp_sum(acc);
-        if (lane == 0) red[wid][c] = acc;
+        const double v = warp_sum4(acc[0], acc[1], acc[2], acc[3], lane);
+        if ((lane & 7) == 0) red[wid][c + lane / 8] = v;
     }
     __syncthreads();
     for (int c = threadIdx.x; c < ncols; c += blockDim.x) {
@@ -1324,10 +1332,9 @@ __global__ void __launch_bounds__(kDotThreads) k_multidot(const double *__restri
     if (threadIdx.x == 0) last = atomicAdd(&tickets[r], 1u) == (unsigned)(nblk - 1);
     __syncthreads();
     if (!last) return;
-    for (int c = threadIdx.x; c < ncols; c += blockDim.x) {
-        double s = 0.0;
-        for (int b = 0; b < nblk; ++b) s += __ldcg(partial + ((int64_t)r * nblk + b) * kMaxCols + c);
-        out[(int64_t)r * ostride + c] = s;
+    for (int c = wid; c < ncols; c += kDotThreads / 32) {
+        const double s = partials_sum(partial, r, nblk, c, lane);
+        if (lane == 0) out[(int64_t)r * ostride + c] = s;
     }
     if (threadIdx.x == 0) tickets[r] = 0u;
 }
@@ -1375,12 +1382,17 @@ __global__ void k_sub(const double *__restrict__ a, const double *__restrict__ b
         out[i] = a[i] - b[i];
 }
 
-// dst_r = src_r * scale_r (scale_r = 1/norm; zero norm -> zero vector)
+// dst_r = src_r / norm_r (zero norm -> zero vector); one division a block
 __global__ void k_scale_vec(const double *__restrict__ src, int64_t sstride, double *__restrict__ dst,
                             int64_t dstride, const double *__restrict__ nrm, int64_t nstride, int64_t n3) {
+    __shared__ double sf;
     const int r = blockIdx.y;
-    const double v = nrm[r * nstride];
-    const double f = v != 0.0 ? 1.0 / v : 0.0;
+    if (threadIdx.x == 0) {
+        const double v = nrm[r * nstride];
+        sf = v != 0.0 ? 1.0 / v : 0.0;
+    }
+    __syncthreads();
+    const double f = sf;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n3; i += (int64_t)gridDim.x * blockDim.x)
         dst[r * dstride + i] = src[r * sstride + i] * f;
 }
@@ -1440,48 +1452,227 @@ __global__ void k_cycle_start(GmresState st, int restart, int nrhs) {
     st.kfull[r] = 0;
 }
 
-// Arnoldi column j: H[:,j] = h1 + h2, H[j+1,j] = ||w||, then Givens rotations.
-__global__ void k_arnoldi_givens(GmresState st, int restart, int j, int nrhs, const int32_t *__restrict__ frozen,
-                                 const int32_t *__restrict__ jd = nullptr) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nrhs) return;
-    if (frozen[r]) return;
-    if (jd) j = *jd;
+// Loop control of a step captured in a graph (handle set, jd the step counter on the device): the last system to finish
+// freezes the systems that reached the tolerance, advances the counter, and repeats the loop body while some system is
+// active and j < restart.
+struct LoopCtl {
+    int32_t *jd = nullptr;
+    const double *tol = nullptr;
+    unsigned *done = nullptr;   // systems finished in this step
+    int nrhs = 0;
+    cudaGraphConditionalHandle handle{};
+};
+
+// Arnoldi column j of system r, by one block: H[:,j] = h1 + h2, H[j+1,j] = ||w||, then the Givens rotations.  Leaves
+// 1 / ||w|| in nrm2 (0 for a zero norm or a frozen system: the next basis vector is zero).  wn2 = ||w||^2.
+struct GivensShared {
+    double h[kMaxCols + 1], cs[kMaxCols], sn[kMaxCols];
+};
+__device__ void arnoldi_column(const GmresState &st, int restart, int j, int r, double wn2,
+                               int32_t *__restrict__ frozen, GivensShared &sh) {
     const int ld = restart + 1;
+    const bool live = !frozen[r];
+    for (int i = threadIdx.x; i <= j && live; i += blockDim.x) {
+        sh.h[i] = st.h1[r * kMaxCols + i] + st.h2[r * kMaxCols + i];
+        if (i < j) {
+            sh.cs[i] = st.cs[r * restart + i];
+            sh.sn[i] = st.sn[r * restart + i];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    if (!live) {
+        st.nrm2[r] = 0.0;
+        return;
+    }
+    const double wn = sqrt(wn2);
+    st.nrm2[r] = wn != 0.0 ? 1.0 / wn : 0.0;
     double *Hc = st.H + (int64_t)r * ld * restart + (int64_t)j * ld;
-    for (int i = 0; i <= j; ++i) Hc[i] = st.h1[r * kMaxCols + i] + st.h2[r * kMaxCols + i];
-    const double wn = sqrt(st.nrm2[r]);
-    st.nrm2[r] = wn;  // the following normalisation of w divides by the norm
-    Hc[j + 1] = wn;
-    double *cs = st.cs + r * restart, *sn = st.sn + r * restart, *g = st.g + r * ld;
+    double a = sh.h[0];
     for (int i = 0; i < j; ++i) {
-        const double t = cs[i] * Hc[i] + sn[i] * Hc[i + 1];
-        Hc[i + 1] = -sn[i] * Hc[i] + cs[i] * Hc[i + 1];
-        Hc[i] = t;
+        const double b = sh.h[i + 1];
+        Hc[i] = sh.cs[i] * a + sh.sn[i] * b;
+        a = -sh.sn[i] * a + sh.cs[i] * b;
     }
-    const double a = Hc[j], b = Hc[j + 1];
-    const double den = hypot(a, b);
-    if (den == 0.0) {
-        cs[j] = 1.0;
-        sn[j] = 0.0;
-    } else {
-        cs[j] = a / den;
-        sn[j] = b / den;
-    }
-    Hc[j] = cs[j] * a + sn[j] * b;
+    const double den = hypot(a, wn);
+    const double c = den == 0.0 ? 1.0 : a / den, s = den == 0.0 ? 0.0 : wn / den;
+    st.cs[r * restart + j] = c;
+    st.sn[r * restart + j] = s;
+    Hc[j] = c * a + s * wn;
     Hc[j + 1] = 0.0;
+    double *g = st.g + r * ld;
     const double gj = g[j];
-    g[j] = cs[j] * gj;
-    g[j + 1] = -sn[j] * gj;
+    g[j] = c * gj;
+    g[j + 1] = -s * gj;
     // the cycle keeps its best iterate: the least-squares solution over the first k columns, k where the
     // residual estimate last decreased strictly (EW/capacitance.py:174-191); the estimate never rises in exact
     // arithmetic, so k = j + 1 unless it stagnates
-    const double est = st.bnorm[r] > 0 ? fabs(g[j + 1]) / st.bnorm[r] : 0.0;
+    const double est = st.bnorm[r] > 0 ? fabs(s * gj) / st.bnorm[r] : 0.0;
     st.kfull[r] = j + 1;
     if (est < st.res[r]) {
         st.res[r] = est;
         st.kcount[r] = j + 1;
     }
+}
+
+// After a system's column, by one thread of its last block.
+__device__ void loop_control(const GmresState &st, int restart, int j, int32_t *__restrict__ frozen,
+                             const LoopCtl &lc) {
+    if (!lc.jd) return;
+    __threadfence();
+    if (atomicAdd(lc.done, 1u) != (unsigned)(lc.nrhs - 1)) return;
+    __threadfence();
+    const double t = *lc.tol;
+    bool active = false;
+    for (int r = 0; r < lc.nrhs; ++r) {
+        if (!frozen[r] && __ldcg(st.res + r) <= t) frozen[r] = 1;
+        active = active || !frozen[r];
+    }
+    *lc.done = 0u;
+    *lc.jd = j + 1;
+    cudaGraphSetConditional(lc.handle, (active && j + 1 < restart) ? 1u : 0u);
+}
+
+// End of an Arnoldi step: w_r -= sum_c V_r[c] h_r[c] (h the last Gram-Schmidt pass's dots) and its norm in one pass; the
+// last block of each system does the column's rotations and the loop control.
+__global__ void __launch_bounds__(kDotThreads) k_arnoldi_end(const double *__restrict__ V, int64_t ldv, int64_t n3,
+                                                             double *__restrict__ w, const double *__restrict__ h,
+                                                             GmresState st, int restart, int j,
+                                                             int32_t *__restrict__ frozen,
+                                                             double *__restrict__ partial, int nblk,
+                                                             unsigned *__restrict__ tickets, LoopCtl lc) {
+    __shared__ double hs[kMaxCols], red[kDotThreads / 32];
+    __shared__ GivensShared gsh;
+    __shared__ bool last;
+    const int r = blockIdx.y;
+    if (lc.jd) j = *lc.jd;
+    for (int c = threadIdx.x; c <= j; c += blockDim.x) hs[c] = h[(int64_t)r * kMaxCols + c];
+    __syncthreads();
+    const int64_t i0 = (int64_t)blockIdx.x * kDotChunk + threadIdx.x;
+    const double *Vr = V + (int64_t)r * n3 + i0;
+    double *wr = w + (int64_t)r * n3 + i0;
+    double acc[kDotItems];
+#pragma unroll
+    for (int k = 0; k < kDotItems; ++k) acc[k] = i0 + k * kDotThreads < n3 ? wr[k * kDotThreads] : 0.0;
+    for (int c = 0; c <= j; ++c) {
+        const double *Vc = Vr + (int64_t)c * ldv;
+        const double hc = hs[c];
+#pragma unroll
+        for (int k = 0; k < kDotItems; ++k)
+            if (i0 + k * kDotThreads < n3) acc[k] -= Vc[k * kDotThreads] * hc;
+    }
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < kDotItems; ++k) {
+        if (i0 + k * kDotThreads < n3) wr[k * kDotThreads] = acc[k];
+        s += acc[k] * acc[k];
+    }
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    s = warp_sum(s);
+    if (lane == 0) red[wid] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int q = 0; q < kDotThreads / 32; ++q) t += red[q];
+        partial[((int64_t)r * nblk + blockIdx.x) * kMaxCols] = t;
+        __threadfence();
+        last = atomicAdd(&tickets[r], 1u) == (unsigned)(nblk - 1);
+    }
+    __syncthreads();
+    if (!last) return;
+    if (wid == 0) {
+        const double t = partials_sum(partial, r, nblk, 0, lane);
+        if (lane == 0) red[0] = t;
+    }
+    __syncthreads();
+    arnoldi_column(st, restart, j, r, red[0], frozen, gsh);
+    if (threadIdx.x == 0) {
+        tickets[r] = 0u;
+        loop_control(st, restart, j, frozen, lc);
+    }
+}
+
+// A whole Arnoldi step after the matvec for systems of at most kSmallRows rows, one block a system with w in registers:
+// the Gram-Schmidt passes, the rotations, the next basis vector (also to vin when given) and the loop control.  One SM's
+// float64 rate bounds it, and every warp of the block pays its part of the reductions: eight rows a thread, so that the
+// block has no more warps than it needs (1500 rows, one to five columns, two passes: 28 us in seven launches -> 15 us).
+// Beyond 2048 rows more SMs are worth the launches (3000 rows, three systems, four columns: 27 us here, 25 there, and
+// the columns' work grows four times as fast here).
+constexpr int kSmallThreads = 256;
+constexpr int kSmallRows = kSmallThreads * kDotItems;
+
+__global__ void __launch_bounds__(kSmallThreads) k_arnoldi_small(double *__restrict__ V, int64_t ldv, int64_t n3,
+                                                                 const double *__restrict__ w, double *__restrict__ vin,
+                                                                 GmresState st, int restart, int j, int passes,
+                                                                 int32_t *__restrict__ frozen, LoopCtl lc) {
+    __shared__ double red[kSmallThreads / 32][kMaxCols], hs[kMaxCols], rn[kSmallThreads / 32 + 1];
+    __shared__ GivensShared gsh;
+    const int r = blockIdx.x;
+    if (lc.jd) j = *lc.jd;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5, rows = (int)n3;
+    const int stride = blockDim.x;
+    // the rows of this thread: threadIdx.x + k blockDim.x, k < kDotItems
+    const int mine = rows > (int)threadIdx.x ? (rows - (int)threadIdx.x + stride - 1) / stride : 0;
+    double *Vr = V + (int64_t)r * n3 + threadIdx.x;
+    double wv[kDotItems];
+#pragma unroll
+    for (int k = 0; k < kDotItems; ++k) wv[k] = k < mine ? w[r * n3 + threadIdx.x + k * stride] : 0.0;
+    for (int pass = 0; pass < passes; ++pass) {
+        for (int c = 0; c <= j; c += 4) {
+            double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (c + q <= j) {
+                    const double *Vc = Vr + (int64_t)(c + q) * ldv;
+#pragma unroll
+                    for (int k = 0; k < kDotItems; ++k)
+                        if (k < mine) acc[q] += Vc[k * stride] * wv[k];
+                }
+            }
+            const double v = warp_sum4(acc[0], acc[1], acc[2], acc[3], lane);
+            if ((lane & 7) == 0) red[wid][c + lane / 8] = v;
+        }
+        __syncthreads();
+        if ((int)threadIdx.x <= j) {
+            const int c = threadIdx.x;
+            double s = 0.0;
+            for (int q = 0; q < nwarp; ++q) s += red[q][c];
+            hs[c] = s;
+            (pass == 0 ? st.h1 : st.h2)[r * kMaxCols + c] = s;
+        }
+        __syncthreads();
+        for (int c = 0; c <= j; ++c) {
+            const double *Vc = Vr + (int64_t)c * ldv;
+            const double hc = hs[c];
+#pragma unroll
+            for (int k = 0; k < kDotItems; ++k)
+                if (k < mine) wv[k] -= Vc[k * stride] * hc;
+        }
+    }
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < kDotItems; ++k)
+        if (k < mine) s += wv[k] * wv[k];
+    s = warp_sum(s);
+    if (lane == 0) rn[wid] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s = 0.0;
+        for (int q = 0; q < nwarp; ++q) s += rn[q];
+        rn[kSmallThreads / 32] = s;
+    }
+    __syncthreads();
+    arnoldi_column(st, restart, j, r, rn[kSmallThreads / 32], frozen, gsh);
+    __syncthreads();
+    const double f = st.nrm2[r];
+    double *dst = Vr + (int64_t)(j + 1) * ldv;
+#pragma unroll
+    for (int k = 0; k < kDotItems; ++k)
+        if (k < mine) {
+            dst[k * stride] = wv[k] * f;
+            if (vin) vin[r * n3 + threadIdx.x + k * stride] = wv[k] * f;
+        }
+    if (threadIdx.x == 0) loop_control(st, restart, j, frozen, lc);
 }
 
 // Coefficients u (length k+1) of the least-squares residual b - A x_k = V_{k+1} u:
@@ -1530,8 +1721,8 @@ static char *carve_ws(char *&p, size_t bytes) {
 }
 
 // Dots of the first ncols basis vectors with w, for every system.  The scratch
-// holds nrhs * nblk * kMaxCols partials followed by nrhs zeroed tickets
-// (multidot_bytes / multidot_init).
+// holds nrhs * nblk * kMaxCols partials followed by nrhs + 1 zeroed tickets
+// (multidot_bytes / multidot_init; the last counts systems for the loop control).
 static int multidot(const double *V, int64_t ldv, int64_t vstride, int ncols, const double *w, int64_t wstride,
                     int64_t n3, int nrhs, double *partial, double *out, int64_t ostride, cudaStream_t s,
                     const int32_t *jd = nullptr) {
@@ -1551,7 +1742,7 @@ static size_t multidot_bytes(int64_t n3, int nrhs) {
 
 static int multidot_init(double *partial, int64_t n3, int nrhs, cudaStream_t s) {
     const int nblk = (int)((n3 + kDotChunk - 1) / kDotChunk);
-    MPS_CUDA_TRY(cudaMemsetAsync(partial + (size_t)nrhs * nblk * kMaxCols, 0, sizeof(unsigned) * (size_t)nrhs, s));
+    MPS_CUDA_TRY(cudaMemsetAsync(partial + (size_t)nrhs * nblk * kMaxCols, 0, sizeof(unsigned) * (size_t)(nrhs + 1), s));
     return MPS_OK;
 }
 
@@ -1565,38 +1756,21 @@ static int multidot_init(double *partial, int64_t n3, int nrhs, cudaStream_t s) 
 // restart - j0 steps.  The host reads the estimates once per graph launch.
 // ---------------------------------------------------------------------------
 
-// V[j+1]_r = w_r / nrm_r (j = *jd; zero norm -> zero vector), copied to vin as well.
-__global__ void k_next_basis(const double *__restrict__ w, double *__restrict__ V, int64_t ldv,
-                             const int32_t *__restrict__ jd, const double *__restrict__ nrm, double *__restrict__ vin,
+// V[j+1]_r = w_r inv_r, copied to vin as well when given.  In the graph form the step counter has been advanced
+// already: the new vector is column *jd.
+__global__ void k_next_basis(const double *__restrict__ w, double *__restrict__ V, int64_t ldv, int col,
+                             const int32_t *__restrict__ jd, const double *__restrict__ inv, double *__restrict__ vin,
                              int64_t n3) {
     const int r = blockIdx.y;
-    const double v = nrm[r];
-    const double f = v != 0.0 ? 1.0 / v : 0.0;
-    double *dst = V + (int64_t)(*jd + 1) * ldv + (int64_t)r * n3;
-    double *d2 = vin + (int64_t)r * n3;
+    const double f = inv[r];
+    if (jd) col = *jd;
+    double *dst = V + (int64_t)col * ldv + (int64_t)r * n3;
     const double *src = w + (int64_t)r * n3;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n3; i += (int64_t)gridDim.x * blockDim.x) {
         const double x = src[i] * f;
         dst[i] = x;
-        d2[i] = x;
+        if (vin) vin[(int64_t)r * n3 + i] = x;
     }
-}
-
-// End of a step: freeze the systems that reached the tolerance, advance j, and
-// repeat the body while some system is active and j < restart.
-__global__ void k_loop_ctrl(const double *__restrict__ res, int32_t *__restrict__ frozen,
-                            const double *__restrict__ tol, int nrhs, int32_t *__restrict__ jd, int restart,
-                            cudaGraphConditionalHandle h) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    const double t = *tol;
-    bool active = false;
-    for (int r = 0; r < nrhs; ++r) {
-        if (!frozen[r] && res[r] <= t) frozen[r] = 1;
-        active = active || !frozen[r];
-    }
-    const int j = *jd + 1;
-    *jd = j;
-    cudaGraphSetConditional(h, (active && j < restart) ? 1u : 0u);
 }
 
 __global__ void k_graph_enter(int32_t *__restrict__ jd, int j0, double *__restrict__ tol_d, double tol) {
@@ -1669,6 +1843,49 @@ static bool graphs_enabled(const mps_system *s) {
     return !(v && v[0] == '0');
 }
 
+// Everything of an Arnoldi step after its matvec (w = A V[j]): Gram-Schmidt (twice with reorth), the column's rotations,
+// V[j + 1], and, in the graph form (lc.jd set; j ignored), the copy to vin and the loop control.
+static int arnoldi_step(const GmresWs &W, int64_t n3, int nrhs, int restart, int j, bool reorth, const LoopCtl &lc,
+                        cudaStream_t st) {
+    const int64_t ldv = (int64_t)nrhs * n3;
+    const int ncols = lc.jd ? 1 : j + 1;
+    double *vin = lc.jd ? W.vin : nullptr;
+    if (n3 <= kSmallRows) {
+        const int threads = std::max(64, ((int)n3 + 32 * kDotItems - 1) / (32 * kDotItems) * 32);   // > kMaxCols - 1 columns
+        k_arnoldi_small<<<nrhs, threads, 0, st>>>(W.V, ldv, n3, W.w, vin, W.S, restart, j, reorth ? 2 : 1, W.frozen,
+                                                        lc);
+        MPS_LAUNCH_CHECK();
+        return MPS_OK;
+    }
+    const dim3 vgrid(grid_for(n3, 256, 152 * 8), nrhs);
+    MPS_TRY(multidot(W.V, ldv, n3, ncols, W.w, n3, n3, nrhs, W.partial, W.S.h1, kMaxCols, st, lc.jd));
+    if (reorth) {
+        k_sub_basis<<<vgrid, 256, 0, st>>>(W.V, ldv, n3, ncols, W.S.h1, kMaxCols, W.w, n3, n3, lc.jd);
+        MPS_LAUNCH_CHECK();
+        MPS_TRY(multidot(W.V, ldv, n3, ncols, W.w, n3, n3, nrhs, W.partial, W.S.h2, kMaxCols, st, lc.jd));
+    }
+    const int nblk = (int)((n3 + kDotChunk - 1) / kDotChunk);
+    unsigned *tickets = (unsigned *)(W.partial + (size_t)nrhs * nblk * kMaxCols);
+    k_arnoldi_end<<<dim3(nblk, nrhs), kDotThreads, 0, st>>>(W.V, ldv, n3, W.w, reorth ? W.S.h2 : W.S.h1, W.S, restart, j,
+                                                            W.frozen, W.partial, nblk, tickets, lc);
+    MPS_LAUNCH_CHECK();
+    k_next_basis<<<vgrid, 256, 0, st>>>(W.w, W.V, ldv, j + 1, lc.jd, W.S.nrm2, vin, n3);
+    MPS_LAUNCH_CHECK();
+    return MPS_OK;
+}
+
+// The loop control of a captured step (its counter sits behind the dots' tickets).
+static LoopCtl loop_ctl(const GmresWs &W, int64_t n3, int nrhs, cudaGraphConditionalHandle h) {
+    const int nblk = (int)((n3 + kDotChunk - 1) / kDotChunk);
+    LoopCtl lc;
+    lc.jd = W.jd;
+    lc.tol = W.tol_d;
+    lc.done = (unsigned *)(W.partial + (size_t)nrhs * nblk * kMaxCols) + nrhs;
+    lc.nrhs = nrhs;
+    lc.handle = h;
+    return lc;
+}
+
 static int matvec_any(mps_system *s, const double *m, double *out, int nrhs, int precision, cudaStream_t st);
 
 // Captures the step body for g's configuration on the system's capture stream
@@ -1676,7 +1893,6 @@ static int matvec_any(mps_system *s, const double *m, double *out, int nrhs, int
 // marks g failed and returns MPS_OK: the caller keeps the host-driven steps.
 static int arnoldi_graph_build(mps_system *s, ArnoldiGraph &g, const GmresWs &W, int64_t n3) {
     const int nrhs = g.nrhs, restart = g.restart;
-    const int64_t ldv = (int64_t)nrhs * n3;
     if (!s->cap) MPS_CUDA_TRY(cudaStreamCreateWithFlags(&s->cap, cudaStreamNonBlocking));
     cudaGraph_t graph = nullptr;
     MPS_CUDA_TRY(cudaGraphCreate(&graph, 0));
@@ -1698,43 +1914,12 @@ static int arnoldi_graph_build(mps_system *s, ArnoldiGraph &g, const GmresWs &W,
     }
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     cudaStream_t cs = s->cap;
-    const dim3 vgrid(grid_for(n3, 256, 152 * 8), nrhs);
     capture_count_begin();
     ce = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     int e = ce == cudaSuccess ? MPS_OK : MPS_CUDA_ERR;
     if (e == MPS_OK) {
-        auto launched = [&]() { return cudaGetLastError() == cudaSuccess ? MPS_OK : MPS_CUDA_ERR; };
         e = matvec_any(s, W.vin, W.w, nrhs, g.precision, cs);
-        if (e == MPS_OK) e = multidot(W.V, ldv, n3, 1, W.w, n3, n3, nrhs, W.partial, W.S.h1, kMaxCols, cs, W.jd);
-        if (e == MPS_OK) {
-            k_sub_basis<<<vgrid, 256, 0, cs>>>(W.V, ldv, n3, 1, W.S.h1, kMaxCols, W.w, n3, n3, W.jd);
-            count_launch();
-            e = launched();
-        }
-        if (e == MPS_OK && g.reorth) {
-            e = multidot(W.V, ldv, n3, 1, W.w, n3, n3, nrhs, W.partial, W.S.h2, kMaxCols, cs, W.jd);
-            if (e == MPS_OK) {
-                k_sub_basis<<<vgrid, 256, 0, cs>>>(W.V, ldv, n3, 1, W.S.h2, kMaxCols, W.w, n3, n3, W.jd);
-                count_launch();
-                e = launched();
-            }
-        }
-        if (e == MPS_OK) e = multidot(W.w, n3, n3, 1, W.w, n3, n3, nrhs, W.partial, W.S.nrm2, 1, cs);
-        if (e == MPS_OK) {
-            k_arnoldi_givens<<<(nrhs + 31) / 32, 32, 0, cs>>>(W.S, restart, 0, nrhs, W.frozen, W.jd);
-            count_launch();
-            e = launched();
-        }
-        if (e == MPS_OK) {
-            k_next_basis<<<vgrid, 256, 0, cs>>>(W.w, W.V, ldv, W.jd, W.S.nrm2, W.vin, n3);
-            count_launch();
-            e = launched();
-        }
-        if (e == MPS_OK) {
-            k_loop_ctrl<<<1, 32, 0, cs>>>(W.S.res, W.frozen, W.tol_d, nrhs, W.jd, restart, h);
-            count_launch();
-            e = launched();
-        }
+        if (e == MPS_OK) e = arnoldi_step(W, n3, nrhs, restart, 0, g.reorth, loop_ctl(W, n3, nrhs, h), cs);
         cudaGraph_t out = nullptr;
         ce = cudaStreamEndCapture(cs, &out);
         if (ce != cudaSuccess) e = MPS_CUDA_ERR;
@@ -1937,19 +2122,7 @@ static int gmres_core(mps_system *s, const double *b, double *x, int nrhs, doubl
             }
             queued = false;
             // classical Gram-Schmidt, twice (once for the inner solves of the mixed refinement)
-            GM_TRY(multidot(V, ldv, n3, j + 1, w, n3, n3, nrhs, partial, S.h1, kMaxCols, st));
-            k_sub_basis<<<vgrid, 256, 0, st>>>(V, ldv, n3, j + 1, S.h1, kMaxCols, w, n3, n3);
-            GM_LAUNCH();
-            if (fl.reorth) {
-                GM_TRY(multidot(V, ldv, n3, j + 1, w, n3, n3, nrhs, partial, S.h2, kMaxCols, st));
-                k_sub_basis<<<vgrid, 256, 0, st>>>(V, ldv, n3, j + 1, S.h2, kMaxCols, w, n3, n3);
-                GM_LAUNCH();
-            }
-            GM_TRY(multidot(w, n3, n3, 1, w, n3, n3, nrhs, partial, S.nrm2, 1, st));
-            k_arnoldi_givens<<<(nrhs + 31) / 32, 32, 0, st>>>(S, restart, j, nrhs, frozen);
-            GM_LAUNCH();
-            k_scale_vec<<<vgrid, 256, 0, st>>>(w, n3, V + (int64_t)(j + 1) * ldv, n3, S.nrm2, 1, n3);
-            GM_LAUNCH();
+            GM_TRY(arnoldi_step(W, n3, nrhs, restart, j, fl.reorth, LoopCtl(), st));
             GM_CUDA(cudaMemcpyAsync(hres, S.res, sizeof(double) * nrhs, cudaMemcpyDeviceToHost, st));
             if (may_speculate && j + 1 < restart && likely_continues()) {
                 if (!s->ev_res) GM_CUDA(cudaEventCreateWithFlags(&s->ev_res, cudaEventDisableTiming));
