@@ -614,65 +614,102 @@ __device__ __forceinline__ void store_pair(PairData<T> &pd, int64_t w, int32_t b
     pd.rz[w] = (T)rh[2];
 }
 
-// Same traversal as k_csr_count; kept lanes write at the ballot prefix, so a
-// row lists its pairs by neighbour-cell offset, then by particle id.
-__global__ void __launch_bounds__(256) k_csr_fill(const double *__restrict__ x, const float *__restrict__ xf,
-                                                  PairScreen ps,
-                                                  const int32_t *__restrict__ sorted, const int32_t *__restrict__ lin,
-                                                  const int32_t *__restrict__ counts,
-                                                  const int64_t *__restrict__ starts, int64_t n, int64_t ncx,
-                                                  int64_t ncy, int64_t ncz, const int64_t *__restrict__ off27,
-                                                  const double *__restrict__ perp, const double *__restrict__ para,
-                                                  const double *__restrict__ rv, int64_t ntab, double inv_dr,
-                                                  PairData<double> p64, PairData<float> p32, int *__restrict__ err) {
-    const int lane = threadIdx.x & 31;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; s < n; s += nw) {
-        const int32_t a = sorted[s];
-        const CellWalk cw = cell_walk(lin[a], lane, counts, starts, ncx, ncy, ncz);
-        int64_t w = off27[(int64_t)a * 27];   // the row's pairs follow in (cell offset, position) order
-        for (int j0 = 0; j0 < cw.total; j0 += 32) {
-            const int j = j0 + lane;
+// Traversal of the cells around particle a in the order of k_csr_count, shared by the fill kernels: the screen only
+// decides which candidates are kept (float screen, float64 for the few in its margin band) and queues their ids per warp
+// in shared memory, in traversal order; drain(cnt, w) then computes the pairs w .. w + cnt - 1 of the row from the queue,
+// one per lane (cnt <= 32), instead of by the few lanes of each round that kept one (about one candidate in six is
+// kept).  The row lists its pairs by neighbour-cell offset, then by particle id.
+constexpr int kFillWarps = 8;
+
+template <class F>
+__device__ __forceinline__ void csr_row_walk(const double *__restrict__ x, const float *__restrict__ xf,
+                                             const PairScreen &ps, const CellWalk &cw,
+                                             const int32_t *__restrict__ sorted, int32_t a, int lane, int64_t w,
+                                             int32_t *q_b, F &&drain) {
+    int qn = 0;                           // kept pairs waiting in the queue (warp-uniform, < 32 between rounds)
+    // two candidates per lane per iteration (candidates j0 + lane and j0 + 32 + lane, queued in that order)
+    for (int j0 = 0; j0 < cw.total; j0 += 64) {
+        int32_t bb[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int j = j0 + 32 * h + lane;
             int o;
             int64_t pos;
             walk_at(cw, j < cw.total ? j : cw.total - 1, o, pos);
             (void)o;
+            bb[h] = j < cw.total ? sorted[pos] : a;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int32_t b = bb[h];
             bool keep = false;
-            int32_t b = -1;
-            double r[3] = {0, 0, 0}, s2 = 0.0;
-            if (j < cw.total) {
-                b = sorted[pos];
-                const int sc = b != a ? pair_screen(xf, a, b, ps) : SCREEN_OUT;
-                if (sc != SCREEN_OUT) {
-                    bool big = false;
-                    s2 = pair_diff2(x, a, b, ps, r, &big);
-                    if (big) {
-                        const double de = pair_exact(x, a, b, ps, r);
-                        s2 = __dmul_rn(de, de);
-                        keep = de < ps.rc;
-                    } else {
-                        // inside the screen's inner margin: kept for sure; near rc: the
-                        // correctly rounded separation decides, as in the count pass
-                        keep = sc == SCREEN_IN || __dsqrt_rn(s2) < ps.rc;
-                    }
-                }
+            const int sc = b != a ? pair_screen(xf, a, b, ps) : SCREEN_OUT;
+            if (sc == SCREEN_IN) {
+                keep = true;
+            } else if (sc == SCREEN_NEAR) {   // the correctly rounded float64 separation decides
+                double r64[3];
+                keep = pair_exact(x, a, b, ps, r64) < ps.rc;
             }
             const unsigned mask = __ballot_sync(0xffffffffu, keep);
-            if (keep) {
-                const int64_t wp = w + __popc(mask & ((1u << lane) - 1u));
-                // the float64 division and square root are the slow part of this
-                // kernel on GB300: Newton iterations from float32 seeds instead
-                const double y = rsqrt_newton(s2);
-                const double d = s2 * y;
-                const double rh[3] = {r[0] * y, r[1] * y, r[2] * y};
-                double A = 0.0, B = 0.0;
-                // ntab == 0: the couplings are filled in afterwards from the separations
-                if (ntab > 0 && !table_lerp_fast(perp, para, rv, ntab, d, &A, &B, inv_dr)) atomicExch(err, 1);
-                store_pair(p64, wp, b, A, B, rh, d);
-                store_pair(p32, wp, b, A, B, rh, d);
-            }
-            w += __popc(mask);
+            if (keep) q_b[qn + __popc(mask & ((1u << lane) - 1u))] = b;
+            qn += __popc(mask);
         }
+        __syncwarp();
+        while (qn >= 32) {
+            drain(32, w);
+            w += 32;
+            qn -= 32;
+            __syncwarp();
+            if (lane < qn) q_b[lane] = q_b[32 + lane];   // the rest to the front (qn < 64 here)
+            if (lane + 32 < qn) q_b[lane + 32] = q_b[64 + lane];
+            __syncwarp();
+        }
+    }
+    if (qn > 0) drain(qn, w);
+    __syncwarp();
+}
+
+// Float64 pair list of the quadrupole and polydisperse operators (50,000 spheres, 60 of about 380 candidates: 1.77 ms
+// with the pair terms in the walk, 0.45 ms queued).
+__global__ void __launch_bounds__(kFillWarps * 32) k_csr_fill(const double *__restrict__ x,
+                                                              const float *__restrict__ xf, PairScreen ps,
+                                                              const int32_t *__restrict__ sorted,
+                                                              const int32_t *__restrict__ lin,
+                                                              const int32_t *__restrict__ counts,
+                                                              const int64_t *__restrict__ starts, int64_t n,
+                                                              int64_t ncx, int64_t ncy, int64_t ncz,
+                                                              const int64_t *__restrict__ off27,
+                                                              const double *__restrict__ perp,
+                                                              const double *__restrict__ para,
+                                                              const double *__restrict__ rv, int64_t ntab,
+                                                              double inv_dr, PairData<double> p64,
+                                                              PairData<float> p32, int *__restrict__ err) {
+    __shared__ int32_t q_b[kFillWarps][128];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; s < n; s += nw) {
+        const int32_t a = sorted[s];
+        const CellWalk cw = cell_walk(lin[a], lane, counts, starts, ncx, ncy, ncz);
+        csr_row_walk(x, xf, ps, cw, sorted, a, lane, off27[(int64_t)a * 27], q_b[wid], [&](int cnt, int64_t w) {
+            if (lane >= cnt) return;
+            const int32_t b = q_b[wid][lane];
+            double r[3];
+            bool big = false;
+            double s2 = pair_diff2(x, a, b, ps, r, &big);
+            if (big) {   // far-wrapped: the general rule
+                const double de = pair_exact(x, a, b, ps, r);
+                s2 = __dmul_rn(de, de);
+            }
+            // the float64 division and square root are slow on GB300: Newton iterations from float32 seeds instead
+            const double y = rsqrt_newton(s2);
+            const double d = s2 * y;
+            const double rh[3] = {r[0] * y, r[1] * y, r[2] * y};
+            double A = 0.0, B = 0.0;
+            // ntab == 0: the couplings are filled in afterwards from the separations
+            if (ntab > 0 && !table_lerp_fast(perp, para, rv, ntab, d, &A, &B, inv_dr)) atomicExch(err, 1);
+            store_pair(p64, w + lane, b, A, B, rh, d);
+            store_pair(p32, w + lane, b, A, B, rh, d);
+        });
     }
 }
 
@@ -795,16 +832,9 @@ __device__ __forceinline__ void df_pair_out(const DfTab &tab, PairData<dfv> &pdf
     store_pair_df(pdf, p32, wp, b, A, B, rh, d);
 }
 
-// Same traversal and pair order as k_csr_fill.  About one candidate in six is
-// kept, so the screen only decides which candidates are kept (float screen, float64
-// for the few in its margin band) and queues their ids per warp in shared memory,
-// in traversal order; the double-float separations and couplings are then computed
-// 32 kept pairs at a time, one per lane, instead of by the few lanes of each round
-// that kept one.  The values are those of the per-round form: the keep decision is
-// the same (inside the screen's inner margin the float64 distance is below rc too),
-// and so is the separation (double-float difference, float64 for a far-wrapped pair).
-constexpr int kFillWarps = 8;
-
+// Double-float pair list of the dipole operator, as k_csr_fill.  The keep decision is that of the float64 form (inside
+// the screen's inner margin the float64 distance is below rc too), and so is the separation (double-float difference,
+// float64 for a far-wrapped pair).
 __global__ void __launch_bounds__(kFillWarps * 32) k_csr_fill_df(const double *__restrict__ x,
                                                                  const float *__restrict__ xf,
                                                                  const float2 *__restrict__ xdf, PairScreen ps,
@@ -854,48 +884,8 @@ __global__ void __launch_bounds__(kFillWarps * 32) k_csr_fill_df(const double *_
     for (int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; s < n; s += nw) {
         const int32_t a = sorted[s];
         const CellWalk cw = cell_walk(lin[a], lane, counts, starts, ncx, ncy, ncz);
-        int64_t w = off27[(int64_t)a * 27];   // the row's pairs follow in (cell offset, position) order
-        int qn = 0;                           // kept pairs waiting in the queue (warp-uniform, < 32 between rounds)
-        // two candidates per lane per iteration (candidates j0 + lane and j0 + 32 + lane, queued in that order)
-        for (int j0 = 0; j0 < cw.total; j0 += 64) {
-            int32_t bb[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int j = j0 + 32 * h + lane;
-                int o;
-                int64_t pos;
-                walk_at(cw, j < cw.total ? j : cw.total - 1, o, pos);
-                (void)o;
-                bb[h] = j < cw.total ? sorted[pos] : a;
-            }
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int32_t b = bb[h];
-                bool keep = false;
-                const int sc = b != a ? pair_screen(xf, a, b, ps) : SCREEN_OUT;
-                if (sc == SCREEN_IN) {
-                    keep = true;
-                } else if (sc == SCREEN_NEAR) {   // the correctly rounded float64 separation decides
-                    double r64[3];
-                    keep = pair_exact(x, a, b, ps, r64) < ps.rc;
-                }
-                const unsigned mask = __ballot_sync(0xffffffffu, keep);
-                if (keep) q_b[wid][qn + __popc(mask & ((1u << lane) - 1u))] = b;
-                qn += __popc(mask);
-            }
-            __syncwarp();
-            while (qn >= 32) {
-                drain(a, 32, w);
-                w += 32;
-                qn -= 32;
-                __syncwarp();
-                if (lane < qn) q_b[wid][lane] = q_b[wid][32 + lane];   // the rest to the front (qn < 64 here)
-                if (lane + 32 < qn) q_b[wid][lane + 32] = q_b[wid][64 + lane];
-                __syncwarp();
-            }
-        }
-        if (qn > 0) drain(a, qn, w);
-        __syncwarp();
+        csr_row_walk(x, xf, ps, cw, sorted, a, lane, off27[(int64_t)a * 27], q_b[wid],
+                     [&](int cnt, int64_t w) { drain(a, cnt, w); });
     }
 }
 
@@ -1052,7 +1042,7 @@ int csr_pairs_fill(const double *x, const float *xf, double maxabs, const double
         MPS_CUDA_TRY(cudaStreamSynchronize(s));
     }
     const double inv_dr = rv_last > 0 ? (double)(ntab - 1) / rv_last : 0.0;
-    k_csr_fill<<<grid_for(n * 32, 256, 152 * 64), 256, 0, s>>>(x, xf, make_screen(box, rc, maxabs), cb.sorted, cb.lin, cb.counts,
+    k_csr_fill<<<grid_for(n * 32, kFillWarps * 32, 152 * 64), kFillWarps * 32, 0, s>>>(x, xf, make_screen(box, rc, maxabs), cb.sorted, cb.lin, cb.counts,
                                                      cb.starts, n, cb.ncell[0], cb.ncell[1], cb.ncell[2], off27,
                                                      perp, para, rv, ntab, inv_dr, p64, p32, err);
     MPS_LAUNCH_CHECK();
