@@ -55,6 +55,42 @@ __device__ __forceinline__ T warp_sum(T v) {
     return v;
 }
 
+// C sums over the warp (C <= 32), one to a lane: each halving of the warp halves the values a lane still carries, so C sums
+// take about C + 4 shuffles and additions instead of 5 C, and what follows (the conversion to float64, the scaling, the
+// store) is one instruction for all of them: on GB300 a float64 instruction of a warp, a conversion too, costs the same
+// for one active lane as for 32.  Each sum adds the same pairs in the same order as warp_sum.  warp_sums_index tells
+// which sum a lane holds (-1: none, or the same as another lane).
+template <int C, int O = 16, typename T>
+__device__ __forceinline__ T warp_sums(const T (&v)[C], int lane) {
+    if constexpr (O == 0) {
+        static_assert(C == 1, "more sums than lanes");
+        return v[0];
+    } else {
+        constexpr int H = (C + 1) / 2;
+        const bool hi = lane & O;
+        T u[H];
+#pragma unroll
+        for (int k = 0; k < H; ++k) {
+            const T up = v[k + H < C ? k + H : k];
+            u[k] = (hi ? up : v[k]) + __shfl_xor_sync(0xffffffffu, hi ? v[k] : up, O);
+        }
+        return warp_sums<H, O / 2>(u, lane);
+    }
+}
+
+template <int C, int O = 16>
+__device__ __forceinline__ int warp_sums_index(int lane) {
+    if constexpr (O == 0) {
+        return 0;
+    } else {
+        constexpr int H = (C + 1) / 2;
+        const int i = warp_sums_index<H, O / 2>(lane);
+        if (C == 1) return (lane & O) ? -1 : i;
+        const int k = i + ((lane & O) ? H : 0);
+        return i < 0 || k >= C ? -1 : k;
+    }
+}
+
 // Four sums over the warp in 6 additions instead of 20 (float64 additions are what a warp's reductions cost on GB300):
 // halves of the warp take half of the values each.  Lane 0 returns a's sum, lane 8 b's, lane 16 c's, lane 24 d's.
 template <typename T>

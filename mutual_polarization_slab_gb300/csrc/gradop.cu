@@ -335,6 +335,7 @@ __global__ void __launch_bounds__(256, 3) k_contract_grad_warp(const float *__re
                                                             const float *__restrict__ w, const float *__restrict__ g,
                                                             GridParams gp, double *__restrict__ out) {
     const int lane = threadIdx.x & 31;
+    const int oc = warp_sums_index<3 * NR>(lane);   // the output component this lane writes
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int P = gp.P;
@@ -381,14 +382,8 @@ __global__ void __launch_bounds__(256, 3) k_contract_grad_warp(const float *__re
                 acc[3 * r + 2] += wx * wy * s1[r];
             }
         }
-#pragma unroll
-        for (int c = 0; c < 3 * NR; ++c) acc[c] = warp_sum(acc[c]);
-        if (lane == 0)
-#pragma unroll
-            for (int r = 0; r < NR; ++r)
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-                    out[((int64_t)(r0 + r) * n + a) * 3 + c] = (double)acc[3 * r + c] * gp.hprod;
+        const float v = warp_sums(acc, lane);
+        if (oc >= 0) out[((int64_t)(r0 + oc / 3) * n + a) * 3 + oc % 3] = float_to_double(v) * gp.hprod;
     }
 }
 
@@ -402,8 +397,10 @@ __global__ void __launch_bounds__(256, 3) k_contract_grad_warp(const float *__re
 // is a template parameter, so the z runs unroll completely with the z factors in
 // registers and the shared-memory offsets are immediates.  A node is staged by about
 // (R / kHomeBlock)^3 blocks (9.6 at P = 10), all from L2.
-// With one vector a CTA takes 2 x 2 home blocks (5.2 stagings a node): 0.256 -> 0.156 ms for N = 2e5 on 192^3, with the
-// region staged row by row (the wraps worked out once a row, not once a node).
+// With one vector a CTA takes 2 x 2 home blocks (5.2 stagings a node): 0.256 -> 0.156 ms for N = 2e5 on 240^3, with the
+// region staged row by row (the wraps worked out once a row, not once a node).  The sums end one to a lane, converted and
+// scaled together: lane 0's 3 NR conversions and multiplications had cost a warp 6 NR float64 instructions a particle
+// (0.209 -> 0.174 ms for N = 1e5, three vectors, 192^3; 0.155 -> 0.144 for N = 2e5, one vector, 240^3).
 // 67 KB of shared memory at P = 10 and 3 vectors, 3 blocks per SM (80 registers): the mixed step at the bench
 // workload took 19.25 ms against 20.08 with the warp gather; float4 nodes (the 3 vectors interleaved, 87 KB,
 // 2 blocks per SM) took 20.17.
@@ -460,6 +457,7 @@ __global__ void __launch_bounds__(256, NR == 1 ? 4 : 3) k_contract_grad_home(
     const int X0 = bx0 * kHomeBlock, Y0 = by0 * kHomeBlock, Z0 = bz * kHomeBlock;
     const float *g0 = grid + (int64_t)r0 * G;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int oc = warp_sums_index<3 * NR>(lane);   // the output component this lane writes
     // origin + offset < 3 N (the host requires it): at most two wraps
     auto wrap2 = [](int i, int N) {
         i -= i >= N ? N : 0;
@@ -557,14 +555,8 @@ __global__ void __launch_bounds__(256, NR == 1 ? 4 : 3) k_contract_grad_home(
                     acc[3 * r + 2] += wx * wy * s1[r];
                 }
             }
-#pragma unroll
-            for (int c = 0; c < 3 * NR; ++c) acc[c] = warp_sum(acc[c]);
-            if (lane == 0)
-#pragma unroll
-                for (int r = 0; r < NR; ++r)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c)
-                        out[((int64_t)(r0 + r) * n + a) * 3 + c] = (double)acc[3 * r + c] * gp.hprod;
+            const float v = warp_sums(acc, lane);
+            if (oc >= 0) out[((int64_t)(r0 + oc / 3) * n + a) * 3 + oc % 3] = float_to_double(v) * gp.hprod;
         }
         __syncthreads();   // this chunk's particle data is read before the next chunk overwrites it
     }
