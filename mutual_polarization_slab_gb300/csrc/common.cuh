@@ -55,6 +55,14 @@ __device__ __forceinline__ T warp_sum(T v) {
     return v;
 }
 
+// One float from global to shared memory without a register in between: a staging loop issues all its loads at once
+// (copy_async_wait before the barrier that publishes them).
+__device__ __forceinline__ void copy_async(float *smem, const float *gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // C sums over the warp (C <= 32), one to a lane: each halving of the warp halves the values a lane still carries, so C sums
 // take about C + 4 shuffles and additions instead of 5 C, and what follows (the conversion to float64, the scaling, the
 // store) is one instruction for all of them: on GB300 a float64 instruction of a warp, a conversion too, costs the same

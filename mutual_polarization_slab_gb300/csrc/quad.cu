@@ -18,6 +18,9 @@
 
 namespace mps {
 
+__device__ __forceinline__ double to_double(float v) { return float_to_double(v); }
+__device__ __forceinline__ double to_double(double v) { return v; }
+
 // ---------------------------------------------------------------------------
 // Spread / contract for ncomp (<= 8) moment components per particle.
 // ---------------------------------------------------------------------------
@@ -73,6 +76,7 @@ __global__ void __launch_bounds__(256) k_contract_gen(const T *__restrict__ grid
     const int P = gp.P;
     const int Nx = gp.N[0], Ny = gp.N[1], Nz = gp.N[2];
     const int64_t G = gp.G;
+    const int oc = warp_sums_index<8>(lane);   // the component this lane writes
     for (int64_t t = warp; t < n * nrhs; t += nw) {
         const int64_t a = gp.order ? (int64_t)gp.order[t % n] : t % n;
         const int r = (int)(t / n);
@@ -102,29 +106,138 @@ __global__ void __launch_bounds__(256) k_contract_gen(const T *__restrict__ grid
                     if (c < ncomp) acc[c] += wv * g0[c * G + node];
             }
         }
+        const T v = warp_sums(acc, lane);
+        if (oc >= 0 && oc < ncomp) out[((int64_t)r * n + a) * ncomp + oc] = to_double(v) * gp.hprod;
+    }
+}
+
+// Contraction of the eight float32 grids of a vector by home blocks: a block takes the particles whose stencils start in
+// one 8^3 block of nodes and four of the components; it stages the nodes that they reach, the block grown by P - 1 per
+// axis, as float4 (the four components side by side), then a warp per particle sums over its stencil from shared memory,
+// the lanes on the P^2 columns.  Rows of P + 8 nodes: consecutive columns of a warp then lie 16 bytes apart modulo the
+// banks, whatever P.  The gather from the grids (k_contract_gen) reads a line per row, plane and component of every
+// particle through L1, which bounds it; here the staging does (the blocks' chains of loads).  N = 50,320, 90 x 90 x 96,
+// P = 6: 96 us by the gather (with its sums converted by one lane), 60 so (with an interleaved copy of the grids, staged
+// 16 bytes at a time or gathered from, 63 and 68).
+constexpr int kHome8Chunk = 32;
+constexpr int kHome8Warps = 8;
+
+__global__ void __launch_bounds__(kHome8Warps * 32, 5) k_contract_home8(
+    const float *__restrict__ grid, int64_t n, const int64_t *__restrict__ hstart,
+    const int32_t *__restrict__ hentries, int nbx, int nby, const int32_t *__restrict__ start,
+    const float *__restrict__ w, GridParams gp, double *__restrict__ out) {
+    const int P = gp.P, F = 3 * P;
+    const int R = kHomeBlock + P - 1, RS = R + 1, RP = R * RS;   // nodes per axis, row and plane strides
+    extern __shared__ float4 s_reg4[];                            // [R][R][RS]
+    float *s_w = (float *)(s_reg4 + R * RP);                      // [kHome8Chunk][3 P]
+    int *s_p = (int *)(s_w + kHome8Chunk * F);                    // [kHome8Chunk][2]: first node in the region, particle id
+    const int64_t hb = blockIdx.x;
+    const int64_t e0 = hstart[hb], e1 = hstart[hb + 1];
+    if (e0 == e1) return;   // the whole block leaves: no barrier is left waiting
+    const int Nx = gp.N[0], Ny = gp.N[1], Nz = gp.N[2];
+    const int X0 = (int)(hb % nbx) * kHomeBlock, Y0 = (int)((hb / nbx) % nby) * kHomeBlock,
+              Z0 = (int)(hb / ((int64_t)nbx * nby)) * kHomeBlock;
+    const int r = blockIdx.y >> 1, c0 = 4 * (blockIdx.y & 1);
+    const int64_t G = gp.G;
+    const float *g0 = grid + (int64_t)blockIdx.y * 4 * G;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    // origin + offset < 3 N (the host requires N >= 8 and N >= P): at most two wraps
+    auto wrap2 = [](int i, int N) {
+        i -= i >= N ? N : 0;
+        return i - (i >= N ? N : 0);
+    };
+    const int LX = R <= 16 ? 16 : 32, x = lane & (LX - 1);
+    if (x < R) {
+        const float *gx = g0 + wrap2(X0 + x, Nx);
+        const int rpw = 32 / LX;   // rows a warp takes at a time
+        for (int row = wid * rpw + lane / LX; row < R * R; row += kHome8Warps * rpw) {
+            const int z = row / R, y = row - z * R;
+            const float *src = gx + ((int64_t)wrap2(Z0 + z, Nz) * Ny + wrap2(Y0 + y, Ny)) * Nx;
+            float *dst = (float *)(s_reg4 + row * RS + x);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) acc[c] = warp_sum(acc[c]);
-        if (lane == 0)
-            for (int c = 0; c < ncomp; ++c) out[((int64_t)r * n + a) * ncomp + c] = (double)acc[c] * gp.hprod;
+            for (int c = 0; c < 4; ++c) copy_async(dst + c, src + c * G);
+        }
+    }
+    const int full = P * P / 32 * 32, rem = P * P - full;   // columns of the whole rounds and of the last one,
+    const int lz = rem ? 32 / rem : 1;                      // whose lanes share a column's planes
+    const int lcol = rem ? full + lane / lz : 0, lsub = lane - lane / lz * lz;
+    const int ljy = lcol / P, ljx = lcol - ljy * P;
+    const int oc = warp_sums_index<4>(lane);
+    for (int64_t b0 = e0; b0 < e1; b0 += kHome8Chunk) {
+        const int cnt = (int)min((int64_t)kHome8Chunk, e1 - b0);
+        for (int q = threadIdx.x; q < cnt * F; q += kHome8Warps * 32) {
+            const int p = q / F;
+            s_w[q] = w[(int64_t)hentries[b0 + p] * F + (q - p * F)];
+        }
+        if (threadIdx.x < cnt) {
+            const int32_t a = hentries[b0 + threadIdx.x];
+            const int32_t *sa = start + 3 * (int64_t)a;
+            s_p[2 * threadIdx.x] = (sa[2] - Z0) * RP + (sa[1] - Y0) * RS + sa[0] - X0;
+            s_p[2 * threadIdx.x + 1] = a;
+        }
+        copy_async_wait();
+        __syncthreads();   // the region (first pass) and this chunk's particles are in place
+        for (int p = wid; p < cnt; p += kHome8Warps) {
+            const float *wa = s_w + p * F;
+            const float4 *base = s_reg4 + s_p[2 * p];
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int q = lane; q < full; q += 32) {
+                const int jy = q / P, jx = q - jy * P;
+                const float4 *col = base + jy * RS + jx;
+                float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+                for (int jz = 0; jz < P; ++jz) {
+                    const float wz = wa[2 * P + jz];
+                    const float4 v = col[jz * RP];
+                    s[0] += wz * v.x;
+                    s[1] += wz * v.y;
+                    s[2] += wz * v.z;
+                    s[3] += wz * v.w;
+                }
+                const float wxy = wa[jx] * wa[P + jy];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[c] += wxy * s[c];
+            }
+            if (rem && lcol < P * P) {
+                const float4 *col = base + ljy * RS + ljx;
+                const float wxy = wa[ljx] * wa[P + ljy];
+                for (int jz = lsub; jz < P; jz += lz) {
+                    const float wv = wxy * wa[2 * P + jz];
+                    const float4 v = col[jz * RP];
+                    acc[0] += wv * v.x;
+                    acc[1] += wv * v.y;
+                    acc[2] += wv * v.z;
+                    acc[3] += wv * v.w;
+                }
+            }
+            __syncwarp();
+            const float v = warp_sums(acc, lane);
+            if (oc >= 0) out[((int64_t)r * n + s_p[2 * p + 1]) * 8 + c0 + oc] = float_to_double(v) * gp.hprod;
+        }
+        __syncthreads();   // this chunk's particles are read before the next overwrites them
     }
 }
 
 // ---------------------------------------------------------------------------
 // Wave space
 // ---------------------------------------------------------------------------
-__global__ void k_quad_kcoef(GridParams gp, double *__restrict__ c64, float *__restrict__ c32) {
-    const int Nxh = gp.N[0] / 2 + 1;
-    const int64_t Gc = (int64_t)Nxh * gp.N[1] * gp.N[2];
+// The couplings depend on k only through its components' squares: worked out once for the quarter spectrum and written
+// for its mirror images.  The float32 table holds the unit wave vector too (the float64 square root and division of a
+// point cost the float32 scale kernel more than reading 16 bytes: 25 -> 12 us on 90 x 90 x 96); the float64 kernel works
+// it out.
+__global__ void k_quad_kcoef(GridParams gp, double *__restrict__ c64, float4 *__restrict__ c32) {
+    const HalfQuarter hq(gp.N);
     const double invG = 1.0 / (double)gp.G;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < Gc; t += (int64_t)gridDim.x * blockDim.x) {
-        const int ix = (int)(t % Nxh);
-        const int iy = (int)((t / Nxh) % gp.N[1]);
-        const int iz = (int)(t / ((int64_t)Nxh * gp.N[1]));
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < hq.size();
+         t += (int64_t)gridDim.x * blockDim.x) {
+        int ix, iy, iz;
+        hq.point(t, &ix, &iy, &iz);
         const double kx = fft_freq(ix, gp.N[0]) * gp.kfac[0];
         const double ky = fft_freq(iy, gp.N[1]) * gp.kfac[1];
         const double kz = fft_freq(iz, gp.N[2]) * gp.kfac[2];
         const double k2 = kx * kx + ky * ky + kz * kz;
         double v[4] = {0, 0, 0, 0};
+        float q[3] = {0, 0, 0};
         if (k2 > 0) {
             const double k = sqrt(k2);
             const double s = sin(k), c = cos(k);
@@ -136,13 +249,21 @@ __global__ void k_quad_kcoef(GridParams gp, double *__restrict__ c64, float *__r
             v[1] = -22.5 * j1 * j2 * g;      // HEQ / i
             v[2] = 45.0 * j2 * j1 * g;       // HGS / i
             v[3] = 112.5 * j2 * j2 * g;      // HGQ
-            for (int q = 0; q < 4; ++q)
-                if (!isfinite(v[q])) v[q] = 0.0;
+            for (int i = 0; i < 4; ++i)
+                if (!isfinite(v[i])) v[i] = 0.0;
+            const double inv = 1.0 / k;
+            q[0] = (float)(kx * inv);
+            q[1] = (float)(ky * inv);
+            q[2] = (float)(kz * inv);
         }
-        for (int q = 0; q < 4; ++q) {
-            c64[4 * t + q] = v[q];
-            if (c32) c32[4 * t + q] = (float)v[q];
-        }
+        const float4 lo = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
+        mirror_points(hq, ix, iy, iz, [&](int64_t lin, int sy, int sz) {
+            for (int i = 0; i < 4; ++i) c64[4 * lin + i] = v[i];
+            if (c32) {
+                c32[2 * lin] = lo;
+                c32[2 * lin + 1] = make_float4(q[0], sy * q[1], sz * q[2], 0.f);
+            }
+        });
     }
 }
 
@@ -203,23 +324,36 @@ __global__ void k_scale_quad(typename C2T<T>::type *__restrict__ spec, int nrhs,
         const int ix = (int)(t % Nxh);
         const int iy = (int)((t / Nxh) % gp.N[1]);
         const int iz = (int)(t / ((int64_t)Nxh * gp.N[1]));
-        const double kx = fft_freq(ix, gp.N[0]) * gp.kfac[0];
-        const double ky = fft_freq(iy, gp.N[1]) * gp.kfac[1];
-        const double kz = fft_freq(iz, gp.N[2]) * gp.kfac[2];
-        const double k2 = kx * kx + ky * ky + kz * kz;
-        T q[3] = {0, 0, 0};
-        if (k2 > 0) {
-            const double inv = 1.0 / sqrt(k2);
-            q[0] = (T)(kx * inv);
-            q[1] = (T)(ky * inv);
-            q[2] = (T)(kz * inv);
+        T q[3] = {0, 0, 0}, cf[4];
+        if constexpr (sizeof(T) == 4) {
+            const float4 *c4 = (const float4 *)coef + 2 * t;
+            const float4 lo = c4[0], hi = c4[1];
+            cf[0] = lo.x;
+            cf[1] = lo.y;
+            cf[2] = lo.z;
+            cf[3] = lo.w;
+            q[0] = hi.x;
+            q[1] = hi.y;
+            q[2] = hi.z;
+        } else {
+            const double kx = fft_freq(ix, gp.N[0]) * gp.kfac[0];
+            const double ky = fft_freq(iy, gp.N[1]) * gp.kfac[1];
+            const double kz = fft_freq(iz, gp.N[2]) * gp.kfac[2];
+            const double k2 = kx * kx + ky * ky + kz * kz;
+            if (k2 > 0) {
+                const double inv = 1.0 / sqrt(k2);
+                q[0] = kx * inv;
+                q[1] = ky * inv;
+                q[2] = kz * inv;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) cf[i] = coef[4 * t + i];
         }
         const bool ny[3] = {(gp.N[0] % 2 == 0) && ix == gp.N[0] / 2, (gp.N[1] % 2 == 0) && iy == gp.N[1] / 2,
                             (gp.N[2] % 2 == 0) && iz == gp.N[2] / 2};
         const bool nyq = ny[0] || ny[1] || ny[2];
         // conjugate partner: non-Nyquist components flip sign
         const T qp[3] = {ny[0] ? q[0] : -q[0], ny[1] ? q[1] : -q[1], ny[2] ? q[2] : -q[2]};
-        const T cf[4] = {coef[4 * t], coef[4 * t + 1], coef[4 * t + 2], coef[4 * t + 3]};
         for (int r = 0; r < nrhs; ++r) {
             C *s = spec + (int64_t)(8 * r) * Gc + t;
             C f[8], o1[8];
@@ -244,6 +378,22 @@ __global__ void k_scale_quad(typename C2T<T>::type *__restrict__ spec, int nrhs,
 // ---------------------------------------------------------------------------
 // Real space
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void load8(const float *__restrict__ p, float v[8]) {   // 32-byte aligned rows
+    const float4 a = ((const float4 *)p)[0], b = ((const float4 *)p)[1];
+    v[0] = a.x;
+    v[1] = a.y;
+    v[2] = a.z;
+    v[3] = a.w;
+    v[4] = b.x;
+    v[5] = b.y;
+    v[6] = b.z;
+    v[7] = b.w;
+}
+__device__ __forceinline__ void load8(const double *__restrict__ p, double v[8]) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = p[i];
+}
+
 __device__ __forceinline__ int64_t qsearch(const double *__restrict__ rv, int64_t n, double d, double inv_dr) {
     double gf = d * inv_dr;
     int64_t g = gf < 0 ? 0 : (gf > (double)(n - 1) ? n - 1 : (int64_t)gf);
@@ -269,7 +419,7 @@ __device__ __forceinline__ int64_t qsearch(const double *__restrict__ rv, int64_
     return lo;
 }
 
-// coef[p][9] = (A, B, C, D, E, F, G, H, I) interpolated at the pair separation.
+// coef[9][np] = (A, B, C, D, E, F, G, H, I) interpolated at the pair separations.
 __global__ void k_quad_pair_coefs(const double *__restrict__ dist, int64_t np, const double *__restrict__ perp,
                                   const double *__restrict__ para, const double *__restrict__ qt,
                                   const double *__restrict__ rv, int64_t ntab, double inv_dr,
@@ -288,38 +438,63 @@ __global__ void k_quad_pair_coefs(const double *__restrict__ dist, int64_t np, c
             for (int k = 0; k < 7; ++k) v[2 + k] = qt[k * ntab + i - 1] * u + qt[k * ntab + i] * t;
         }
         for (int k = 0; k < 9; ++k) {
-            c64[9 * p + k] = v[k];
-            if (c32) c32[9 * p + k] = (float)v[k];
+            c64[k * np + p] = v[k];
+            if (c32) c32[k * np + p] = (float)v[k];
         }
     }
 }
 
+// Float32 copy of the moments for the pair sum: a pair converts nothing (eight conversions a pair on the float64 pipe
+// had been two thirds of the float32 sum) and gathers two aligned float4 instead of eight doubles.
+__global__ void k_moments8(const double *__restrict__ m, int64_t total, float *__restrict__ m32) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
+        m32[i] = (float)m[i];
+}
+
+// mp: the moments the pairs read (T), m: those of the diagonal.  G lanes to a row, its pairs in turn; the couplings are
+// nine arrays of n_pairs, so a row's reads are contiguous.  The row's eight sums end one to a lane.  3 million pairs in
+// 50,320 rows: 79 us with the conversions, 48 so (memory bound at 26; a warp to a row took 66).
 template <typename T, int G>
-__global__ void __launch_bounds__(256) k_rs_quad(const double *__restrict__ m, double *__restrict__ out, int64_t n,
-                                                 int nrhs, const int64_t *__restrict__ row_ptr,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_rs_quad(const double *__restrict__ m, const T *__restrict__ mp,
+                                                 double *__restrict__ out, int64_t n,
+                                                 int nrhs, int64_t np, const int64_t *__restrict__ row_ptr,
                                                  const int32_t *__restrict__ nbr, const T *__restrict__ rxs,
                                                  const T *__restrict__ rys, const T *__restrict__ rzs,
                                                  const T *__restrict__ coef, const double *__restrict__ diagS,
                                                  const double *__restrict__ diagQ,
                                                  const int32_t *__restrict__ diag_of_rhs) {
     const int lane = threadIdx.x % G;
+    const int oc = warp_sums_index<8, G / 2>(lane);
     const int64_t grp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
     const int64_t ngrp = ((int64_t)gridDim.x * blockDim.x) / G;
-    for (int64_t t = grp; t < n * nrhs; t += ngrp) {
-        const int64_t a = t % n;
-        const int r = (int)(t / n);
+    // every lane of a warp walks its rows the same number of times: the sums at the end take all of them
+    const int64_t trips = (n * nrhs + ngrp - 1) / ngrp;
+    for (int64_t it = 0; it < trips; ++it) {
+        const int64_t t = it * ngrp + grp;
+        const bool on = t < n * nrhs;
+        const int64_t a = on ? t % n : 0;
+        const int r = on ? (int)(t / n) : 0;
         T acc[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) acc[c] = (T)0;
-        for (int64_t e = row_ptr[a] + lane; e < row_ptr[a + 1]; e += G) {
-            const int32_t b = nbr[e];
+        const int64_t e1 = on ? row_ptr[a + 1] : 0;
+        int64_t e = on ? row_ptr[a] + lane : 0;
+        int32_t next = e < e1 ? nbr[e] : 0;
+        // what the row's end takes, loaded before its pairs
+        const bool wr = on && oc >= 0;
+        const int64_t di0 = (int64_t)(diag_of_rhs && on ? diag_of_rhs[r] : 0) * n + a, o = ((int64_t)r * n + a) * 8 + oc;
+        const double d = wr ? (oc < 3 ? diagS[di0] : diagQ[di0]) : 0.0, mo = wr ? m[o] : 0.0, prev = wr ? out[o] : 0.0;
+        for (; e < e1; e += G) {
+            const int32_t b = next;
+            next = e + G < e1 ? nbr[e + G] : 0;   // the neighbour's moments wait for its id only once a row
             const T rx = rxs[e], ry = rys[e], rz = rzs[e];
-            const T *cf = coef + 9 * e;
-            const T A = cf[0], B = cf[1], Cc = cf[2], D = cf[3], E = cf[4], F = cf[5], Gg = cf[6], H = cf[7],
-                    I = cf[8];
-            const double *mb = m + ((int64_t)r * n + b) * 8;
-            const T Sx = (T)mb[0], Sy = (T)mb[1], Sz = (T)mb[2];
-            const T Q0 = (T)mb[3], Q1 = (T)mb[4], Q2 = (T)mb[5], Q3 = (T)mb[6], Q4 = (T)mb[7];
+            const T *cf = coef + e;
+            const T A = cf[0], B = cf[np], Cc = cf[2 * np], D = cf[3 * np], E = cf[4 * np], F = cf[5 * np],
+                    Gg = cf[6 * np], H = cf[7 * np], I = cf[8 * np];
+            T mb[8];
+            load8(mp + ((int64_t)r * n + b) * 8, mb);
+            const T Sx = mb[0], Sy = mb[1], Sz = mb[2];
+            const T Q0 = mb[3], Q1 = mb[4], Q2 = mb[5], Q3 = mb[6], Q4 = mb[7];
             const T sr = Sx * rx + Sy * ry + Sz * rz;
             const T Qr0 = Q0 * rx + Q1 * ry + Q2 * rz;
             const T Qr1 = Q1 * rx + Q3 * ry + Q4 * rz;
@@ -346,18 +521,8 @@ __global__ void __launch_bounds__(256) k_rs_quad(const double *__restrict__ m, d
                 acc[3 + k] += v;
             }
         }
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-#pragma unroll
-            for (int o = G / 2; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o, G);
-        if (lane == 0) {
-            const int64_t di0 = (int64_t)(diag_of_rhs ? diag_of_rhs[r] : 0) * n + a;
-            const double ds = diagS[di0], dq = diagQ[di0];
-            const double *ma = m + ((int64_t)r * n + a) * 8;
-            double *o = out + ((int64_t)r * n + a) * 8;
-            for (int c = 0; c < 3; ++c) o[c] += ds * ma[c] + (double)acc[c];
-            for (int c = 3; c < 8; ++c) o[c] += dq * ma[c] + (double)acc[c];
-        }
+        const T v = warp_sums<8, G / 2>(acc, lane);
+        if (wr) out[o] = prev + (d * mo + to_double(v));
     }
 }
 
@@ -388,6 +553,32 @@ int contract_gen(const T *grid, int64_t n, int nrhs, int ncomp, const int32_t *s
     return MPS_OK;
 }
 
+// The staging costs so much a block, the gather so much a particle; on 96^3 with P = 6 (10) 33 us and 0.53 a thousand
+// particles (87 and 1.8) against 1.8 (5.0) a thousand: even at 16 particles a block.
+bool contract_home8_pays(const GridParams &gp, int64_t n) {
+    if (gp.P > kMaxP) return false;
+    int64_t blocks = 1;
+    for (int d = 0; d < 3; ++d) {
+        if (gp.N[d] < kHomeBlock || gp.N[d] < gp.P) return false;
+        blocks *= (gp.N[d] + kHomeBlock - 1) / kHomeBlock;
+    }
+    return n >= 16 * blocks;
+}
+
+int contract_home8(const float *grid, int64_t n, int nrhs, const int32_t *start, const float *w, const GridParams &gp,
+                   const TileBins &tb, double *out, cudaStream_t s) {
+    if (!tb.has_home) return MPS_BAD_ARG;
+    const int R = kHomeBlock + gp.P - 1;
+    const size_t smem = sizeof(float4) * (size_t)R * R * (R + 1) + sizeof(float) * (size_t)kHome8Chunk * 3 * gp.P +
+                        sizeof(int) * 2 * kHome8Chunk;
+    if (smem > 48 * 1024)
+        MPS_CUDA_TRY(cudaFuncSetAttribute(k_contract_home8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_contract_home8<<<dim3((unsigned)tb.nhome, 2 * nrhs), kHome8Warps * 32, smem, s>>>(
+        grid, n, tb.hstart, tb.hentries, tb.nhb[0], tb.nhb[1], start, w, gp, out);
+    MPS_LAUNCH_CHECK();
+    return MPS_OK;
+}
+
 int quad_diag(const double *lam, int64_t total, const double *gq2, double *diag, cudaStream_t s) {
     double self_q = 0.0;
     MPS_CUDA_TRY(cudaMemcpyAsync(&self_q, gq2, sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -398,8 +589,7 @@ int quad_diag(const double *lam, int64_t total, const double *gq2, double *diag,
 }
 
 int quad_kcoef(const GridParams &gp, double *c64, float *c32, cudaStream_t s) {
-    const int64_t Gc = (int64_t)(gp.N[0] / 2 + 1) * gp.N[1] * gp.N[2];
-    k_quad_kcoef<<<grid_for(Gc, 256), 256, 0, s>>>(gp, c64, c32);
+    k_quad_kcoef<<<grid_for(HalfQuarter(gp.N).size(), 128), 128, 0, s>>>(gp, c64, (float4 *)c32);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
 }
@@ -425,12 +615,21 @@ int quad_pair_coefs(const double *dist, int64_t np, const double *perp, const do
 }
 
 template <typename T>
-int real_space_quad(const double *m, double *out, int64_t n, int nrhs, const int64_t *row_ptr, const int32_t *nbr,
-                    const T *rx, const T *ry, const T *rz, const T *coef, const double *diagS, const double *diagQ,
-                    const int32_t *diag_of_rhs, cudaStream_t s) {
+int real_space_quad(const double *m, float *m32, double *out, int64_t n, int nrhs, const int64_t *row_ptr, int64_t np,
+                    const int32_t *nbr, const T *rx, const T *ry, const T *rz, const T *coef, const double *diagS,
+                    const double *diagQ, const int32_t *diag_of_rhs, cudaStream_t s) {
+    const T *mp;
+    if constexpr (sizeof(T) == 4) {
+        const int64_t total = 8 * n * nrhs;
+        k_moments8<<<grid_for(total, 256), 256, 0, s>>>(m, total, m32);
+        MPS_LAUNCH_CHECK();
+        mp = m32;
+    } else {
+        mp = m;
+    }
     constexpr int G = 8;
-    k_rs_quad<T, G><<<grid_for(n * nrhs * G, 256, 152 * 64), 256, 0, s>>>(m, out, n, nrhs, row_ptr, nbr, rx, ry, rz,
-                                                                          coef, diagS, diagQ, diag_of_rhs);
+    k_rs_quad<T, G><<<grid_for(n * nrhs * G, 256, 152 * 64), 256, 0, s>>>(m, mp, out, n, nrhs, np, row_ptr, nbr, rx, ry,
+                                                                          rz, coef, diagS, diagQ, diag_of_rhs);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
 }
@@ -445,11 +644,11 @@ template int contract_gen<double>(const double *, int64_t, int, int, const int32
                                   const GridParams &, double *, cudaStream_t);
 template int scale_quad<float>(void *, int, const GridParams &, const float *, cudaStream_t);
 template int scale_quad<double>(void *, int, const GridParams &, const double *, cudaStream_t);
-template int real_space_quad<float>(const double *, double *, int64_t, int, const int64_t *, const int32_t *,
-                                    const float *, const float *, const float *, const float *, const double *,
-                                    const double *, const int32_t *, cudaStream_t);
-template int real_space_quad<double>(const double *, double *, int64_t, int, const int64_t *, const int32_t *,
-                                     const double *, const double *, const double *, const double *, const double *,
-                                     const double *, const int32_t *, cudaStream_t);
+template int real_space_quad<float>(const double *, float *, double *, int64_t, int, const int64_t *, int64_t,
+                                    const int32_t *, const float *, const float *, const float *, const float *,
+                                    const double *, const double *, const int32_t *, cudaStream_t);
+template int real_space_quad<double>(const double *, float *, double *, int64_t, int, const int64_t *, int64_t,
+                                     const int32_t *, const double *, const double *, const double *, const double *,
+                                     const double *, const double *, const int32_t *, cudaStream_t);
 
 }  // namespace mps

@@ -162,11 +162,11 @@ struct mps_system {
     // gradient/quadrupole diagonal
     int kind = 0;
     int ndof = 3;
-    double *qcoef = nullptr;        // n_pairs x 9 (A..I) float64
+    double *qcoef = nullptr;        // 9 x n_pairs (A..I) float64
     float *qcoef32 = nullptr;
     double *diagq = nullptr;        // n_diag x n: 15/(8 pi (eps-1)) + grad_quad_2(0)/2
     double *qkcoef = nullptr;       // half spectrum x 4: HES, HEQ/i, HGS/i, HGQ (with 1/G)
-    float *qkcoef32 = nullptr;
+    float *qkcoef32 = nullptr;      // half spectrum x 8: the same and the unit wave vector
     // polydisperse operator (kind 2): one scalar grid per vector, kernel values
     // K(d)/d of every particle's stencil, base offset node0 h - x per particle
     double *cs_base = nullptr;      // n x 3
@@ -688,7 +688,9 @@ static int ensure_tiles(mps_system *s, int use, cudaStream_t st, bool *used) {
 // Tiles of the node spread, built once where the grid and the support allow it.
 static int ensure_nodes(mps_system *s, cudaStream_t st, bool *used) {
     *used = nodes_supported(s->gp);
-    if (*used && !s->tbn.mem) MPS_TRY(node_bins_build(s->start, s->n, s->gp, s->max_rhs, s->tbn, st));
+    // blocks to a tile: three vectors share one, a vector of dipole and quadrupole moments takes one
+    const int groups = s->kind == MPS_DIPOLE_QUADRUPOLE ? s->max_rhs : (s->max_rhs + 2) / 3;
+    if (*used && !s->tbn.mem) MPS_TRY(node_bins_build(s->start, s->n, s->gp, groups, s->tbn, st));
     return MPS_OK;
 }
 
@@ -957,6 +959,11 @@ static bool df_usable(mps_system *s) {
 template <typename T>
 static int matvec_quad(mps_system *s, const double *m, double *out, int nrhs, cudaStream_t st) {
     const bool dbl = sizeof(T) == 8;
+    bool nodes = false;
+    MPS_TRY(ensure_nodes(s, st, &nodes));
+    const bool home = !dbl && nodes && contract_home8_pays(s->gp, s->n);
+    if (home) MPS_TRY(tile_bins_home(s->start, s->n, s->gp, s->tbn, st));
+    if (!dbl && !s->m32) MPS_TRY(dalloc(&s->m32, sizeof(float) * 8 * (size_t)s->n * s->max_rhs, st));
     MPS_TRY(ensure_grids(s, dbl ? MPS_FP64 : MPS_FP32, st));
     T *grid = dbl ? (T *)s->grid64 : (T *)s->grid32;
     void *spec = dbl ? s->spec64 : s->spec32;
@@ -967,7 +974,10 @@ static int matvec_quad(mps_system *s, const double *m, double *out, int nrhs, cu
     StageEvents *ev = nullptr;
     MPS_TRY(stage_begin(s, dbl ? MPS_FP64 : MPS_FP32, &ev, st));
     STAGE_MARK(1);
-    MPS_TRY(spread_gen<T>(m, s->n, nrhs, 8, s->start, w, s->gp, grid, st));
+    if (nodes)
+        MPS_TRY(spread_nodes8<T>(m, s->n, nrhs, s->start, w, s->gp, s->tbn, grid, st));
+    else
+        MPS_TRY(spread_gen<T>(m, s->n, nrhs, 8, s->start, w, s->gp, grid, st));
     STAGE_MARK(2);
     MPS_TRY(exec_plan(s, dbl ? CUFFT_D2Z : CUFFT_R2C, 8 * nrhs, grid, spec, 0, st));
     STAGE_MARK(3);
@@ -975,10 +985,13 @@ static int matvec_quad(mps_system *s, const double *m, double *out, int nrhs, cu
     STAGE_MARK(4);
     MPS_TRY(exec_plan(s, dbl ? CUFFT_Z2D : CUFFT_C2R, 8 * nrhs, spec, grid, 0, st));
     STAGE_MARK(5);
-    MPS_TRY(contract_gen<T>(grid, s->n, nrhs, 8, s->start, w, s->gp, out, st));
+    if (home)
+        MPS_TRY(contract_home8((const float *)grid, s->n, nrhs, s->start, (const float *)w, s->gp, s->tbn, out, st));
+    else
+        MPS_TRY(contract_gen<T>(grid, s->n, nrhs, 8, s->start, w, s->gp, out, st));
     STAGE_MARK(6);
-    MPS_TRY(real_space_quad<T>(m, out, s->n, nrhs, s->row_ptr, pd.nbr, pd.rx, pd.ry, pd.rz, pc, s->diag, s->diagq,
-                               s->diag_idx, st));
+    MPS_TRY(real_space_quad<T>(m, s->m32, out, s->n, nrhs, s->row_ptr, s->n_pairs, pd.nbr, pd.rx, pd.ry, pd.rz, pc,
+                               s->diag, s->diagq, s->diag_idx, st));
     STAGE_MARK(7);
     return MPS_OK;
 }
@@ -2754,7 +2767,7 @@ extern "C" int mps_system_create(const mps_system_desc *d, mps_system **out, mps
         if (!rc) rc = dalloc(&s->diagq, sizeof(double) * n * d->n_diag, st);
         if (!rc) rc = quad_diag(d->lambdap, n * d->n_diag, d->quad_tables + 4 * d->n_tab, s->diagq, st);
         if (!rc) rc = dalloc(&s->qkcoef, sizeof(double) * 4 * s->Gc, st);
-        if (!rc) rc = dalloc(&s->qkcoef32, sizeof(float) * 4 * s->Gc, st);
+        if (!rc) rc = dalloc(&s->qkcoef32, sizeof(float) * 8 * s->Gc, st);
         if (!rc) rc = quad_kcoef(s->gp, s->qkcoef, s->qkcoef32, st);
     }
     if (rc) {

@@ -452,29 +452,30 @@ __global__ void __launch_bounds__(256) k_spread_tiled(const double *__restrict__
 // from shared memory costs as much; there a lane takes two nodes along z at once, with one list for both (11 of 10
 // planes) and one read.  Measured against the tiled double-float spread: one vector, N = 200,000, 240^3, P = 10
 // 1165 -> 646 us; one vector, N = 8228 in half of a 60 x 72 x 160 grid, P = 8 65 -> 28 us.
+// Float32 moments of eight components (dipole and quadrupole) take pairs of nodes too; against float atomics from a warp a
+// particle, N = 50,320, 90 x 90 x 96, P = 6: 118 us and the zeroing -> 54 us.
 constexpr int kNodeTile = 8;
 constexpr int kNodeChunk = 96;      // 3 mask words
 constexpr int kNodeWords = kNodeChunk / 32;
 
 // Depth 8 (two nodes a thread) unless that leaves fewer than two blocks for every SM, then 4 (one node a thread: there
-// the length of a lane's list is the time a block takes).
-static int node_tile_depth(const GridParams &gp, int nrhs) {
+// the length of a lane's list is the time a block takes).  groups: blocks to a tile.
+static int node_tile_depth(const GridParams &gp, int groups) {
     const int64_t nxy = (int64_t)((gp.N[0] + kNodeTile - 1) / kNodeTile) * ((gp.N[1] + kNodeTile - 1) / kNodeTile);
-    return nxy * ((gp.N[2] + 7) / 8) * ((nrhs + 2) / 3) >= 304 ? 8 : 4;
+    return nxy * ((gp.N[2] + 7) / 8) * groups >= 304 ? 8 : 4;
 }
 
 bool nodes_supported(const GridParams &gp) {
     return gp.P >= 1 && gp.P <= kMaxP && gp.N[0] >= kNodeTile && gp.N[1] >= kNodeTile && gp.N[2] >= kNodeTile;
 }
 
-int node_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int nrhs, TileBins &tb, cudaStream_t s) {
+int node_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int groups, TileBins &tb, cudaStream_t s) {
     if (!nodes_supported(gp) || n < 1) return MPS_BAD_ARG;
-    return bins_build(start, n, gp, kNodeTile, kNodeTile, node_tile_depth(gp, nrhs), tb, s);
+    return bins_build(start, n, gp, kNodeTile, kNodeTile, node_tile_depth(gp, groups), tb, s);
 }
 
-template <typename T, int NR, int TZ>
+template <typename T, int C, int TZ>
 struct NodeStage {
-    static constexpr int C = 3 * NR;
     T mwx[kNodeChunk][kNodeTile * C + 1];           // m_c wx at the tile's columns (odd stride: no bank conflicts)
     T wyz[kNodeChunk][kNodeTile + TZ + 1];          // wy at its rows, wz at its planes
     unsigned mask[kNodeWords][2 * kNodeTile + TZ];  // particles that reach a column, row, plane
@@ -482,17 +483,19 @@ struct NodeStage {
 
 constexpr int kNodeThreads = 256;
 
-template <typename T, int NR, int TZ>
-__global__ void __launch_bounds__(kNodeThreads) k_spread_nodes(const double *__restrict__ m, int64_t n, int rfirst,
+// NR vectors of NC components each to a block.
+template <typename T, int NR, int TZ, int NC>
+__global__ void __launch_bounds__(kNodeThreads, std::is_same<T, float>::value ? 4 : 1) k_spread_nodes(const double *__restrict__ m, int64_t n, int rfirst,
                                                           const int32_t *__restrict__ start,
                                                           const T *__restrict__ w, GridParams gp,
                                                           const int64_t *__restrict__ tstart,
                                                           const int32_t *__restrict__ entries, int ntx, int nty,
                                                           T *__restrict__ grid) {
-    constexpr int C = 3 * NR, NQ = TZ / 4;
-    constexpr bool PAIR = std::is_same<T, dfv>::value && NQ == 2;   // a lane's two nodes share a list
+    constexpr int C = NC * NR, NQ = TZ / 4;
+    constexpr bool PAIR = (std::is_same<T, dfv>::value || std::is_same<T, float>::value) && NQ == 2;   // a lane's two
+                                                                                                       // nodes share a list
     extern __shared__ __align__(16) unsigned char smem_nodes[];
-    NodeStage<T, NR, TZ> &st = *reinterpret_cast<NodeStage<T, NR, TZ> *>(smem_nodes);
+    NodeStage<T, C, TZ> &st = *reinterpret_cast<NodeStage<T, C, TZ> *>(smem_nodes);
     const int r0 = rfirst + NR * (int)blockIdx.y;
     const int64_t t = blockIdx.x;
     const int X0 = (int)(t % ntx) * kNodeTile, Y0 = (int)((t / ntx) % nty) * kNodeTile,
@@ -517,6 +520,10 @@ __global__ void __launch_bounds__(kNodeThreads) k_spread_nodes(const double *__r
             const int word = task / 3, d = task - 3 * word, pp = 32 * word + lane;
             const int origin = d == 0 ? X0 : (d == 1 ? Y0 : Z0), Nd = d == 0 ? Nx : (d == 1 ? Ny : Nz);
             const int len = d == 2 ? TZ : kNodeTile;
+            if (32 * word >= cnt) {   // no particle left for this word
+                if (lane < len) st.mask[word][d * kNodeTile + lane] = 0u;
+                continue;
+            }
             const bool in = pp < cnt;
             const int32_t a = in ? entries[cb + pp] : 0;
             int j = in ? origin - start[3 * (int64_t)a + d] : 0;   // stencil index of the tile's first node
@@ -535,7 +542,8 @@ __global__ void __launch_bounds__(kNodeThreads) k_spread_nodes(const double *__r
 #pragma unroll
                 for (int r = 0; r < NR; ++r)
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) mv[3 * r + c] = in ? (T)m[((int64_t)(r0 + r) * n + a) * 3 + c] : (T)0;
+                    for (int c = 0; c < NC; ++c)
+                        mv[NC * r + c] = in ? (T)m[((int64_t)(r0 + r) * n + a) * NC + c] : (T)0;
             }
 #pragma unroll
             for (int k = 0; k < kNodeTile; ++k) {
@@ -600,7 +608,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_spread_nodes(const double *__r
         for (int q = 0; q < NQ; ++q) {
             const int gz = Z0 + zb + ZQ * q;
             if (gz < Nz) {
-                T *g = grid + (int64_t)3 * r0 * gp.G + ((int64_t)gz * Ny + Y0 + y) * Nx + X0 + x;
+                T *g = grid + (int64_t)NC * r0 * gp.G + ((int64_t)gz * Ny + Y0 + y) * Nx + X0 + x;
 #pragma unroll
                 for (int c = 0; c < C; ++c) g[c * gp.G] = acc[q][c].get();
             }
@@ -608,14 +616,14 @@ __global__ void __launch_bounds__(kNodeThreads) k_spread_nodes(const double *__r
     }
 }
 
-template <typename T, int NR, int TZ>
+template <typename T, int NR, int TZ, int NC = 3>
 static int nodes_launch(const double *m, int64_t n, int r0, int groups, const int32_t *start, const T *w,
                         const GridParams &gp, const TileBins &tb, T *grid, cudaStream_t s) {
-    const size_t smem = sizeof(NodeStage<T, NR, TZ>);
+    const size_t smem = sizeof(NodeStage<T, NC * NR, TZ>);
     if (smem > 48 * 1024)
-        MPS_CUDA_TRY(cudaFuncSetAttribute(k_spread_nodes<T, NR, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        MPS_CUDA_TRY(cudaFuncSetAttribute(k_spread_nodes<T, NR, TZ, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
-    k_spread_nodes<T, NR, TZ><<<dim3((unsigned)tb.ntiles, groups), kNodeThreads, smem, s>>>(
+    k_spread_nodes<T, NR, TZ, NC><<<dim3((unsigned)tb.ntiles, groups), kNodeThreads, smem, s>>>(
         m, n, r0, start, w, gp, tb.tile_start, tb.entries, tb.ntx, tb.nty, grid);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
@@ -641,6 +649,20 @@ int spread_nodes(const double *m, int64_t n, int nrhs, const int32_t *start, con
     return MPS_BAD_ARG;
 }
 
+// Dipole and quadrupole moments: eight components to a vector, one vector to a block.
+template <typename T>
+int spread_nodes8(const double *m, int64_t n, int nrhs, const int32_t *start, const T *w, const GridParams &gp,
+                  const TileBins &tb, T *grid, cudaStream_t s) {
+    if (tb.tx != kNodeTile || tb.ty != kNodeTile) return MPS_BAD_ARG;
+    if (tb.tz == 8) return nodes_launch<T, 1, 8, 8>(m, n, 0, nrhs, start, w, gp, tb, grid, s);
+    if (tb.tz == 4) return nodes_launch<T, 1, 4, 8>(m, n, 0, nrhs, start, w, gp, tb, grid, s);
+    return MPS_BAD_ARG;
+}
+
+template int spread_nodes8<float>(const double *, int64_t, int, const int32_t *, const float *, const GridParams &,
+                                  const TileBins &, float *, cudaStream_t);
+template int spread_nodes8<double>(const double *, int64_t, int, const int32_t *, const double *, const GridParams &,
+                                   const TileBins &, double *, cudaStream_t);
 template int spread_nodes<double>(const double *, int64_t, int, const int32_t *, const double *, const GridParams &,
                                   const TileBins &, double *, cudaStream_t);
 template int spread_nodes<dfv>(const double *, int64_t, int, const int32_t *, const dfv *, const GridParams &,

@@ -38,8 +38,8 @@ constexpr int kHomeBlock = 8;
 
 bool tiles_supported(const GridParams &gp, int tz);
 int tile_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tz, TileBins &tb, cudaStream_t s);
-// Bins for spread_nodes: 8 x 8 tiles of the depth that node_tile_depth gives.
-int node_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int nrhs, TileBins &tb, cudaStream_t s);
+// Bins for spread_nodes and spread_nodes8: 8 x 8 tiles, of depth 8 or 4 by the number of blocks (groups to a tile).
+int node_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int groups, TileBins &tb, cudaStream_t s);
 bool nodes_supported(const GridParams &gp);
 // Fills tb.pentry (once) for the gathers of the tiled contractions.
 int tile_bins_pentry(const int32_t *start, const GridParams &gp, TileBins &tb, cudaStream_t s);
@@ -57,6 +57,11 @@ int spread_tiled(const double *m, int64_t n, int nrhs, const int32_t *start, con
 template <typename T>
 int spread_nodes(const double *m, int64_t n, int nrhs, const int32_t *start, const T *w, const GridParams &gp,
                  const TileBins &tb, T *grid, cudaStream_t s);
+
+// Eight components a vector (m [r][a][8], grid[(r*8+c)][G]).
+template <typename T>
+int spread_nodes8(const double *m, int64_t n, int nrhs, const int32_t *start, const T *w, const GridParams &gp,
+                  const TileBins &tb, T *grid, cudaStream_t s);
 
 // out[r][a][c] = hprod * sum over the stencil (overwrites); partial: nentries * 3 * min(nrhs,3) of T.
 template <typename T>
