@@ -400,7 +400,8 @@ __global__ void __launch_bounds__(256, 3) k_contract_grad_warp(const float *__re
 // With one vector a CTA takes 2 x 2 home blocks (5.2 stagings a node): 0.256 -> 0.156 ms for N = 2e5 on 240^3, with the
 // region staged row by row (the wraps worked out once a row, not once a node).  The sums end one to a lane, converted and
 // scaled together: lane 0's 3 NR conversions and multiplications had cost a warp 6 NR float64 instructions a particle
-// (0.209 -> 0.174 ms for N = 1e5, three vectors, 192^3; 0.155 -> 0.144 for N = 2e5, one vector, 240^3).
+// (0.209 -> 0.174 ms for N = 1e5, three vectors, 192^3; 0.155 -> 0.144 for N = 2e5, one vector, 240^3; 0.168 and 0.136
+// with the staging copies asynchronous).
 // 67 KB of shared memory at P = 10 and 3 vectors, 3 blocks per SM (80 registers): the mixed step at the bench
 // workload took 19.25 ms against 20.08 with the warp gather; float4 nodes (the 3 vectors interleaved, 87 KB,
 // 2 blocks per SM) took 20.17.
@@ -469,12 +470,11 @@ __global__ void __launch_bounds__(256, NR == 1 ? 4 : 3) k_contract_grad_home(
     {
         const int x = lane % LX, gx = wrap2(X0 + x, Nx);
         if (x < RX) {
-#pragma unroll 4
             for (int row = wid * ROWS + lane / LX; row < RY * RZ; row += 8 * ROWS) {
                 const int z = row / RY, y = row - z * RY;
                 const float *src = g0 + ((int64_t)wrap2(Z0 + z, Nz) * Ny + wrap2(Y0 + y, Ny)) * Nx + gx;
 #pragma unroll
-                for (int r = 0; r < NR; ++r) s_reg[r * VOL + row * RX + x] = __ldg(src + r * G);
+                for (int r = 0; r < NR; ++r) copy_async(s_reg + r * VOL + row * RX + x, src + r * G);
             }
         }
         if (RX > LX) {
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(256, NR == 1 ? 4 : 3) k_contract_grad_home(
                 const int z = row / RY, y = row - z * RY;
                 const float *src = g0 + ((int64_t)wrap2(Z0 + z, Nz) * Ny + wrap2(Y0 + y, Ny)) * Nx + gl;
 #pragma unroll
-                for (int r = 0; r < NR; ++r) s_reg[r * VOL + row * RX + LX] = __ldg(src + r * G);
+                for (int r = 0; r < NR; ++r) copy_async(s_reg + r * VOL + row * RX + LX, src + r * G);
             }
         }
     }
@@ -503,6 +503,7 @@ __global__ void __launch_bounds__(256, NR == 1 ? 4 : 3) k_contract_grad_home(
             s_p[4 * threadIdx.x + 2] = start[3 * a + 2] - Z0;
             s_p[4 * threadIdx.x + 3] = (int)a;
         }
+        copy_async_wait();
         __syncthreads();   // the region (first pass) and this chunk's particle data are in place
         for (int pp = wid; pp < cnt; pp += 8) {
             const int ox = s_p[4 * pp], oy = s_p[4 * pp + 1], oz = s_p[4 * pp + 2];
