@@ -296,13 +296,16 @@ __global__ void __launch_bounds__(256, MB) k_spread_cs(const double *__restrict_
         const int r0 = (int)(t / n) * RB;
         const int cnt = min(RB, nrhs - r0);
         const int sx = start[3 * a], sy = start[3 * a + 1], sz = start[3 * a + 2];
+        // a lane loads (and converts) one component, shuffles hand them round
+        static_assert(3 * RB <= 32, "a lane a component");
+        const int lq = lane / 3;
+        const T mv = lq < cnt ? (T)m[((int64_t)(r0 + lq) * n + a) * 3 + lane - 3 * lq] : (T)0;
         T px[RB], py[RB], pz[RB];
 #pragma unroll
         for (int q = 0; q < RB; ++q) {
-            const double *ma = m + ((int64_t)(r0 + (q < cnt ? q : 0)) * n + a) * 3;
-            px[q] = (T)ma[0];
-            py[q] = (T)ma[1];
-            pz[q] = (T)ma[2];
+            px[q] = __shfl_sync(0xffffffffu, mv, 3 * q);
+            py[q] = __shfl_sync(0xffffffffu, mv, 3 * q + 1);
+            pz[q] = __shfl_sync(0xffffffffu, mv, 3 * q + 2);
         }
         const T bx = (T)(base[3 * a] - lo * gp.h[0]), by = (T)(base[3 * a + 1] - lo * gp.h[1]),
                 bz = (T)(base[3 * a + 2] - lo * gp.h[2]);
@@ -380,6 +383,7 @@ __global__ void __launch_bounds__(256, MB) k_contract_cs(const T *__restrict__ g
     const int Nx = gp.N[0], Ny = gp.N[1], Nz = gp.N[2];
     const int64_t P3 = (int64_t)P * P * P;
     const int nblk = (nrhs + RB - 1) / RB;
+    const int oc = warp_sums_index<3 * RB>(lane);   // the sum this lane writes
     for (int64_t t = warp; t < n * nblk; t += nw) {
         const int64_t a = gp.order ? (int64_t)gp.order[t % n] : t % n;
         const int r0 = (int)(t / n) * RB;
@@ -390,9 +394,9 @@ __global__ void __launch_bounds__(256, MB) k_contract_cs(const T *__restrict__ g
         const T hx = (T)gp.h[0], hy = (T)gp.h[1], hz = (T)gp.h[2];
         const T *ga = g + a * P3;
         const T *gr = grid + (int64_t)r0 * gp.G;
-        T ax[RB], ay[RB], az[RB];
+        T acc[3 * RB];
 #pragma unroll
-        for (int q = 0; q < RB; ++q) ax[q] = ay[q] = az[q] = 0;
+        for (int q = 0; q < 3 * RB; ++q) acc[q] = 0;
         for (int row0 = 0; row0 < P * P; row0 += 32) {
             int idx, sub, lpp;
             if (!stencil_row(row0, P, lane, &idx, &sub, &lpp)) continue;
@@ -410,34 +414,277 @@ __global__ void __launch_bounds__(256, MB) k_contract_cs(const T *__restrict__ g
                 int iz = sz + jz;
                 if (iz >= Nz) iz -= Nz;
                 const T wv = ga[jx + P * (jy + P * jz)];
-                const T rz = bz + (T)jz * hz;
+                const T wz = wv * (bz + (T)jz * hz);
                 const T *node = gr + rowb + (int64_t)Nx * Ny * iz;
 #pragma unroll
                 for (int q = 0; q < RB; ++q) {
                     if (q < cnt) {
-                        const T v = wv * node[(int64_t)q * gp.G];
-                        sxy[q] += v;
-                        szz[q] += v * rz;
+                        const T v = node[(int64_t)q * gp.G];
+                        sxy[q] += wv * v;
+                        szz[q] += wz * v;
                     }
                 }
             }
 #pragma unroll
             for (int q = 0; q < RB; ++q) {
-                ax[q] += rx * sxy[q];
-                ay[q] += ry * sxy[q];
-                az[q] += szz[q];
+                acc[3 * q] += rx * sxy[q];
+                acc[3 * q + 1] += ry * sxy[q];
+                acc[3 * q + 2] += szz[q];
             }
         }
+        const T v = warp_sums(acc, lane);
+        if (oc >= 0 && oc < 3 * cnt) out[((int64_t)(r0 + oc / 3) * n + a) * 3 + oc % 3] = (double)v * gp.hprod;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Many vectors (a spectrum or sweep batch).
+//
+// Spread: a block owns an 8 x 4 x 2 tile of nodes and walks the particles whose stencils reach it (TileBins), 32 at a time
+// with their moments in shared memory; a warp owns a row of 8 nodes, four lanes to a node, and takes the particles that
+// reach its row (a ballot) one after the other: one weight K(d)/d a node serves 16 vectors a group, V groups to a block.
+// Every node is written once, in the planes that the transforms read, in a fixed order of sums: no atomics, no zeroing.
+// 48 vectors, 3,000 spheres, 40^3, P = 8: 87 us with float atomics from a warp a particle (78 with four-vector atomics on
+// interleaved grids), 54 so; a lane keeps two nodes along z (one: 73), the moments read from shared
+// memory being what bounds it.
+//
+// Contraction: the grids lie side by side, node by node, four vectors to a float4.  From planes, a warp touched a line in
+// L1 for every vector and row of the stencil; here four lanes take a node's 16 vectors (64 contiguous bytes), eight nodes
+// of the stencil at a time, the weights are read once for all 16, and no sum crosses more than eight lanes.  103 -> 50 us,
+// the L2's bandwidth, and 7 us for the transposition.
+// ---------------------------------------------------------------------------
+constexpr int kCsGroup = 16;
+constexpr int kCsTileX = 8, kCsTileY = 4, kCsTileZ = 4, kCsChunk = 32;
+
+// mv[a][axis][v] = m[v][a][axis], v < 4 vq (zeros beyond nrhs).
+__global__ void k_cs_moments(const double *__restrict__ m, int64_t n, int nrhs, int vq, float *__restrict__ mv) {
+    const int64_t total = n * 12 * vq;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t a3 = t / (4 * vq);   // 3 a + axis
+        const int v = (int)(t - a3 * (4 * vq));
+        mv[t] = v < nrhs ? (float)m[(int64_t)v * n * 3 + a3] : 0.f;
+    }
+}
+
+template <int V>
+__global__ void __launch_bounds__(256, 4) k_spread_cs_nodes(const float4 *__restrict__ mv, int nrhs, int vq,
+                                                         const int32_t *__restrict__ start,
+                                                         const double *__restrict__ base, const float *__restrict__ g,
+                                                         GridParams gp, const int64_t *__restrict__ tstart,
+                                                         const int32_t *__restrict__ entries, int ntx, int nty,
+                                                         float *__restrict__ grid) {
+    __shared__ float4 s_m[kCsChunk][3][4 * V];
+    __shared__ float4 s_b[kCsChunk];    // node0 - x of the stencil's first node, particle id
+    __shared__ int s_o[kCsChunk][3];    // stencil index of the tile's first node
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, lv = lane & 3, xn = lane >> 2;
+    const int64_t t = blockIdx.x;
+    const int X0 = (int)(t % ntx) * kCsTileX, Y0 = (int)((t / ntx) % nty) * kCsTileY,
+              Z0 = (int)(t / ((int64_t)ntx * nty)) * kCsTileZ;
+    const int yr = wid & (kCsTileY - 1), zr = 2 * (wid / kCsTileY);   // the warp's rows: (yr, zr) and (yr, zr + 1)
+    const int P = gp.P, lo = (P - 1) / 2;
+    const int Nx = gp.N[0], Ny = gp.N[1], Nz = gp.N[2];
+    const bool inx = X0 + xn < Nx, row_in = Y0 + yr < Ny && Z0 + zr < Nz;
+    const int q0 = (int)blockIdx.y * 4 * V;   // first float4 of the block's vectors
+    const float hx = (float)gp.h[0], hy = (float)gp.h[1], hz = (float)gp.h[2];
+    float acc[2][V][4];
 #pragma unroll
-        for (int q = 0; q < RB; ++q) {
-            const T sxq = warp_sum(ax[q]), syq = warp_sum(ay[q]), szq = warp_sum(az[q]);
-            if (lane == 0 && q < cnt) {
-                double *o = out + ((int64_t)(r0 + q) * n + a) * 3;
-                o[0] = (double)sxq * gp.hprod;
-                o[1] = (double)syq * gp.hprod;
-                o[2] = (double)szq * gp.hprod;
+    for (int v = 0; v < V; ++v)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[0][v][k] = acc[1][v][k] = 0.f;
+    const int64_t e0 = tstart[t], e1 = tstart[t + 1];
+    for (int64_t cb = e0; cb < e1; cb += kCsChunk) {
+        const int cnt = (int)min((int64_t)kCsChunk, e1 - cb);
+        // a warp copies four particles' moments; the first works out the geometry too
+        int32_t id[kCsChunk / 8];
+#pragma unroll
+        for (int k = 0; k < kCsChunk / 8; ++k) id[k] = wid + 8 * k < cnt ? entries[cb + wid + 8 * k] : -1;
+#pragma unroll
+        for (int k = 0; k < kCsChunk / 8; ++k)
+            if (id[k] >= 0)
+                for (int i = lane; i < 12 * V; i += 32) {
+                    const int c = i / (4 * V), q = i - c * (4 * V);
+                    if (q0 + q < vq)
+                        copy_async(&s_m[wid + 8 * k][c][q], mv + (3 * (int64_t)id[k] + c) * vq + q0 + q);
+                    else
+                        s_m[wid + 8 * k][c][q] = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+        if (threadIdx.x < cnt) {
+            const int32_t a = entries[cb + threadIdx.x];
+            const double *b = base + 3 * (int64_t)a;
+            s_b[threadIdx.x] = make_float4((float)(b[0] - lo * gp.h[0]), (float)(b[1] - lo * gp.h[1]),
+                                           (float)(b[2] - lo * gp.h[2]), __int_as_float(a));
+            const int32_t *sa = start + 3 * (int64_t)a;
+            s_o[threadIdx.x][0] = X0 - sa[0] + (X0 < sa[0] ? Nx : 0);
+            s_o[threadIdx.x][1] = Y0 - sa[1] + (Y0 < sa[1] ? Ny : 0);
+            s_o[threadIdx.x][2] = Z0 - sa[2] + (Z0 < sa[2] ? Nz : 0);
+        }
+        copy_async_wait();
+        __syncthreads();
+        // the chunk's particles whose stencils hold one of the rows
+        bool on = false;
+        if (lane < cnt && row_in) {
+            int jy = s_o[lane][1] + yr, jz = s_o[lane][2] + zr;
+            jy -= jy >= Ny ? Ny : 0;
+            jz -= jz >= Nz ? Nz : 0;
+            on = jy < P && (jz < P || jz == Nz - 1);   // (the second row holds the stencil's first plane)
+        }
+        unsigned list = __ballot_sync(0xffffffffu, on);
+        // four particles at a time: each of a node's lanes works out one of them, shuffles hand its weights round
+        while (list) {
+            int pk[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                pk[k] = __ffs(list) - 1;   // -1 when the list is done
+                list &= list - 1;
+            }
+            const int p = lv == 0 ? pk[0] : lv == 1 ? pk[1] : lv == 2 ? pk[2] : pk[3];
+            float wx[2] = {0.f, 0.f}, wy[2] = {0.f, 0.f}, wz[2] = {0.f, 0.f};
+            if (p >= 0) {
+                int jx = s_o[p][0] + xn, jy = s_o[p][1] + yr, jz = s_o[p][2] + zr;
+                jx -= jx >= Nx ? Nx : 0;
+                jy -= jy >= Ny ? Ny : 0;
+                jz -= jz >= Nz ? Nz : 0;
+                const float4 b = s_b[p];
+                const float *ga = g + ((int64_t)__float_as_int(b.w) * P * P + jy) * P + jx;
+                const bool in = inx && jx < P;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float wv = in && jz < P ? ga[jz * P * P] : 0.f;
+                    wx[h] = wv * (b.x + (float)jx * hx);
+                    wy[h] = wv * (b.y + (float)jy * hy);
+                    wz[h] = wv * (b.z + (float)jz * hz);
+                    if (++jz >= Nz) jz = 0;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (pk[k] < 0) break;   // the whole warp
+                const int src = (lane & 28) | k;
+                float u[2][3];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    u[h][0] = __shfl_sync(0xffffffffu, wx[h], src);
+                    u[h][1] = __shfl_sync(0xffffffffu, wy[h], src);
+                    u[h][2] = __shfl_sync(0xffffffffu, wz[h], src);
+                }
+#pragma unroll
+                for (int v = 0; v < V; ++v)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        const float4 mc = s_m[pk[k]][c][4 * v + lv];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            acc[h][v][0] += u[h][c] * mc.x;
+                            acc[h][v][1] += u[h][c] * mc.y;
+                            acc[h][v][2] += u[h][c] * mc.z;
+                            acc[h][v][3] += u[h][c] * mc.w;
+                        }
+                    }
             }
         }
+        __syncthreads();
+    }
+    if (inx && row_in) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (Z0 + zr + h >= Nz) break;
+            float *o = grid + ((int64_t)(Z0 + zr + h) * Ny + Y0 + yr) * Nx + X0 + xn;
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int r = 4 * (q0 + 4 * v + lv) + k;
+                    if (r < nrhs) o[r * gp.G] = acc[h][v][k];
+                }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256) k_contract_cs_il(const float4 *__restrict__ il, int64_t n, int nrhs, int vq,
+                                                        const int32_t *__restrict__ start,
+                                                        const double *__restrict__ base, const float *__restrict__ g,
+                                                        GridParams gp, double *__restrict__ out) {
+    const int lane = threadIdx.x & 31, lv = lane & 3, ni = lane >> 2;
+    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int P = gp.P, PP = P * P, lo = (P - 1) / 2;
+    const int Nx = gp.N[0], Ny = gp.N[1], Nz = gp.N[2];
+    const int64_t plane = (int64_t)Nx * Ny * vq;
+    const int nblk = (nrhs + kCsGroup - 1) / kCsGroup;
+    for (int64_t t = warp; t < n * nblk; t += nw) {
+        const int64_t a = gp.order ? (int64_t)gp.order[t % n] : t % n;
+        const int r0 = (int)(t / n) * kCsGroup, vec = min(r0 / 4 + lv, vq - 1);   // (surplus lanes repeat the last four)
+        const int sx = start[3 * a], sy = start[3 * a + 1], sz = start[3 * a + 2];
+        const float bx = (float)(base[3 * a] - lo * gp.h[0]), by = (float)(base[3 * a + 1] - lo * gp.h[1]),
+                    bz = (float)(base[3 * a + 2] - lo * gp.h[2]);
+        const float hx = (float)gp.h[0], hy = (float)gp.h[1], hz = (float)gp.h[2];
+        const float *ga = g + a * PP * P;
+        float acc[12];   // 3 vector + axis
+#pragma unroll
+        for (int k = 0; k < 12; ++k) acc[k] = 0.f;
+        for (int col = ni; col < PP; col += 8) {
+            const int jy = col / P, jx = col - jy * P;
+            int ix = sx + jx, iy = sy + jy;
+            if (ix >= Nx) ix -= Nx;
+            if (iy >= Ny) iy -= Ny;
+            const float rx = bx + (float)jx * hx, ry = by + (float)jy * hy;
+            const float4 *row = il + ((int64_t)ix + (int64_t)Nx * iy) * vq + vec;
+            float s[4] = {0.f, 0.f, 0.f, 0.f}, z[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+            for (int jz = 0; jz < P; ++jz) {
+                int iz = sz + jz;
+                if (iz >= Nz) iz -= Nz;
+                const float wv = ga[col + PP * jz], wz = wv * (bz + (float)jz * hz);
+                const float4 v = __ldg(row + plane * iz);
+                s[0] += wv * v.x;
+                s[1] += wv * v.y;
+                s[2] += wv * v.z;
+                s[3] += wv * v.w;
+                z[0] += wz * v.x;
+                z[1] += wz * v.y;
+                z[2] += wz * v.z;
+                z[3] += wz * v.w;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                acc[3 * k] += rx * s[k];
+                acc[3 * k + 1] += ry * s[k];
+                acc[3 * k + 2] += z[k];
+            }
+        }
+        // sums over the eight node lanes, halving what a lane carries: 12 -> 6 -> 3 -> one or two
+        const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
+        float b[6], c[3];
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+            b[k] = (h16 ? acc[k + 6] : acc[k]) + __shfl_xor_sync(0xffffffffu, h16 ? acc[k] : acc[k + 6], 16);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) c[k] = (h8 ? b[k + 3] : b[k]) + __shfl_xor_sync(0xffffffffu, h8 ? b[k] : b[k + 3], 8);
+        const float d0 = (h4 ? c[2] : c[0]) + __shfl_xor_sync(0xffffffffu, h4 ? c[0] : c[2], 4);
+        const float d1 = c[1] + __shfl_xor_sync(0xffffffffu, c[1], 4);
+        const int k0 = (h16 ? 2 : 0) + (h8 ? 1 : 0), r = r0 + 4 * lv + k0;
+        if (r < nrhs) {
+            double *o = out + ((int64_t)r * n + a) * 3;
+            o[h4 ? 2 : 0] = (double)d0 * gp.hprod;
+            if (!h4) o[1] = (double)d1 * gp.hprod;
+        }
+    }
+}
+
+// Planes to interleaved: 32 nodes and 64 vectors of them to a block, through shared memory.
+__global__ void __launch_bounds__(256) k_cs_interleave(const float *__restrict__ grid, int nrhs, int64_t G, int vq,
+                                                       float4 *__restrict__ il) {
+    __shared__ float s[64][33];
+    const int64_t t0 = (int64_t)blockIdx.x * 32;
+    const int v0 = (int)blockIdx.y * 64, lane = threadIdx.x & 31;
+    for (int v = threadIdx.x >> 5; v < 64; v += 8)
+        s[v][lane] = v0 + v < nrhs && t0 + lane < G ? grid[(int64_t)(v0 + v) * G + t0 + lane] : 0.f;
+    __syncthreads();
+    for (int e = threadIdx.x; e < 32 * 16; e += 256) {
+        const int node = e >> 4, q = e & 15;
+        if (t0 + node < G && v0 / 4 + q < vq)
+            il[(t0 + node) * vq + v0 / 4 + q] = make_float4(s[4 * q][node], s[4 * q + 1][node], s[4 * q + 2][node],
+                                                            s[4 * q + 3][node]);
     }
 }
 
@@ -447,8 +694,8 @@ __global__ void __launch_bounds__(256, MB) k_contract_cs(const T *__restrict__ g
 int cs_pair_coefs(const int64_t *row_ptr, const int32_t *nbr, const double *dist, int64_t n, const double *radius,
                   const int32_t *cls, int64_t M, const double *tab, const double *rv, int64_t ntab, double xi,
                   PairData<double> p64, PairData<float> p32, int *err, cudaStream_t s) {
-    k_cs_pair_coefs<<<grid_for(n * 32, 128), 128, 0, s>>>(row_ptr, nbr, dist, n, radius, cls, M, tab, rv, ntab, xi, p64.A,
-                                                    p64.BA, p32.A, p32.BA, err);
+    k_cs_pair_coefs<<<grid_for(n * 32, 128), 128, 0, s>>>(row_ptr, nbr, dist, n, radius, cls, M, tab, rv, ntab, xi,
+                                                         p64.A, p64.BA, p32.A, p32.BA, err);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
 }
@@ -486,6 +733,56 @@ int spread_cs(const double *m, int64_t n, int nrhs, const int32_t *start, const 
     // unbounded); double: unbounded (a 64-register cap spills it)
     constexpr int MB = sizeof(T) == 4 ? 4 : 1;
     k_spread_cs<T, 8, MB><<<grid_for(items * 32, 256, 152 * 64), 256, 0, s>>>(m, n, nrhs, start, base, g, gp, grid);
+    MPS_LAUNCH_CHECK();
+    return MPS_OK;
+}
+
+// Below a group of vectors lanes are idle; with fewer than two tiles for every SM a tile's list is the time it takes.
+// Spread and contraction by these kernels and by the others: 16 vectors, 40^3, 3,000 spheres, P = 8 62 us against 91;
+// P = 5 37 against 45; 34^3, 300 spheres 25 against 25; 48 vectors, 20^3, 400 spheres 60 against 41.
+bool cs_many(const GridParams &gp, int64_t n, int nrhs) {
+    return nrhs >= kCsGroup && n >= 1 && 3 * n <= gp.G && gp.G >= 300 * kCsTileX * kCsTileY * kCsTileZ && gp.P <= kMaxP && gp.N[0] >= kCsTileX && gp.N[1] >= kCsTileY &&
+           gp.N[2] >= kCsTileZ && gp.N[0] >= gp.P && gp.N[1] >= gp.P && gp.N[2] >= gp.P;
+}
+
+size_t cs_many_floats(int nrhs, int64_t G) { return (size_t)((nrhs + 3) / 4) * 4 * (size_t)G; }
+
+int cs_bins_build(const int32_t *start, int64_t n, const GridParams &gp, TileBins &tb, cudaStream_t s) {
+    return bins_build(start, n, gp, kCsTileX, kCsTileY, kCsTileZ, tb, s);
+}
+
+int spread_cs_many(const double *m, int64_t n, int nrhs, const int32_t *start, const double *base, const float *g,
+                   const GridParams &gp, const TileBins &tb, float *scratch, float *grid, cudaStream_t s) {
+    if (tb.tx != kCsTileX || tb.ty != kCsTileY || tb.tz != kCsTileZ) return MPS_BAD_ARG;
+    const int vq = (nrhs + 3) / 4, groups = (nrhs + kCsGroup - 1) / kCsGroup;
+    k_cs_moments<<<grid_for(n * 12 * vq, 256), 256, 0, s>>>(m, n, nrhs, vq, scratch);
+    MPS_LAUNCH_CHECK();
+    const float4 *mv = (const float4 *)scratch;
+    // as many groups to a block as leave the fewest lanes without a vector, more rather than fewer
+    const int V = groups % 3 == 0 || groups > 4 ? 3 : (groups % 2 == 0 ? 2 : 1);
+    const dim3 blocks((unsigned)tb.ntiles, (groups + V - 1) / V);
+    if (V == 3)
+        k_spread_cs_nodes<3><<<blocks, 256, 0, s>>>(mv, nrhs, vq, start, base, g, gp, tb.tile_start, tb.entries, tb.ntx,
+                                                    tb.nty, grid);
+    else if (V == 2)
+        k_spread_cs_nodes<2><<<blocks, 256, 0, s>>>(mv, nrhs, vq, start, base, g, gp, tb.tile_start, tb.entries, tb.ntx,
+                                                    tb.nty, grid);
+    else
+        k_spread_cs_nodes<1><<<blocks, 256, 0, s>>>(mv, nrhs, vq, start, base, g, gp, tb.tile_start, tb.entries, tb.ntx,
+                                                    tb.nty, grid);
+    MPS_LAUNCH_CHECK();
+    return MPS_OK;
+}
+
+int contract_cs_many(const float *grid, int64_t n, int nrhs, const int32_t *start, const double *base, const float *g,
+                     const GridParams &gp, float *scratch, double *out, cudaStream_t s) {
+    const int vq = (nrhs + 3) / 4;
+    k_cs_interleave<<<dim3((unsigned)((gp.G + 31) / 32), (vq + 15) / 16), 256, 0, s>>>(grid, nrhs, gp.G, vq,
+                                                                                       (float4 *)scratch);
+    MPS_LAUNCH_CHECK();
+    const int64_t items = n * ((nrhs + kCsGroup - 1) / kCsGroup);
+    k_contract_cs_il<<<grid_for(items * 32, 256, 152 * 64), 256, 0, s>>>((const float4 *)scratch, n, nrhs, vq, start,
+                                                                         base, g, gp, out);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
 }

@@ -2,6 +2,7 @@
 
 #include "cells.cuh"
 #include "grid.cuh"
+#include "tiles.cuh"
 
 namespace mps {
 
@@ -21,5 +22,13 @@ int scale_cs(void *spec, int nrhs, const GridParams &gp, const T *coef, cudaStre
 template <typename T>
 int contract_cs(const T *grid, int64_t n, int nrhs, const int32_t *start, const double *base, const T *g,
                 const GridParams &gp, double *out, cudaStream_t s);
+// The float32 spread and contraction of many vectors (scratch of cs_many_floats, 16-byte aligned; tb from cs_bins_build).
+bool cs_many(const GridParams &gp, int64_t n, int nrhs);
+size_t cs_many_floats(int nrhs, int64_t G);
+int cs_bins_build(const int32_t *start, int64_t n, const GridParams &gp, TileBins &tb, cudaStream_t s);
+int spread_cs_many(const double *m, int64_t n, int nrhs, const int32_t *start, const double *base, const float *g,
+                   const GridParams &gp, const TileBins &tb, float *scratch, float *grid, cudaStream_t s);
+int contract_cs_many(const float *grid, int64_t n, int nrhs, const int32_t *start, const double *base, const float *g,
+                     const GridParams &gp, float *scratch, double *out, cudaStream_t s);
 
 }  // namespace mps

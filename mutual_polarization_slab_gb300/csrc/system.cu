@@ -213,7 +213,8 @@ struct mps_system {
     size_t fft_work_bytes = 0;
     TileBins tb32;              // tiles of the float32 reference form's spread and contraction (tuned depth)
     TileBins tbg;               // tiles of the gradient-form spread (depth 12 where the grid allows it)
-    TileBins tbn;               // tiles of the float64 and double-float node spread
+    TileBins tbn;               // tiles of the node spread (float64, double-float, eight moments)
+    TileBins tbc;               // tiles of the polydisperse node spread of many vectors
     TileBins tb64;              // tiles of the tiled double-float contraction (A/B form)
     double *partial64 = nullptr;
     float *partial32 = nullptr;
@@ -335,6 +336,7 @@ static void free_system(mps_system *s) {
     tile_bins_free(s->tb32, s->stream);
     tile_bins_free(s->tbg, s->stream);
     tile_bins_free(s->tbn, s->stream);
+    tile_bins_free(s->tbc, s->stream);
     if (s->partial64) cudaFreeAsync(s->partial64, s->stream);
     if (s->partial32) cudaFreeAsync(s->partial32, s->stream);
     if (s->partialg) cudaFreeAsync(s->partialg, s->stream);
@@ -473,7 +475,10 @@ static int ensure_grids(mps_system *s, int precision, cudaStream_t st) {
         if (!s->spec64) MPS_TRY(dalloc(&s->spec64, nr * s->Gc * 2 * sizeof(double), st));
     } else {
         if (!s->grid32) MPS_TRY(dalloc(&s->grid32, nr * s->gp.G * sizeof(float), st));
-        if (!s->spec32) MPS_TRY(dalloc(&s->spec32, nr * s->Gc * 2 * sizeof(float), st));
+        // the polydisperse operator's interleaved grids pass through the spectra, which are a little larger
+        size_t floats = nr * s->Gc * 2;
+        if (s->kind == MPS_POLYDISPERSE) floats = std::max(floats, cs_many_floats(s->max_rhs, s->gp.G));
+        if (!s->spec32) MPS_TRY(dalloc(&s->spec32, floats * sizeof(float), st));
     }
     return MPS_OK;
 }
@@ -1047,6 +1052,8 @@ static int pair_sum_join(mps_system *s, double *out, int nrhs, cudaStream_t st) 
 template <typename T>
 static int matvec_cs(mps_system *s, const double *m, double *out, int nrhs, cudaStream_t st) {
     const bool dbl = sizeof(T) == 8;
+    const bool many = !dbl && cs_many(s->gp, s->n, nrhs);
+    if (many && !s->tbc.mem) MPS_TRY(cs_bins_build(s->start, s->n, s->gp, s->tbc, st));
     MPS_TRY(ensure_grids(s, dbl ? MPS_FP64 : MPS_FP32, st));
     T *grid = dbl ? (T *)s->grid64 : (T *)s->grid32;
     void *spec = dbl ? s->spec64 : s->spec32;
@@ -1057,7 +1064,11 @@ static int matvec_cs(mps_system *s, const double *m, double *out, int nrhs, cuda
     const bool beside = !dbl && pair_sum_beside(ev);
     if (beside) MPS_TRY(pair_sum_fork(s, m, nrhs, st, false));
     STAGE_MARK(1);
-    MPS_TRY(spread_cs<T>(m, s->n, nrhs, s->start, s->cs_base, g, s->gp, grid, st));
+    if (many)
+        MPS_TRY(spread_cs_many(m, s->n, nrhs, s->start, s->cs_base, (const float *)g, s->gp, s->tbc, (float *)spec,
+                               (float *)grid, st));
+    else
+        MPS_TRY(spread_cs<T>(m, s->n, nrhs, s->start, s->cs_base, g, s->gp, grid, st));
     STAGE_MARK(2);
     MPS_TRY(exec_plan(s, dbl ? CUFFT_D2Z : CUFFT_R2C, nrhs, grid, spec, 0, st));
     STAGE_MARK(3);
@@ -1065,7 +1076,11 @@ static int matvec_cs(mps_system *s, const double *m, double *out, int nrhs, cuda
     STAGE_MARK(4);
     MPS_TRY(exec_plan(s, dbl ? CUFFT_Z2D : CUFFT_C2R, nrhs, spec, grid, 0, st));
     STAGE_MARK(5);
-    MPS_TRY(contract_cs<T>(grid, s->n, nrhs, s->start, s->cs_base, g, s->gp, out, st));
+    if (many)
+        MPS_TRY(contract_cs_many((const float *)grid, s->n, nrhs, s->start, s->cs_base, (const float *)g, s->gp,
+                               (float *)spec, out, st));
+    else
+        MPS_TRY(contract_cs<T>(grid, s->n, nrhs, s->start, s->cs_base, g, s->gp, out, st));
     STAGE_MARK(6);
     if (dbl)
         MPS_TRY(real_space_csr<double>(m, out, s->n, nrhs, s->row_ptr, s->p64, s->diag, s->diag_idx, s->slab, true, st));

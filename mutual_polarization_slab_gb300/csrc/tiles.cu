@@ -26,7 +26,7 @@
 
 namespace mps {
 
-constexpr int kMaxTileList = 8;  // distinct tiles per axis touched by one stencil (ceil((P-1)/T)+2)
+constexpr int kMaxTileList = 10;  // distinct tiles per axis touched by one stencil (axis_tile_bound, T >= 2)
 // particles staged per spread iteration (one barrier interval): 96 measured 1.42 ms for the double-float spread
 // at the bench workload against 1.57 for 32 and 1.46 for 64 (fewer barriers; the warps' shares even out)
 constexpr int kChunk = 96;
@@ -172,7 +172,7 @@ static int64_t axis_tile_bound(int N, int T, int P) {
 
 // Tile lists without a host round trip: the entry arrays are sized by the per-particle bound (nentries holds that
 // capacity), the offsets and totals stay on the device.
-static int bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tx, int ty, int tz, TileBins &tb,
+int bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tx, int ty, int tz, TileBins &tb,
                       cudaStream_t s) {
     tile_bins_free(tb, s);
     TileGeom tg;

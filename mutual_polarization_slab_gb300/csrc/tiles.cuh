@@ -38,6 +38,9 @@ constexpr int kHomeBlock = 8;
 
 bool tiles_supported(const GridParams &gp, int tz);
 int tile_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tz, TileBins &tb, cudaStream_t s);
+// Bins of tiles of 2 to 16 nodes an axis, without a host round trip.
+int bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tx, int ty, int tz, TileBins &tb,
+               cudaStream_t s);
 // Bins for spread_nodes and spread_nodes8: 8 x 8 tiles, of depth 8 or 4 by the number of blocks (groups to a tile).
 int node_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int groups, TileBins &tb, cudaStream_t s);
 bool nodes_supported(const GridParams &gp);
