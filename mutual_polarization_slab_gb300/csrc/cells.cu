@@ -949,6 +949,15 @@ void compute_ncell(const double *box, double rmax, int64_t *ncell) {
     }
 }
 
+bool cells_fit(const int64_t *ncell) {
+    int64_t ncells = 1;
+    for (int d = 0; d < 3; ++d) {
+        if (ncell[d] > INT32_MAX / ncells) return false;
+        ncells *= ncell[d];
+    }
+    return true;
+}
+
 size_t cell_bins_bytes(int64_t n, int64_t ncells) {
     size_t b = 0;
     b += 256 + (size_t)n * 4;         // lin
@@ -1119,6 +1128,7 @@ int probe_real_space(const double *xe, int64_t ne, const double *xp, const doubl
     if (ntab < 2) return MPS_BAD_ARG;
     int64_t ncell[3];
     compute_ncell(box, rc, ncell);
+    if (!cells_fit(ncell)) return MPS_BAD_ARG;
     const int64_t ncells = ncell[0] * ncell[1] * ncell[2];
     int64_t *cell_p = nullptr, *cell_e = nullptr;
     void *bins = nullptr;
@@ -1174,6 +1184,7 @@ int probe_real_space_quad(const double *xe, int64_t ne, const double *xp, const 
     if (ntab < 2) return MPS_BAD_ARG;
     int64_t ncell[3];
     compute_ncell(box, rc, ncell);
+    if (!cells_fit(ncell)) return MPS_BAD_ARG;
     const int64_t ncells = ncell[0] * ncell[1] * ncell[2];
     int64_t *cell_p = nullptr, *cell_e = nullptr;
     void *bins = nullptr;
@@ -1229,6 +1240,7 @@ int probe_real_space_cs(const double *xe, int64_t ne, const double *xp, const do
     if (ntab < 2 || M < 1 || cmin < 0 || cmin >= M) return MPS_BAD_ARG;
     int64_t ncell[3];
     compute_ncell(box, rc, ncell);
+    if (!cells_fit(ncell)) return MPS_BAD_ARG;
     const int64_t ncells = ncell[0] * ncell[1] * ncell[2];
     int64_t *cell_p = nullptr, *cell_e = nullptr;
     void *bins = nullptr;

@@ -34,6 +34,8 @@ struct Box3 {
 };
 
 void compute_ncell(const double *box, double rmax, int64_t *ncell);
+// Whether 32-bit cell ids hold the grid: a cutoff that small for its box is refused before anything is sized from it.
+bool cells_fit(const int64_t *ncell);
 size_t cell_bins_bytes(int64_t n, int64_t ncells);
 int cell_assign(const double *x, int64_t n, const double *box, const int64_t *ncell, int64_t *cell3, cudaStream_t s);
 int cell_bins_build(const int64_t *cell3, int64_t n, const int64_t *ncell, void *ws, CellBins &cb, cudaStream_t s);

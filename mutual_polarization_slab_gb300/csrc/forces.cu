@@ -82,6 +82,7 @@ extern "C" int mps_dipole_forces(const double *pos, const double *dip, int64_t n
     cudaStream_t s = (cudaStream_t)stream;
     int64_t ncell[3];
     compute_ncell(box, r_cut, ncell);
+    if (!cells_fit(ncell)) return MPS_BAD_ARG;
     const int64_t ncells = ncell[0] * ncell[1] * ncell[2];
     int64_t *cell3 = nullptr;
     void *bins = nullptr;

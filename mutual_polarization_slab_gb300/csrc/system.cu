@@ -2631,6 +2631,7 @@ extern "C" int mps_system_create(const mps_system_desc *d, mps_system **out, mps
     }
     // cell list + pair CSR
     compute_ncell(d->box, d->rc, s->ncell);
+    if (!cells_fit(s->ncell)) CR_TRY(MPS_BAD_ARG);
     const int64_t ncells = s->ncell[0] * s->ncell[1] * s->ncell[2];
     int64_t *cell3 = nullptr, *cnt27 = nullptr, *off27 = nullptr;
     void *bins = nullptr, *scan_tmp = nullptr;
