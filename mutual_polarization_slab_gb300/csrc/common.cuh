@@ -55,10 +55,14 @@ __device__ __forceinline__ T warp_sum(T v) {
     return v;
 }
 
-// One float (or four, aligned) from global to shared memory without a register in between: a staging loop issues all its loads at once
+// One float (or two or four, aligned) from global to shared memory without a register in between: a staging loop issues all its loads at once
 // (copy_async_wait before the barrier that publishes them).
 __device__ __forceinline__ void copy_async(float *smem, const float *gmem) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async(float2 *smem, const float2 *gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
                  : "memory");
 }
 __device__ __forceinline__ void copy_async(float4 *smem, const float4 *gmem) {

@@ -13,16 +13,21 @@ namespace mps {
 
 constexpr int kDfMaxStages = 12;
 
-// One axis: N = product of radices (4, 3, 5, 2), Stockham stage s reads
-// in[j + r N/R] and writes out[(j / Ns) Ns R + j % Ns + r Ns].
+// One axis: N = product of radices (2 .. 8), Stockham stage s reads in[j + r N/R] and writes
+// out[(j / Ns) Ns R + j % Ns + r Ns].
 struct DfAxisPlan {
     int N = 0;
-    int nst = 0;
+    int nst = 0, ntw = 0;
     int R[kDfMaxStages];
     int Ns[kDfMaxStages];
-    int twoff[kDfMaxStages];   // offset of stage s's twiddles (Ns x R) in the table
-    int ntw = 0;
+    int twoff[kDfMaxStages];     // offset of stage s's twiddles ((R - 1) x Ns) in the table
+    unsigned mNR[kDfMaxStages], mNs[kDfMaxStages], mN, mNh;   // multipliers for division by N / R, Ns, N, N / 2 + 1
     const float4 *tw = nullptr;  // device table: (cos hi, cos lo, -sin hi, -sin lo) of 2 pi jm r / (Ns R)
+};
+
+// Wave-number step of each axis as double-float numbers.
+struct DfStep {
+    float hi[3], lo[3];
 };
 
 struct DfPlan3 {
@@ -35,18 +40,18 @@ struct DfPlan3 {
 // axis is longer than 1024.
 int df_plan(const GridParams &gp, DfPlan3 *out);
 
-// Forward: double-float real grids ((hi, lo) float pairs, ncomp x [Nz][Ny][Nx]) -> double-float half
-// spectra (ncomp x [Nz][Ny][Nx/2+1], float4 per complex value) in spec.
+// Forward (x and y): double-float real grids ((hi, lo) float pairs, ncomp x [Nz][Ny][Nx]) -> double-float half
+// spectra (ncomp x [Nz][Ny][Nx/2+1], float4 per complex value; twice the transforms' values) in spec.
 // Inverse: the reverse, unnormalised.  For the dipole operator the z pass of the
 // forward transform, the Green's scale and the z pass of the inverse run in one
 // kernel (scale_dipole): spec then never holds the unscaled z-transformed data.
 int df_forward_xy(const float2 *grid, float4 *spec, int ncomp, const GridParams &gp, const DfPlan3 &pl,
                   cudaStream_t s);
-int df_z_scale_dipole(float4 *spec, int nrhs, const GridParams &gp, const DfPlan3 &pl, const double *H,
-                      const float2 *tm6, cudaStream_t s);
-// The scale tensor of the double-float z pass, 6 double-float entries per
-// half-spectrum point (6 x Gc float2), built once per grid.
-int df_scale_table(const GridParams &gp, const double *H, float2 *tm6, cudaStream_t s);
+int df_z_scale_dipole(float4 *spec, int nrhs, const GridParams &gp, const DfPlan3 &pl, const float2 *hs,
+                      cudaStream_t s);
+// The scale of the double-float z pass, 0.5 H / |k|^2 as a double-float entry per half-spectrum point, built once per
+// grid.
+int df_scale_table(const GridParams &gp, const double *H, float2 *hs, cudaStream_t s);
 int df_inverse_yx(float4 *spec, float2 *grid, int ncomp, const GridParams &gp, const DfPlan3 &pl, cudaStream_t s);
 
 // The same transforms in float32 (float2 per complex value) for the float32

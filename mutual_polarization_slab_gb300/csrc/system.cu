@@ -75,18 +75,18 @@ struct GreenCoef {
     double *h64 = nullptr;
     float *h32 = nullptr;
     float *hs32 = nullptr;   // H / |k|^2 of the gradient-form float32 operator (built on first use)
-    float2 *tm6 = nullptr;   // double-float scale tensor H q q^T, 6 x Gc (built on first use)
+    float2 *hsdf = nullptr;  // 0.5 H / |k|^2 in double-float (built on first use)
     double *hs64 = nullptr;  // 0.5 H / |k|^2 of the float64 transforms (built on first use)
-    cudaEvent_t ev_h = nullptr, ev_hs32 = nullptr, ev_tm6 = nullptr, ev_hs64 = nullptr;   // recorded after each fill
+    cudaEvent_t ev_h = nullptr, ev_hs32 = nullptr, ev_hsdf = nullptr, ev_hs64 = nullptr;   // recorded after each fill
     ~GreenCoef() {
         if (h64) cudaFree(h64);
         if (h32) cudaFree(h32);
         if (hs32) cudaFree(hs32);
-        if (tm6) cudaFree(tm6);
+        if (hsdf) cudaFree(hsdf);
         if (hs64) cudaFree(hs64);
         if (ev_h) cudaEventDestroy(ev_h);
         if (ev_hs32) cudaEventDestroy(ev_hs32);
-        if (ev_tm6) cudaEventDestroy(ev_tm6);
+        if (ev_hsdf) cudaEventDestroy(ev_hsdf);
         if (ev_hs64) cudaEventDestroy(ev_hs64);
     }
 };
@@ -233,8 +233,8 @@ struct mps_system {
     int resid_prec = MPS_FP64;   // operator of the refinement residuals
     float *g32 = nullptr;        // gradient factors dw_d/dr of the gradient-form operator, n x 3 x P
     int inner_prec = MPS_FP32;   // operator of the mixed solve's inner GMRES
-    // this system's stream has waited for the shared lazily built Green's buffers (hs32, tm6)
-    bool hs32_ready = false, tm6_ready = false, hs64_ready = false;
+    // this system's stream has waited for the shared lazily built Green's buffers (hs32, hs64, hsdf)
+    bool hs32_ready = false, hsdf_ready = false, hs64_ready = false;
     InnerGrid *inner = nullptr;      // coarser inner discretisation of the gradient-form operator, or null
     // Arnoldi-step graphs (captured on their own stream once every lazily built buffer of the matvec exists:
     // after the first matvec of that precision and batch width outside a capture)
@@ -854,7 +854,7 @@ static int matvec_f32(mps_system *s, const double *m, double *out, int nrhs, cud
 // tiled spread and contraction accumulate in double-float arithmetic (float64
 // weights and grids), the FFTs and Green's scale are the double-float transforms
 // of dffft.cu; the pair sum is the float64 kernel.
-// First-use setup of the double-float operator: weights, tile bins (autotuned depth), grids, scale tensor.
+// First-use setup of the double-float operator: weights, tile bins, grids, scale.
 static int df_prepare(mps_system *s, cudaStream_t st, bool *nodes_out) {
     const int64_t nw = (int64_t)s->n * 3 * s->gp.P;
     if (!s->wdf) {
@@ -863,18 +863,18 @@ static int df_prepare(mps_system *s, cudaStream_t st, bool *nodes_out) {
     }
     MPS_TRY(ensure_nodes(s, st, nodes_out));
     MPS_TRY(ensure_grids(s, MPS_FP64, st));
-    if (!s->tm6_ready) {
+    if (!s->hsdf_ready) {
         std::lock_guard<std::mutex> lk(g_green_mu);
-        if (!s->green->tm6) {
+        if (!s->green->hsdf) {
             float2 *tm = nullptr;
-            MPS_TRY(dalloc_persistent(&tm, sizeof(float2) * 6 * s->Gc));
+            MPS_TRY(dalloc_persistent(&tm, sizeof(float2) * s->Gc));
             MPS_TRY(df_scale_table(s->gp, s->green->h64, tm, st));
-            MPS_TRY(green_mark_filled(&s->green->ev_tm6, st));
-            s->green->tm6 = tm;
+            MPS_TRY(green_mark_filled(&s->green->ev_hsdf, st));
+            s->green->hsdf = tm;
         } else {
-            MPS_CUDA_TRY(cudaStreamWaitEvent(st, s->green->ev_tm6, 0));   // filled by another system
+            MPS_CUDA_TRY(cudaStreamWaitEvent(st, s->green->ev_hsdf, 0));   // filled by another system
         }
-        s->tm6_ready = true;
+        s->hsdf_ready = true;
     }
     return MPS_OK;
 }
@@ -897,7 +897,7 @@ static int df_field_grids(mps_system *s, const double *m, int nrhs, StageEvents 
     STAGE_MARK(2);
     MPS_TRY(df_forward_xy((const float2 *)grid, spec, 3 * nrhs, s->gp, s->dfp, st));
     STAGE_MARK(3);
-    MPS_TRY(df_z_scale_dipole(spec, nrhs, s->gp, s->dfp, s->h64, s->green->tm6, st));
+    MPS_TRY(df_z_scale_dipole(spec, nrhs, s->gp, s->dfp, s->green->hsdf, st));
     STAGE_MARK(4);
     MPS_TRY(df_inverse_yx(spec, (float2 *)grid, 3 * nrhs, s->gp, s->dfp, st));
     STAGE_MARK(5);
@@ -2304,7 +2304,7 @@ static int refine_mixed(mps_system *s, const double *b, double *x, int nrhs, con
     int rc = MPS_NOT_CONVERGED;
     int step = 0;
     int e = MPS_OK;
-    // The double-float residual's first-use set-up (weights, tiles, grids, scale tensor) runs on the system's
+    // The double-float residual's first-use set-up (weights, tiles, grids, scale) runs on the system's
     // prep stream beside the first inner solve.
     cudaEvent_t ev_prep = nullptr;
     if (s->resid_prec == MPS_DF && df_usable(s) && !s->wdf) {
