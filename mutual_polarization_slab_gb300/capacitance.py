@@ -24,7 +24,7 @@ import numpy as np
 import torch
 
 from . import ewald
-from .system import SpectralEwaldSystem, as_device, spectral_parameters, to_host
+from .system import SpectralEwaldSystem, as_device, spectral_parameters, to_host, unit_field_systems
 
 __all__ = ["gmres_restarted", "magnetic_dipole", "capacitance", "run_capacitance", "capacitance_tensor",
            "capacitance_tensor_spectrum", "dilute_guess", "default_table"]
@@ -358,7 +358,6 @@ def capacitance_tensor_spectrum(x, box, eps_p, xi, errortol=1e-3, *, slab_factor
     # complex permittivities (frequency-dependent eps, which the MATLAB driver allows) give complex C and p
     cplx = np.iscomplexobj(eps)
     eps = eps.astype(np.complex128 if cplx else np.float64)
-    tdt = torch.complex128 if cplx else torch.float64
     if eps.ndim == 1:
         eps = eps[:, None]
     N, F = xn.shape[0], xn.shape[2]
@@ -370,27 +369,21 @@ def capacitance_tensor_spectrum(x, box, eps_p, xi, errortol=1e-3, *, slab_factor
     restart = min(3 * N, 10) if restart is None else int(restart)
     maxit = min(3 * N, 100) if maxit is None else int(maxit)
     C = np.zeros((3, 3, F, K), dtype=eps.dtype)
-    p = np.zeros((N, 3, 3, K, F), dtype=eps.dtype)
+    p = np.empty((N, 3, 3, K, F), dtype=eps.dtype)
     for f in range(F):
         lam = eps.T.copy()                                   # (K, N) permittivity sets
         sysm = SpectralEwaldSystem(xn[:, :, f], lam, box, xi, rc, Ngrid, P, perp, para, rv,
                                    slab_factor=slab_factor, eta=eta, max_rhs=3 * K,
                                    inner=_inner(precision, "grad", inner_grid))
-        b = torch.zeros((3 * K, N, 3), dtype=tdt, device="cuda")
-        x0 = torch.zeros_like(b)
-        diag_index = []
-        for k in range(K):
-            amp = torch.as_tensor(dilute_guess(eps[:, k], phi, [1.0, 0.0, 0.0])[:, 0], dtype=tdt, device="cuda")
-            for i in range(3):
-                b[3 * k + i, :, i] = 1.0
-                x0[3 * k + i, :, i] = amp
-                diag_index.append(k)
+        b, x0, diag_index = unit_field_systems(np.stack([dilute_guess(v, phi, [1.0, 0.0, 0.0])[:, 0] for v in eps.T]))
         sol, _ = sysm.solve(b, x0, tol=errortol, restart=restart, maxit=maxit, precision=precision,
                             inner_tol=inner_tol, inner_maxit=inner_maxit, diag_index=diag_index)
-        sol = sol.reshape(K, 3, N, 3).cpu().numpy()
-        for k in range(K):
-            for i in range(3):
-                C[i, :, f, k] = sol[k, i].mean(axis=0)
-                p[:, :, i, k, f] = sol[k, i]
+        sol = sol.reshape(K, 3, N, 3)
+        C[:, :, f, :] = sol.mean(dim=2).permute(1, 2, 0).cpu().numpy()
+        pf = to_host(sol.permute(2, 3, 1, 0).contiguous())
+        if F == 1:
+            p = pf[..., None]
+        else:
+            p[..., f] = pf
         sysm.close()
     return C.mean(axis=2), p

@@ -30,7 +30,7 @@ import torch
 
 from . import _lib as L
 from . import ewald
-from .system import SpectralEwaldSystem, as_device, fft_size, spectral_parameters
+from .system import SpectralEwaldSystem, as_device, fft_size, spectral_parameters, to_host, unit_field_systems
 
 __all__ = ["TABLE_ORDER", "real_space_table", "default_table", "QuadrupoleSystem", "matrix_vector_multiply",
            "matrix_vector_multiply_flat", "matrix_vector_solve", "capacitance_tensor",
@@ -251,25 +251,15 @@ def capacitance_tensor_spectrum(x, box, eps_p, xi, errortol=1e-3, *, rc=None, Ng
     for f in range(F):
         sysm = QuadrupoleSystem(xn[:, :, f], eps.T.copy(), box, xi, errortol, tables, r_vals, rc=rc, Ngrid=Ngrid,
                                 P=P, max_rhs=3 * K)
-        b = torch.zeros((3 * K, N, 8), dtype=torch.float64, device="cuda")
-        x0 = torch.zeros_like(b)
-        diag_index = []
-        for k in range(K):
-            with np.errstate(invalid="ignore"):
-                beta = (eps[:, k] - 1.0) / (eps[:, k] + 2.0)
-            beta[np.isinf(eps[:, k])] = 1.0
-            amp = torch.as_tensor(4 * np.pi * beta / (1 - beta * phi), device="cuda")
-            for i in range(3):
-                b[3 * k + i, :, i] = 1.0
-                x0[3 * k + i, :, i] = amp
-                diag_index.append(k)
+        with np.errstate(invalid="ignore"):
+            beta = (eps.T - 1.0) / (eps.T + 2.0)
+        beta[np.isinf(eps.T)] = 1.0
+        b, x0, diag_index = unit_field_systems(4 * np.pi * beta / (1 - beta * phi), 8)
         sol, _ = sysm.solve(b, x0, tol=errortol, restart=restart, maxit=maxit, precision=precision,
                             inner_tol=inner_tol, inner_maxit=inner_maxit, diag_index=diag_index)
-        sol = sol.reshape(K, 3, N, 8).cpu().numpy()
-        for k in range(K):
-            for i in range(3):
-                C[:, i, f, k] = sol[k, i, :, :3].mean(axis=0)
-                p[:, :, i, k, f] = sol[k, i, :, :3]
-                Qo[:, :, i, k, f] = sol[k, i, :, 3:]
+        sol = sol.reshape(K, 3, N, 8)
+        C[:, :, f, :] = sol[..., :3].mean(dim=2).permute(2, 1, 0).cpu().numpy()
+        sol = to_host(sol.permute(2, 3, 1, 0).contiguous())
+        p[..., f], Qo[..., f] = sol[:, :3], sol[:, 3:]
         sysm.close()
     return C.mean(axis=2), p, Qo

@@ -27,7 +27,7 @@ import numpy as np
 import torch
 
 from . import _lib as L
-from .system import SpectralEwaldSystem, as_device
+from .system import SpectralEwaldSystem, as_device, to_host, unit_field_systems
 
 __all__ = ["unique_radii", "real_space_table", "default_r_table", "spectral_parameters", "PolydisperseSystem",
            "compute_field", "compute_dipole", "capacitance_tensor", "capacitance_tensor_spectrum", "dipole",
@@ -233,22 +233,12 @@ def capacitance_tensor_spectrum(x, box, a, eps_p, xi, *, tol=1e-3, precision="fp
     p = np.zeros((N, 9, F, K))
     for f in range(F):
         sysm = PolydisperseSystem(xn[:, :, f], a_np, eps.T.copy(), box, xi, tol, rt, perp, para, max_rhs=3 * K)
-        b = torch.zeros((3 * K, N, 3), dtype=torch.float64, device="cuda")
-        x0 = torch.zeros_like(b)
-        diag_index = []
-        for k in range(K):
-            amp = torch.as_tensor(_guess_amplitude(a_np, eps[:, k], phi), device="cuda")
-            for i in range(3):
-                b[3 * k + i, :, i] = 1.0
-                x0[3 * k + i, :, i] = amp
-                diag_index.append(k)
+        b, x0, diag_index = unit_field_systems(np.stack([_guess_amplitude(a_np, v, phi) for v in eps.T]))
         sol, _ = sysm.solve(b, x0, tol=tol, restart=restart, maxit=maxit, precision=precision,
                             diag_index=diag_index)
-        sol = sol.reshape(K, 3, N, 3).cpu().numpy()
-        for k in range(K):
-            for i in range(3):
-                C[3 * i:3 * i + 3, f, k] = sol[k, i].mean(axis=0)
-                p[:, 3 * i:3 * i + 3, f, k] = sol[k, i]
+        sol = sol.reshape(K, 3, N, 3)
+        C[:, f, :] = sol.mean(dim=2).reshape(K, 9).T.cpu().numpy()
+        p[:, :, f, :] = to_host(sol.permute(2, 1, 3, 0).reshape(N, 9, K).contiguous())
         sysm.close()
     return C.mean(axis=1).T, p.transpose(0, 1, 3, 2)
 
