@@ -352,7 +352,7 @@ struct CsCplx<double> {
 
 // spec[r][k] *= coef[k]: a thread takes one spectrum point of a few vectors (blockIdx.y), with one complex (8 or 16 byte)
 // load and store per value; with all vectors to a thread a small grid's points filled the chip too thinly (48 vectors on
-// 40^3: 13.7 -> @SC@ us).
+// 40^3: 13.7 -> 4.0 us).
 constexpr int kScaleVec = 4;
 
 template <typename T>
