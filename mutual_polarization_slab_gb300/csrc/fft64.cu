@@ -9,14 +9,16 @@
 //             the x and y components enter only as a = kx fx + ky fy: two transforms each way instead of three
 //   butterflies  of all lines of a block are numbered through and dealt to its threads, so no lane idles for a line
 //             length that is no multiple of 32; radices up to 12 run in registers
-//   primes    a radix p above 5 runs as p - 1 multiply-adds a point on the sums and differences x_r +- x_{p-r}
+//   primes    a radix p above 5 runs as p - 1 multiply-adds a point on the sums and differences x_r +- x_{p-r}; where
+//             (p - 1) / 2 = 3 q with q prime to 3, five for every nine of them (stage64_thirds)
 // The passes run at the float64 rate (x and y on 192^3: 24 operations a point in 97 % of the time that the measured
 // 5.0e11 multiply-adds a second would take).  Against cuFFT's D2Z / Z2D with the scale as a pass of its own, both ways,
-// float64: three vectors on 192^3 14.96 -> 8.33 ms, on 64^3 0.40 -> 0.32; one vector on 86^3 1.22 -> 0.59, on 240^3
+// float64: three vectors on 192^3 14.96 -> 8.33 ms, on 64^3 0.40 -> 0.32; one vector on 86^3 1.22 -> 0.46, on 240^3
 // 12.6 -> 6.3, on 96^3 0.65 -> 0.36 ms; twelve on 25^3 0.147 -> 0.135, on 43^3 0.93 -> 0.79 ms.
 #include "fft64.cuh"
 
 #include <math.h>
+#include <string.h>
 
 #include <map>
 #include <mutex>
@@ -245,6 +247,87 @@ __device__ __forceinline__ void stage64_prime(double2 *in, double2 *out, int nl,
     }
 }
 
+// Prime radix R with (R - 1) / 2 = 3 q, q prime to 3.  With r = g^T, k = g^S (g a generator), the sums over r of
+// a_r cos(2 pi k r / R) and d_r sin(2 pi k r / R) are correlations over the exponents, Z_3 x Z_2q: the coefficient depends
+// on (s1 + t1 mod 3, s2 + t2) only (and changes sign, the sine's, or not with s2 + t2 -> + q), t1 in Z_3, t2 < q standing
+// for the pairs r, R - r.  In the direction of 3, with c_u = c' + c~_u, c' their mean,
+//   y_s = c' (a_0 + a_1 + a_2) + z_s,  z_0 = alpha c~_0 + beta c~_1,  z_1 = alpha c~_1 + beta c~_2,  z_2 = -(z_0 + z_1),
+// alpha = a_0 - a_2, beta = a_1 - a_2 (the c~ sum to zero): five multiplications instead of nine.
+//   1  sums and differences of the pairs, then sum, alpha and beta of each triple of them, in place
+//   2  a thread takes one part (cosine, sine), one component (re, im) and one s2 of a butterfly: three outputs
+//   3  the outputs k and R - k from their two parts
+// tab: q triples r (packed integers), then for the cosines and the sines 2 q entries (c', c~_0, c~_1, c~_2).
+// Both ways, one vector on 86^3 (2 x 43) 0.58 -> 0.46 ms, 36 on 31^3 0.60 -> 0.54, one on 103^3 1.78 -> 1.15.
+__device__ __forceinline__ void stage64_thirds(double2 *in, double2 *out, int nl, int ld, int N, int R, int q, int Ns,
+                                               const double2 *__restrict__ tw, const double2 *__restrict__ tab) {
+    const unsigned NR = N / R, nb = nl * NR;
+    for (unsigned w = threadIdx.x; w < nb * q; w += blockDim.x) {
+        const unsigned t = w / nb, lj = w - t * nb, line = lj / NR, j = lj - line * NR, jm = j % Ns;
+        double2 *a = in + line * ld + j;
+        const double2 pr = tab[t];
+        const int r[3] = {__double2loint(pr.x), __double2hiint(pr.x), __double2loint(pr.y)};
+        double2 s[3], d[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            double2 u = a[r[c] * NR], v = a[(R - r[c]) * NR];
+            if (Ns > 1) {
+                u = zmul(u, tw[jm * R + r[c]]);
+                v = zmul(v, tw[jm * R + R - r[c]]);
+            }
+            s[c] = zadd(u, v);
+            d[c] = zsub(u, v);
+        }
+        a[r[0] * NR] = zadd(zadd(s[0], s[1]), s[2]);
+        a[r[1] * NR] = zsub(s[0], s[2]);
+        a[r[2] * NR] = zsub(s[1], s[2]);
+        a[(R - r[0]) * NR] = zadd(zadd(d[0], d[1]), d[2]);
+        a[(R - r[1]) * NR] = zsub(d[0], d[2]);
+        a[(R - r[2]) * NR] = zsub(d[1], d[2]);
+    }
+    __syncthreads();
+    for (unsigned w = threadIdx.x; w < nb * (4 * q + 2); w += blockDim.x) {
+        const unsigned e = w / nb, lj = w - e * nb, line = lj / NR, j = lj - line * NR, jq = j / Ns, jm = j - jq * Ns;
+        const unsigned comp = e & 1, s2 = e >> 2;
+        const bool sine = e & 2;
+        const double *a = (const double *)(in + line * ld + j) + comp;
+        double *o = (double *)(out + line * ld + jq * Ns * R + jm) + comp;
+        if (s2 == (unsigned)q) {   // X_0
+            double m = a[0];
+            for (int t = 0; t < q; ++t) m += a[2 * NR * __double2loint(tab[t].x)];
+            o[0] = m;
+            continue;
+        }
+        const double2 *c = tab + q + (sine ? 4 * q : 0) + 2 * s2;
+        double m = sine ? 0.0 : a[0], z0 = 0.0, z1 = 0.0;
+#pragma unroll 2
+        for (int t = 0; t < q; ++t) {
+            const double2 pr = tab[t], c0 = c[2 * t], c1 = c[2 * t + 1];   // (c', c~0), (c~1, c~2)
+            const int r0 = __double2loint(pr.x), r1 = __double2hiint(pr.x), r2 = __double2loint(pr.y);
+            const double sum = a[2 * NR * (sine ? R - r0 : r0)], al = a[2 * NR * (sine ? R - r1 : r1)],
+                         be = a[2 * NR * (sine ? R - r2 : r2)];
+            m = fma(sum, c0.x, m);
+            z0 = fma(al, c0.y, fma(be, c1.x, z0));
+            z1 = fma(al, c1.x, fma(be, c1.y, z1));
+        }
+        const double2 pk = tab[s2];
+        const int k0 = __double2loint(pk.x), k1 = __double2hiint(pk.x), k2 = __double2loint(pk.y);
+        o[2 * Ns * (sine ? R - k0 : k0)] = m + z0;
+        o[2 * Ns * (sine ? R - k1 : k1)] = m + z1;
+        o[2 * Ns * (sine ? R - k2 : k2)] = m - (z0 + z1);
+    }
+    __syncthreads();
+    for (unsigned w = threadIdx.x; w < nb * 3 * q; w += blockDim.x) {
+        const unsigned e = w / nb, lj = w - e * nb, line = lj / NR, j = lj - line * NR, jq = j / Ns, jm = j - jq * Ns;
+        const unsigned t = e / 3, c = e - 3 * t;
+        const double2 pr = tab[t];
+        const int k = c == 0 ? __double2loint(pr.x) : (c == 1 ? __double2hiint(pr.x) : __double2loint(pr.y));
+        double2 *o = out + line * ld + jq * Ns * R + jm;
+        const double2 u = o[k * Ns], v = o[(R - k) * Ns];
+        o[k * Ns] = make_double2(u.x + v.y, u.y - v.x);
+        o[(R - k) * Ns] = make_double2(u.x - v.y, u.y + v.x);
+    }
+}
+
 // Forward transform of the nl lines in a (b: scratch of the same size); returns the buffer with the result.  All
 // threads of the block call it; the lines are complete in a, and the result is complete on return.
 __device__ double2 *fft64_lines(double2 *a, double2 *b, int nl, int ld, const F64Axis &p) {
@@ -262,7 +345,12 @@ __device__ double2 *fft64_lines(double2 *a, double2 *b, int nl, int ld, const F6
             F64_STAGE(10)
             F64_STAGE(12)
 #undef F64_STAGE
-            default: stage64_prime(a, b, nl, ld, p.N, p.R[s], p.Ns[s], t, p.tw + p.rtoff[s]); break;
+            default:
+                if (p.third[s])
+                    stage64_thirds(a, b, nl, ld, p.N, p.R[s], p.third[s], p.Ns[s], t, p.tw + p.rtoff[s]);
+                else
+                    stage64_prime(a, b, nl, ld, p.N, p.R[s], p.Ns[s], t, p.tw + p.rtoff[s]);
+                break;
         }
         __syncthreads();
         double2 *x = a;
@@ -523,6 +611,48 @@ static std::vector<int> f64_radices(int n, bool first) {
     return best;
 }
 
+// q of a prime whose (R - 1) / 2 = 3 q with q prime to 3; below q = 5 the split costs what it saves.
+static int f64_third(int R) {
+    const int q = (R - 1) / 6;
+    return (R - 1) % 6 == 0 && q % 3 != 0 && q >= 5 ? q : 0;
+}
+
+// The table of stage64_thirds.
+static void f64_thirds_table(int R, int q, std::vector<double2> &tw) {
+    std::vector<int> power(R - 1);   // g^e mod R of the smallest generator g
+    for (int g = 2;; ++g) {
+        int x = 1, e = 0;
+        do {
+            power[e++] = x;
+            x = x * g % R;
+        } while (x != 1);
+        if (e == R - 1) break;
+    }
+    auto at = [&](int u1, int u2) {   // the element whose exponent is u1 mod 3 and u2 mod 2 q
+        int e = u2 % (2 * q);
+        while (e % 3 != u1 % 3) e += 2 * q;
+        return power[e];
+    };
+    auto pack = [](int lo, int hi) {
+        const uint64_t b = (uint64_t)(uint32_t)lo | ((uint64_t)(uint32_t)hi << 32);
+        double d;
+        memcpy(&d, &b, sizeof d);
+        return d;
+    };
+    for (int t = 0; t < q; ++t) tw.push_back(make_double2(pack(at(0, t), at(1, t)), pack(at(2, t), 0)));
+    for (int sine = 0; sine < 2; ++sine)
+        for (int u = 0; u < 2 * q; ++u) {
+            double c[3];
+            for (int k = 0; k < 3; ++k) {
+                const double ang = 2.0 * M_PI * (double)at(k, u) / (double)R;
+                c[k] = sine ? sin(ang) : cos(ang);
+            }
+            const double mean = (c[0] + c[1] + c[2]) / 3.0;
+            tw.push_back(make_double2(mean, c[0] - mean));
+            tw.push_back(make_double2(c[1] - mean, c[2] - mean));
+        }
+}
+
 static bool f64_axis(int N, int dev, F64Axis *out) {
     if (N < 2 || N > kF64MaxN) return false;
     std::lock_guard<std::mutex> lk(g_f64_mu);
@@ -561,7 +691,11 @@ static bool f64_axis(int N, int dev, F64Axis *out) {
                 tw.push_back(make_double2(cos(ang), sin(ang)));
             }
         p.rtoff[s] = (int)tw.size();
-        if (s < (int)(radices.size() - rest.size()))
+        const bool prime = s < (int)(radices.size() - rest.size());
+        p.third[s] = prime ? f64_third(R) : 0;
+        if (p.third[s])
+            f64_thirds_table(R, p.third[s], tw);
+        else if (prime)
             for (int r = 0; r < R; ++r) {
                 const double ang = 2.0 * M_PI * (double)r / (double)R;
                 tw.push_back(make_double2(cos(ang), sin(ang)));

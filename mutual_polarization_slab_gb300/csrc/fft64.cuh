@@ -13,10 +13,11 @@ constexpr int kF64MaxN = 1024;
 constexpr int kF64MaxPrime = 127;
 
 // Mixed-radix plan of one axis: stage s has radix R[s], Ns[s] = R[0] ... R[s-1].  tw holds each stage's twiddles
-// exp(-2 pi i jm r / (Ns R)) at twoff[s] + jm R + r, and, for a prime radix above 5, its R roots at rtoff[s].
+// exp(-2 pi i jm r / (Ns R)) at twoff[s] + jm R + r, and, for a prime radix above 5, its R roots at rtoff[s] or, where
+// third[s] = q > 0, the permutation and coefficients of the split into thirds (stage64_thirds).
 struct F64Axis {
     int N = 0, nst = 0;
-    int R[kF64MaxStages], Ns[kF64MaxStages], twoff[kF64MaxStages], rtoff[kF64MaxStages];
+    int R[kF64MaxStages], Ns[kF64MaxStages], twoff[kF64MaxStages], rtoff[kF64MaxStages], third[kF64MaxStages];
     const double2 *tw = nullptr;
 };
 
