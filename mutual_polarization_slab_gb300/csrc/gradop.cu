@@ -321,6 +321,41 @@ __global__ void k_contract_grad_gather(const float *__restrict__ partial, int64_
     }
 }
 
+// The columns of a stencil by rounds of a warp, for the contractions below: lane's column (jx, jy) of a round, the planes
+// sub, sub + lpp, ... of it; false: none.  For the supports of the staged contraction (8 and 10) the columns that a round
+// reads together lie in different banks of its region, whose rows are 20 floats apart: 8 x 4 columns of every other row,
+// then the edge of 10 x 10, 24 columns and 12 with two lanes each.  Elsewhere 32 consecutive columns a round.
+__host__ __device__ constexpr int grad_rounds(int P) { return P == 8 ? 2 : (P == 10 ? 4 : (P * P + 31) / 32); }
+
+__device__ __forceinline__ bool grad_column(int P, int round, int lane, int *jx, int *jy, int *sub, int *lpp) {
+    *sub = 0;
+    *lpp = 1;
+    if (P != 8 && P != 10) {
+        int idx;
+        if (!stencil_row(32 * round, P, lane, &idx, sub, lpp)) return false;
+        *jx = idx % P;
+        *jy = idx / P;
+        return true;
+    }
+    if (round < 2) {
+        *jx = lane & 7;
+        *jy = 2 * (lane >> 3) + round;
+        return true;
+    }
+    if (round == 2) {
+        const int e = lane - 16;   // columns 8 and 9 of rows 0, 1, 2, 5
+        *jx = e < 0 ? lane & 7 : 8 + (e & 1);
+        *jy = e < 0 ? 8 + (lane >> 3) : (e < 6 ? e >> 1 : 5);
+        return lane < 24;
+    }
+    const int c = lane < 12 ? lane : lane - 12, q = c >> 1;   // columns 8 and 9 of rows 3, 4, 6, 7, 8, 9
+    *jx = 8 + (c & 1);
+    *jy = q < 2 ? 3 + q : 4 + q;
+    *sub = lane < 12 ? 0 : 1;
+    *lpp = 2;
+    return lane < 24;
+}
+
 // Contraction as a warp-per-particle gather: the grids of the gradient form (one
 // per vector) are small enough to be read mostly from L2.  Lanes take the (x, y)
 // columns of the stencil, each runs its z column; fixed summation order.  Warps
@@ -348,10 +383,9 @@ __global__ void __launch_bounds__(256, 3) k_contract_grad_warp(const float *__re
         float acc[3 * NR];
 #pragma unroll
         for (int c = 0; c < 3 * NR; ++c) acc[c] = 0.f;
-        for (int row0 = 0; row0 < P * P; row0 += 32) {
-            int idx, sub, lpp;
-            if (!stencil_row(row0, P, lane, &idx, &sub, &lpp)) continue;
-            const int jx = idx % P, jy = idx / P;
+        for (int round = 0; round < grad_rounds(P); ++round) {
+            int jx, jy, sub, lpp;
+            if (!grad_column(P, round, lane, &jx, &jy, &sub, &lpp)) continue;
             int ix = sx + jx;
             if (ix >= Nx) ix -= Nx;
             int iy = sy + jy;
@@ -387,60 +421,57 @@ __global__ void __launch_bounds__(256, 3) k_contract_grad_warp(const float *__re
     }
 }
 
-// Contraction by home blocks (the default where the support is 8 or 10): one CTA per
-// kHomeBlock^3 block of grid nodes stages every node its particles' stencils can
-// reach -- the block grown by P - 1 nodes per axis, R = kHomeBlock + P - 1 per axis,
-// one plane of R^3 floats per vector -- in shared memory with coalesced loads, and
-// its particles' offsets and per-axis factors (kHomeChunk particles at a time).  One
-// warp per particle then runs the sums of k_contract_grad_warp in the same order,
-// from shared memory and registers instead of L2: the results are bit-identical.  P
-// is a template parameter, so the z runs unroll completely with the z factors in
-// registers and the shared-memory offsets are immediates.  A node is staged by about
-// (R / kHomeBlock)^3 blocks (9.6 at P = 10), all from L2.
-// With one vector a CTA takes 2 x 2 home blocks (5.2 stagings a node): 0.256 -> 0.156 ms for N = 2e5 on 240^3, with the
-// region staged row by row (the wraps worked out once a row, not once a node).  The sums end one to a lane, converted and
-// scaled together: lane 0's 3 NR conversions and multiplications had cost a warp 6 NR float64 instructions a particle
-// (0.209 -> 0.174 ms for N = 1e5, three vectors, 192^3; 0.155 -> 0.144 for N = 2e5, one vector, 240^3; 0.168 and 0.136
-// with the staging copies asynchronous).
-// 67 KB of shared memory at P = 10 and 3 vectors, 3 blocks per SM (80 registers): the mixed step at the bench
-// workload took 19.25 ms against 20.08 with the warp gather; float4 nodes (the 3 vectors interleaved, 87 KB,
-// 2 blocks per SM) took 20.17.
-constexpr int kHomeChunk = 32;
+// Contraction by home blocks (the default where the support is 8 or 10): one CTA per kHomeBlock^3 block of grid nodes
+// stages every node its particles' stencils can reach -- the block grown by P - 1 nodes per axis, one plane of nodes per
+// vector -- in shared memory, and its particles' offsets and per-axis factors (kHomeChunk particles at a time).  One warp
+// per particle then runs the sums of k_contract_grad_warp in the same order, from shared memory and registers instead of
+// L2: the results are bit-identical.  P is a template parameter, so the z runs unroll completely with the z factors in
+// registers and the shared-memory offsets are immediates.  A node is staged by about (1 + (P - 1) / 8)^3 blocks (9.6 at
+// P = 10), all from L2; with one vector a CTA takes three home blocks along y (6.2).
+// Shared memory bounds it (a node's read and its staging), so the rows lie 20 floats apart: the columns that a round of the
+// warp reads together then hit different banks (grad_column), and a row is staged by five 16-byte copies.  The sums end
+// one to a lane, converted and scaled together: lane 0's 3 NR conversions and multiplications had cost a warp 6 NR float64
+// instructions a particle.  Three vectors of N = 1e5 on 144^3 / one of N = 2e5 on 192^3: 0.209 / 0.155 ms with two-way bank
+// conflicts, staging by single floats and lane 0's epilogue; 0.168 / 0.136 with the sums one to a lane and asynchronous
+// copies; 0.118 / 0.109 so.
+// 78 KB of shared memory at P = 10 and 3 vectors, 3 blocks per SM (80 registers); float4 nodes (the 3 vectors interleaved,
+// 2 blocks per SM) were slower.
+constexpr int kHomeChunk = 24;
+constexpr int kHomeRow = 20;   // floats from one row of the region to the next (grad_column), whole 16-byte pieces
 
-// A CTA covers BX x BY home blocks: the margin of P - 1 nodes is staged once for all of them.
-template <int NR, int P, int BX, int BY>
+// A CTA covers BY home blocks along y: the margin of P - 1 nodes is staged once for all of them.
+template <int NR, int P, int BY>
 struct HomeTile {
-    static constexpr int RX = BX * kHomeBlock + P - 1, RY = BY * kHomeBlock + P - 1, RZ = kHomeBlock + P - 1;
-    static constexpr int VOL = RX * RY * RZ;
+    static constexpr int RX = kHomeBlock + P - 1, RY = BY * kHomeBlock + P - 1, RZ = kHomeBlock + P - 1;
+    static constexpr int VOL = kHomeRow * RY * RZ;
+    static_assert(RX <= kHomeRow, "a row holds the region's columns");
     static constexpr size_t smem =
         sizeof(float) * ((size_t)NR * VOL + 2 * kHomeChunk * 3 * P) + sizeof(int) * 4 * kHomeChunk;
 };
 
-template <int NR, int P, int BX, int BY>
+template <int NR, int P, int BY>
 __global__ void __launch_bounds__(256, NR == 1 ? 4 : 3) k_contract_grad_home(
     const float *__restrict__ grid, int64_t n, int r0, const int64_t *__restrict__ hstart,
     const int32_t *__restrict__ hentries, int nbx, int nby, const int32_t *__restrict__ start,
     const float *__restrict__ w, const float *__restrict__ g, GridParams gp, double *__restrict__ out) {
-    using HT = HomeTile<NR, P, BX, BY>;
-    constexpr int RX = HT::RX, RY = HT::RY, RZ = HT::RZ, VOL = HT::VOL, RR = RX * RY;
+    using HT = HomeTile<NR, P, BY>;
+    constexpr int RX = HT::RX, RY = HT::RY, RZ = HT::RZ, VOL = HT::VOL, RS = kHomeRow, RR = RS * RY;
     constexpr int F = 3 * P;                        // per-axis factors of one particle
-    constexpr int NB = BX * BY;
-    extern __shared__ float s_reg[];                // [NR][VOL] nodes, x fastest
+    extern __shared__ __align__(16) float s_reg[];  // [NR][VOL] nodes, x fastest
     float *s_w = s_reg + NR * VOL;                  // [kHomeChunk][F]
     float *s_g = s_w + kHomeChunk * F;              // [kHomeChunk][F]
     int *s_p = (int *)(s_g + kHomeChunk * F);       // [kHomeChunk][4]: offsets in the block, particle id
-    const int tbx = (nbx + BX - 1) / BX, tby = (nby + BY - 1) / BY;
+    const int tby = (nby + BY - 1) / BY;
     const int64_t b = blockIdx.x;
-    const int bx0 = (int)(b % tbx) * BX, by0 = (int)((b / tbx) % tby) * BY, bz = (int)(b / ((int64_t)tbx * tby));
+    const int bx = (int)(b % nbx), by0 = (int)((b / nbx) % tby) * BY, bz = (int)(b / ((int64_t)nbx * tby));
     // the home blocks' particle lists, one after the other
-    int64_t first[NB];
-    int upto[NB], total = 0;
+    int64_t first[BY];
+    int upto[BY], total = 0;
 #pragma unroll
-    for (int k = 0; k < NB; ++k) {
-        const int bx = bx0 + k % BX, by = by0 + k / BX;
+    for (int k = 0; k < BY; ++k) {
         first[k] = 0;
-        if (bx < nbx && by < nby) {
-            const int64_t hb = ((int64_t)bz * nby + by) * nbx + bx;
+        if (by0 + k < nby) {
+            const int64_t hb = ((int64_t)bz * nby + by0 + k) * nbx + bx;
             first[k] = hstart[hb] - total;
             total += (int)(hstart[hb + 1] - hstart[hb]);
         }
@@ -450,12 +481,12 @@ __global__ void __launch_bounds__(256, NR == 1 ? 4 : 3) k_contract_grad_home(
     auto entry = [&](int q) {
         int64_t e = first[0];
 #pragma unroll
-        for (int k = 1; k < NB; ++k) e = q >= upto[k - 1] ? first[k] : e;
+        for (int k = 1; k < BY; ++k) e = q >= upto[k - 1] ? first[k] : e;
         return (int64_t)hentries[e + q];
     };
     const int Nx = gp.N[0], Ny = gp.N[1], Nz = gp.N[2];
     const int64_t G = gp.G;
-    const int X0 = bx0 * kHomeBlock, Y0 = by0 * kHomeBlock, Z0 = bz * kHomeBlock;
+    const int X0 = bx * kHomeBlock, Y0 = by0 * kHomeBlock, Z0 = bz * kHomeBlock;
     const float *g0 = grid + (int64_t)r0 * G;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int oc = warp_sums_index<3 * NR>(lane);   // the output component this lane writes
@@ -464,27 +495,21 @@ __global__ void __launch_bounds__(256, NR == 1 ? 4 : 3) k_contract_grad_home(
         i -= i >= N ? N : 0;
         return i - (i >= N ? N : 0);
     };
-    // rows of the region: LX lanes a row (a 17th column goes by itself), the x wrap worked out once
-    constexpr int LX = RX <= 17 ? 16 : 32, ROWS = 32 / LX;
-    static_assert(RX <= LX + 1, "one column at most is left over");
-    {
-        const int x = lane % LX, gx = wrap2(X0 + x, Nx);
-        if (x < RX) {
-            for (int row = wid * ROWS + lane / LX; row < RY * RZ; row += 8 * ROWS) {
-                const int z = row / RY, y = row - z * RY;
-                const float *src = g0 + ((int64_t)wrap2(Z0 + z, Nz) * Ny + wrap2(Y0 + y, Ny)) * Nx + gx;
+    if (Nx % 4 == 0) {   // rows by 16-byte pieces: X0 is a multiple of 8, so no piece wraps within
+        constexpr int PC = RS / 4;
+        for (int i = threadIdx.x; i < RY * RZ * PC; i += 256) {
+            const int row = i / PC, c = i - row * PC, z = row / RY, y = row - z * RY;
+            const float *src = g0 + ((int64_t)wrap2(Z0 + z, Nz) * Ny + wrap2(Y0 + y, Ny)) * Nx + wrap2(X0 + 4 * c, Nx);
 #pragma unroll
-                for (int r = 0; r < NR; ++r) copy_async(s_reg + r * VOL + row * RX + x, src + r * G);
-            }
+            for (int r = 0; r < NR; ++r)
+                copy_async((float4 *)(s_reg + r * VOL + row * RS + 4 * c), (const float4 *)(src + r * G));
         }
-        if (RX > LX) {
-            const int gl = wrap2(X0 + LX, Nx);
-            for (int row = threadIdx.x; row < RY * RZ; row += 256) {
-                const int z = row / RY, y = row - z * RY;
-                const float *src = g0 + ((int64_t)wrap2(Z0 + z, Nz) * Ny + wrap2(Y0 + y, Ny)) * Nx + gl;
+    } else {
+        for (int i = threadIdx.x; i < RY * RZ * RX; i += 256) {
+            const int row = i / RX, x = i - row * RX, z = row / RY, y = row - z * RY;
+            const float *src = g0 + ((int64_t)wrap2(Z0 + z, Nz) * Ny + wrap2(Y0 + y, Ny)) * Nx + wrap2(X0 + x, Nx);
 #pragma unroll
-                for (int r = 0; r < NR; ++r) copy_async(s_reg + r * VOL + row * RX + LX, src + r * G);
-            }
+            for (int r = 0; r < NR; ++r) copy_async(s_reg + r * VOL + row * RS + x, src + r * G);
         }
     }
     for (int c0 = 0; c0 < total; c0 += kHomeChunk) {
@@ -497,7 +522,7 @@ __global__ void __launch_bounds__(256, NR == 1 ? 4 : 3) k_contract_grad_home(
         }
         if (threadIdx.x < cnt) {
             const int64_t a = entry(c0 + threadIdx.x);
-            // a home block holds the stencil's first node: offsets in [0, BX kHomeBlock) and so on
+            // a home block holds the stencil's first node: offsets in [0, kHomeBlock), in y [0, BY kHomeBlock)
             s_p[4 * threadIdx.x + 0] = start[3 * a] - X0;
             s_p[4 * threadIdx.x + 1] = start[3 * a + 1] - Y0;
             s_p[4 * threadIdx.x + 2] = start[3 * a + 2] - Z0;
@@ -519,11 +544,10 @@ __global__ void __launch_bounds__(256, NR == 1 ? 4 : 3) k_contract_grad_home(
 #pragma unroll
             for (int c = 0; c < 3 * NR; ++c) acc[c] = 0.f;
 #pragma unroll
-            for (int row0 = 0; row0 < P * P; row0 += 32) {
-                int idx, sub, lpp;   // lpp is a constant of each unrolled round
-                if (!stencil_row(row0, P, lane, &idx, &sub, &lpp)) continue;
-                const int jx = idx % P, jy = idx / P;
-                const float *col = s_reg + (oz * RY + oy + jy) * RX + ox + jx;
+            for (int round = 0; round < grad_rounds(P); ++round) {
+                int jx, jy, sub, lpp;   // lpp is a constant of each unrolled round
+                if (!grad_column(P, round, lane, &jx, &jy, &sub, &lpp)) continue;
+                const float *col = s_reg + (oz * RY + oy + jy) * RS + ox + jx;
                 float s0[NR], s1[NR];
 #pragma unroll
                 for (int r = 0; r < NR; ++r) s0[r] = s1[r] = 0.f;
@@ -570,33 +594,32 @@ bool contract_grad_home_supported(const GridParams &gp) {
     return true;
 }
 
-template <int NR, int P, int BX, int BY>
+template <int NR, int P, int BY>
 static int home_launch(const float *grid, int64_t n, int r0, const int32_t *start, const float *w, const float *g,
                        const GridParams &gp, const TileBins &tb, double *out, cudaStream_t s) {
-    constexpr size_t smem = HomeTile<NR, P, BX, BY>::smem;
+    constexpr size_t smem = HomeTile<NR, P, BY>::smem;
     if (smem > 48 * 1024)
-        MPS_CUDA_TRY(cudaFuncSetAttribute(k_contract_grad_home<NR, P, BX, BY>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned blocks = (unsigned)((tb.nhb[0] + BX - 1) / BX) * (unsigned)((tb.nhb[1] + BY - 1) / BY) *
-                            (unsigned)tb.nhb[2];
-    k_contract_grad_home<NR, P, BX, BY><<<blocks, 256, smem, s>>>(grid, n, r0, tb.hstart, tb.hentries, tb.nhb[0],
+        MPS_CUDA_TRY(cudaFuncSetAttribute(k_contract_grad_home<NR, P, BY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)smem));
+    const unsigned blocks = (unsigned)tb.nhb[0] * (unsigned)((tb.nhb[1] + BY - 1) / BY) * (unsigned)tb.nhb[2];
+    k_contract_grad_home<NR, P, BY><<<blocks, 256, smem, s>>>(grid, n, r0, tb.hstart, tb.hentries, tb.nhb[0],
                                                                   tb.nhb[1], start, w, g, gp, out);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
 }
 
-// One vector leaves room for four home blocks to a CTA: taken where every SM still gets four CTAs and the wider region
+// One vector leaves room for three home blocks to a CTA: taken where every SM still gets four CTAs and the longer region
 // wraps at most twice.
 template <int P>
 static int home_dispatch(const float *grid, int64_t n, int nrhs, const int32_t *start, const float *w, const float *g,
                          const GridParams &gp, const TileBins &tb, double *out, cudaStream_t s) {
-    const bool wide = tb.nhome >= 4 * 4 * 152 && gp.N[0] >= 16 && gp.N[1] >= 16;
+    const bool wide = tb.nhome >= 3 * 4 * 152 && gp.N[1] >= 16;
     for (int r0 = 0; r0 < nrhs; r0 += 3) {
         const int nr = min(3, nrhs - r0);
-        const int rc = nr == 3   ? home_launch<3, P, 1, 1>(grid, n, r0, start, w, g, gp, tb, out, s)
-                       : nr == 2 ? home_launch<2, P, 1, 1>(grid, n, r0, start, w, g, gp, tb, out, s)
-                       : wide    ? home_launch<1, P, 2, 2>(grid, n, r0, start, w, g, gp, tb, out, s)
-                                 : home_launch<1, P, 1, 1>(grid, n, r0, start, w, g, gp, tb, out, s);
+        const int rc = nr == 3   ? home_launch<3, P, 1>(grid, n, r0, start, w, g, gp, tb, out, s)
+                       : nr == 2 ? home_launch<2, P, 1>(grid, n, r0, start, w, g, gp, tb, out, s)
+                       : wide    ? home_launch<1, P, 3>(grid, n, r0, start, w, g, gp, tb, out, s)
+                                 : home_launch<1, P, 1>(grid, n, r0, start, w, g, gp, tb, out, s);
         if (rc) return rc;
     }
     return MPS_OK;
