@@ -2636,10 +2636,10 @@ extern "C" int mps_system_create(const mps_system_desc *d, mps_system **out, mps
     int64_t *cell3 = nullptr, *cnt27 = nullptr, *off27 = nullptr;
     void *bins = nullptr, *scan_tmp = nullptr;
     int *err = nullptr;
-    float *xf = nullptr;
+    float4 *xf = nullptr;   // float positions and ids in cell order
     unsigned *maxbits = nullptr;
     double maxabs = 0.0;
-    CR_TRY(dalloc(&xf, sizeof(float) * 3 * n, st));
+    CR_TRY(dalloc(&xf, sizeof(float4) * n, st));
     CR_TRY(dalloc(&maxbits, sizeof(unsigned) * 4, st));
     CR_TRY(dalloc(&cell3, sizeof(int64_t) * 3 * n, st));
     CR_TRY(dalloc(&bins, cell_bins_bytes(n, ncells), st));
@@ -2666,7 +2666,7 @@ extern "C" int mps_system_create(const mps_system_desc *d, mps_system **out, mps
         rc = MPS_CUDA_ERR;
     if (!rc) s->gp.order = s->order;
     int64_t np = 0;
-    if (!rc) rc = positions_f32(s->x, n, xf, maxbits, &maxabs, st);
+    if (!rc) rc = positions_f32(s->x, cb.sorted, n, xf, maxbits, &maxabs, st);
     int64_t *last2 = reinterpret_cast<int64_t *>(s->host_scr);   // page-locked, free until the first solve
     if (!rc) rc = csr_pairs_count(s->x, xf, maxabs, d->box, d->rc, cb, cnt27, off27, scan_tmp, last2, st);
     // the grid geometry and k-space (side stream) and the inner grid (the capture stream, idle until the first
