@@ -58,8 +58,9 @@ __device__ __forceinline__ int64_t seg_index(const double *__restrict__ rv, int6
 
 // One group of 8 lanes per particle over its CSR row (N = 200,000, 12 million pairs: 1.75 ms and 0.39 for the float64
 // copy of the list before, 1.21 ms with the slopes from a table, the guessed index, no division and the list read as it
-// is).  T: the pair data's type; the double-float list of a system that
-// has made no float64 copy is read as it is, its values joined by one float64 addition each.
+// is; 1.04 with the part along the particle's own moment summed as a scalar and one multiply-add a term).  T: the pair
+// data's type; the double-float list of a system that has made no float64 copy is read as it is, its values joined by one
+// float64 addition each.
 template <typename T>
 __global__ void __launch_bounds__(256) k_rs_force(const double *__restrict__ m, int64_t n,
                                                   const int64_t *__restrict__ row_ptr, PairData<T> pd,
@@ -68,13 +69,14 @@ __global__ void __launch_bounds__(256) k_rs_force(const double *__restrict__ m, 
                                                   double *__restrict__ F, int *__restrict__ err) {
     constexpr int G = 8;
     const int lane = threadIdx.x % G;
+    const int oc = warp_sums_index<4, G / 2>(lane);   // the sum this lane holds at the end
     const int64_t grp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
     const int64_t ngrp = ((int64_t)gridDim.x * blockDim.x) / G;
     const double inv_dr = slope[0].x;
     for (int64_t i0 = grp; i0 < n; i0 += ngrp) {
         const int64_t a = order ? (int64_t)order[i0] : i0;
         const double amx = m[3 * a], amy = m[3 * a + 1], amz = m[3 * a + 2];
-        double fx = 0.0, fy = 0.0, fz = 0.0;
+        double f[4] = {0.0, 0.0, 0.0, 0.0};   // the force without its part along the particle's own moment; that part
         for (int64_t e = row_ptr[a] + lane; e < row_ptr[a + 1]; e += G) {
             const int32_t b = pd.nbr[e];
             const double d = (double)pd.dist[e];
@@ -97,21 +99,16 @@ __global__ void __launch_bounds__(256) k_rs_force(const double *__restrict__ m, 
             // grad_r [A (ma.mb) + (B - A)(ma.r)(mb.r)]
             const double cr = sl.x * ab + (sl.y - sl.x - 2.0 * s) * arbr;
             const double sb = s * br, sa = s * ar;
-            fx -= cr * rx + sb * amx + sa * mbx;
-            fy -= cr * ry + sb * amy + sa * mby;
-            fz -= cr * rz + sb * amz + sa * mbz;
+            f[0] -= cr * rx;
+            f[1] -= cr * ry;
+            f[2] -= cr * rz;
+            f[0] -= sa * mbx;
+            f[1] -= sa * mby;
+            f[2] -= sa * mbz;
+            f[3] -= sb;
         }
-#pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) {
-            fx += __shfl_xor_sync(0xffffffffu, fx, o, G);
-            fy += __shfl_xor_sync(0xffffffffu, fy, o, G);
-            fz += __shfl_xor_sync(0xffffffffu, fz, o, G);
-        }
-        if (lane == 0) {
-            F[3 * a] = fx;
-            F[3 * a + 1] = fy;
-            F[3 * a + 2] = fz;
-        }
+        const double v = warp_sums<4, G / 2>(f, lane), own = __shfl_sync(0xffffffffu, v, 6, G);   // lane 6 holds f[3]
+        if (oc >= 0 && oc < 3) F[3 * a + oc] = v + own * (oc == 0 ? amx : (oc == 1 ? amy : amz));
     }
 }
 

@@ -183,7 +183,10 @@ __global__ void __launch_bounds__(128) k_probe_real(const double *__restrict__ x
             const double *m = p + 3 * (int64_t)b;
             const double ba = (B - A) * ((m[0] * r[0] + m[1] * r[1] + m[2] * r[2]) * y) * y;
 #pragma unroll
-            for (int k = 0; k < 3; ++k) acc[k] += A * m[k] + ba * r[k];
+            for (int k = 0; k < 3; ++k) {   // (two multiply-adds, not three instructions)
+                acc[k] += A * m[k];
+                acc[k] += ba * r[k];
+            }
         });
         const double v = warp_sum4(acc[0], acc[1], acc[2], 0.0, lane);
         if ((lane & 7) == 0 && lane < 24) out[3 * e + lane / 8] = v;
@@ -240,9 +243,15 @@ __global__ void __launch_bounds__(128) k_probe_real_quad(const double *__restric
             const double rQr = Q0 * (rx * rx - rz * rz) + 2 * Q1 * rx * ry + 2 * Q2 * rx * rz +
                                Q3 * (ry * ry - rz * rz) + 2 * Q4 * ry * rz;
             const double sE = (B - A) * sr - 0.5 * Cc * rQr;
-            acc[0] += A * Sx + sE * rx - D * Qr0;
-            acc[1] += A * Sy + sE * ry - D * Qr1;
-            acc[2] += A * Sz + sE * rz - D * Qr2;
+            acc[0] += A * Sx;
+            acc[1] += A * Sy;
+            acc[2] += A * Sz;
+            acc[0] += sE * rx;
+            acc[1] += sE * ry;
+            acc[2] += sE * rz;
+            acc[0] -= D * Qr0;
+            acc[1] -= D * Qr1;
+            acc[2] -= D * Qr2;
             const double q5[5] = {rx * rx, rx * ry, rx * rz, ry * ry, ry * rz};
             const double srs[5] = {2 * Sx * rx, Sx * ry + rx * Sy, Sx * rz + rx * Sz, 2 * Sy * ry, Sy * rz + ry * Sz};
             const double qq[5] = {4 * Qr0 * rx, 2 * (Qr0 * ry + rx * Qr1), 2 * (Qr0 * rz + rx * Qr2), 4 * Qr1 * ry,
@@ -250,11 +259,14 @@ __global__ void __launch_bounds__(128) k_probe_real_quad(const double *__restric
             const double Qv[5] = {Q0, Q1, Q2, Q3, Q4};
             const double cq = Cc * sr + 0.5 * I * rQr;
             const double di = (D + E) * sr + 0.5 * (F + H) * rQr;
+            const double hG = 0.5 * Gg, hH = 0.5 * H;
 #pragma unroll
             for (int k = 0; k < 5; ++k) {
-                double v = cq * q5[k] + D * srs[k] + 0.5 * (Gg * Qv[k] + H * qq[k]);
-                if (k == 0 || k == 3) v += di;
-                acc[3 + k] += v;
+                acc[3 + k] += cq * q5[k];
+                acc[3 + k] += D * srs[k];
+                acc[3 + k] += hG * Qv[k];
+                acc[3 + k] += hH * qq[k];
+                if (k == 0 || k == 3) acc[3 + k] += di;
             }
         });
         const double v = warp_sum4(acc[0], acc[1], acc[2], acc[3], lane), w = warp_sum4(acc[4], acc[5], acc[6], acc[7], lane);
@@ -311,7 +323,10 @@ __global__ void __launch_bounds__(128) k_probe_real_cs(const double *__restrict_
             const double *m = p + 3 * (int64_t)b;
             const double ba = (B - A) * ((m[0] * r[0] + m[1] * r[1] + m[2] * r[2]) * y) * y;
 #pragma unroll
-            for (int k = 0; k < 3; ++k) acc[k] += A * m[k] + ba * r[k];
+            for (int k = 0; k < 3; ++k) {   // (two multiply-adds, not three instructions)
+                acc[k] += A * m[k];
+                acc[k] += ba * r[k];
+            }
         });
         const double v = warp_sum4(acc[0], acc[1], acc[2], 0.0, lane);
         if ((lane & 7) == 0 && lane < 24) out[3 * e + lane / 8] = v;

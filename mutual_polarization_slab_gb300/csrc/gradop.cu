@@ -79,6 +79,8 @@ __global__ void k_grad_scale_coef(GridParams gp, const double *__restrict__ H, f
 // divisions, no shared-memory atomics); the warps then walk only the particles that reach their patch, from ballots.
 // Alone, at depth 12: 0.288 -> 0.217 ms a launch for three vectors of N = 1e5 on 144^3, 0.387 -> 0.241 for one of
 // N = 2e5 on 192^3.
+// An update of two multiply-adds (not a product, a multiply-add and an addition): 0.223 -> 0.200 ms for the three
+// vectors beside the pair sum, 0.244 -> 0.241 for the one.
 // particles staged per barrier interval: 96 measured 0.300 ms per launch at the bench workload against 0.323
 // for 32 (fewer barriers, and the warps' uneven shares of a chunk even out), 0.306 for 64 and 0.301 for 128
 constexpr int kGChunk = 96;
@@ -174,7 +176,10 @@ __global__ void __launch_bounds__(256, TZ > 12 ? 3 : (TZ > 8 ? 4 : 5)) k_spread_
                     for (int z = z0; z < z0 + 4 && z < TZ; ++z) {
                         const float2 fz = s_f[pp][kTileX + kTileY + z];
 #pragma unroll
-                        for (int r = 0; r < NR; ++r) acc[z][r] += cA[r] * fz.x + cB[r] * fz.y;
+                        for (int r = 0; r < NR; ++r) {   // (one sum a + b on the right is three instructions, this two)
+                            acc[z][r] += cA[r] * fz.x;
+                            acc[z][r] += cB[r] * fz.y;
+                        }
                     }
                 }
             }

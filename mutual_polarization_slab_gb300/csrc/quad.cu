@@ -503,9 +503,15 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_rs_quad(const d
                           2 * Q4 * ry * rz;
             // field: A S + (B-A)(S.r) r - (C rQr r)/2 - D Q.r
             const T sE = (B - A) * sr - (T)0.5 * Cc * rQr;
-            acc[0] += A * Sx + sE * rx - D * Qr0;
-            acc[1] += A * Sy + sE * ry - D * Qr1;
-            acc[2] += A * Sz + sE * rz - D * Qr2;
+            acc[0] += A * Sx;
+            acc[1] += A * Sy;
+            acc[2] += A * Sz;
+            acc[0] += sE * rx;
+            acc[1] += sE * ry;
+            acc[2] += sE * rz;
+            acc[0] -= D * Qr0;
+            acc[1] -= D * Qr1;
+            acc[2] -= D * Qr2;
             // gradient, 5-component (xx, xy, xz, yy, yz)
             const T q5[5] = {rx * rx, rx * ry, rx * rz, ry * ry, ry * rz};
             const T srs[5] = {2 * Sx * rx, Sx * ry + rx * Sy, Sx * rz + rx * Sz, 2 * Sy * ry, Sy * rz + ry * Sz};
@@ -514,11 +520,14 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_rs_quad(const d
             const T Qv[5] = {Q0, Q1, Q2, Q3, Q4};
             const T cq = Cc * sr + (T)0.5 * I * rQr;
             const T di = (D + E) * sr + (T)0.5 * (F + H) * rQr;
+            const T hG = (T)0.5 * Gg, hH = (T)0.5 * H;
 #pragma unroll
             for (int k = 0; k < 5; ++k) {
-                T v = cq * q5[k] + D * srs[k] + (T)0.5 * (Gg * Qv[k] + H * qq[k]);
-                if (k == 0 || k == 3) v += di;
-                acc[3 + k] += v;
+                acc[3 + k] += cq * q5[k];
+                acc[3 + k] += D * srs[k];
+                acc[3 + k] += hG * Qv[k];
+                acc[3 + k] += hH * qq[k];
+                if (k == 0 || k == 3) acc[3 + k] += di;
             }
         }
         const T v = warp_sums<8, G / 2>(acc, lane);

@@ -226,9 +226,13 @@ __global__ void __launch_bounds__(256) k_rs_csr(const double *__restrict__ m, do
                     const TM *mb = mT + ((int64_t)(r0 + r) * n + b) * 3;
                     const T mx = (T)mb[0], my = (T)mb[1], mz = (T)mb[2];
                     const T s = ba * (mx * rx + my * ry + mz * rz);
-                    acc[r][0] += av * mx + s * rx;
-                    acc[r][1] += av * my + s * ry;
-                    acc[r][2] += av * mz + s * rz;
+                    // (one multiply-add each; acc += av * mx + s * rx would take three instructions a component)
+                    acc[r][0] += av * mx;
+                    acc[r][1] += av * my;
+                    acc[r][2] += av * mz;
+                    acc[r][0] += s * rx;
+                    acc[r][1] += s * ry;
+                    acc[r][2] += s * rz;
                 }
             }
         }
@@ -385,9 +389,12 @@ __global__ void __launch_bounds__(256) k_rs_csr_f32(const double *__restrict__ m
             const float rx = pd.rx[e], ry = pd.ry[e], rz = pd.rz[e];
             const float4 v = __ldg(mf + (int64_t)b * nrhs + rc);
             const float s = ba * (v.x * rx + v.y * ry + v.z * rz);
-            ax += av * v.x + s * rx;
-            ay += av * v.y + s * ry;
-            az += av * v.z + s * rz;
+            ax += av * v.x;
+            ay += av * v.y;
+            az += av * v.z;
+            ax += s * rx;
+            ay += s * ry;
+            az += s * rz;
         }
 #pragma unroll
         for (int o = RL; o < 32; o <<= 1) {
