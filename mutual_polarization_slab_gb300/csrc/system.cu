@@ -3056,11 +3056,11 @@ extern "C" int mps_field_map(const double *x_e, int64_t n_e, const double *x_p, 
     const GridParams gp = make_grid_params(Ngrid, box, xi, eta, P);
     const int64_t Gc = (int64_t)(gp.N[0] / 2 + 1) * gp.N[1] * gp.N[2];
     int32_t *start_p = nullptr, *start_e = nullptr;
-    double *w_p = nullptr, *w_e = nullptr, *grid = nullptr, *spec = nullptr, *H = nullptr, *wave = nullptr,
-           *real = nullptr;
+    double *w_p = nullptr, *w_e = nullptr, *grid = nullptr, *spec = nullptr, *H = nullptr, *hs = nullptr,
+           *wave = nullptr, *real = nullptr;
     void *work = nullptr;
     auto cleanup = [&]() {
-        void *ptrs[] = {start_p, start_e, w_p, w_e, grid, spec, H, wave, real, work};
+        void *ptrs[] = {start_p, start_e, w_p, w_e, grid, spec, H, hs, wave, real, work};
         for (void *q : ptrs)
             if (q) cudaFreeAsync(q, st);
     };
@@ -3074,26 +3074,36 @@ extern "C" int mps_field_map(const double *x_e, int64_t n_e, const double *x_p, 
     if (!rc_) rc_ = dalloc(&H, sizeof(double) * (size_t)Gc, st);
     if (!rc_) rc_ = dalloc(&wave, sizeof(double) * 3 * (size_t)n_e, st);
     if (!rc_) rc_ = dalloc(&real, sizeof(double) * 3 * (size_t)n_e, st);
-    // wave space: spread the source dipoles, D2Z, H k^k^ scale, Z2D, contract at the probes
+    // wave space: spread the source dipoles, transform, H k^k^ scale, transform back, contract at the probes
     if (!rc_) rc_ = grid_geometry(x_p, n_p, gp, start_p, w_p, nullptr, st);
     if (!rc_) rc_ = spread<double>(p, n_p, 1, start_p, w_p, gp, grid, st);
     if (!rc_) rc_ = green_half(gp, H, nullptr, st);
-    CachedPlan fwd{}, inv{};
-    if (!rc_) rc_ = get_plan(CUFFT_D2Z, gp, 3, &fwd);
-    if (!rc_) rc_ = get_plan(CUFFT_Z2D, gp, 3, &inv);
-    if (!rc_) rc_ = dalloc(&work, std::max(fwd.work, inv.work) + 16, st);
-    if (!rc_) {
-        std::lock_guard<std::mutex> lk(g_plan_mu);
-        if (cufftSetWorkArea(fwd.h, work) != CUFFT_SUCCESS || cufftSetStream(fwd.h, st) != CUFFT_SUCCESS ||
-            cufftExecD2Z(fwd.h, (cufftDoubleReal *)grid, (cufftDoubleComplex *)spec) != CUFFT_SUCCESS)
-            rc_ = MPS_CUFFT_ERR;
-    }
-    if (!rc_) rc_ = scale_half<double>(spec, 1, gp, H, st);
-    if (!rc_) {
-        std::lock_guard<std::mutex> lk(g_plan_mu);
-        if (cufftSetWorkArea(inv.h, work) != CUFFT_SUCCESS || cufftSetStream(inv.h, st) != CUFFT_SUCCESS ||
-            cufftExecZ2D(inv.h, (cufftDoubleComplex *)spec, (cufftDoubleReal *)grid) != CUFFT_SUCCESS)
-            rc_ = MPS_CUFFT_ERR;
+    F64Plan3 f64;
+    if (!rc_) rc_ = f64_plan(gp, &f64);
+    if (f64.ok) {   // the transforms of the float64 operator; cuFFT where an axis is longer or has a larger prime
+        if (!rc_) rc_ = dalloc(&hs, sizeof(double) * (size_t)Gc, st);
+        if (!rc_) rc_ = f64_scale_coef(gp, H, hs, st);
+        if (!rc_) rc_ = f64_forward_xy(grid, spec, 3, gp, f64, st);
+        if (!rc_) rc_ = f64_z_scale_dipole(spec, 1, gp, f64, hs, st);
+        if (!rc_) rc_ = f64_inverse_yx(spec, grid, 3, gp, f64, st);
+    } else {
+        CachedPlan fwd{}, inv{};
+        if (!rc_) rc_ = get_plan(CUFFT_D2Z, gp, 3, &fwd);
+        if (!rc_) rc_ = get_plan(CUFFT_Z2D, gp, 3, &inv);
+        if (!rc_) rc_ = dalloc(&work, std::max(fwd.work, inv.work) + 16, st);
+        if (!rc_) {
+            std::lock_guard<std::mutex> lk(g_plan_mu);
+            if (cufftSetWorkArea(fwd.h, work) != CUFFT_SUCCESS || cufftSetStream(fwd.h, st) != CUFFT_SUCCESS ||
+                cufftExecD2Z(fwd.h, (cufftDoubleReal *)grid, (cufftDoubleComplex *)spec) != CUFFT_SUCCESS)
+                rc_ = MPS_CUFFT_ERR;
+        }
+        if (!rc_) rc_ = scale_half<double>(spec, 1, gp, H, st);
+        if (!rc_) {
+            std::lock_guard<std::mutex> lk(g_plan_mu);
+            if (cufftSetWorkArea(inv.h, work) != CUFFT_SUCCESS || cufftSetStream(inv.h, st) != CUFFT_SUCCESS ||
+                cufftExecZ2D(inv.h, (cufftDoubleComplex *)spec, (cufftDoubleReal *)grid) != CUFFT_SUCCESS)
+                rc_ = MPS_CUFFT_ERR;
+        }
     }
     if (!rc_) rc_ = grid_geometry(x_e, n_e, gp, start_e, w_e, nullptr, st);
     if (!rc_) rc_ = contract<double>(grid, n_e, 1, start_e, w_e, gp, wave, st);
