@@ -767,9 +767,9 @@ static int f64_x(bool fwd, const double *gin, double *gout, double2 *spec, int n
     return MPS_OK;
 }
 
-static int f64_y(double2 *spec, int ncomp, const GridParams &gp, const F64Axis &py, int inverse, cudaStream_t s) {
-    const int64_t nplanes = (int64_t)ncomp * gp.N[2];
-    const int Nxh = gp.N[0] / 2 + 1, L = f64_lines(py.N, 1, nplanes * Nxh), nblk = (Nxh + L - 1) / L;
+// Transform along the middle axis of nplanes arrays of p.N x Nxh: y of every z plane, or z of whole spectra.
+static int f64_y(double2 *spec, int64_t nplanes, int Nxh, const F64Axis &py, int inverse, cudaStream_t s) {
+    const int L = f64_lines(py.N, 1, nplanes * Nxh), nblk = (Nxh + L - 1) / L;
     const size_t smem = sizeof(double2) * 2 * (size_t)L * (py.N | 1);
     const int rc = f64_smem(k_f64_y, smem);
     if (rc) return rc;
@@ -782,13 +782,18 @@ int f64_forward_xy(const double *grid, void *spec, int ncomp, const GridParams &
                    cudaStream_t s) {
     if (!pl.ok) return MPS_BAD_ARG;
     const int rc = f64_x(true, grid, nullptr, (double2 *)spec, ncomp, gp, pl.ax[0], s);
-    return rc ? rc : f64_y((double2 *)spec, ncomp, gp, pl.ax[1], 0, s);
+    return rc ? rc : f64_y((double2 *)spec, (int64_t)ncomp * gp.N[2], gp.N[0] / 2 + 1, pl.ax[1], 0, s);
 }
 
 int f64_inverse_yx(void *spec, double *grid, int ncomp, const GridParams &gp, const F64Plan3 &pl, cudaStream_t s) {
     if (!pl.ok) return MPS_BAD_ARG;
-    const int rc = f64_y((double2 *)spec, ncomp, gp, pl.ax[1], 1, s);
+    const int rc = f64_y((double2 *)spec, (int64_t)ncomp * gp.N[2], gp.N[0] / 2 + 1, pl.ax[1], 1, s);
     return rc ? rc : f64_x(false, nullptr, grid, (double2 *)spec, ncomp, gp, pl.ax[0], s);
+}
+
+int f64_z(void *spec, int ncomp, const GridParams &gp, const F64Plan3 &pl, int inverse, cudaStream_t s) {
+    if (!pl.ok) return MPS_BAD_ARG;
+    return f64_y((double2 *)spec, ncomp, (gp.N[0] / 2 + 1) * gp.N[1], pl.ax[2], inverse, s);
 }
 
 int f64_z_scale_dipole(void *spec, int nrhs, const GridParams &gp, const F64Plan3 &pl, const double *hs,

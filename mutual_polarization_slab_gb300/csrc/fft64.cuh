@@ -38,6 +38,8 @@ int f64_forward_xy(const double *grid, void *spec, int ncomp, const GridParams &
 // z transform, the dipole operator's scale H k k^T / |k|^2 (Nyquist rule) and the inverse z transform.
 int f64_z_scale_dipole(void *spec, int nrhs, const GridParams &gp, const F64Plan3 &pl, const double *hs,
                        cudaStream_t s);
+// The z transform by itself, of ncomp spectra (forward, or inverse and unnormalised), for scales of other operators.
+int f64_z(void *spec, int ncomp, const GridParams &gp, const F64Plan3 &pl, int inverse, cudaStream_t s);
 int f64_inverse_yx(void *spec, double *grid, int ncomp, const GridParams &gp, const F64Plan3 &pl, cudaStream_t s);
 
 }  // namespace mps

@@ -316,7 +316,7 @@ __device__ __forceinline__ void quad_couple(const T q[3], const T cf[4], bool cc
 
 template <typename T>
 __global__ void k_scale_quad(typename C2T<T>::type *__restrict__ spec, int nrhs, GridParams gp,
-                             const T *__restrict__ coef) {
+                             const T *__restrict__ coef, double factor) {
     using C = typename C2T<T>::type;
     const int Nxh = gp.N[0] / 2 + 1;
     const int64_t Gc = (int64_t)Nxh * gp.N[1] * gp.N[2];
@@ -347,7 +347,7 @@ __global__ void k_scale_quad(typename C2T<T>::type *__restrict__ spec, int nrhs,
                 q[2] = kz * inv;
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) cf[i] = coef[4 * t + i];
+            for (int i = 0; i < 4; ++i) cf[i] = factor * coef[4 * t + i];
         }
         const bool ny[3] = {(gp.N[0] % 2 == 0) && ix == gp.N[0] / 2, (gp.N[1] % 2 == 0) && iy == gp.N[1] / 2,
                             (gp.N[2] % 2 == 0) && iz == gp.N[2] / 2};
@@ -604,9 +604,9 @@ int quad_kcoef(const GridParams &gp, double *c64, float *c32, cudaStream_t s) {
 }
 
 template <typename T>
-int scale_quad(void *spec, int nrhs, const GridParams &gp, const T *coef, cudaStream_t s) {
+int scale_quad(void *spec, int nrhs, const GridParams &gp, const T *coef, cudaStream_t s, double factor) {
     const int64_t Gc = (int64_t)(gp.N[0] / 2 + 1) * gp.N[1] * gp.N[2];
-    k_scale_quad<T><<<grid_for(Gc, 256), 256, 0, s>>>((typename C2T<T>::type *)spec, nrhs, gp, coef);
+    k_scale_quad<T><<<grid_for(Gc, 256), 256, 0, s>>>((typename C2T<T>::type *)spec, nrhs, gp, coef, factor);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
 }
@@ -651,8 +651,8 @@ template int contract_gen<float>(const float *, int64_t, int, int, const int32_t
                                  double *, cudaStream_t);
 template int contract_gen<double>(const double *, int64_t, int, int, const int32_t *, const double *,
                                   const GridParams &, double *, cudaStream_t);
-template int scale_quad<float>(void *, int, const GridParams &, const float *, cudaStream_t);
-template int scale_quad<double>(void *, int, const GridParams &, const double *, cudaStream_t);
+template int scale_quad<float>(void *, int, const GridParams &, const float *, cudaStream_t, double);
+template int scale_quad<double>(void *, int, const GridParams &, const double *, cudaStream_t, double);
 template int real_space_quad<float>(const double *, float *, double *, int64_t, int, const int64_t *, int64_t,
                                     const int32_t *, const float *, const float *, const float *, const float *,
                                     const double *, const double *, const int32_t *, cudaStream_t);

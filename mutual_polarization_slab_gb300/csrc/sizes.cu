@@ -356,12 +356,12 @@ struct CsCplx<double> {
 constexpr int kScaleVec = 4;
 
 template <typename T>
-__global__ void k_scale_cs(T *__restrict__ spec, int nrhs, int64_t Gc, const T *__restrict__ coef) {
+__global__ void k_scale_cs(T *__restrict__ spec, int nrhs, int64_t Gc, const T *__restrict__ coef, T factor) {
     using C = typename CsCplx<T>::type;
     const int r0 = blockIdx.y * kScaleVec, cnt = min(kScaleVec, nrhs - r0);
     C *sp = reinterpret_cast<C *>(spec) + (int64_t)r0 * Gc;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < Gc; t += (int64_t)gridDim.x * blockDim.x) {
-        const T c = coef[t];
+        const T c = factor * coef[t];
         C v[kScaleVec];
 #pragma unroll
         for (int r = 0; r < kScaleVec; ++r)
@@ -797,9 +797,10 @@ int contract_cs_many(const float *grid, int64_t n, int nrhs, const int32_t *star
 }
 
 template <typename T>
-int scale_cs(void *spec, int nrhs, const GridParams &gp, const T *coef, cudaStream_t s) {
+int scale_cs(void *spec, int nrhs, const GridParams &gp, const T *coef, cudaStream_t s, double factor) {
     const int64_t Gc = (int64_t)(gp.N[0] / 2 + 1) * gp.N[1] * gp.N[2];
-    k_scale_cs<T><<<dim3(grid_for(Gc, 256), (nrhs + kScaleVec - 1) / kScaleVec), 256, 0, s>>>((T *)spec, nrhs, Gc, coef);
+    k_scale_cs<T><<<dim3(grid_for(Gc, 256), (nrhs + kScaleVec - 1) / kScaleVec), 256, 0, s>>>((T *)spec, nrhs, Gc, coef,
+                                                                                                   (T)factor);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
 }
@@ -822,8 +823,8 @@ template int spread_cs<float>(const double *, int64_t, int, const int32_t *, con
                               const GridParams &, float *, cudaStream_t);
 template int spread_cs<double>(const double *, int64_t, int, const int32_t *, const double *, const double *,
                                const GridParams &, double *, cudaStream_t);
-template int scale_cs<float>(void *, int, const GridParams &, const float *, cudaStream_t);
-template int scale_cs<double>(void *, int, const GridParams &, const double *, cudaStream_t);
+template int scale_cs<float>(void *, int, const GridParams &, const float *, cudaStream_t, double);
+template int scale_cs<double>(void *, int, const GridParams &, const double *, cudaStream_t, double);
 template int contract_cs<float>(const float *, int64_t, int, const int32_t *, const double *, const float *,
                                 const GridParams &, double *, cudaStream_t);
 template int contract_cs<double>(const double *, int64_t, int, const int32_t *, const double *, const double *,

@@ -18,7 +18,7 @@ template <typename T>
 int spread_cs(const double *m, int64_t n, int nrhs, const int32_t *start, const double *base, const T *g,
               const GridParams &gp, T *grid, cudaStream_t s);
 template <typename T>
-int scale_cs(void *spec, int nrhs, const GridParams &gp, const T *coef, cudaStream_t s);
+int scale_cs(void *spec, int nrhs, const GridParams &gp, const T *coef, cudaStream_t s, double factor = 1.0);
 template <typename T>
 int contract_cs(const T *grid, int64_t n, int nrhs, const int32_t *start, const double *base, const T *g,
                 const GridParams &gp, double *out, cudaStream_t s);

@@ -984,11 +984,22 @@ static int matvec_quad(mps_system *s, const double *m, double *out, int nrhs, cu
     else
         MPS_TRY(spread_gen<T>(m, s->n, nrhs, 8, s->start, w, s->gp, grid, st));
     STAGE_MARK(2);
-    MPS_TRY(exec_plan(s, dbl ? CUFFT_D2Z : CUFFT_R2C, 8 * nrhs, grid, spec, 0, st));
+    const bool own = dbl && f64_usable(s);
+    if (own) {   // (twice the spectra: the scale takes on the factor)
+        MPS_TRY(f64_forward_xy(s->grid64, spec, 8 * nrhs, s->gp, s->f64p, st));
+        MPS_TRY(f64_z(spec, 8 * nrhs, s->gp, s->f64p, 0, st));
+    } else {
+        MPS_TRY(exec_plan(s, dbl ? CUFFT_D2Z : CUFFT_R2C, 8 * nrhs, grid, spec, 0, st));
+    }
     STAGE_MARK(3);
-    MPS_TRY(scale_quad<T>(spec, nrhs, s->gp, kc, st));
+    MPS_TRY(scale_quad<T>(spec, nrhs, s->gp, kc, st, own ? 0.5 : 1.0));
     STAGE_MARK(4);
-    MPS_TRY(exec_plan(s, dbl ? CUFFT_Z2D : CUFFT_C2R, 8 * nrhs, spec, grid, 0, st));
+    if (own) {
+        MPS_TRY(f64_z(spec, 8 * nrhs, s->gp, s->f64p, 1, st));
+        MPS_TRY(f64_inverse_yx(spec, s->grid64, 8 * nrhs, s->gp, s->f64p, st));
+    } else {
+        MPS_TRY(exec_plan(s, dbl ? CUFFT_Z2D : CUFFT_C2R, 8 * nrhs, spec, grid, 0, st));
+    }
     STAGE_MARK(5);
     if (home)
         MPS_TRY(contract_home8((const float *)grid, s->n, nrhs, s->start, (const float *)w, s->gp, s->tbn, out, st));
@@ -1070,11 +1081,22 @@ static int matvec_cs(mps_system *s, const double *m, double *out, int nrhs, cuda
     else
         MPS_TRY(spread_cs<T>(m, s->n, nrhs, s->start, s->cs_base, g, s->gp, grid, st));
     STAGE_MARK(2);
-    MPS_TRY(exec_plan(s, dbl ? CUFFT_D2Z : CUFFT_R2C, nrhs, grid, spec, 0, st));
+    const bool own = dbl && f64_usable(s);
+    if (own) {   // (twice the spectra: the scale takes on the factor)
+        MPS_TRY(f64_forward_xy(s->grid64, spec, nrhs, s->gp, s->f64p, st));
+        MPS_TRY(f64_z(spec, nrhs, s->gp, s->f64p, 0, st));
+    } else {
+        MPS_TRY(exec_plan(s, dbl ? CUFFT_D2Z : CUFFT_R2C, nrhs, grid, spec, 0, st));
+    }
     STAGE_MARK(3);
-    MPS_TRY(scale_cs<T>(spec, nrhs, s->gp, hc, st));
+    MPS_TRY(scale_cs<T>(spec, nrhs, s->gp, hc, st, own ? 0.5 : 1.0));
     STAGE_MARK(4);
-    MPS_TRY(exec_plan(s, dbl ? CUFFT_Z2D : CUFFT_C2R, nrhs, spec, grid, 0, st));
+    if (own) {
+        MPS_TRY(f64_z(spec, nrhs, s->gp, s->f64p, 1, st));
+        MPS_TRY(f64_inverse_yx(spec, s->grid64, nrhs, s->gp, s->f64p, st));
+    } else {
+        MPS_TRY(exec_plan(s, dbl ? CUFFT_Z2D : CUFFT_C2R, nrhs, spec, grid, 0, st));
+    }
     STAGE_MARK(5);
     if (many)
         MPS_TRY(contract_cs_many((const float *)grid, s->n, nrhs, s->start, s->cs_base, (const float *)g, s->gp,
