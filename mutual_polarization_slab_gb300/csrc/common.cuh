@@ -76,6 +76,11 @@ __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_
 // store) is one instruction for all of them: on GB300 a float64 instruction of a warp, a conversion too, costs the same
 // for one active lane as for 32.  Each sum adds the same pairs in the same order as warp_sum.  warp_sums_index tells
 // which sum a lane holds (-1: none, or the same as another lane).
+template <typename T>
+__device__ __forceinline__ T lane_xor(T v, int o) {
+    return __shfl_xor_sync(0xffffffffu, v, o);
+}
+
 template <int C, int O = 16, typename T>
 __device__ __forceinline__ T warp_sums(const T (&v)[C], int lane) {
     if constexpr (O == 0) {
@@ -88,7 +93,7 @@ __device__ __forceinline__ T warp_sums(const T (&v)[C], int lane) {
 #pragma unroll
         for (int k = 0; k < H; ++k) {
             const T up = v[k + H < C ? k + H : k];
-            u[k] = (hi ? up : v[k]) + __shfl_xor_sync(0xffffffffu, hi ? v[k] : up, O);
+            u[k] = (hi ? up : v[k]) + lane_xor(hi ? v[k] : up, O);
         }
         return warp_sums<H, O / 2>(u, lane);
     }

@@ -64,12 +64,13 @@ __device__ __forceinline__ dfv &operator+=(dfv &a, dfv b) {
     return a;
 }
 
+__device__ __forceinline__ dfv lane_xor(dfv v, int o) {
+    return dfv(__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o));
+}
+
 __device__ __forceinline__ dfv warp_sum(dfv v) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const dfv w(__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o));
-        v = v + w;
-    }
+    for (int o = 16; o > 0; o >>= 1) v = v + lane_xor(v, o);
     return v;
 }
 

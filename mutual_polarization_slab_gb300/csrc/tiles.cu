@@ -866,7 +866,8 @@ int contract_tiled_df(const dfv *grid, int64_t n, int nrhs, const int32_t *start
 // column), then the column sums are weighted by wx*wy in double-float.  Fixed
 // summation order: deterministic.  Bounds of 3 blocks per SM let ptxas keep more
 // loads in flight (72 registers for one vector; 1.19 ms per residual matvec at the
-// bench workload against 1.30 ms with 56 registers under the default heuristic).
+// bench workload against 1.30 ms with 56 registers under the default heuristic).  The sums end one to a lane (N = 100,000,
+// P = 10 on 192^3: 393 -> 381 us a vector); deeper unrolling or other bounds were slower (399 to 451).
 template <int NR>
 __global__ void __launch_bounds__(256, 3) k_contract_df_warp(const dfv *__restrict__ grid, int64_t n, int r0,
                                                           const int32_t *__restrict__ order,
@@ -876,6 +877,7 @@ __global__ void __launch_bounds__(256, 3) k_contract_df_warp(const dfv *__restri
     constexpr int C = 3 * NR;
     __shared__ dfv s_w[8][3 * kMaxP];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int oc = warp_sums_index<C>(lane);
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int P = gp.P;
@@ -917,11 +919,8 @@ __global__ void __launch_bounds__(256, 3) k_contract_df_warp(const dfv *__restri
 #pragma unroll
             for (int c = 0; c < C; ++c) acc[c] += wxy * col[c].get();
         }
-#pragma unroll
-        for (int c = 0; c < C; ++c) acc[c] = warp_sum(acc[c]);
-        if (lane == 0)
-#pragma unroll
-            for (int c = 0; c < C; ++c) out[((int64_t)r0 * n + a) * 3 + (c / 3) * n * 3 + c % 3] = (double)acc[c] * gp.hprod;
+        const dfv v = warp_sums(acc, lane);   // one sum to a lane, its conversion and scaling one instruction for all
+        if (oc >= 0) out[((int64_t)(r0 + oc / 3) * n + a) * 3 + oc % 3] = (double)v * gp.hprod;
     }
 }
 
