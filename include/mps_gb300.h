@@ -433,7 +433,7 @@ int mps_system_profile(mps_system *sys, int32_t enable);
  * Resets the accumulators. */
 int mps_system_stage_times(mps_system *sys, double *ms, int64_t *count);
 
-/* Drops the process's cache of Green's coefficients and scale tensors (keyed by
+/* Drops the process's cache of Green's coefficients and their scales (keyed by
  * device, grid, box, xi and eta; shared by systems built on the same grid), so
  * the next system built recomputes its k-space data, as the reference does on
  * every capacitance() call (EW/capacitance.py:385).  Systems that hold

@@ -68,7 +68,7 @@ def unit_field_systems(amp, ndof: int = 3):
 
 
 def clear_kspace_cache():
-    """Drop the process's cached Green's coefficients and scale tensors (shared by
+    """Drop the process's cached Green's coefficients and their scales (shared by
     systems built on the same device, grid, box, xi and eta), so the next system
     recomputes its k-space data as the reference does on every ``capacitance()``
     call (``CPU - Ewald test/capacitance.py:385``).  Existing systems keep theirs."""
@@ -410,7 +410,7 @@ class SpectralEwaldSystem:
         double-float FFTs) or float64 iterative refinement around a float32-operator
         GMRES (``'mixed'``) for R right-hand sides at once.  The refinement
         residuals use ``residual_precision`` ('df': double-float FFTs, the default;
-        'fp64': cuFFT float64); operators without a double-float path use float64.
+        'fp64': float64); operators without a double-float path use float64.
         ``inner_operator='grad'`` runs the inner GMRES on the gradient form of the
         float32 operator (one FFT pair per vector; it differs from the reference
         operator by ~1e-5, which the refinement removes).
