@@ -18,8 +18,8 @@
 //            is of rank one, x and y enter only as kx fx + ky fy: two transforms each way instead of three
 // The float32 issue rate bounds it (some 220 instructions a point and transform in double-float).  Against one warp to a
 // line, radices up to 5, three z transforms and the six-entry scale tensor, three vectors on 192^3: x 0.52 and 0.46 ->
-// 0.39 and 0.45 ms, y 0.61 -> 0.38, z 1.29 -> 0.66 (with the x and y passes twice 3.49 -> 2.26); one vector on 240^3
-// 2.17 -> 1.65 ms, on 60 x 72 x 160 156 -> 105 us.
+// 0.39 and 0.45 ms, y 0.61 -> 0.38, z 1.29 -> 0.61 (with the x and y passes twice 3.49 -> 2.20); one vector on 240^3
+// 2.17 -> 1.65 ms, on 60 x 72 x 160 156 -> 102 us.
 #include <math.h>
 
 #include <algorithm>
@@ -489,40 +489,46 @@ __global__ void __launch_bounds__(kDfThreads, kDfBlocks) k_fft_z_scale(typename 
             }
             copy_async_wait();
             __syncthreads();
-            typename A::S *Z = fft_lines<A>(buf, other, (two ? 2 : 3) * cols, ld, pz, sm);
-            if (mine) {
+            // both transforms from one call: two copies of the stages overflow the instruction cache (three vectors on
+            // 192^3 0.65 -> 0.61 ms)
+            typename A::S *Z = buf;
+#pragma unroll 1
+            for (int pass = 0; pass < 2; ++pass) {
+                Z = fft_lines<A>(Z, Z == buf ? other : buf, (two ? 2 : 3) * cols, ld, pz, sm);
+                if (pass) break;
+                if (mine) {
 #pragma unroll 2
-                for (unsigned z = z0; z < (unsigned)Nz; z += zstep) {
-                    const Rr qz = A::freq(fft_freq(z, Nz), q.hi[2], q.lo[2]);
-                    const bool nyz = 2 * (int)z == Nz;
-                    const Rr hc = A::coef(h[z * zs + col], qx, qy, qz);
-                    typename A::S *o = Z + t * ld + at<A>(z);
-                    if (two) {
-                        const V a = A::ld(o[0]), b = A::mulr(A::ld(o[bs]), qz);
-                        const bool same = nyz == nyy;   // nyy == nyx here
-                        const V s = A::add(a, b);
-                        o[0] = A::st(A::mulr(same ? s : a, hc));
-                        o[bs] = A::st(A::mulr(same ? s : b, A::rmul(hc, qz)));
-                    } else {
-                        const bool ny[3] = {2 * kx == Nx, nyy, nyz};
-                        const Rr qc[3] = {qx, qy, qz};
-                        V s0 = A::zero(), s1 = A::zero();   // off and on the Nyquist bins
+                    for (unsigned z = z0; z < (unsigned)Nz; z += zstep) {
+                        const Rr qz = A::freq(fft_freq(z, Nz), q.hi[2], q.lo[2]);
+                        const bool nyz = 2 * (int)z == Nz;
+                        const Rr hc = A::coef(h[z * zs + col], qx, qy, qz);
+                        typename A::S *o = Z + t * ld + at<A>(z);
+                        if (two) {
+                            const V a = A::ld(o[0]), b = A::mulr(A::ld(o[bs]), qz);
+                            const bool same = nyz == nyy;   // nyy == nyx here
+                            const V s = A::add(a, b);
+                            o[0] = A::st(A::mulr(same ? s : a, hc));
+                            o[bs] = A::st(A::mulr(same ? s : b, A::rmul(hc, qz)));
+                        } else {
+                            const bool ny[3] = {2 * kx == Nx, nyy, nyz};
+                            const Rr qc[3] = {qx, qy, qz};
+                            V s0 = A::zero(), s1 = A::zero();   // off and on the Nyquist bins
 #pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            const V v = A::mulr(A::ld(o[c * bs]), qc[c]);
-                            if (ny[c])
-                                s1 = A::add(s1, v);
-                            else
-                                s0 = A::add(s0, v);
+                            for (int c = 0; c < 3; ++c) {
+                                const V v = A::mulr(A::ld(o[c * bs]), qc[c]);
+                                if (ny[c])
+                                    s1 = A::add(s1, v);
+                                else
+                                    s0 = A::add(s0, v);
+                            }
+#pragma unroll
+                            for (int c = 0; c < 3; ++c)
+                                o[c * bs] = A::st(A::mulr(ny[c] ? s1 : s0, A::rmul(hc, qc[c])));
                         }
-#pragma unroll
-                        for (int c = 0; c < 3; ++c)
-                            o[c * bs] = A::st(A::mulr(ny[c] ? s1 : s0, A::rmul(hc, qc[c])));
                     }
                 }
+                __syncthreads();
             }
-            __syncthreads();
-            Z = fft_lines<A>(Z, Z == buf ? other : buf, (two ? 2 : 3) * cols, ld, pz, sm);
             if (mine)
                 for (unsigned z = z0; z < (unsigned)Nz; z += zstep) {
                     typename A::S *f = base + z * zs;
