@@ -13,7 +13,7 @@
 //             (p - 1) / 2 = 3 q with q prime to 3, five for every nine of them (stage64_thirds)
 // The passes run at the float64 rate (x and y on 192^3: 24 operations a point in 97 % of the time that the measured
 // 5.0e11 multiply-adds a second would take).  Against cuFFT's D2Z / Z2D with the scale as a pass of its own, both ways,
-// float64: three vectors on 192^3 14.96 -> 8.33 ms, on 64^3 0.40 -> 0.32; one vector on 86^3 1.22 -> 0.46, on 240^3
+// float64: three vectors on 192^3 14.96 -> 8.33 ms, on 64^3 0.40 -> 0.30; one vector on 86^3 1.22 -> 0.46, on 240^3
 // 12.6 -> 6.3, on 96^3 0.65 -> 0.36 ms; twelve on 25^3 0.147 -> 0.135, on 43^3 0.93 -> 0.79 ms.
 #include "fft64.cuh"
 
@@ -431,20 +431,28 @@ __global__ void __launch_bounds__(kF64Threads, kF64Blocks) k_f64_x_inv(const dou
 }
 
 // ---------------------------------------------------------------------------
-// y pass: L consecutive kx columns of one (component, z) plane
+// y pass: L consecutive columns of the (component, z) planes, numbered through all planes: a tile of the one column that
+// 33 leave over beside four times eight would cost a warp's float64 instruction as much as a whole one (three vectors on
+// 64^3 54.9 -> 50.9 us a pass)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kF64Threads, kF64Blocks) k_f64_y(double2 *__restrict__ spec, int64_t nplanes, int Nxh, F64Axis py,
                                                        int L, int inverse) {
     extern __shared__ double2 sm64[];
-    const int Ny = py.N, ld = Ny | 1, nblk = (Nxh + L - 1) / L;
+    const int Ny = py.N, ld = Ny | 1;
     const double sg = inverse ? -1.0 : 1.0;
-    for (int64_t tile = blockIdx.x; tile < nplanes * nblk; tile += gridDim.x) {
-        const int64_t plane = tile / nblk;
-        const int kx0 = (int)(tile % nblk) * L, nl = min(L, Nxh - kx0);
-        double2 *base = spec + plane * Ny * (int64_t)Nxh + kx0;
+    const int64_t total = nplanes * Nxh, plane_len = (int64_t)Ny * Nxh;
+    for (int64_t tile = blockIdx.x; tile * L < total; tile += gridDim.x) {
+        const int64_t c0 = tile * L, p0 = c0 / Nxh;
+        const unsigned k0 = (unsigned)(c0 - p0 * Nxh);
+        const int nl = (int)min((int64_t)L, total - c0);
+        double2 *base = spec + p0 * plane_len;
+        auto column = [&](unsigned t) {   // offset of the tile's column t
+            const unsigned k = k0 + t, w = k / (unsigned)Nxh;
+            return (int64_t)w * plane_len + (k - w * (unsigned)Nxh);
+        };
         for (unsigned i = threadIdx.x; i < (unsigned)(nl * Ny); i += blockDim.x) {
             const unsigned y = i / nl, t = i - y * nl;
-            const double2 v = base[(int64_t)y * Nxh + t];
+            const double2 v = base[column(t) + (int64_t)y * Nxh];
             sm64[t * ld + y] = make_double2(v.x, sg * v.y);
         }
         __syncthreads();
@@ -452,7 +460,7 @@ __global__ void __launch_bounds__(kF64Threads, kF64Blocks) k_f64_y(double2 *__re
         for (unsigned i = threadIdx.x; i < (unsigned)(nl * Ny); i += blockDim.x) {
             const unsigned y = i / nl, t = i - y * nl;
             const double2 v = Z[t * ld + y];
-            base[(int64_t)y * Nxh + t] = make_double2(v.x, sg * v.y);
+            base[column(t) + (int64_t)y * Nxh] = make_double2(v.x, sg * v.y);
         }
         __syncthreads();
     }
@@ -769,11 +777,11 @@ static int f64_x(bool fwd, const double *gin, double *gout, double2 *spec, int n
 
 // Transform along the middle axis of nplanes arrays of p.N x Nxh: y of every z plane, or z of whole spectra.
 static int f64_y(double2 *spec, int64_t nplanes, int Nxh, const F64Axis &py, int inverse, cudaStream_t s) {
-    const int L = f64_lines(py.N, 1, nplanes * Nxh), nblk = (Nxh + L - 1) / L;
+    const int L = f64_lines(py.N, 1, nplanes * Nxh);
     const size_t smem = sizeof(double2) * 2 * (size_t)L * (py.N | 1);
     const int rc = f64_smem(k_f64_y, smem);
     if (rc) return rc;
-    k_f64_y<<<grid_for(nplanes * nblk, 1, INT32_MAX), kF64Threads, smem, s>>>(spec, nplanes, Nxh, py, L, inverse);
+    k_f64_y<<<grid_for((nplanes * Nxh + L - 1) / L, 1, INT32_MAX), kF64Threads, smem, s>>>(spec, nplanes, Nxh, py, L, inverse);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
 }
