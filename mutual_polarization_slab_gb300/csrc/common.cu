@@ -34,6 +34,15 @@ void set_last_error(cudaError_t e, const char *what, const char *file, int line)
     snprintf(g_last_error, sizeof(g_last_error), "%s: %s (%s:%d)", what, cudaGetErrorString(e), file, line);
 }
 
+bool upload_complete(void *out, const void *host, size_t bytes) {
+    cudaStream_t s = nullptr;   // a stream of its own: waiting for the legacy stream would wait for other threads' work too
+    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return false;
+    const bool ok = cudaMemcpyAsync(out, host, bytes, cudaMemcpyHostToDevice, s) == cudaSuccess &&
+                    cudaStreamSynchronize(s) == cudaSuccess;
+    cudaStreamDestroy(s);
+    return ok;
+}
+
 // ---------------------------------------------------------------------------
 // Exclusive scan.  Tile = 1024 threads x 4 items.  Phase 1 writes tile sums,
 // phase 2 scans the tile sums in one block (looping over chunks), phase 3

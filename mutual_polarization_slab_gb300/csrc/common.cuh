@@ -41,6 +41,11 @@ void capture_count_begin();
 long long capture_count_end();
 void add_launches(long long k);
 
+// Copies bytes of host memory into out (device), complete on return, whatever stream reads it next: a plain cudaMemcpy from
+// pageable memory may return with the device's write still pending on the legacy stream, which no non-blocking stream
+// waits for.
+bool upload_complete(void *out, const void *host, size_t bytes);
+
 inline unsigned grid_for(int64_t work, int block, int64_t cap = 152 * 32) {
     int64_t g = (work + block - 1) / block;
     if (g < 1) g = 1;

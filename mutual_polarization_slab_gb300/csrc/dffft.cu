@@ -646,7 +646,7 @@ static bool df_axis(int N, int dev, DfAxisPlan *out) {
         cudaGetLastError();
         return false;
     }
-    if (cudaMemcpy(d, tw.data(), sizeof(float4) * tw.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (!upload_complete(d, tw.data(), sizeof(float4) * tw.size())) {   // before another thread can find the plan
         cudaFree(d);
         return false;
     }

@@ -715,7 +715,7 @@ static bool f64_axis(int N, int dev, F64Axis *out) {
         cudaGetLastError();
         return false;
     }
-    if (cudaMemcpy(d, tw.data(), sizeof(double2) * tw.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (!upload_complete(d, tw.data(), sizeof(double2) * tw.size())) {   // before another thread can find the plan
         cudaFree(d);
         return false;
     }
