@@ -176,6 +176,33 @@ __device__ __forceinline__ void mirror_points(const HalfQuarter &q, int ix, int 
             f(((int64_t)(b ? mz : iz) * q.Ny + (a ? my : iy)) * q.Nxh + ix, a ? -1 : 1, b ? -1 : 1);
 }
 
+// Rows of stacked grids taken two at a time as the real and the imaginary part of one complex line.  No pair reaches from
+// one grid into the next (a grid with an odd number of rows ends with a row by itself): the two rows share a rounding
+// error, and an infinity or NaN, and grids of different vectors have nothing to do with each other.
+struct RowPairs {
+    unsigned rows, pairs;   // of one grid
+    __host__ __device__ explicit RowPairs(int64_t grid_rows)
+        : rows((unsigned)grid_rows), pairs((unsigned)((grid_rows + 1) / 2)) {}
+    // The lines from pair p0 on: first row of the first one, and of line l after that; two = it has a second row.
+    struct Lines {
+        unsigned q0, pairs;
+        bool odd;
+        int64_t row0;
+        __device__ __forceinline__ unsigned row(unsigned l, bool *two) const {
+            *two = true;
+            if (!odd) return 2 * l;
+            const unsigned c = (q0 + l) / pairs;
+            *two = q0 + l - c * pairs != pairs - 1;
+            return 2 * l - c;
+        }
+    };
+    __device__ __forceinline__ Lines from(int64_t p0) const {
+        const bool odd = rows & 1;
+        const int64_t c0 = odd ? p0 / pairs : 0;
+        return {(unsigned)(p0 - c0 * pairs), pairs, odd, 2 * p0 - c0};
+    }
+};
+
 __device__ __forceinline__ int64_t wrap_index(int64_t i, int64_t n) {
     int64_t r = i % n;
     return r < 0 ? r + n : r;

@@ -339,38 +339,42 @@ __device__ __forceinline__ typename A::S *lines_after_twiddles(float4 *sm, const
 }
 
 // ---------------------------------------------------------------------------
-// x pass (Rl: real type of the grids): rows 2 t and 2 t + 1 of the stacked grids (nrows rows of Nx) are one line
+// x pass (Rl: real type of the grids): two rows of Nx of a grid are one line (npairs lines over all the stacked grids)
 // ---------------------------------------------------------------------------
 template <class A, typename Rl>
 __global__ void __launch_bounds__(kDfThreads, kDfBlocks) k_fft_x_fwd(const Rl *__restrict__ grid, typename A::S *__restrict__ spec,
-                                                             int64_t nrows, DfAxisPlan px, int L, int ld) {
+                                                             int64_t npairs, RowPairs rp, DfAxisPlan px, int L, int ld) {
     extern __shared__ float4 sm[];
     typename A::S *buf = lines_after_twiddles<A>(sm, px);
     const int Nx = px.N, Nxh = Nx / 2 + 1;
-    const int64_t npairs = (nrows + 1) / 2, ntiles = (npairs + L - 1) / L;
+    const int64_t ntiles = (npairs + L - 1) / L;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int64_t p0 = tile * L;
         const int nl = (int)min((int64_t)L, npairs - p0);
-        const Rl *rows = grid + 2 * p0 * Nx;
-        const int avail = (int)min((int64_t)2 * nl, nrows - 2 * p0);   // rows that exist
+        const RowPairs::Lines ln = rp.from(p0);
+        const Rl *rows = grid + ln.row0 * Nx;
         for (unsigned i = threadIdx.x; i < (unsigned)(nl * Nx); i += kDfThreads) {
             const unsigned line = div16(i, px.mN), n = i - line * Nx;
             Rl *d = reinterpret_cast<Rl *>(buf + line * ld + at<A>(n));   // (re, im)
-            copy_async(d, rows + (int64_t)(2 * line) * Nx + n);
-            if ((int)(2 * line + 1) < avail)
-                copy_async(d + 1, rows + (int64_t)(2 * line + 1) * Nx + n);
+            bool two;
+            const Rl *row = rows + (int64_t)ln.row(line, &two) * Nx + n;
+            copy_async(d, row);
+            if (two)
+                copy_async(d + 1, row + Nx);
             else
                 d[1] = Rl{};
         }
         copy_async_wait();
         __syncthreads();
         const typename A::S *Z = fft_lines<A>(buf, buf + L * ld, nl, ld, px, sm);
-        typename A::S *o = spec + 2 * p0 * Nxh;
+        typename A::S *out = spec + ln.row0 * Nxh;
         for (unsigned i = threadIdx.x; i < (unsigned)(nl * Nxh); i += kDfThreads) {
             const unsigned line = div16(i, px.mNh), k = i - line * Nxh;
             const auto zk = A::ld(Z[line * ld + at<A>(k)]), zc = A::conj(A::ld(Z[line * ld + at<A>(k ? Nx - k : 0)]));
-            o[(int64_t)(2 * line) * Nxh + k] = A::st(A::add(zk, zc));
-            if ((int)(2 * line + 1) < avail) o[(int64_t)(2 * line + 1) * Nxh + k] = A::st(A::mi(A::sub(zk, zc)));
+            bool two;
+            typename A::S *o = out + (int64_t)ln.row(line, &two) * Nxh + k;
+            o[0] = A::st(A::add(zk, zc));
+            if (two) o[Nxh] = A::st(A::mi(A::sub(zk, zc)));
         }
         __syncthreads();
     }
@@ -378,22 +382,23 @@ __global__ void __launch_bounds__(kDfThreads, kDfBlocks) k_fft_x_fwd(const Rl *_
 
 template <class A, typename Rl>
 __global__ void __launch_bounds__(kDfThreads, kDfBlocks) k_fft_x_inv(const typename A::S *__restrict__ spec, Rl *__restrict__ grid,
-                                                             int64_t nrows, DfAxisPlan px, int L, int ld) {
+                                                             int64_t npairs, RowPairs rp, DfAxisPlan px, int L, int ld) {
     extern __shared__ float4 sm[];
     typename A::S *buf = lines_after_twiddles<A>(sm, px);
     const int Nx = px.N, Nxh = Nx / 2 + 1;
-    const int64_t npairs = (nrows + 1) / 2, ntiles = (npairs + L - 1) / L;
+    const int64_t ntiles = (npairs + L - 1) / L;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int64_t p0 = tile * L;
         const int nl = (int)min((int64_t)L, npairs - p0);
-        const typename A::S *in = spec + 2 * p0 * Nxh;
-        const int avail = (int)min((int64_t)2 * nl, nrows - 2 * p0);
+        const RowPairs::Lines ln = rp.from(p0);
+        const typename A::S *in = spec + ln.row0 * Nxh;
         // X0 + i X1 at k and, from the Hermitian halves, at N - k; the real bins' imaginary parts are dropped
 #pragma unroll 4
         for (unsigned i = threadIdx.x; i < (unsigned)(nl * Nxh); i += kDfThreads) {
             const unsigned line = div16(i, px.mNh), k = i - line * Nxh;
-            auto x0 = A::ld(in[(int64_t)(2 * line) * Nxh + k]);
-            auto x1 = (int)(2 * line + 1) < avail ? A::ld(in[(int64_t)(2 * line + 1) * Nxh + k]) : A::zero();
+            bool two;
+            const typename A::S *row = in + (int64_t)ln.row(line, &two) * Nxh + k;
+            auto x0 = A::ld(row[0]), x1 = two ? A::ld(row[Nxh]) : A::zero();
             const bool real_bin = k == 0 || 2 * k == (unsigned)Nx;
             if (real_bin) {
                 x0 = A::zero_im(x0);
@@ -405,12 +410,14 @@ __global__ void __launch_bounds__(kDfThreads, kDfBlocks) k_fft_x_inv(const typen
         copy_async_wait();
         __syncthreads();
         const typename A::S *Z = fft_lines<A>(buf, buf + L * ld, nl, ld, px, sm);
-        Rl *rows = grid + 2 * p0 * Nx;
+        Rl *rows = grid + ln.row0 * Nx;
         for (unsigned i = threadIdx.x; i < (unsigned)(nl * Nx); i += kDfThreads) {
             const unsigned line = div16(i, px.mN), n = i - line * Nx;
             const Rl *z = reinterpret_cast<const Rl *>(Z + line * ld + at<A>(n ? Nx - n : 0));
-            rows[(int64_t)(2 * line) * Nx + n] = z[0];
-            if ((int)(2 * line + 1) < avail) rows[(int64_t)(2 * line + 1) * Nx + n] = z[1];
+            bool two;
+            Rl *row = rows + (int64_t)ln.row(line, &two) * Nx + n;
+            row[0] = z[0];
+            if (two) row[Nx] = z[1];
         }
         __syncthreads();
     }
@@ -698,7 +705,8 @@ static int set_smem(K kernel, size_t bytes) {
 template <class A, typename Rl>
 static int launch_x(bool fwd, const Rl *gin, Rl *gout, typename A::S *spec, int ncomp, const GridParams &gp,
                     const DfAxisPlan &px, cudaStream_t s) {
-    const int64_t nrows = (int64_t)ncomp * gp.N[2] * gp.N[1], npairs = (nrows + 1) / 2;
+    const RowPairs rp((int64_t)gp.N[2] * gp.N[1]);
+    const int64_t npairs = (int64_t)ncomp * rp.pairs;
     const int ld = line_stride<A>(px.N);
     const size_t column = sizeof(typename A::S) * 2 * (size_t)ld;
     const int L = lines_per_block(column, npairs);
@@ -706,10 +714,10 @@ static int launch_x(bool fwd, const Rl *gin, Rl *gout, typename A::S *spec, int 
     const size_t smem = sizeof(float4) * px.ntw + column * L;
     if (fwd) {
         MPS_TRY_STATUS((set_smem<A>(k_fft_x_fwd<A, Rl>, smem)));
-        k_fft_x_fwd<A, Rl><<<blocks, kDfThreads, smem, s>>>(gin, spec, nrows, px, L, ld);
+        k_fft_x_fwd<A, Rl><<<blocks, kDfThreads, smem, s>>>(gin, spec, npairs, rp, px, L, ld);
     } else {
         MPS_TRY_STATUS((set_smem<A>(k_fft_x_inv<A, Rl>, smem)));
-        k_fft_x_inv<A, Rl><<<blocks, kDfThreads, smem, s>>>(spec, gout, nrows, px, L, ld);
+        k_fft_x_inv<A, Rl><<<blocks, kDfThreads, smem, s>>>(spec, gout, npairs, rp, px, L, ld);
     }
     MPS_LAUNCH_CHECK();
     return MPS_OK;

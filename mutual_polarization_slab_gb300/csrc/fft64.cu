@@ -3,8 +3,8 @@
 // GB300 issues two float64 multiply-adds a clock on an SM, so one float64 warp instruction holds its scheduler's
 // float64 pipe for some 64 cycles: everything else in these kernels (shared-memory passes, index arithmetic, twiddle
 // loads) hides behind the arithmetic, and the float64 operations per point are what there is to save.
-//   x pass    two real rows make one complex line (half the work of a complex transform a row; rows are paired over the
-//             whole array, so odd row counts waste nothing), separated without the factor 1/2, which the scale holds
+//   x pass    two real rows of a grid make one complex line (half the work of a complex transform a row), separated
+//             without the factor 1/2, which the scale holds
 //   z pass    forward transform, scale and inverse transform in one kernel.  Because the scale is k (k . f) H / |k|^2,
 //             the x and y components enter only as a = kx fx + ky fy: two transforms each way instead of three
 //   butterflies  of all lines of a block are numbered through and dealt to its threads, so no lane idles for a line
@@ -361,57 +361,60 @@ __device__ double2 *fft64_lines(double2 *a, double2 *b, int nl, int ld, const F6
 }
 
 // ---------------------------------------------------------------------------
-// x pass: rows 2 t and 2 t + 1 of the stacked grids (nrows rows of Nx) are one complex line
+// x pass: two rows of Nx of a grid are one complex line (npairs lines over all the stacked grids)
 // ---------------------------------------------------------------------------
 // 5 blocks an SM (96 registers): 8.33 ms for three vectors on 192^3 against 8.35 at 4 blocks; with radices 15 and 16 as
 // well (128 registers, 4 blocks) 8.56, with none above 8 8.61.
 constexpr int kF64Threads = 128, kF64Blocks = 5;
 
 __global__ void __launch_bounds__(kF64Threads, kF64Blocks) k_f64_x_fwd(const double *__restrict__ grid,
-                                                           double2 *__restrict__ spec, int64_t nrows, F64Axis px,
+                                                           double2 *__restrict__ spec, int64_t npairs, RowPairs rp, F64Axis px,
                                                            int L) {
     extern __shared__ double2 sm64[];
     const int Nx = px.N, Nxh = Nx / 2 + 1, ld = Nx | 1;
-    const int64_t npairs = (nrows + 1) / 2, ntiles = (npairs + L - 1) / L;
+    const int64_t ntiles = (npairs + L - 1) / L;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int64_t p0 = tile * L;
         const int nl = (int)min((int64_t)L, npairs - p0);
-        const double *rows = grid + 2 * p0 * Nx;
-        const int avail = (int)min((int64_t)2 * nl, nrows - 2 * p0);   // rows that exist
+        const RowPairs::Lines ln = rp.from(p0);
+        const double *rows = grid + ln.row0 * Nx;
         for (unsigned i = threadIdx.x; i < (unsigned)(nl * Nx); i += blockDim.x) {
             const unsigned line = i / Nx, n = i - line * Nx;
-            sm64[line * ld + n] = make_double2(rows[(int64_t)(2 * line) * Nx + n],
-                                               (int)(2 * line + 1) < avail ? rows[(int64_t)(2 * line + 1) * Nx + n] : 0.0);
+            bool two;
+            const double *row = rows + (int64_t)ln.row(line, &two) * Nx + n;
+            sm64[line * ld + n] = make_double2(row[0], two ? row[Nx] : 0.0);
         }
         __syncthreads();
         const double2 *Z = fft64_lines(sm64, sm64 + L * ld, nl, ld, px);
-        double2 *o = spec + 2 * p0 * Nxh;
+        double2 *out = spec + ln.row0 * Nxh;
         for (unsigned i = threadIdx.x; i < (unsigned)(nl * Nxh); i += blockDim.x) {
             const unsigned line = i / Nxh, k = i - line * Nxh;
             const double2 a = Z[line * ld + k], b = Z[line * ld + (k ? Nx - k : 0)];
-            o[(int64_t)(2 * line) * Nxh + k] = make_double2(a.x + b.x, a.y - b.y);
-            if ((int)(2 * line + 1) < avail)
-                o[(int64_t)(2 * line + 1) * Nxh + k] = make_double2(a.y + b.y, b.x - a.x);
+            bool two;
+            double2 *o = out + (int64_t)ln.row(line, &two) * Nxh + k;
+            o[0] = make_double2(a.x + b.x, a.y - b.y);
+            if (two) o[Nxh] = make_double2(a.y + b.y, b.x - a.x);
         }
         __syncthreads();
     }
 }
 
 __global__ void __launch_bounds__(kF64Threads, kF64Blocks) k_f64_x_inv(const double2 *__restrict__ spec, double *__restrict__ grid,
-                                                           int64_t nrows, F64Axis px, int L) {
+                                                           int64_t npairs, RowPairs rp, F64Axis px, int L) {
     extern __shared__ double2 sm64[];
     const int Nx = px.N, Nxh = Nx / 2 + 1, ld = Nx | 1;
-    const int64_t npairs = (nrows + 1) / 2, ntiles = (npairs + L - 1) / L;
+    const int64_t ntiles = (npairs + L - 1) / L;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int64_t p0 = tile * L;
         const int nl = (int)min((int64_t)L, npairs - p0);
-        const double2 *in = spec + 2 * p0 * Nxh;
-        const int avail = (int)min((int64_t)2 * nl, nrows - 2 * p0);
+        const RowPairs::Lines ln = rp.from(p0);
+        const double2 *in = spec + ln.row0 * Nxh;
         // conj(X0 + i X1) at k and, from the Hermitian halves, at N - k; the real bins' imaginary parts are dropped
         for (unsigned i = threadIdx.x; i < (unsigned)(nl * Nxh); i += blockDim.x) {
             const unsigned line = i / Nxh, k = i - line * Nxh;
-            double2 a = in[(int64_t)(2 * line) * Nxh + k];
-            double2 b = (int)(2 * line + 1) < avail ? in[(int64_t)(2 * line + 1) * Nxh + k] : make_double2(0.0, 0.0);
+            bool two;
+            const double2 *row = in + (int64_t)ln.row(line, &two) * Nxh + k;
+            double2 a = row[0], b = two ? row[Nxh] : make_double2(0.0, 0.0);
             const bool real_bin = k == 0 || 2 * k == (unsigned)Nx;
             if (real_bin) a.y = b.y = 0.0;
             sm64[line * ld + k] = make_double2(a.x - b.y, -(a.y + b.x));
@@ -419,12 +422,14 @@ __global__ void __launch_bounds__(kF64Threads, kF64Blocks) k_f64_x_inv(const dou
         }
         __syncthreads();
         const double2 *Z = fft64_lines(sm64, sm64 + L * ld, nl, ld, px);
-        double *rows = grid + 2 * p0 * Nx;
+        double *rows = grid + ln.row0 * Nx;
         for (unsigned i = threadIdx.x; i < (unsigned)(nl * Nx); i += blockDim.x) {
             const unsigned line = i / Nx, n = i - line * Nx;
             const double2 z = Z[line * ld + n];   // conj of the inverse transform
-            rows[(int64_t)(2 * line) * Nx + n] = z.x;
-            if ((int)(2 * line + 1) < avail) rows[(int64_t)(2 * line + 1) * Nx + n] = -z.y;
+            bool two;
+            double *row = rows + (int64_t)ln.row(line, &two) * Nx + n;
+            row[0] = z.x;
+            if (two) row[Nx] = -z.y;
         }
         __syncthreads();
     }
@@ -758,18 +763,19 @@ static int f64_smem(K kernel, size_t bytes) {
 
 static int f64_x(bool fwd, const double *gin, double *gout, double2 *spec, int ncomp, const GridParams &gp,
                  const F64Axis &px, cudaStream_t s) {
-    const int64_t nrows = (int64_t)ncomp * gp.N[2] * gp.N[1], npairs = (nrows + 1) / 2;
+    const RowPairs rp((int64_t)gp.N[2] * gp.N[1]);
+    const int64_t npairs = (int64_t)ncomp * rp.pairs;
     const int L = f64_lines(px.N, 1, npairs);
     const size_t smem = sizeof(double2) * 2 * (size_t)L * (px.N | 1);
     const unsigned blocks = grid_for((npairs + L - 1) / L, 1, INT32_MAX);
     if (fwd) {
         const int rc = f64_smem(k_f64_x_fwd, smem);
         if (rc) return rc;
-        k_f64_x_fwd<<<blocks, kF64Threads, smem, s>>>(gin, spec, nrows, px, L);
+        k_f64_x_fwd<<<blocks, kF64Threads, smem, s>>>(gin, spec, npairs, rp, px, L);
     } else {
         const int rc = f64_smem(k_f64_x_inv, smem);
         if (rc) return rc;
-        k_f64_x_inv<<<blocks, kF64Threads, smem, s>>>(spec, gout, nrows, px, L);
+        k_f64_x_inv<<<blocks, kF64Threads, smem, s>>>(spec, gout, npairs, rp, px, L);
     }
     MPS_LAUNCH_CHECK();
     return MPS_OK;
