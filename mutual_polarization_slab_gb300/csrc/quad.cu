@@ -574,14 +574,20 @@ bool contract_home8_pays(const GridParams &gp, int64_t n) {
     return n >= 16 * blocks;
 }
 
+static size_t home8_smem(int P) {
+    const size_t R = kHomeBlock + P - 1;
+    return sizeof(float4) * R * R * (R + 1) + sizeof(float) * kHome8Chunk * 3 * P + sizeof(int) * 2 * kHome8Chunk;
+}
+
 int contract_home8(const float *grid, int64_t n, int nrhs, const int32_t *start, const float *w, const GridParams &gp,
                    const TileBins &tb, double *out, cudaStream_t s) {
     if (!tb.has_home) return MPS_BAD_ARG;
-    const int R = kHomeBlock + gp.P - 1;
-    const size_t smem = sizeof(float4) * (size_t)R * R * (R + 1) + sizeof(float) * (size_t)kHome8Chunk * 3 * gp.P +
-                        sizeof(int) * 2 * kHome8Chunk;
+    const size_t smem = home8_smem(gp.P);
+    // one limit for every launch (the largest support's): a thread that sets its own lower one between another's request
+    // and launch would make that launch fail
     if (smem > 48 * 1024)
-        MPS_CUDA_TRY(cudaFuncSetAttribute(k_contract_home8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        MPS_CUDA_TRY(cudaFuncSetAttribute(k_contract_home8, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)home8_smem(kMaxP)));
     k_contract_home8<<<dim3((unsigned)tb.nhome, 2 * nrhs), kHome8Warps * 32, smem, s>>>(
         grid, n, tb.hstart, tb.hentries, tb.nhb[0], tb.nhb[1], start, w, gp, out);
     MPS_LAUNCH_CHECK();
