@@ -34,13 +34,26 @@ void set_last_error(cudaError_t e, const char *what, const char *file, int line)
     snprintf(g_last_error, sizeof(g_last_error), "%s: %s (%s:%d)", what, cudaGetErrorString(e), file, line);
 }
 
-bool upload_complete(void *out, const void *host, size_t bytes) {
+int upload_table(const void *host, size_t bytes, void **out) {
+    void *d = nullptr;
+    if (cudaError_t e = cudaMalloc(&d, bytes); e != cudaSuccess) {
+        set_last_error(e, "cudaMalloc", __FILE__, __LINE__);
+        cudaGetLastError();   // the next launch check is not to find it
+        return e == cudaErrorMemoryAllocation ? MPS_NO_MEMORY : MPS_CUDA_ERR;
+    }
     cudaStream_t s = nullptr;   // a stream of its own: waiting for the legacy stream would wait for other threads' work too
-    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return false;
-    const bool ok = cudaMemcpyAsync(out, host, bytes, cudaMemcpyHostToDevice, s) == cudaSuccess &&
-                    cudaStreamSynchronize(s) == cudaSuccess;
-    cudaStreamDestroy(s);
-    return ok;
+    cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d, host, bytes, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (s) cudaStreamDestroy(s);
+    if (e != cudaSuccess) {
+        set_last_error(e, "table upload", __FILE__, __LINE__);
+        cudaGetLastError();
+        cudaFree(d);
+        return MPS_CUDA_ERR;
+    }
+    *out = d;
+    return MPS_OK;
 }
 
 // ---------------------------------------------------------------------------

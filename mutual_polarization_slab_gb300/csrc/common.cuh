@@ -41,10 +41,10 @@ void capture_count_begin();
 long long capture_count_end();
 void add_launches(long long k);
 
-// Copies bytes of host memory into out (device), complete on return, whatever stream reads it next: a plain cudaMemcpy from
-// pageable memory may return with the device's write still pending on the legacy stream, which no non-blocking stream
-// waits for.
-bool upload_complete(void *out, const void *host, size_t bytes);
+// A device copy of bytes of host memory (cudaMalloc), complete on return, whatever stream reads it next: a plain cudaMemcpy
+// from pageable memory may return with the device's write still pending on the legacy stream, which no non-blocking stream
+// waits for.  MPS_NO_MEMORY or MPS_CUDA_ERR (and no copy) otherwise.
+int upload_table(const void *host, size_t bytes, void **out);
 
 inline unsigned grid_for(int64_t work, int block, int64_t cap = 152 * 32) {
     int64_t g = (work + block - 1) / block;

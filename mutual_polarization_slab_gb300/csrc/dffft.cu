@@ -612,18 +612,22 @@ static std::vector<int> df_radices(int n) {
 
 static unsigned div16_mul(unsigned d) { return d == 1 ? 0u : (unsigned)(((1ull << 32) + d - 1) / d); }
 
-static bool df_axis(int N, int dev, DfAxisPlan *out) {
-    if (N < 2 || N > 1024) return false;
+// MPS_OK with supported = false for a length that the transforms do not take; other status codes are failures that say
+// nothing about the length.
+static int df_axis(int N, int dev, DfAxisPlan *out, bool *supported) {
+    *supported = false;
+    if (N < 2 || N > 1024) return MPS_OK;
     std::lock_guard<std::mutex> lk(g_df_mu);
     auto it = g_df_axes.find({dev, N});
     if (it != g_df_axes.end()) {
         *out = it->second;
-        return true;
+        *supported = true;
+        return MPS_OK;
     }
     int m = N;
     for (int f : {2, 3, 5})
         while (m % f == 0) m /= f;
-    if (m != 1) return false;
+    if (m != 1) return MPS_OK;
     DfAxisPlan p;
     p.N = N;
     p.mN = div16_mul(N);
@@ -649,19 +653,15 @@ static bool df_axis(int N, int dev, DfAxisPlan *out) {
     }
     if (tw.empty()) tw.push_back(make_float4(1.f, 0.f, 0.f, 0.f));
     float4 *d = nullptr;
-    if (cudaMalloc((void **)&d, sizeof(float4) * tw.size()) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    if (!upload_complete(d, tw.data(), sizeof(float4) * tw.size())) {   // before another thread can find the plan
-        cudaFree(d);
-        return false;
-    }
+    // before another thread can find the plan
+    const int rc = upload_table(tw.data(), sizeof(float4) * tw.size(), (void **)&d);
+    if (rc) return rc;
     p.tw = d;
     p.ntw = (int)tw.size();
     g_df_axes[{dev, N}] = p;
     *out = p;
-    return true;
+    *supported = true;
+    return MPS_OK;
 }
 
 int df_plan(const GridParams &gp, DfPlan3 *out) {
@@ -669,8 +669,11 @@ int df_plan(const GridParams &gp, DfPlan3 *out) {
     if (gp.N[0] % 2 != 0) return MPS_OK;
     int dev = 0;
     MPS_CUDA_TRY(cudaGetDevice(&dev));
-    for (int d = 0; d < 3; ++d)
-        if (!df_axis(gp.N[d], dev, &out->ax[d])) return MPS_OK;
+    for (int d = 0; d < 3; ++d) {
+        bool supported;
+        const int rc = df_axis(gp.N[d], dev, &out->ax[d], &supported);
+        if (rc || !supported) return rc;
+    }
     out->ok = true;
     return MPS_OK;
 }

@@ -666,13 +666,17 @@ static void f64_thirds_table(int R, int q, std::vector<double2> &tw) {
         }
 }
 
-static bool f64_axis(int N, int dev, F64Axis *out) {
-    if (N < 2 || N > kF64MaxN) return false;
+// MPS_OK with supported = false for a length that the transforms do not take; other status codes are failures that say
+// nothing about the length.
+static int f64_axis(int N, int dev, F64Axis *out, bool *supported) {
+    *supported = false;
+    if (N < 2 || N > kF64MaxN) return MPS_OK;
     std::lock_guard<std::mutex> lk(g_f64_mu);
     auto it = g_f64_axes.find({dev, N});
     if (it != g_f64_axes.end()) {
         *out = it->second;
-        return true;
+        *supported = true;
+        return MPS_OK;
     }
     F64Axis p;
     p.N = N;
@@ -684,13 +688,13 @@ static bool f64_axis(int N, int dev, F64Axis *out) {
     const int smooth = N / m;
     for (int f = 7; f <= m; f += 2)
         while (m % f == 0) {
-            if (f > kF64MaxPrime) return false;
+            if (f > kF64MaxPrime) return MPS_OK;
             radices.push_back(f);
             m /= f;
         }
     const std::vector<int> rest = f64_radices(smooth, radices.empty());
     radices.insert(radices.end(), rest.begin(), rest.end());
-    if (radices.size() > (size_t)kF64MaxStages) return false;
+    if (radices.size() > (size_t)kF64MaxStages) return MPS_OK;
     std::vector<double2> tw;
     int ns = 1;
     for (int R : radices) {
@@ -716,26 +720,25 @@ static bool f64_axis(int N, int dev, F64Axis *out) {
         ns *= R;
     }
     double2 *d = nullptr;
-    if (cudaMalloc((void **)&d, sizeof(double2) * tw.size()) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    if (!upload_complete(d, tw.data(), sizeof(double2) * tw.size())) {   // before another thread can find the plan
-        cudaFree(d);
-        return false;
-    }
+    // before another thread can find the plan
+    const int rc = upload_table(tw.data(), sizeof(double2) * tw.size(), (void **)&d);
+    if (rc) return rc;
     p.tw = d;
     g_f64_axes[{dev, N}] = p;
     *out = p;
-    return true;
+    *supported = true;
+    return MPS_OK;
 }
 
 int f64_plan(const GridParams &gp, F64Plan3 *out) {
     out->ok = false;
     int dev = 0;
     MPS_CUDA_TRY(cudaGetDevice(&dev));
-    for (int d = 0; d < 3; ++d)
-        if (!f64_axis(gp.N[d], dev, &out->ax[d])) return MPS_OK;
+    for (int d = 0; d < 3; ++d) {
+        bool supported;
+        const int rc = f64_axis(gp.N[d], dev, &out->ax[d], &supported);
+        if (rc || !supported) return rc;
+    }
     out->ok = true;
     return MPS_OK;
 }

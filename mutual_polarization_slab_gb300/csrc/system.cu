@@ -699,16 +699,18 @@ static int ensure_nodes(mps_system *s, cudaStream_t st, bool *used) {
     return MPS_OK;
 }
 
-static bool df_usable(mps_system *s);
+static int df_usable(mps_system *s, bool *usable);
 
 // The float64 transforms of fft64.cu take every axis up to 1024 whose prime factors are at most 127 (measured faster
-// than cuFFT at every length tried, see there); other grids keep cuFFT.
-static bool f64_usable(mps_system *s) {
+// than cuFFT at every length tried, see there); other grids keep cuFFT.  A failure to plan decides nothing: it is the
+// caller's status, and the next call plans again.
+static int f64_usable(mps_system *s, bool *usable) {
     if (s->f64_state == 0) {
-        if (f64_plan(s->gp, &s->f64p) != MPS_OK) return false;
+        MPS_TRY(f64_plan(s->gp, &s->f64p));
         s->f64_state = s->f64p.ok ? 1 : -1;
     }
-    return s->f64_state == 1;
+    *usable = s->f64_state == 1;
+    return MPS_OK;
 }
 
 // The scale coefficient of the float64 transforms, from the process cache or computed on stream st.
@@ -764,8 +766,8 @@ static bool own_fft32() {
 // Wave-space field grids of nrhs moment vectors in float64 (spread, transforms, dipole scale), left in s->grid64.  Stage
 // marks 2..5 of the calling matvec (ev may be null).
 static int f64_field_grids(mps_system *s, const double *m, int nrhs, StageEvents *ev, cudaStream_t st) {
-    const bool own = f64_usable(s);
-    bool nodes = false;
+    bool own = false, nodes = false;
+    MPS_TRY(f64_usable(s, &own));
     if (own) MPS_TRY(f64_prepare(s, st));
     MPS_TRY(ensure_nodes(s, st, &nodes));
     MPS_TRY(ensure_grids(s, MPS_FP64, st));
@@ -808,8 +810,8 @@ static int matvec_f64(mps_system *s, const double *m, double *out, int nrhs, cud
 
 // The reference discretisation in float32.
 static int matvec_f32(mps_system *s, const double *m, double *out, int nrhs, cudaStream_t st) {
-    const bool own_fft = own_fft32() && df_usable(s);
-    bool use_tiles = false;
+    bool own_fft = false, use_tiles = false;
+    if (own_fft32()) MPS_TRY(df_usable(s, &own_fft));
     MPS_TRY(ensure_tiles(s, kTileRef32, st, &use_tiles));
     MPS_TRY(ensure_grids(s, MPS_FP32, st));
     float *grid = s->grid32;
@@ -949,13 +951,15 @@ static int matvec_df(mps_system *s, const double *m, double *out, int nrhs, cuda
     return MPS_OK;
 }
 
-static bool df_usable(mps_system *s) {
-    if (s->kind != MPS_DIPOLE) return false;
+static int df_usable(mps_system *s, bool *usable) {
+    *usable = false;
+    if (s->kind != MPS_DIPOLE) return MPS_OK;
     if (s->df_state == 0) {
-        if (df_plan(s->gp, &s->dfp) != MPS_OK) return false;
+        MPS_TRY(df_plan(s->gp, &s->dfp));
         s->df_state = s->dfp.ok ? 1 : -1;
     }
-    return s->df_state == 1;
+    *usable = s->df_state == 1;
+    return MPS_OK;
 }
 
 // Dipole + quadrupole operator (8 moments per sphere, CQ/MatrixVectorMultiply.m:31-77):
@@ -984,7 +988,8 @@ static int matvec_quad(mps_system *s, const double *m, double *out, int nrhs, cu
     else
         MPS_TRY(spread_gen<T>(m, s->n, nrhs, 8, s->start, w, s->gp, grid, st));
     STAGE_MARK(2);
-    const bool own = dbl && f64_usable(s);
+    bool own = false;
+    if (dbl) MPS_TRY(f64_usable(s, &own));
     if (own) {   // (twice the spectra: the scale takes on the factor)
         MPS_TRY(f64_forward_xy(s->grid64, spec, 8 * nrhs, s->gp, s->f64p, st));
         MPS_TRY(f64_z(spec, 8 * nrhs, s->gp, s->f64p, 0, st));
@@ -1081,7 +1086,8 @@ static int matvec_cs(mps_system *s, const double *m, double *out, int nrhs, cuda
     else
         MPS_TRY(spread_cs<T>(m, s->n, nrhs, s->start, s->cs_base, g, s->gp, grid, st));
     STAGE_MARK(2);
-    const bool own = dbl && f64_usable(s);
+    bool own = false;
+    if (dbl) MPS_TRY(f64_usable(s, &own));
     if (own) {   // (twice the spectra: the scale takes on the factor)
         MPS_TRY(f64_forward_xy(s->grid64, spec, nrhs, s->gp, s->f64p, st));
         MPS_TRY(f64_z(spec, nrhs, s->gp, s->f64p, 0, st));
@@ -1255,7 +1261,9 @@ static int matvec_grad_inner(mps_system *s, const double *m, double *out, int nr
 static int matvec_real(mps_system *s, const double *m, double *out, int nrhs, int precision, cudaStream_t st) {
     if (precision == MPS_FP32_GRAD) return matvec_grad(s, m, out, nrhs, st);
     if (precision == MPS_DF) {
-        if (df_usable(s)) return matvec_df(s, m, out, nrhs, st);
+        bool df = false;
+        MPS_TRY(df_usable(s, &df));
+        if (df) return matvec_df(s, m, out, nrhs, st);
         precision = MPS_FP64;
     }
     if (s->kind == MPS_POLYDISPERSE)
@@ -2329,7 +2337,12 @@ static int refine_mixed(mps_system *s, const double *b, double *x, int nrhs, con
     // The double-float residual's first-use set-up (weights, tiles, grids, scale) runs on the system's
     // prep stream beside the first inner solve.
     cudaEvent_t ev_prep = nullptr;
-    if (s->resid_prec == MPS_DF && df_usable(s) && !s->wdf) {
+    bool df = false;
+    if (s->resid_prec == MPS_DF && (e = df_usable(s, &df)) != MPS_OK) {
+        cudaFreeAsync(buf, st);
+        return e;
+    }
+    if (df && !s->wdf) {
         cudaEvent_t ev_in = nullptr;
         bool ok = (s->prep || cudaStreamCreateWithFlags(&s->prep, cudaStreamNonBlocking) == cudaSuccess) &&
                   cudaEventCreateWithFlags(&ev_in, cudaEventDisableTiming) == cudaSuccess &&
@@ -3377,7 +3390,9 @@ extern "C" int mps_adjoint_forces(mps_system *sys, const double *m, const double
     // wave space: phi = IFFT(scale(FFT(spread(m)))), float64-accurate, then the weight-gradient contraction.
     // Grids the double-float FFTs support take the double-float pipeline (float64 issue is slow on GB300) and
     // convert phi to float64 in place; the others use the float64 stages.
-    if (!rc && df_usable(sys)) {
+    bool df = false;
+    if (!rc) rc = df_usable(sys, &df);
+    if (!rc && df) {
         rc = df_field_grids(sys, m, 1, nullptr, st);
         if (!rc) rc = dfv_to_f64_inplace(sys->grid64, 3 * sys->gp.G, st);
     } else if (!rc) {
