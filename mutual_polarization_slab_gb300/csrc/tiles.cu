@@ -26,7 +26,7 @@
 
 namespace mps {
 
-constexpr int kMaxTileList = 10;  // distinct tiles per axis touched by one stencil (axis_tile_bound, T >= 2)
+constexpr int kMaxTileList = 8;  // distinct tiles per axis that a stencil may touch (axis_tile_bound: 6 for P = kMaxP, T = 4)
 // particles staged per spread iteration (one barrier interval): 96 measured 1.42 ms for the double-float spread
 // at the bench workload against 1.57 for 32 and 1.46 for 64 (fewer barriers; the warps' shares even out)
 constexpr int kChunk = 96;
@@ -59,8 +59,7 @@ struct TileGeom {
     int P;
 };
 
-__global__ void k_tile_count(const int32_t *__restrict__ start, int64_t n, TileGeom tg, int32_t *__restrict__ tcount,
-                             int64_t *__restrict__ pcount) {
+__global__ void k_tile_count(const int32_t *__restrict__ start, int64_t n, TileGeom tg, int32_t *__restrict__ tcount) {
     for (int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; a < n; a += (int64_t)gridDim.x * blockDim.x) {
         int L[3][kMaxTileList];
         int c[3];
@@ -69,7 +68,16 @@ __global__ void k_tile_count(const int32_t *__restrict__ start, int64_t n, TileG
             for (int iy = 0; iy < c[1]; ++iy)
                 for (int ix = 0; ix < c[0]; ++ix)
                     atomicAdd(&tcount[((int64_t)L[2][iz] * tg.nt[1] + L[1][iy]) * tg.nt[0] + L[0][ix]], 1);
-        pcount[a] = (int64_t)c[0] * c[1] * c[2];
+    }
+}
+
+// Tiles that each particle's stencil touches.
+__global__ void k_tile_pcount(const int32_t *__restrict__ start, int64_t n, TileGeom tg, int64_t *__restrict__ pcount) {
+    for (int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; a < n; a += (int64_t)gridDim.x * blockDim.x) {
+        int L[kMaxTileList];
+        int64_t c = 1;
+        for (int d = 0; d < 3; ++d) c *= axis_tiles(start[3 * a + d], tg.P, tg.N[d], tg.T[d], L);
+        pcount[a] = c;
     }
 }
 
@@ -170,25 +178,37 @@ static int64_t axis_tile_bound(int N, int T, int P) {
     return std::min<int64_t>(nt, (P - 1) / T + 2 + (N % T != 0 ? 1 : 0));
 }
 
-// Tile lists without a host round trip: the entry arrays are sized by the per-particle bound (nentries holds that
-// capacity), the offsets and totals stay on the device.
-int bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tx, int ty, int tz, TileBins &tb,
-                      cudaStream_t s) {
-    tile_bins_free(tb, s);
+static TileGeom tile_geom(const GridParams &gp, const TileBins &tb) {
     TileGeom tg;
     tg.P = gp.P;
-    tg.T[0] = tx;
-    tg.T[1] = ty;
-    tg.T[2] = tz;
-    int64_t per = 1;
+    tg.T[0] = tb.tx;
+    tg.T[1] = tb.ty;
+    tg.T[2] = tb.tz;
     for (int d = 0; d < 3; ++d) {
         tg.N[d] = gp.N[d];
         tg.nt[d] = (gp.N[d] + tg.T[d] - 1) / tg.T[d];
-        per *= axis_tile_bound(gp.N[d], tg.T[d], gp.P);
     }
+    return tg;
+}
+
+// Tile lists without a host round trip: the entry arrays are sized by the per-particle bound (nentries holds that
+// capacity), the offsets and totals stay on the device.
+int bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tx, int ty, int tz, TileBins &tb,
+               cudaStream_t s) {
+    tile_bins_free(tb, s);
+    const int T3[3] = {tx, ty, tz};
+    int64_t per = 1;
+    for (int d = 0; d < 3; ++d) {
+        const int64_t bound = axis_tile_bound(gp.N[d], T3[d], gp.P);
+        if (bound > kMaxTileList) return MPS_BAD_ARG;
+        per *= bound;
+    }
+    if (n < 1) return MPS_BAD_ARG;
     tb.tx = tx;
     tb.ty = ty;
     tb.tz = tz;
+    tb.n = n;
+    const TileGeom tg = tile_geom(gp, tb);
     tb.ntx = tg.nt[0];
     tb.nty = tg.nt[1];
     tb.ntz = tg.nt[2];
@@ -196,36 +216,28 @@ int bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tx, in
     const int64_t T = tb.ntiles;
     const int64_t Emax = n * per;
     tb.nentries = Emax;
-    // temporaries: tile counts and cursors, per-particle counts, scan scratch, the unsorted lists
-    size_t tmp_bytes = 256 * 5 + (size_t)T * 4 * 2 + (size_t)n * 8 + scan_workspace(std::max(T, n) + 1) +
-                       (size_t)Emax * 4;
+    // temporaries: tile counts and cursors, scan scratch, the unsorted lists
+    size_t tmp_bytes = 256 * 4 + (size_t)T * 4 * 2 + scan_workspace(T + 1) + (size_t)Emax * 4;
     char *tmp = nullptr;
     MPS_CUDA_TRY(cudaMallocAsync((void **)&tmp, tmp_bytes, s));
     char *p = tmp;
     int32_t *tcount = (int32_t *)carve_t(p, (size_t)T * 4);
     int32_t *cursor = (int32_t *)carve_t(p, (size_t)T * 4);
-    int64_t *pcount = (int64_t *)carve_t(p, (size_t)n * 8);
-    void *scan_tmp = carve_t(p, scan_workspace(std::max(T, n) + 1));
+    void *scan_tmp = carve_t(p, scan_workspace(T + 1));
     int32_t *unsorted = (int32_t *)carve_t(p, (size_t)Emax * 4);
     // persistent arrays
-    size_t bytes = 256 * 4 + (size_t)(T + 1) * 8 + (size_t)Emax * 4 + (size_t)(n + 1) * 8 + (size_t)Emax * 4;
+    size_t bytes = 256 * 2 + (size_t)(T + 1) * 8 + (size_t)Emax * 4;
     MPS_CUDA_TRY(cudaMallocAsync(&tb.mem, bytes, s));
     p = (char *)tb.mem;
     tb.tile_start = (int64_t *)carve_t(p, (size_t)(T + 1) * 8);
     tb.entries = (int32_t *)carve_t(p, (size_t)Emax * 4);
-    tb.pstart = (int64_t *)carve_t(p, (size_t)(n + 1) * 8);
-    tb.pentry = (int32_t *)carve_t(p, (size_t)Emax * 4);
     MPS_CUDA_TRY(cudaMemsetAsync(tcount, 0, (size_t)T * 4, s));
     MPS_CUDA_TRY(cudaMemsetAsync(cursor, 0, (size_t)T * 4, s));
-    k_tile_count<<<grid_for(n, 256), 256, 0, s>>>(start, n, tg, tcount, pcount);
+    k_tile_count<<<grid_for(n, 256), 256, 0, s>>>(start, n, tg, tcount);
     MPS_LAUNCH_CHECK();
     int r = exclusive_scan_i32_to_i64(tcount, tb.tile_start, T, scan_tmp, s);
     if (r) return r;
     k_scan_total<int32_t><<<1, 32, 0, s>>>(tcount, tb.tile_start, T);
-    MPS_LAUNCH_CHECK();
-    r = exclusive_scan_i64(pcount, tb.pstart, n, scan_tmp, s);
-    if (r) return r;
-    k_scan_total<int64_t><<<1, 32, 0, s>>>(pcount, tb.pstart, n);
     MPS_LAUNCH_CHECK();
     k_tile_fill<<<grid_for(n, 256), 256, 0, s>>>(start, n, tg, tb.tile_start, cursor, unsorted);
     MPS_LAUNCH_CHECK();
@@ -241,7 +253,7 @@ int bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tx, in
 }
 
 int tile_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tz, TileBins &tb, cudaStream_t s) {
-    if (!tiles_supported(gp, tz) || n < 1) return MPS_BAD_ARG;
+    if (!tiles_supported(gp, tz)) return MPS_BAD_ARG;
     return bins_build(start, n, gp, kTileX, kTileY, tz, tb, s);
 }
 
@@ -261,15 +273,24 @@ __global__ void k_tile_pentry(const int64_t *__restrict__ tstart, int64_t ntiles
 
 int tile_bins_pentry(const int32_t *start, const GridParams &gp, TileBins &tb, cudaStream_t s) {
     if (tb.has_pentry || !tb.mem) return MPS_OK;
-    TileGeom tg;
-    tg.P = gp.P;
-    tg.T[0] = tb.tx;
-    tg.T[1] = tb.ty;
-    tg.T[2] = tb.tz;
-    for (int d = 0; d < 3; ++d) {
-        tg.N[d] = gp.N[d];
-        tg.nt[d] = (gp.N[d] + tg.T[d] - 1) / tg.T[d];
-    }
+    const TileGeom tg = tile_geom(gp, tb);
+    char *tmp = nullptr;
+    MPS_CUDA_TRY(cudaMallocAsync((void **)&tmp, 256 * 2 + (size_t)tb.n * 8 + scan_workspace(tb.n + 1), s));
+    char *p = tmp;
+    int64_t *pcount = (int64_t *)carve_t(p, (size_t)tb.n * 8);
+    void *scan_tmp = carve_t(p, scan_workspace(tb.n + 1));
+    if (!tb.pmem)
+        MPS_CUDA_TRY(cudaMallocAsync(&tb.pmem, 256 * 2 + (size_t)(tb.n + 1) * 8 + (size_t)tb.nentries * 4, s));
+    p = (char *)tb.pmem;
+    tb.pstart = (int64_t *)carve_t(p, (size_t)(tb.n + 1) * 8);
+    tb.pentry = (int32_t *)carve_t(p, (size_t)tb.nentries * 4);
+    k_tile_pcount<<<grid_for(tb.n, 256), 256, 0, s>>>(start, tb.n, tg, pcount);
+    MPS_LAUNCH_CHECK();
+    const int r = exclusive_scan_i64(pcount, tb.pstart, tb.n, scan_tmp, s);
+    if (r) return r;
+    k_scan_total<int64_t><<<1, 32, 0, s>>>(pcount, tb.pstart, tb.n);
+    MPS_LAUNCH_CHECK();
+    cudaFreeAsync(tmp, s);
     k_tile_pentry<<<grid_for(tb.ntiles * 32, 256), 256, 0, s>>>(tb.tile_start, tb.ntiles, tb.entries, start, tg,
                                                                tb.pstart, tb.pentry);
     MPS_LAUNCH_CHECK();
@@ -335,6 +356,7 @@ int tile_bins_home(const int32_t *start, int64_t n, const GridParams &gp, TileBi
 
 void tile_bins_free(TileBins &tb, cudaStream_t s) {
     if (tb.mem) cudaFreeAsync(tb.mem, s);
+    if (tb.pmem) cudaFreeAsync(tb.pmem, s);
     if (tb.hmem) cudaFreeAsync(tb.hmem, s);
     tb = TileBins();
 }
@@ -470,7 +492,7 @@ bool nodes_supported(const GridParams &gp) {
 }
 
 int node_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int groups, TileBins &tb, cudaStream_t s) {
-    if (!nodes_supported(gp) || n < 1) return MPS_BAD_ARG;
+    if (!nodes_supported(gp)) return MPS_BAD_ARG;
     return bins_build(start, n, gp, kNodeTile, kNodeTile, node_tile_depth(gp, groups), tb, s);
 }
 

@@ -17,13 +17,16 @@ struct TileBins {
     int tz = 0;                     // tile depth (z)
     int ntx = 0, nty = 0, ntz = 0;
     int64_t ntiles = 0;
-    int64_t nentries = 0;
+    int64_t n = 0;                   // particles
+    int64_t nentries = 0;            // capacity of the lists (an upper bound of the entries)
     int64_t *tile_start = nullptr;   // ntiles + 1
     int32_t *entries = nullptr;      // particle id per (tile, particle) entry, tiles in order, ids ascending
+    void *mem = nullptr;             // single allocation backing the arrays above
+    // Each particle's own list (on demand, tile_bins_pentry: the tiled contractions' gathers need it, spreads do not).
     int64_t *pstart = nullptr;       // n + 1: each particle's entries ...
     int32_t *pentry = nullptr;       // ... listed here (entry indices), in the particle's tile order
-    bool has_pentry = false;         // pentry filled (the tiled contractions' gathers need it; spreads do not)
-    void *mem = nullptr;             // single allocation backing the arrays above
+    void *pmem = nullptr;            // single allocation backing the two
+    bool has_pentry = false;         // both filled
     // Home bins (on demand, tile_bins_home): every particle once, under the kHomeBlock^3 block of grid nodes that
     // holds the first node of its stencil; the stencil then lies inside the block grown by P - 1 nodes per axis.
     bool has_home = false;
@@ -38,13 +41,14 @@ constexpr int kHomeBlock = 8;
 
 bool tiles_supported(const GridParams &gp, int tz);
 int tile_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tz, TileBins &tb, cudaStream_t s);
-// Bins of tiles of 2 to 16 nodes an axis, without a host round trip.
+// Bins of tiles of tx x ty x tz nodes (4 or more an axis with P up to kMaxP; MPS_BAD_ARG where a stencil could touch more
+// tiles of an axis than the builder's lists hold), without a host round trip.
 int bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tx, int ty, int tz, TileBins &tb,
                cudaStream_t s);
 // Bins for spread_nodes and spread_nodes8: 8 x 8 tiles, of depth 8 or 4 by the number of blocks (groups to a tile).
 int node_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int groups, TileBins &tb, cudaStream_t s);
 bool nodes_supported(const GridParams &gp);
-// Fills tb.pentry (once) for the gathers of the tiled contractions.
+// Builds tb.pstart and tb.pentry (once) for the gathers of the tiled contractions.
 int tile_bins_pentry(const int32_t *start, const GridParams &gp, TileBins &tb, cudaStream_t s);
 // Fills the home bins (once) for the staged contractions.
 int tile_bins_home(const int32_t *start, int64_t n, const GridParams &gp, TileBins &tb, cudaStream_t s);
