@@ -316,7 +316,7 @@ __device__ __forceinline__ void quad_couple(const T q[3], const T cf[4], bool cc
 
 template <typename T>
 __global__ void k_scale_quad(typename C2T<T>::type *__restrict__ spec, int nrhs, GridParams gp,
-                             const T *__restrict__ coef, double factor) {
+                             const T *__restrict__ coef, T factor) {
     using C = typename C2T<T>::type;
     const int Nxh = gp.N[0] / 2 + 1;
     const int64_t Gc = (int64_t)Nxh * gp.N[1] * gp.N[2];
@@ -328,10 +328,10 @@ __global__ void k_scale_quad(typename C2T<T>::type *__restrict__ spec, int nrhs,
         if constexpr (sizeof(T) == 4) {
             const float4 *c4 = (const float4 *)coef + 2 * t;
             const float4 lo = c4[0], hi = c4[1];
-            cf[0] = lo.x;
-            cf[1] = lo.y;
-            cf[2] = lo.z;
-            cf[3] = lo.w;
+            cf[0] = factor * lo.x;
+            cf[1] = factor * lo.y;
+            cf[2] = factor * lo.z;
+            cf[3] = factor * lo.w;
             q[0] = hi.x;
             q[1] = hi.y;
             q[2] = hi.z;
@@ -612,7 +612,8 @@ int quad_kcoef(const GridParams &gp, double *c64, float *c32, cudaStream_t s) {
 template <typename T>
 int scale_quad(void *spec, int nrhs, const GridParams &gp, const T *coef, cudaStream_t s, double factor) {
     const int64_t Gc = (int64_t)(gp.N[0] / 2 + 1) * gp.N[1] * gp.N[2];
-    k_scale_quad<T><<<grid_for(Gc, 256), 256, 0, s>>>((typename C2T<T>::type *)spec, nrhs, gp, coef, factor);
+    k_scale_quad<T><<<grid_for(Gc, 256), 256, 0, s>>>((typename C2T<T>::type *)spec, nrhs, gp, coef,
+                                                        (T)factor);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
 }

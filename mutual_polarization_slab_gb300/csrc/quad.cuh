@@ -18,7 +18,7 @@ int contract_home8(const float *grid, int64_t n, int nrhs, const int32_t *start,
 int quad_diag(const double *lam, int64_t total, const double *gq2, double *diag, cudaStream_t s);
 // c64: half spectrum x 4, c32 (optional): half spectrum x 8 (the same and the unit wave vector).
 int quad_kcoef(const GridParams &gp, double *c64, float *c32, cudaStream_t s);
-// factor: a power of two that the float64 scale takes on (1/2 for spectra of twice the transform).
+// factor: a power of two that the scale takes on (1/2 for spectra of twice the transform).
 template <typename T>
 int scale_quad(void *spec, int nrhs, const GridParams &gp, const T *coef, cudaStream_t s, double factor = 1.0);
 int quad_pair_coefs(const double *dist, int64_t np, const double *perp, const double *para, const double *qt,
