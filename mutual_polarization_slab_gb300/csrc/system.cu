@@ -968,9 +968,12 @@ static int df_usable(mps_system *s, bool *usable) {
 template <typename T>
 static int matvec_quad(mps_system *s, const double *m, double *out, int nrhs, cudaStream_t st) {
     const bool dbl = sizeof(T) == 8;
+    // float64 moments go up by atomics (spread_gen): by nodes, eight float64 sums a node and particle took about twice as
+    // long wherever the time counts (one vector, N = 3500, 64^3, P = 6 28 us against 54; three, N = 1041, 25^3, P = 12 121
+    // against 412)
     bool nodes = false;
-    MPS_TRY(ensure_nodes(s, st, &nodes));
-    const bool home = !dbl && nodes && contract_home8_pays(s->gp, s->n);
+    if (!dbl) MPS_TRY(ensure_nodes(s, st, &nodes));
+    const bool home = nodes && contract_home8_pays(s->gp, s->n);
     if (home) MPS_TRY(tile_bins_home(s->start, s->n, s->gp, s->tbn, st));
     if (!dbl && !s->m32) MPS_TRY(dalloc(&s->m32, sizeof(float) * 8 * (size_t)s->n * s->max_rhs, st));
     MPS_TRY(ensure_grids(s, dbl ? MPS_FP64 : MPS_FP32, st));
@@ -984,7 +987,7 @@ static int matvec_quad(mps_system *s, const double *m, double *out, int nrhs, cu
     MPS_TRY(stage_begin(s, dbl ? MPS_FP64 : MPS_FP32, &ev, st));
     STAGE_MARK(1);
     if (nodes)
-        MPS_TRY(spread_nodes8<T>(m, s->n, nrhs, s->start, w, s->gp, s->tbn, grid, st));
+        MPS_TRY(spread_nodes8(m, s->n, nrhs, s->start, (const float *)w, s->gp, s->tbn, (float *)grid, st));
     else
         MPS_TRY(spread_gen<T>(m, s->n, nrhs, 8, s->start, w, s->gp, grid, st));
     STAGE_MARK(2);

@@ -672,19 +672,14 @@ int spread_nodes(const double *m, int64_t n, int nrhs, const int32_t *start, con
 }
 
 // Dipole and quadrupole moments: eight components to a vector, one vector to a block.
-template <typename T>
-int spread_nodes8(const double *m, int64_t n, int nrhs, const int32_t *start, const T *w, const GridParams &gp,
-                  const TileBins &tb, T *grid, cudaStream_t s) {
+int spread_nodes8(const double *m, int64_t n, int nrhs, const int32_t *start, const float *w, const GridParams &gp,
+                  const TileBins &tb, float *grid, cudaStream_t s) {
     if (tb.tx != kNodeTile || tb.ty != kNodeTile) return MPS_BAD_ARG;
-    if (tb.tz == 8) return nodes_launch<T, 1, 8, 8>(m, n, 0, nrhs, start, w, gp, tb, grid, s);
-    if (tb.tz == 4) return nodes_launch<T, 1, 4, 8>(m, n, 0, nrhs, start, w, gp, tb, grid, s);
+    if (tb.tz == 8) return nodes_launch<float, 1, 8, 8>(m, n, 0, nrhs, start, w, gp, tb, grid, s);
+    if (tb.tz == 4) return nodes_launch<float, 1, 4, 8>(m, n, 0, nrhs, start, w, gp, tb, grid, s);
     return MPS_BAD_ARG;
 }
 
-template int spread_nodes8<float>(const double *, int64_t, int, const int32_t *, const float *, const GridParams &,
-                                  const TileBins &, float *, cudaStream_t);
-template int spread_nodes8<double>(const double *, int64_t, int, const int32_t *, const double *, const GridParams &,
-                                   const TileBins &, double *, cudaStream_t);
 template int spread_nodes<double>(const double *, int64_t, int, const int32_t *, const double *, const GridParams &,
                                   const TileBins &, double *, cudaStream_t);
 template int spread_nodes<dfv>(const double *, int64_t, int, const int32_t *, const dfv *, const GridParams &,

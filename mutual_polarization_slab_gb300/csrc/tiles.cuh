@@ -65,10 +65,9 @@ template <typename T>
 int spread_nodes(const double *m, int64_t n, int nrhs, const int32_t *start, const T *w, const GridParams &gp,
                  const TileBins &tb, T *grid, cudaStream_t s);
 
-// Eight components a vector (m [r][a][8], grid[(r*8+c)][G]).
-template <typename T>
-int spread_nodes8(const double *m, int64_t n, int nrhs, const int32_t *start, const T *w, const GridParams &gp,
-                  const TileBins &tb, T *grid, cudaStream_t s);
+// Eight float32 components a vector (m [r][a][8], grid[(r*8+c)][G]).
+int spread_nodes8(const double *m, int64_t n, int nrhs, const int32_t *start, const float *w, const GridParams &gp,
+                  const TileBins &tb, float *grid, cudaStream_t s);
 
 // out[r][a][c] = hprod * sum over the stencil (overwrites); partial: nentries * 3 * min(nrhs,3) of T.
 template <typename T>
