@@ -701,13 +701,13 @@ static int ensure_nodes(mps_system *s, cudaStream_t st, bool *used) {
 
 static int df_usable(mps_system *s, bool *usable);
 
-// The float64 transforms of fft64.cu take every axis up to 1024 whose prime factors are at most 127 (measured faster
-// than cuFFT at every length tried, see there); other grids keep cuFFT.  A failure to plan decides nothing: it is the
+// The float64 transforms of fft64.cu take every axis up to 1024 whose prime factors are at most 127; grids on which they do
+// not pay (f64_pays) and other grids keep cuFFT.  A failure to plan decides nothing: it is the
 // caller's status, and the next call plans again.
 static int f64_usable(mps_system *s, bool *usable) {
     if (s->f64_state == 0) {
         MPS_TRY(f64_plan(s->gp, &s->f64p));
-        s->f64_state = s->f64p.ok ? 1 : -1;
+        s->f64_state = s->f64p.ok && f64_pays(s->gp, s->kind == MPS_DIPOLE) ? 1 : -1;
     }
     *usable = s->f64_state == 1;
     return MPS_OK;
@@ -3118,7 +3118,7 @@ extern "C" int mps_field_map(const double *x_e, int64_t n_e, const double *x_p, 
     if (!rc_) rc_ = green_half(gp, H, nullptr, st);
     F64Plan3 f64;
     if (!rc_) rc_ = f64_plan(gp, &f64);
-    if (f64.ok) {   // the transforms of the float64 operator; cuFFT where an axis is longer or has a larger prime
+    if (f64.ok && f64_pays(gp, true)) {   // the transforms of the float64 operator; cuFFT where they do not apply or pay
         if (!rc_) rc_ = dalloc(&hs, sizeof(double) * (size_t)Gc, st);
         if (!rc_) rc_ = f64_scale_coef(gp, H, hs, st);
         if (!rc_) rc_ = f64_forward_xy(grid, spec, 3, gp, f64, st);
