@@ -5,6 +5,7 @@
 #include "realspace.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace mps {
 
@@ -226,13 +227,21 @@ __global__ void __launch_bounds__(256) k_rs_csr(const double *__restrict__ m, do
                     const TM *mb = mT + ((int64_t)(r0 + r) * n + b) * 3;
                     const T mx = (T)mb[0], my = (T)mb[1], mz = (T)mb[2];
                     const T s = ba * (mx * rx + my * ry + mz * rz);
-                    // (one multiply-add each; acc += av * mx + s * rx would take three instructions a component)
-                    acc[r][0] += av * mx;
-                    acc[r][1] += av * my;
-                    acc[r][2] += av * mz;
-                    acc[r][0] += s * rx;
-                    acc[r][1] += s * ry;
-                    acc[r][2] += s * rz;
+                    if constexpr (std::is_same<T, dfv>::value && R < 3) {
+                        // double-float sums are long chains: one or two vectors wait for them (one vector, N = 30,000,
+                        // 150 neighbours 92 -> 71 us), three keep the lanes busy (159 against 134 by the form below)
+                        acc[r][0] += av * mx + s * rx;
+                        acc[r][1] += av * my + s * ry;
+                        acc[r][2] += av * mz + s * rz;
+                    } else {
+                        // (one multiply-add each; acc += av * mx + s * rx would take three instructions a component)
+                        acc[r][0] += av * mx;
+                        acc[r][1] += av * my;
+                        acc[r][2] += av * mz;
+                        acc[r][0] += s * rx;
+                        acc[r][1] += s * ry;
+                        acc[r][2] += s * rz;
+                    }
                 }
             }
         }
@@ -265,13 +274,14 @@ __global__ void __launch_bounds__(256) k_rs_csr(const double *__restrict__ m, do
 }
 
 template <typename T>
-int real_space_csr(const double *m, double *out, int64_t n, int nrhs, const int64_t *row_ptr, PairData<T> pd,
-                   const double *diag, const int32_t *diag_of_rhs, const double *slab, bool accumulate,
+int real_space_csr(const double *m, double *out, int64_t n, int nrhs, const int64_t *row_ptr, int64_t np,
+                   PairData<T> pd, const double *diag, const int32_t *diag_of_rhs, const double *slab, bool accumulate,
                    cudaStream_t s) {
-    // Up to four vectors share a pass over the pair data, 8 lanes to a row.  Where that fills less than two blocks of
-    // every SM, a warp takes one row of one vector, in blocks of 4 warps (N = 500, one
-    // vector: 12.2 -> 5.9 us).
-    if (n * 8 * ((nrhs + 3) / 4) < 152 * 2 * 256) {
+    // Up to four vectors share a pass over the pair data, 8 lanes to a row.  Where that leaves most SMs without work, a
+    // warp takes one row of one vector, in blocks of 4 warps, and reads the pairs once a vector: N = 400, 62 neighbours,
+    // 1, 3, 12 and 24 vectors 1.6, 2.8, 1.6 and 1.0 times as fast, N = 1000, 18 neighbours, 1, 4, 12 vectors 1.1, 1.4, 0.7;
+    // N = 2000, 3 vectors with 5, 19, 73 neighbours 0.7, 0.9, 1.3.
+    if (n * std::max(nrhs, 4) <= (np >= 48 * n ? 10000 : 6000)) {
         for (int r0 = 0; r0 < nrhs; r0 += 32768) {
             k_rs_csr<T, 32, 1><<<dim3(grid_for(n * 32, 128, 152 * 64), min(32768, nrhs - r0)), 128, 0, s>>>(
                 m, out, n, nrhs, r0, row_ptr, pd, diag, diag_of_rhs, slab, accumulate, m, nullptr);
@@ -301,19 +311,21 @@ int real_space_csr(const double *m, double *out, int64_t n, int nrhs, const int6
     return MPS_OK;
 }
 
-template int real_space_csr<double>(const double *, double *, int64_t, int, const int64_t *, PairData<double>,
+template int real_space_csr<double>(const double *, double *, int64_t, int, const int64_t *, int64_t, PairData<double>,
                                     const double *, const int32_t *, const double *, bool, cudaStream_t);
 __global__ void k_to_dfv(const double *__restrict__ m, int64_t total, dfv *__restrict__ md) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
         md[i] = dfv(m[i]);
 }
 
-int real_space_csr_df(const double *m, dfv *mdf, double *out, int64_t n, int nrhs, const int64_t *row_ptr,
+int real_space_csr_df(const double *m, dfv *mdf, double *out, int64_t n, int nrhs, const int64_t *row_ptr, int64_t np,
                       PairData<dfv> pd, const double *diag, const int32_t *diag_of_rhs, const double *slab,
                       bool accumulate, const int32_t *order, cudaStream_t s) {
     k_to_dfv<<<grid_for((int64_t)nrhs * n * 3, 256), 256, 0, s>>>(m, (int64_t)nrhs * n * 3, mdf);
     MPS_LAUNCH_CHECK();
-    if (n * 8 < 152 * 2 * 256) {   // a warp per row and vector, as in float64
+    // a warp per row and vector, as in float64 (3 vectors, N = 2000 and 4000, 20 neighbours 1.15 and 1.0 times as fast; N =
+    // 4000 and 7000, 65 neighbours 1.2 and 1.0)
+    if (n <= (np >= 48 * n ? 6000 : 1500)) {
         for (int r0 = 0; r0 < nrhs; r0 += 32768) {
             k_rs_csr<dfv, 32, 1, dfv><<<dim3(grid_for(n * 32, 128, 152 * 64), min(32768, nrhs - r0)), 128, 0, s>>>(
                 m, out, n, nrhs, r0, row_ptr, pd, diag, diag_of_rhs, slab, accumulate, mdf, order);

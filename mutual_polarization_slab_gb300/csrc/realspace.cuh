@@ -4,13 +4,14 @@
 
 namespace mps {
 
+// np: pairs in the list (row_ptr[n]).
 template <typename T>
-int real_space_csr(const double *m, double *out, int64_t n, int nrhs, const int64_t *row_ptr, PairData<T> pd,
-                   const double *diag, const int32_t *diag_of_rhs, const double *slab, bool accumulate,
+int real_space_csr(const double *m, double *out, int64_t n, int nrhs, const int64_t *row_ptr, int64_t np,
+                   PairData<T> pd, const double *diag, const int32_t *diag_of_rhs, const double *slab, bool accumulate,
                    cudaStream_t s);
 // The same pair sum in double-float arithmetic on double-float pair data; mdf is
 // scratch for the double-float copy of m (nrhs x n x 3).
-int real_space_csr_df(const double *m, dfv *mdf, double *out, int64_t n, int nrhs, const int64_t *row_ptr,
+int real_space_csr_df(const double *m, dfv *mdf, double *out, int64_t n, int nrhs, const int64_t *row_ptr, int64_t np,
                       PairData<dfv> pd, const double *diag, const int32_t *diag_of_rhs, const double *slab,
                       bool accumulate, const int32_t *order, cudaStream_t s);
 // Float32 pair sum on a float copy m32 of the moments (scratch of m32_floats(n, nrhs) floats or more, 16-byte

@@ -803,7 +803,8 @@ static int matvec_f64(mps_system *s, const double *m, double *out, int nrhs, cud
     MPS_TRY(contract<double>(s->grid64, s->n, nrhs, s->start, s->w64, s->gp, out, st));
     STAGE_MARK(6);
     MPS_TRY(ensure_p64(s, st));
-    MPS_TRY(real_space_csr<double>(m, out, s->n, nrhs, s->row_ptr, s->p64, s->diag, s->diag_idx, s->slab, true, st));
+    MPS_TRY(real_space_csr<double>(m, out, s->n, nrhs, s->row_ptr, s->n_pairs, s->p64, s->diag, s->diag_idx, s->slab,
+                                   true, st));
     STAGE_MARK(7);
     return MPS_OK;
 }
@@ -944,7 +945,7 @@ static int matvec_df(mps_system *s, const double *m, double *out, int nrhs, cuda
         MPS_TRY(pair_sum_join(s, out, nrhs, st));
     } else {
         if (!s->mdf) MPS_TRY(dalloc(&s->mdf, sizeof(dfv) * 3 * (size_t)s->n * s->max_rhs, st));
-        MPS_TRY(real_space_csr_df(m, s->mdf, out, s->n, nrhs, s->row_ptr, s->pdf, s->diag, s->diag_idx, s->slab,
+        MPS_TRY(real_space_csr_df(m, s->mdf, out, s->n, nrhs, s->row_ptr, s->n_pairs, s->pdf, s->diag, s->diag_idx, s->slab,
                                   true, s->order, st));
     }
     STAGE_MARK(7);
@@ -1047,7 +1048,7 @@ static int pair_sum_fork(mps_system *s, const double *m, int nrhs, cudaStream_t 
     MPS_CUDA_TRY(cudaEventRecord(s->ev_fork, st));
     MPS_CUDA_TRY(cudaStreamWaitEvent(s->side, s->ev_fork, 0));
     if (df)
-        MPS_TRY(real_space_csr_df(m, s->mdf, s->rs_buf, s->n, nrhs, s->row_ptr, s->pdf, s->diag, s->diag_idx,
+        MPS_TRY(real_space_csr_df(m, s->mdf, s->rs_buf, s->n, nrhs, s->row_ptr, s->n_pairs, s->pdf, s->diag, s->diag_idx,
                                   s->slab, false, s->order, s->side));
     else
         MPS_TRY(real_space_csr_f32(m, s->m32, s->rs_buf, s->n, nrhs, s->row_ptr, s->p32, s->diag, s->diag_idx,
@@ -1114,7 +1115,8 @@ static int matvec_cs(mps_system *s, const double *m, double *out, int nrhs, cuda
         MPS_TRY(contract_cs<T>(grid, s->n, nrhs, s->start, s->cs_base, g, s->gp, out, st));
     STAGE_MARK(6);
     if (dbl)
-        MPS_TRY(real_space_csr<double>(m, out, s->n, nrhs, s->row_ptr, s->p64, s->diag, s->diag_idx, s->slab, true, st));
+        MPS_TRY(real_space_csr<double>(m, out, s->n, nrhs, s->row_ptr, s->n_pairs, s->p64, s->diag, s->diag_idx, s->slab,
+                                   true, st));
     else if (beside)
         MPS_TRY(pair_sum_join(s, out, nrhs, st));
     else
@@ -2914,7 +2916,7 @@ extern "C" int mps_matvec_complex(mps_system *sys, const double *m_ri, double *o
     MPS_TRY(unpack_complex(sys->cgrid, G, sys->rgrid2, st));
     MPS_TRY(contract<double>(sys->rgrid2, sys->n, 2, sys->start, sys->w64, sys->gp, out_ri, st));
     MPS_TRY(ensure_p64(sys, st));
-    return real_space_csr<double>(m_ri, out_ri, sys->n, 2, sys->row_ptr, sys->p64, sys->diag, sys->diag_idx, sys->slab,
+    return real_space_csr<double>(m_ri, out_ri, sys->n, 2, sys->row_ptr, sys->n_pairs, sys->p64, sys->diag, sys->diag_idx, sys->slab,
                                   true, st);
 }
 
