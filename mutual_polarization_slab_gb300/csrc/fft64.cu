@@ -744,15 +744,15 @@ int f64_plan(const GridParams &gp, F64Plan3 *out) {
     return MPS_OK;
 }
 
-// Both ways against cuFFT's, us.  Fused, with the scale: rods behind a short x lose (12 x 12 x 400, 12 and 24 vectors 408
-// against 534 and 767 against 1012; 10 x 20 x 400, 3 vectors 177 against 221), shorter or wider ones do not (10 x 10 x 128,
-// 24 vectors 193 against 286 but 23 % less for the matvec; 14 x 14 x 500 1519 against 1280; 400 x 12 x 12 1118 against 770).
+// Both ways, cuFFT against these, us.  Fused, with the scale: rods behind a short x lose (12 x 12 x 400, 12 and 24 vectors 408
+// against 534 and 767 against 1012; 10 x 20 x 400, 3 vectors 177 against 221), wider ones and longer x do not (12 x 48 x 400,
+// 3 vectors 458 against 438; 14 x 14 x 500, 24 vectors 1519 against 1280; 400 x 12 x 12 1118 against 770).
 // Not fused: 24 grids on 16^3, 20^3, 25^3 78 against 100, 68 and 75, 99 and 116, 96 grids on 16^3, 20^3, 25^3, 28^3 78 and
 // 100, 123 and 188, 259 and 336, 326 and 328, on 24 x 24 x 48 363 and 430; on 30^3, 32^3, 36^3, 48^3 456 against 421, 415
 // and 385, 700 and 627, 1793 and 1250.
 bool f64_pays(const GridParams &gp, bool fused) {
     const int longest = std::max({gp.N[0], gp.N[1], gp.N[2]});
-    if (fused) return gp.N[0] >= 14 || longest < 200;
+    if (fused) return gp.N[0] >= 14 || longest < 200 || std::min(gp.N[1], gp.N[2]) >= 40;
     return gp.N[0] >= 30 && gp.N[1] >= 30 && gp.N[2] >= 30;
 }
 
