@@ -296,16 +296,15 @@ __global__ void __launch_bounds__(256, MB) k_spread_cs(const double *__restrict_
         const int r0 = (int)(t / n) * RB;
         const int cnt = min(RB, nrhs - r0);
         const int sx = start[3 * a], sy = start[3 * a + 1], sz = start[3 * a + 2];
-        // a lane loads (and converts) one component, shuffles hand them round
-        static_assert(3 * RB <= 32, "a lane a component");
-        const int lq = lane / 3;
-        const T mv = lq < cnt ? (T)m[((int64_t)(r0 + lq) * n + a) * 3 + lane - 3 * lq] : (T)0;
+        // every lane loads all the vectors' moments: handed round by shuffles from a lane each, the kernel took up to twice as
+        // long (12 vectors, N = 4000, 64^3, P = 16 215 us so, 430 by shuffles; N = 20,000, 80^3, P = 8 171 and 269)
         T px[RB], py[RB], pz[RB];
 #pragma unroll
         for (int q = 0; q < RB; ++q) {
-            px[q] = __shfl_sync(0xffffffffu, mv, 3 * q);
-            py[q] = __shfl_sync(0xffffffffu, mv, 3 * q + 1);
-            pz[q] = __shfl_sync(0xffffffffu, mv, 3 * q + 2);
+            const double *ma = m + ((int64_t)(r0 + (q < cnt ? q : 0)) * n + a) * 3;
+            px[q] = (T)ma[0];
+            py[q] = (T)ma[1];
+            pz[q] = (T)ma[2];
         }
         const T bx = (T)(base[3 * a] - lo * gp.h[0]), by = (T)(base[3 * a + 1] - lo * gp.h[1]),
                 bz = (T)(base[3 * a + 2] - lo * gp.h[2]);
