@@ -753,7 +753,9 @@ bool cs_many(const GridParams &gp, int64_t n, int nrhs) {
            gp.N[2] >= kCsTileZ && gp.N[0] >= gp.P && gp.N[1] >= gp.P && gp.N[2] >= gp.P;
 }
 
-size_t cs_many_floats(int nrhs, int64_t G) { return (size_t)((nrhs + 3) / 4) * 4 * (size_t)G; }
+size_t cs_many_floats(int nrhs, int64_t G) {
+    return nrhs < kCsGroup ? 0 : (size_t)((nrhs + 3) / 4) * 4 * (size_t)G;   // (fewer vectors never take these kernels)
+}
 
 int cs_bins_build(const int32_t *start, int64_t n, const GridParams &gp, TileBins &tb, cudaStream_t s) {
     return bins_build(start, n, gp, kCsTileX, kCsTileY, kCsTileZ, tb, s);
