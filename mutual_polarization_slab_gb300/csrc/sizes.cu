@@ -745,12 +745,30 @@ int spread_cs(const double *m, int64_t n, int nrhs, const int32_t *start, const 
     return MPS_OK;
 }
 
-// Below a group of vectors lanes are idle; with fewer than two tiles for every SM a tile's list is the time it takes.
-// Spread and contraction by these kernels and by the others: 16 vectors, 40^3, 3,000 spheres, P = 8 62 us against 91;
-// P = 5 37 against 45; 34^3, 300 spheres 25 against 25; 48 vectors, 20^3, 400 spheres 60 against 41.
-bool cs_many(const GridParams &gp, int64_t n, int nrhs) {
-    return nrhs >= kCsGroup && n >= 1 && 3 * n <= gp.G && gp.G >= 300 * kCsTileX * kCsTileY * kCsTileZ && gp.P <= kMaxP && gp.N[0] >= kCsTileX && gp.N[1] >= kCsTileY &&
-           gp.N[2] >= kCsTileZ && gp.N[0] >= gp.P && gp.N[1] >= gp.P && gp.N[2] >= gp.P;
+// What both kernels of many vectors take: a group of vectors, stencils that wrap once, the scratch's size.
+static bool cs_many(const GridParams &gp, int64_t n, int nrhs) {
+    if (nrhs < kCsGroup || n < 1 || 3 * n > gp.G || gp.P > kMaxP) return false;
+    const int T[3] = {kCsTileX, kCsTileY, kCsTileZ};
+    for (int d = 0; d < 3; ++d)
+        if (gp.N[d] < T[d] || gp.N[d] < gp.P) return false;
+    return true;
+}
+
+// Spread by tiles: with fewer than two tiles for every SM a tile's list is the time it takes, and on a large grid with few
+// particles every tile's own time is.  By warps a particle / by tiles, us: 16 vectors, P = 8, 40^3, 3000 and 216 particles
+// 39 / 34 and 21 / 14; 96^3, P = 6, 16 vectors, 1105 particles 27 / 45, 8847 66 / 76; 48 vectors, 500 particles, P = 8
+// 66 / 66.
+bool cs_many_spread(const GridParams &gp, int64_t n, int nrhs) {
+    return cs_many(gp, n, nrhs) && gp.G >= 300 * kCsTileX * kCsTileY * kCsTileZ &&
+           (gp.G < 150000 || (double)n * gp.P * gp.P * gp.P * nrhs >= 30.0 * gp.G);
+}
+
+// Contraction of interleaved grids: the transposition costs by nodes, the gather that it speeds up by particles, and a
+// group that is not full costs as much as a full one.  By planes / interleaved, us: 48 vectors, 40^3, 3000 spheres, P = 8
+// 85 / 60, 216 16 / 25; 16 vectors, 40^3, P = 8, 4000 43 / 37, 1600 23 / 25; 96^3, P = 6, 1105 27 / 69.
+bool cs_many_contract(const GridParams &gp, int64_t n, int nrhs) {
+    const int lanes = (nrhs + kCsGroup - 1) / kCsGroup * kCsGroup;
+    return cs_many(gp, n, nrhs) && (double)n * gp.P * gp.P * (2 * nrhs - lanes) >= 20.0 * gp.G && n * nrhs >= 40000;
 }
 
 size_t cs_many_floats(int nrhs, int64_t G) {

@@ -1072,7 +1072,7 @@ static int pair_sum_join(mps_system *s, double *out, int nrhs, cudaStream_t st) 
 template <typename T>
 static int matvec_cs(mps_system *s, const double *m, double *out, int nrhs, cudaStream_t st) {
     const bool dbl = sizeof(T) == 8;
-    const bool many = !dbl && cs_many(s->gp, s->n, nrhs);
+    const bool many = !dbl && cs_many_spread(s->gp, s->n, nrhs);
     if (many && !s->tbc.mem) MPS_TRY(cs_bins_build(s->start, s->n, s->gp, s->tbc, st));
     MPS_TRY(ensure_grids(s, dbl ? MPS_FP64 : MPS_FP32, st));
     T *grid = dbl ? (T *)s->grid64 : (T *)s->grid32;
@@ -1108,7 +1108,7 @@ static int matvec_cs(mps_system *s, const double *m, double *out, int nrhs, cuda
         MPS_TRY(exec_plan(s, dbl ? CUFFT_Z2D : CUFFT_C2R, nrhs, spec, grid, 0, st));
     }
     STAGE_MARK(5);
-    if (many)
+    if (!dbl && cs_many_contract(s->gp, s->n, nrhs))
         MPS_TRY(contract_cs_many((const float *)grid, s->n, nrhs, s->start, s->cs_base, (const float *)g, s->gp,
                                (float *)spec, out, st));
     else
