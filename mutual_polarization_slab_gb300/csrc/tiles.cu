@@ -671,6 +671,13 @@ int spread_nodes(const double *m, int64_t n, int nrhs, const int32_t *start, con
     return MPS_BAD_ARG;
 }
 
+// Every node of the grid costs, and the lists' set-up does: with stencils that cover less than half of the nodes, or on a
+// small grid, atomics from a warp a particle are no slower (three vectors, 96^3, P = 6, 884, 2949, 8847 particles 32 and 50,
+// 46 and 52, 86 and 65 us by atomics and by nodes; one vector, 16^3, 60 particles 11 and 8, after some 45 for the lists).
+bool spread_nodes8_pays(const GridParams &gp, int64_t n) {
+    return gp.G >= 30000 && 2.0 * n * gp.P * gp.P * gp.P >= (double)gp.G;
+}
+
 // Dipole and quadrupole moments: eight components to a vector, one vector to a block.
 int spread_nodes8(const double *m, int64_t n, int nrhs, const int32_t *start, const float *w, const GridParams &gp,
                   const TileBins &tb, float *grid, cudaStream_t s) {
