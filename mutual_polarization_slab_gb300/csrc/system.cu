@@ -1024,9 +1024,11 @@ static int matvec_quad(mps_system *s, const double *m, double *out, int nrhs, cu
 // The float32 pair sum is independent of the wave-space stages of the same
 // matvec: pair_sum_fork runs it on the system's side stream into rs_buf (from
 // the point the moments are ready on st), pair_sum_join makes st wait for it and
-// adds it into out after the contraction.  MPS_PAIR_STREAM=same keeps it on st
-// after the contraction (A/B timing); so do profiled matvecs (their stage times
-// are taken on st).
+// adds it into out after the contraction.  pair_sum_ready and pair_sum_start are
+// its two halves: kernels enqueued on st in between get their blocks onto the SMs
+// first, and the pair sum, whose blocks fill them, takes what is left.
+// MPS_PAIR_STREAM=same keeps it on st after the contraction (A/B timing); so do
+// profiled matvecs (their stage times are taken on st).
 __global__ void k_axpy1(const double *__restrict__ x, double *__restrict__ y, int64_t total);
 
 static bool pair_sum_beside(const StageEvents *ev) {
@@ -1034,7 +1036,7 @@ static bool pair_sum_beside(const StageEvents *ev) {
     return ev == nullptr && !(ps && strcmp(ps, "same") == 0);
 }
 
-static int pair_sum_fork(mps_system *s, const double *m, int nrhs, cudaStream_t st, bool df) {
+static int pair_sum_ready(mps_system *s, cudaStream_t st, bool df) {
     if (!s->side) {
         MPS_CUDA_TRY(cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking));
         MPS_CUDA_TRY(cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming));
@@ -1046,6 +1048,10 @@ static int pair_sum_fork(mps_system *s, const double *m, int nrhs, cudaStream_t 
     if (!df && !s->m32) MPS_TRY(dalloc(&s->m32, sizeof(float) * m32_floats(s->n, s->max_rhs), st));
     if (df && !s->mdf) MPS_TRY(dalloc(&s->mdf, sizeof(dfv) * 3 * (size_t)s->n * s->max_rhs, st));
     MPS_CUDA_TRY(cudaEventRecord(s->ev_fork, st));
+    return MPS_OK;
+}
+
+static int pair_sum_start(mps_system *s, const double *m, int nrhs, bool df) {
     MPS_CUDA_TRY(cudaStreamWaitEvent(s->side, s->ev_fork, 0));
     if (df)
         MPS_TRY(real_space_csr_df(m, s->mdf, s->rs_buf, s->n, nrhs, s->row_ptr, s->n_pairs, s->pdf, s->diag, s->diag_idx,
@@ -1055,6 +1061,11 @@ static int pair_sum_fork(mps_system *s, const double *m, int nrhs, cudaStream_t 
                                    s->slab, false, s->order, s->side));
     MPS_CUDA_TRY(cudaEventRecord(s->ev_join, s->side));
     return MPS_OK;
+}
+
+static int pair_sum_fork(mps_system *s, const double *m, int nrhs, cudaStream_t st, bool df) {
+    MPS_TRY(pair_sum_ready(s, st, df));
+    return pair_sum_start(s, m, nrhs, df);
 }
 
 static int pair_sum_join(mps_system *s, double *out, int nrhs, cudaStream_t st) {
@@ -1082,13 +1093,17 @@ static int matvec_cs(mps_system *s, const double *m, double *out, int nrhs, cuda
     StageEvents *ev = nullptr;
     MPS_TRY(stage_begin(s, dbl ? MPS_FP64 : MPS_FP32, &ev, st));
     const bool beside = !dbl && pair_sum_beside(ev);
-    if (beside) MPS_TRY(pair_sum_fork(s, m, nrhs, st, false));
+    // the spread of few vectors goes first: the pair sum's blocks kept it from the SMs (one vector, 4000 particles, 40^3,
+    // P = 8 a matvec of 77 -> 74 us; 7400, 48^3, P = 12 182 -> 166); that of many does not (a batch of 48 14.5 -> 15.1 ms)
+    if (beside) MPS_TRY(pair_sum_ready(s, st, false));
+    if (beside && many) MPS_TRY(pair_sum_start(s, m, nrhs, false));
     STAGE_MARK(1);
     if (many)
         MPS_TRY(spread_cs_many(m, s->n, nrhs, s->start, s->cs_base, (const float *)g, s->gp, s->tbc, (float *)spec,
                                (float *)grid, st));
     else
         MPS_TRY(spread_cs<T>(m, s->n, nrhs, s->start, s->cs_base, g, s->gp, grid, st));
+    if (beside && !many) MPS_TRY(pair_sum_start(s, m, nrhs, false));
     STAGE_MARK(2);
     bool own = false;
     if (dbl) MPS_TRY(f64_usable(s, &own));
