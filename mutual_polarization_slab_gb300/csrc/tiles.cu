@@ -481,8 +481,13 @@ constexpr int kNodeChunk = 96;      // 3 mask words
 constexpr int kNodeWords = kNodeChunk / 32;
 
 // Depth 8 (two nodes a thread) unless that leaves fewer than two blocks for every SM, then 4 (one node a thread: there
-// the length of a lane's list is the time a block takes).  groups: blocks to a tile.
+// the length of a lane's list is the time a block takes).  groups: blocks to a tile.  MPS_TILE_DEPTH=4 or 8 fixes the
+// depth (A/B comparisons and tests).
 static int node_tile_depth(const GridParams &gp, int groups) {
+    if (const char *fixed = getenv("MPS_TILE_DEPTH")) {
+        const int depth = atoi(fixed);
+        if (depth == 4 || depth == 8) return depth;
+    }
     const int64_t nxy = (int64_t)((gp.N[0] + kNodeTile - 1) / kNodeTile) * ((gp.N[1] + kNodeTile - 1) / kNodeTile);
     return nxy * ((gp.N[2] + 7) / 8) * groups >= 304 ? 8 : 4;
 }
