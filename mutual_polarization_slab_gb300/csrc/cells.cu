@@ -71,11 +71,17 @@ __global__ void k_cell_rank(const int32_t *__restrict__ unsorted, const int32_t 
     }
 }
 
-// Screen positions (near_position) of the points in sorted order (null: as they come): a walk's candidates are consecutive 16-byte loads.
-__global__ void k_near_positions(const double *__restrict__ x, const int32_t *__restrict__ sorted, int64_t n, Box3 box,
-                                 NearBox nb, float4 *__restrict__ xs) {
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x)
-        xs[s] = near_position(x, sorted ? sorted[s] : s, box, nb);
+// Screen positions (near_position) of n points in sorted order, so that a walk's candidates are consecutive 16-byte loads,
+// and of ne more as they come.
+__global__ void k_near_positions(const double *__restrict__ x, const int32_t *__restrict__ sorted, int64_t n,
+                                 const double *__restrict__ xe, int64_t ne, Box3 box, NearBox nb, float4 *__restrict__ xs,
+                                 float4 *__restrict__ es) {
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n + ne; t += (int64_t)gridDim.x * blockDim.x) {
+        if (t < n)
+            xs[t] = near_position(x, sorted[t], box, nb);
+        else
+            es[t - n] = near_position(xe, t - n, box, nb);
+    }
 }
 
 // Row of the first table separation >= d, at least 1 (the callers have checked d <= rv[ntab - 1]), from the
@@ -1138,9 +1144,65 @@ int pairs_df_to_f64(const PairData<dfv> &pdf, int64_t np, PairData<double> p64, 
 int near_positions(const double *x, const int32_t *sorted, int64_t n, const Box3 &box, const NearBox &nb, float4 *xs,
                    cudaStream_t s) {
     if (n == 0) return MPS_OK;
-    k_near_positions<<<grid_for(n, 256), 256, 0, s>>>(x, sorted, n, box, nb, xs);
+    k_near_positions<<<grid_for(n, 256), 256, 0, s>>>(x, sorted, n, nullptr, 0, box, nb, xs, nullptr);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
+}
+
+// What the walks around the probes read: the sources' cells, the probes' cell coordinates and the screen positions of both, in
+// one allocation (six of them, and a second launch for the positions, had been 4 % of a map of one probe).
+struct ProbeCells {
+    int64_t ncell[3];
+    Box3 box;
+    NearBox nb;
+    CellBins cb;
+    int64_t *cell_e;
+    float4 *xs, *es;
+    int *err;
+    void *mem = nullptr;
+};
+
+static int probe_cells_build(const double *xe, int64_t ne, const double *xp, int64_t np, const double *box, double rc,
+                             ProbeCells &pc, cudaStream_t s) {
+    compute_ncell(box, rc, pc.ncell);
+    if (!cells_fit(pc.ncell)) return MPS_BAD_ARG;
+    const int64_t ncells = pc.ncell[0] * pc.ncell[1] * pc.ncell[2];
+    const size_t bins = cell_bins_bytes(np, ncells);
+    const size_t bytes = 256 * 6 + bins + (sizeof(int64_t) * 3 + sizeof(float4)) * (size_t)(np + ne) + sizeof(int);
+    if (cudaMallocAsync(&pc.mem, bytes, s) != cudaSuccess) {
+        pc.mem = nullptr;
+        cudaGetLastError();
+        return MPS_NO_MEMORY;
+    }
+    char *p = (char *)pc.mem;
+    int64_t *cell_p = (int64_t *)carve(p, sizeof(int64_t) * 3 * (size_t)np);
+    pc.cell_e = (int64_t *)carve(p, sizeof(int64_t) * 3 * (size_t)ne);
+    pc.xs = (float4 *)carve(p, sizeof(float4) * (size_t)np);
+    pc.es = (float4 *)carve(p, sizeof(float4) * (size_t)ne);
+    pc.err = (int *)carve(p, sizeof(int));
+    void *ws = carve(p, bins);
+    const bool periodic[3] = {true, true, true};
+    pc.box = Box3{{box[0], box[1], box[2]}};
+    pc.nb = make_near_box(box, rc, periodic);
+    if (cudaMemsetAsync(pc.err, 0, sizeof(int), s) != cudaSuccess) return MPS_CUDA_ERR;
+    int r = cell_assign(xp, np, box, pc.ncell, cell_p, s);
+    if (!r) r = cell_bins_build(cell_p, np, pc.ncell, ws, pc.cb, s);
+    if (!r) r = cell_assign(xe, ne, box, pc.ncell, pc.cell_e, s);
+    if (r) return r;
+    k_near_positions<<<grid_for(np + ne, 256), 256, 0, s>>>(xp, pc.cb.sorted, np, xe, ne, pc.box, pc.nb, pc.xs, pc.es);
+    MPS_LAUNCH_CHECK();
+    return MPS_OK;
+}
+
+// Status of a probe sum whose kernel has been launched (r: status so far): waits for it.
+static int probe_cells_end(ProbeCells &pc, int r, cudaStream_t s) {
+    int herr = 0;
+    if (!r && cudaGetLastError() != cudaSuccess) r = MPS_CUDA_ERR;
+    if (!r && (cudaMemcpyAsync(&herr, pc.err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+               cudaStreamSynchronize(s) != cudaSuccess))
+        r = MPS_CUDA_ERR;
+    if (pc.mem) cudaFreeAsync(pc.mem, s);
+    return !r && herr ? MPS_TABLE_RANGE : r;
 }
 
 int probe_real_space(const double *xe, int64_t ne, const double *xp, const double *p, int64_t np, const double *box,
@@ -1148,166 +1210,41 @@ int probe_real_space(const double *xe, int64_t ne, const double *xp, const doubl
                      cudaStream_t s) {
     if (ne == 0) return MPS_OK;
     if (ntab < 2) return MPS_BAD_ARG;
-    int64_t ncell[3];
-    compute_ncell(box, rc, ncell);
-    if (!cells_fit(ncell)) return MPS_BAD_ARG;
-    const int64_t ncells = ncell[0] * ncell[1] * ncell[2];
-    int64_t *cell_p = nullptr, *cell_e = nullptr;
-    void *bins = nullptr;
-    int *err = nullptr;
-    float4 *xs = nullptr, *es = nullptr;
-    auto cleanup = [&]() {
-        if (xs) cudaFreeAsync(xs, s);
-        if (es) cudaFreeAsync(es, s);
-        if (cell_p) cudaFreeAsync(cell_p, s);
-        if (cell_e) cudaFreeAsync(cell_e, s);
-        if (bins) cudaFreeAsync(bins, s);
-        if (err) cudaFreeAsync(err, s);
-    };
-    if (cudaMallocAsync((void **)&cell_p, sizeof(int64_t) * 3 * (np > 0 ? np : 1), s) != cudaSuccess ||
-        cudaMallocAsync((void **)&cell_e, sizeof(int64_t) * 3 * ne, s) != cudaSuccess ||
-        cudaMallocAsync(&bins, cell_bins_bytes(np, ncells), s) != cudaSuccess ||
-        cudaMallocAsync((void **)&xs, sizeof(float4) * (np > 0 ? np : 1), s) != cudaSuccess ||
-        cudaMallocAsync((void **)&es, sizeof(float4) * ne, s) != cudaSuccess ||
-        cudaMallocAsync((void **)&err, sizeof(int), s) != cudaSuccess) {
-        cleanup();
-        return MPS_NO_MEMORY;
-    }
-    int rcode = cudaMemsetAsync(err, 0, sizeof(int), s) == cudaSuccess ? MPS_OK : MPS_CUDA_ERR;
-    CellBins cb;
-    if (!rcode) rcode = cell_assign(xp, np, box, ncell, cell_p, s);
-    if (!rcode) rcode = cell_bins_build(cell_p, np, ncell, bins, cb, s);
-    if (!rcode) rcode = cell_assign(xe, ne, box, ncell, cell_e, s);
-    const bool per[3] = {true, true, true};
-    const Box3 b3{{box[0], box[1], box[2]}};
-    const NearBox nb = make_near_box(box, rc, per);
-    if (!rcode) rcode = near_positions(xp, cb.sorted, np, b3, nb, xs, s);
-    if (!rcode) rcode = near_positions(xe, nullptr, ne, b3, nb, es, s);
-    if (!rcode) {
+    ProbeCells pc;
+    const int r = probe_cells_build(xe, ne, xp, np, box, rc, pc, s);
+    if (!r)
         k_probe_real<<<grid_for(ne * 32, 128, 152 * 128), 128, 0, s>>>(
-            xe, ne, cell_e, es, xp, xs, p, cb.counts, cb.starts, ncell[0], ncell[1], ncell[2], b3, nb, rc, perp, para, rv, ntab,
-            out, err);
-        if (cudaGetLastError() != cudaSuccess) rcode = MPS_CUDA_ERR;
-    }
-    int herr = 0;
-    if (!rcode && (cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-                   cudaStreamSynchronize(s) != cudaSuccess))
-        rcode = MPS_CUDA_ERR;
-    cleanup();
-    if (!rcode && herr) rcode = MPS_TABLE_RANGE;
-    return rcode;
+            xe, ne, pc.cell_e, pc.es, xp, pc.xs, p, pc.cb.counts, pc.cb.starts, pc.ncell[0], pc.ncell[1], pc.ncell[2],
+            pc.box, pc.nb, rc, perp, para, rv, ntab, out, pc.err);
+    return probe_cells_end(pc, r, s);
 }
-
 
 int probe_real_space_quad(const double *xe, int64_t ne, const double *xp, const double *sq, int64_t np,
                           const double *box, double rc, const double *tab9, const double *rv, int64_t ntab,
                           double *out, cudaStream_t s) {
     if (ne == 0) return MPS_OK;
     if (ntab < 2) return MPS_BAD_ARG;
-    int64_t ncell[3];
-    compute_ncell(box, rc, ncell);
-    if (!cells_fit(ncell)) return MPS_BAD_ARG;
-    const int64_t ncells = ncell[0] * ncell[1] * ncell[2];
-    int64_t *cell_p = nullptr, *cell_e = nullptr;
-    void *bins = nullptr;
-    int *err = nullptr;
-    float4 *xs = nullptr, *es = nullptr;
-    auto cleanup = [&]() {
-        if (xs) cudaFreeAsync(xs, s);
-        if (es) cudaFreeAsync(es, s);
-        if (cell_p) cudaFreeAsync(cell_p, s);
-        if (cell_e) cudaFreeAsync(cell_e, s);
-        if (bins) cudaFreeAsync(bins, s);
-        if (err) cudaFreeAsync(err, s);
-    };
-    if (cudaMallocAsync((void **)&cell_p, sizeof(int64_t) * 3 * (np > 0 ? np : 1), s) != cudaSuccess ||
-        cudaMallocAsync((void **)&cell_e, sizeof(int64_t) * 3 * ne, s) != cudaSuccess ||
-        cudaMallocAsync(&bins, cell_bins_bytes(np, ncells), s) != cudaSuccess ||
-        cudaMallocAsync((void **)&xs, sizeof(float4) * (np > 0 ? np : 1), s) != cudaSuccess ||
-        cudaMallocAsync((void **)&es, sizeof(float4) * ne, s) != cudaSuccess ||
-        cudaMallocAsync((void **)&err, sizeof(int), s) != cudaSuccess) {
-        cleanup();
-        return MPS_NO_MEMORY;
-    }
-    int rcode = cudaMemsetAsync(err, 0, sizeof(int), s) == cudaSuccess ? MPS_OK : MPS_CUDA_ERR;
-    CellBins cb;
-    if (!rcode) rcode = cell_assign(xp, np, box, ncell, cell_p, s);
-    if (!rcode) rcode = cell_bins_build(cell_p, np, ncell, bins, cb, s);
-    if (!rcode) rcode = cell_assign(xe, ne, box, ncell, cell_e, s);
-    const bool per[3] = {true, true, true};
-    const Box3 b3{{box[0], box[1], box[2]}};
-    const NearBox nb = make_near_box(box, rc, per);
-    if (!rcode) rcode = near_positions(xp, cb.sorted, np, b3, nb, xs, s);
-    if (!rcode) rcode = near_positions(xe, nullptr, ne, b3, nb, es, s);
-    if (!rcode) {
+    ProbeCells pc;
+    const int r = probe_cells_build(xe, ne, xp, np, box, rc, pc, s);
+    if (!r)
         k_probe_real_quad<<<grid_for(ne * 32, 128, 152 * 128), 128, 0, s>>>(
-            xe, ne, cell_e, es, xp, xs, sq, cb.counts, cb.starts, ncell[0], ncell[1], ncell[2], b3, nb, rc, tab9, rv, ntab, out,
-            err);
-        if (cudaGetLastError() != cudaSuccess) rcode = MPS_CUDA_ERR;
-    }
-    int herr = 0;
-    if (!rcode && (cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-                   cudaStreamSynchronize(s) != cudaSuccess))
-        rcode = MPS_CUDA_ERR;
-    cleanup();
-    if (!rcode && herr) rcode = MPS_TABLE_RANGE;
-    return rcode;
+            xe, ne, pc.cell_e, pc.es, xp, pc.xs, sq, pc.cb.counts, pc.cb.starts, pc.ncell[0], pc.ncell[1], pc.ncell[2],
+            pc.box, pc.nb, rc, tab9, rv, ntab, out, pc.err);
+    return probe_cells_end(pc, r, s);
 }
-
 
 int probe_real_space_cs(const double *xe, int64_t ne, const double *xp, const double *p, const int32_t *cls,
                         int32_t cmin, int32_t M, int64_t np, const double *box, double rc, const double *perp,
                         const double *para, const double *rv, int64_t ntab, double *out, cudaStream_t s) {
     if (ne == 0) return MPS_OK;
     if (ntab < 2 || M < 1 || cmin < 0 || cmin >= M) return MPS_BAD_ARG;
-    int64_t ncell[3];
-    compute_ncell(box, rc, ncell);
-    if (!cells_fit(ncell)) return MPS_BAD_ARG;
-    const int64_t ncells = ncell[0] * ncell[1] * ncell[2];
-    int64_t *cell_p = nullptr, *cell_e = nullptr;
-    void *bins = nullptr;
-    int *err = nullptr;
-    float4 *xs = nullptr, *es = nullptr;
-    auto cleanup = [&]() {
-        if (xs) cudaFreeAsync(xs, s);
-        if (es) cudaFreeAsync(es, s);
-        if (cell_p) cudaFreeAsync(cell_p, s);
-        if (cell_e) cudaFreeAsync(cell_e, s);
-        if (bins) cudaFreeAsync(bins, s);
-        if (err) cudaFreeAsync(err, s);
-    };
-    if (cudaMallocAsync((void **)&cell_p, sizeof(int64_t) * 3 * (np > 0 ? np : 1), s) != cudaSuccess ||
-        cudaMallocAsync((void **)&cell_e, sizeof(int64_t) * 3 * ne, s) != cudaSuccess ||
-        cudaMallocAsync(&bins, cell_bins_bytes(np, ncells), s) != cudaSuccess ||
-        cudaMallocAsync((void **)&xs, sizeof(float4) * (np > 0 ? np : 1), s) != cudaSuccess ||
-        cudaMallocAsync((void **)&es, sizeof(float4) * ne, s) != cudaSuccess ||
-        cudaMallocAsync((void **)&err, sizeof(int), s) != cudaSuccess) {
-        cleanup();
-        return MPS_NO_MEMORY;
-    }
-    int rcode = cudaMemsetAsync(err, 0, sizeof(int), s) == cudaSuccess ? MPS_OK : MPS_CUDA_ERR;
-    CellBins cb;
-    if (!rcode) rcode = cell_assign(xp, np, box, ncell, cell_p, s);
-    if (!rcode) rcode = cell_bins_build(cell_p, np, ncell, bins, cb, s);
-    if (!rcode) rcode = cell_assign(xe, ne, box, ncell, cell_e, s);
-    const bool per[3] = {true, true, true};
-    const Box3 b3{{box[0], box[1], box[2]}};
-    const NearBox nb = make_near_box(box, rc, per);
-    if (!rcode) rcode = near_positions(xp, cb.sorted, np, b3, nb, xs, s);
-    if (!rcode) rcode = near_positions(xe, nullptr, ne, b3, nb, es, s);
-    if (!rcode) {
+    ProbeCells pc;
+    const int r = probe_cells_build(xe, ne, xp, np, box, rc, pc, s);
+    if (!r)
         k_probe_real_cs<<<grid_for(ne * 32, 128, 152 * 128), 128, 0, s>>>(
-            xe, ne, cell_e, es, xp, xs, p, cls, cmin, M, cb.counts, cb.starts, ncell[0], ncell[1], ncell[2], b3, nb, rc, perp,
-            para, rv, ntab, out, err);
-        if (cudaGetLastError() != cudaSuccess) rcode = MPS_CUDA_ERR;
-    }
-    int herr = 0;
-    if (!rcode && (cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-                   cudaStreamSynchronize(s) != cudaSuccess))
-        rcode = MPS_CUDA_ERR;
-    cleanup();
-    if (!rcode && herr) rcode = MPS_TABLE_RANGE;
-    return rcode;
+            xe, ne, pc.cell_e, pc.es, xp, pc.xs, p, cls, cmin, M, pc.cb.counts, pc.cb.starts, pc.ncell[0], pc.ncell[1],
+            pc.ncell[2], pc.box, pc.nb, rc, perp, para, rv, ntab, out, pc.err);
+    return probe_cells_end(pc, r, s);
 }
 
 }  // namespace mps

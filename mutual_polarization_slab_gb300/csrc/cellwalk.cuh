@@ -101,7 +101,7 @@ __device__ __forceinline__ float4 near_position(const double *__restrict__ x, in
     return make_float4(v[0], v[1], v[2], __int_as_float((int)i));
 }
 
-// xs[k] = near_position of point sorted[k] (of point k when sorted is null).
+// xs[k] = near_position of point sorted[k].
 int near_positions(const double *x, const int32_t *sorted, int64_t n, const Box3 &box, const NearBox &nb, float4 *xs,
                    cudaStream_t s);
 
