@@ -211,6 +211,8 @@ struct mps_system {
     double *host_scr = nullptr;
     void *fft_work = nullptr;
     size_t fft_work_bytes = 0;
+    bool fft_captured = false;       // a captured step holds fft_work's address
+    std::vector<void *> fft_held;    // outgrown work areas that captured steps hold
     TileBins tb32;              // tiles of the float32 reference form's spread and contraction (tuned depth)
     TileBins tbg;               // tiles of the gradient-form spread (depth 12 where the grid allows it)
     TileBins tbn;               // tiles of the node spread (float64, double-float, eight moments)
@@ -313,6 +315,7 @@ static void free_system(mps_system *s) {
                     s->cx_in, s->cx_out};
     for (void *p : ptrs)
         if (p) cudaFreeAsync(p, s->stream);
+    for (void *p : s->fft_held) cudaFreeAsync(p, s->stream);
     if (s->ev_diag) cudaEventSynchronize(s->ev_diag);   // the last index upload reads the pinned block
     if (s->diag_idx_host) pinned_give(s->diag_idx_host);
     if (s->rs_buf) cudaFreeAsync(s->rs_buf, s->stream);
@@ -430,9 +433,17 @@ static int get_plan(cufftType type, const GridParams &gp, int batch, CachedPlan 
     return MPS_OK;
 }
 
+// A captured step holds the address of the work area of its time (a mixed solve's inner steps are captured before its
+// residual, or a later matvec of more vectors, needs a larger one): such an area stays until the system goes.
 static int ensure_work(mps_system *s, size_t need, cudaStream_t st) {
     if (need <= s->fft_work_bytes) return MPS_OK;
-    if (s->fft_work) cudaFreeAsync(s->fft_work, st);
+    if (s->fft_work) {
+        if (s->fft_captured)
+            s->fft_held.push_back(s->fft_work);
+        else
+            cudaFreeAsync(s->fft_work, st);
+    }
+    s->fft_captured = false;
     s->fft_work = nullptr;
     s->fft_work_bytes = 0;
     MPS_TRY(dalloc(&s->fft_work, need, st));
@@ -2013,6 +2024,7 @@ static int arnoldi_graph_build(mps_system *s, ArnoldiGraph &g, const GmresWs &W,
     }
     g.exec = exec;
     g.body_launches = per_step;
+    s->fft_captured = true;
     return MPS_OK;
 }
 
