@@ -59,8 +59,8 @@ __device__ __forceinline__ int64_t seg_index(const double *__restrict__ rv, int6
 // One group of 8 lanes per particle over its CSR row (N = 200,000, 12 million pairs: 1.75 ms and 0.39 for the float64
 // copy of the list before, 1.21 ms with the slopes from a table, the guessed index, no division and the list read as it
 // is; 1.04 with the part along the particle's own moment summed as a scalar and one multiply-add a term).  T: the pair
-// data's type; the double-float list of a system that has made no float64 copy is read as it is, its values joined by one
-// float64 addition each.
+// data's type; the double-float list of a system that has made no float64 copy is read as it is, its values joined by
+// one float64 addition each.
 template <typename T>
 __global__ void __launch_bounds__(256) k_rs_force(const double *__restrict__ m, int64_t n,
                                                   const int64_t *__restrict__ row_ptr, PairData<T> pd,

@@ -71,8 +71,8 @@ __global__ void k_cell_rank(const int32_t *__restrict__ unsorted, const int32_t 
     }
 }
 
-// Screen positions (near_position) of n points in sorted order, so that a walk's candidates are consecutive 16-byte loads,
-// and of ne more as they come.
+// Screen positions (near_position) of n points in sorted order, so that a walk's candidates are consecutive 16-byte
+// loads, and of ne more as they come.
 __global__ void k_near_positions(const double *__restrict__ x, const int32_t *__restrict__ sorted, int64_t n,
                                  const double *__restrict__ xe, int64_t ne, Box3 box, NearBox nb, float4 *__restrict__ xs,
                                  float4 *__restrict__ es) {
@@ -152,8 +152,8 @@ __device__ __forceinline__ double probe_diff2(const double *__restrict__ xe, int
 // row with rvals >= d); out[e] = sum A m + (B - A) (m . r^) r^ in a fixed order per probe.
 // One candidate in seven lies within rc: the walk screens them in float32 (near_walk) and the float64 pair terms, the
 // only part that GB300's float64 rate bounds, run on 32 kept pairs at a time (90,000 probes and 10,000 spheres, 29 of
-// 203 candidates a probe: 5.62 ms with every candidate in float64, 0.57 ms; the table row comes from the uniform-spacing guess instead of 13 float64
-// comparisons).
+// 203 candidates a probe: 5.62 ms with every candidate in float64, 0.57 ms; the table row comes from the
+// uniform-spacing guess instead of 13 float64 comparisons).
 __global__ void __launch_bounds__(128) k_probe_real(const double *__restrict__ xe, int64_t ne,
                                                     const int64_t *__restrict__ cell_e,
                                                     const float4 *__restrict__ es,
@@ -639,10 +639,10 @@ __device__ __forceinline__ void store_pair(PairData<T> &pd, int64_t w, int32_t b
 }
 
 // Traversal of the cells around particle a in the order of k_csr_count, shared by the fill kernels: the screen only
-// decides which candidates are kept (float screen, float64 for the few in its margin band) and queues their ids per warp
-// in shared memory, in traversal order; drain(cnt, w) then computes the pairs w .. w + cnt - 1 of the row from the queue,
-// one per lane (cnt <= 32), instead of by the few lanes of each round that kept one (about one candidate in six is
-// kept).  The row lists its pairs by neighbour-cell offset, then by particle id.
+// decides which candidates are kept (float screen, float64 for the few in its margin band) and queues their ids per
+// warp in shared memory, in traversal order; drain(cnt, w) then computes the pairs w .. w + cnt - 1 of the row from the
+// queue, one per lane (cnt <= 32), instead of by the few lanes of each round that kept one (about one candidate in six
+// is kept).  The row lists its pairs by neighbour-cell offset, then by particle id.
 constexpr int kFillWarps = 8;
 
 template <class F>
@@ -1149,8 +1149,8 @@ int near_positions(const double *x, const int32_t *sorted, int64_t n, const Box3
     return MPS_OK;
 }
 
-// What the walks around the probes read: the sources' cells, the probes' cell coordinates and the screen positions of both, in
-// one allocation (six of them, and a second launch for the positions, had been 4 % of a map of one probe).
+// What the walks around the probes read: the sources' cells, the probes' cell coordinates and the screen positions of
+// both, in one allocation (six of them, and a second launch for the positions, had been 4 % of a map of one probe).
 struct ProbeCells {
     int64_t ncell[3];
     Box3 box;

@@ -41,9 +41,9 @@ void capture_count_begin();
 long long capture_count_end();
 void add_launches(long long k);
 
-// A device copy of bytes of host memory (cudaMalloc), complete on return, whatever stream reads it next: a plain cudaMemcpy
-// from pageable memory may return with the device's write still pending on the legacy stream, which no non-blocking stream
-// waits for.  MPS_NO_MEMORY or MPS_CUDA_ERR (and no copy) otherwise.
+// A device copy of bytes of host memory (cudaMalloc), complete on return, whatever stream reads it next: a plain
+// cudaMemcpy from pageable memory may return with the device's write still pending on the legacy stream, which no
+// non-blocking stream waits for.  MPS_NO_MEMORY or MPS_CUDA_ERR (and no copy) otherwise.
 int upload_table(const void *host, size_t bytes, void **out);
 
 inline unsigned grid_for(int64_t work, int block, int64_t cap = 152 * 32) {
@@ -60,8 +60,8 @@ __device__ __forceinline__ T warp_sum(T v) {
     return v;
 }
 
-// One float (or two or four, aligned) from global to shared memory without a register in between: a staging loop issues all its loads at once
-// (copy_async_wait before the barrier that publishes them).
+// One float (or two or four, aligned) from global to shared memory without a register in between: a staging loop issues
+// all its loads at once (copy_async_wait before the barrier that publishes them).
 __device__ __forceinline__ void copy_async(float *smem, const float *gmem) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
                  : "memory");
@@ -76,11 +76,11 @@ __device__ __forceinline__ void copy_async(float4 *smem, const float4 *gmem) {
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// C sums over the warp (C <= 32), one to a lane: each halving of the warp halves the values a lane still carries, so C sums
-// take about C + 4 shuffles and additions instead of 5 C, and what follows (the conversion to float64, the scaling, the
-// store) is one instruction for all of them: on GB300 a float64 instruction of a warp, a conversion too, costs the same
-// for one active lane as for 32.  Each sum adds the same pairs in the same order as warp_sum.  warp_sums_index tells
-// which sum a lane holds (-1: none, or the same as another lane).
+// C sums over the warp (C <= 32), one to a lane: each halving of the warp halves the values a lane still carries, so C
+// sums take about C + 4 shuffles and additions instead of 5 C, and what follows (the conversion to float64, the
+// scaling, the store) is one instruction for all of them: on GB300 a float64 instruction of a warp, a conversion too,
+// costs the same for one active lane as for 32.  Each sum adds the same pairs in the same order as warp_sum.
+// warp_sums_index tells which sum a lane holds (-1: none, or the same as another lane).
 template <typename T>
 __device__ __forceinline__ T lane_xor(T v, int o) {
     return __shfl_xor_sync(0xffffffffu, v, o);
@@ -176,9 +176,9 @@ __device__ __forceinline__ void mirror_points(const HalfQuarter &q, int ix, int 
             f(((int64_t)(b ? mz : iz) * q.Ny + (a ? my : iy)) * q.Nxh + ix, a ? -1 : 1, b ? -1 : 1);
 }
 
-// Rows of stacked grids taken two at a time as the real and the imaginary part of one complex line.  No pair reaches from
-// one grid into the next (a grid with an odd number of rows ends with a row by itself): the two rows share a rounding
-// error, and an infinity or NaN, and grids of different vectors have nothing to do with each other.
+// Rows of stacked grids taken two at a time as the real and the imaginary part of one complex line.  No pair reaches
+// from one grid into the next (a grid with an odd number of rows ends with a row by itself): the two rows share a
+// rounding error, and an infinity or NaN, and grids of different vectors have nothing to do with each other.
 struct RowPairs {
     unsigned rows, pairs;   // of one grid
     __host__ __device__ explicit RowPairs(int64_t grid_rows)

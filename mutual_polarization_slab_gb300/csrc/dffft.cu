@@ -5,8 +5,8 @@
 // with __fadd_rn/__fmul_rn/__fmaf_rn so the compiler cannot contract or reorder
 // it.  A complex value is a float4 (re.hi, re.lo, im.hi, im.lo).
 //
-// Transforms: a block holds a few 1-D lines in shared memory and runs a mixed-radix (2 .. 8) Stockham FFT on all of them
-// (stage s reads in[j + r N/R], multiplies by the twiddle w^(r (j mod Ns)) of the Ns R-point DFT and writes
+// Transforms: a block holds a few 1-D lines in shared memory and runs a mixed-radix (2 .. 8) Stockham FFT on all of
+// them (stage s reads in[j + r N/R], multiplies by the twiddle w^(r (j mod Ns)) of the Ns R-point DFT and writes
 // out[(j / Ns) Ns R + j mod Ns + r Ns]; the output is in natural order); the butterflies of all lines are numbered
 // through and dealt to the threads, so no lane idles for a line length that is no multiple of 32.  A line's points lie
 // with one element of padding to every 128 bytes: the first stage's stores, R apart, would otherwise share a bank.
@@ -16,9 +16,9 @@
 //   y pass   tiles of consecutive kx columns, coalesced along kx
 //   z pass   forward FFT, the dipole Green's scale k (k . f) H / |k|^2 and the inverse FFT in one kernel; as the scale
 //            is of rank one, x and y enter only as kx fx + ky fy: two transforms each way instead of three
-// The float32 issue rate bounds it (some 220 instructions a point and transform in double-float).  Against one warp to a
-// line, radices up to 5, three z transforms and the six-entry scale tensor, three vectors on 192^3: x 0.52 and 0.46 ->
-// 0.39 and 0.45 ms, y 0.61 -> 0.38, z 1.29 -> 0.61 (with the x and y passes twice 3.49 -> 2.20); one vector on 240^3
+// The float32 issue rate bounds it (some 220 instructions a point and transform in double-float).  Against one warp to
+// a line, radices up to 5, three z transforms and the six-entry scale tensor, three vectors on 192^3: x 0.52 and 0.46
+// -> 0.39 and 0.45 ms, y 0.61 -> 0.38, z 1.29 -> 0.61 (with the x and y passes twice 3.49 -> 2.20); one vector on 240^3
 // 2.17 -> 1.65 ms, on 60 x 72 x 160 156 -> 102 us.
 #include <math.h>
 
@@ -271,8 +271,9 @@ struct Dft<A, 5> {
 // Stages on the nl lines of a block (p.N points each, line stride ld)
 // ---------------------------------------------------------------------------
 // Six blocks an SM (80 registers, 36 KB of shared memory each), the sums over both passes in x and y and the z pass: on
-// 192^3, 240^3, 60 x 72 x 160 2.26 ms, 1.65 ms, 105 us; five blocks of 44 KB 2.36, 1.64, 103; eight of 27 KB 2.24, 1.91, 97
-// (32-byte rows in z); four of 54 KB with radices 10 and 12 2.52, 1.95, 124; six of 36 KB with them 2.31, 1.85, 112.
+// 192^3, 240^3, 60 x 72 x 160 2.26 ms, 1.65 ms, 105 us; five blocks of 44 KB 2.36, 1.64, 103; eight of 27 KB 2.24,
+// 1.91, 97 (32-byte rows in z); four of 54 KB with radices 10 and 12 2.52, 1.95, 124; six of 36 KB with them 2.31,
+// 1.85, 112.
 constexpr int kDfThreads = 128, kDfBlocks = 6;
 constexpr size_t kDfSmem = 36 * 1024;
 
@@ -307,8 +308,8 @@ __device__ __forceinline__ void df_stage(const typename A::S *in, typename A::S 
     }
 }
 
-// Forward transform of the nl lines in a (b: scratch of the same size); returns the buffer with the result.  All threads
-// of the block call it; the lines are complete in a, and the result is complete on return.
+// Forward transform of the nl lines in a (b: scratch of the same size); returns the buffer with the result.  All
+// threads of the block call it; the lines are complete in a, and the result is complete on return.
 template <class A>
 __device__ typename A::S *fft_lines(typename A::S *a, typename A::S *b, int nl, int ld, const DfAxisPlan &p,
                                     const float4 *tws) {
@@ -330,8 +331,8 @@ __device__ typename A::S *fft_lines(typename A::S *a, typename A::S *b, int nl, 
 }
 
 // The twiddles go to the front of shared memory, the lines behind them.  (From global memory they missed L1, which the
-// lines' shared memory leaves small: with them and the lines' loads waited for one by one, the y pass on 192^3 took 0.58 ms
-// for three vectors.)
+// lines' shared memory leaves small: with them and the lines' loads waited for one by one, the y pass on 192^3 took
+// 0.58 ms for three vectors.)
 template <class A>
 __device__ __forceinline__ typename A::S *lines_after_twiddles(float4 *sm, const DfAxisPlan &p) {
     for (int i = threadIdx.x; i < p.ntw; i += kDfThreads) copy_async(sm + i, p.tw + i);
@@ -342,8 +343,9 @@ __device__ __forceinline__ typename A::S *lines_after_twiddles(float4 *sm, const
 // x pass (Rl: real type of the grids): two rows of Nx of a grid are one line (npairs lines over all the stacked grids)
 // ---------------------------------------------------------------------------
 template <class A, typename Rl>
-__global__ void __launch_bounds__(kDfThreads, kDfBlocks) k_fft_x_fwd(const Rl *__restrict__ grid, typename A::S *__restrict__ spec,
-                                                             int64_t npairs, RowPairs rp, DfAxisPlan px, int L, int ld) {
+__global__ void __launch_bounds__(kDfThreads, kDfBlocks)
+    k_fft_x_fwd(const Rl *__restrict__ grid, typename A::S *__restrict__ spec,
+                int64_t npairs, RowPairs rp, DfAxisPlan px, int L, int ld) {
     extern __shared__ float4 sm[];
     typename A::S *buf = lines_after_twiddles<A>(sm, px);
     const int Nx = px.N, Nxh = Nx / 2 + 1;
@@ -381,8 +383,9 @@ __global__ void __launch_bounds__(kDfThreads, kDfBlocks) k_fft_x_fwd(const Rl *_
 }
 
 template <class A, typename Rl>
-__global__ void __launch_bounds__(kDfThreads, kDfBlocks) k_fft_x_inv(const typename A::S *__restrict__ spec, Rl *__restrict__ grid,
-                                                             int64_t npairs, RowPairs rp, DfAxisPlan px, int L, int ld) {
+__global__ void __launch_bounds__(kDfThreads, kDfBlocks)
+    k_fft_x_inv(const typename A::S *__restrict__ spec, Rl *__restrict__ grid,
+                int64_t npairs, RowPairs rp, DfAxisPlan px, int L, int ld) {
     extern __shared__ float4 sm[];
     typename A::S *buf = lines_after_twiddles<A>(sm, px);
     const int Nx = px.N, Nxh = Nx / 2 + 1;
@@ -427,8 +430,9 @@ __global__ void __launch_bounds__(kDfThreads, kDfBlocks) k_fft_x_inv(const typen
 // y pass: L (a power of two) consecutive kx columns of one (component, z) plane
 // ---------------------------------------------------------------------------
 template <class A>
-__global__ void __launch_bounds__(kDfThreads, kDfBlocks) k_fft_y(typename A::S *__restrict__ spec, int64_t nplanes, int Nxh,
-                                                         DfAxisPlan py, int L, int ld, int inverse) {
+__global__ void __launch_bounds__(kDfThreads, kDfBlocks)
+    k_fft_y(typename A::S *__restrict__ spec, int64_t nplanes, int Nxh,
+            DfAxisPlan py, int L, int ld, int inverse) {
     extern __shared__ float4 sm[];
     typename A::S *buf = lines_after_twiddles<A>(sm, py);
     const int Ny = py.N, nblk = (Nxh + L - 1) / L;
@@ -454,13 +458,14 @@ __global__ void __launch_bounds__(kDfThreads, kDfBlocks) k_fft_y(typename A::S *
 // out = k (k . f) h, the sum over the components whose axis is on its Nyquist bin apart from the others' (the real part
 // of the complex pipeline's coupling).  Columns with both or neither of kx, ky on the Nyquist bin need two lines,
 // a = kx fx + ky fy and b = fz:  out_x = kx t, out_y = ky t, out_z = u with t, u the inverse transforms of h (a + kz b)
-// and h kz (a + kz b); where z is on the other side of the rule than x and y, of h a and h kz^2 b.  A tile that holds one
-// of the few other columns takes three lines a column, fewer columns at a time.
+// and h kz (a + kz b); where z is on the other side of the rule than x and y, of h a and h kz^2 b.  A tile that holds
+// one of the few other columns takes three lines a column, fewer columns at a time.
 // ---------------------------------------------------------------------------
 template <class A>
-__global__ void __launch_bounds__(kDfThreads, kDfBlocks) k_fft_z_scale(typename A::S *__restrict__ spec, int nrhs, GridParams gp,
-                                                               DfAxisPlan pz, DfStep q, const typename A::Coef *__restrict__ h,
-                                                               int L, int ld) {
+__global__ void __launch_bounds__(kDfThreads, kDfBlocks)
+    k_fft_z_scale(typename A::S *__restrict__ spec, int nrhs, GridParams gp,
+                  DfAxisPlan pz, DfStep q, const typename A::Coef *__restrict__ h,
+                  int L, int ld) {
     using V = typename A::V;
     using Rr = typename A::R;
     extern __shared__ float4 sm[];
@@ -585,8 +590,8 @@ int df_scale_table(const GridParams &gp, const double *H, float2 *hs, cudaStream
 static std::map<std::pair<int, int>, DfAxisPlan> g_df_axes;   // per (device, length)
 static std::mutex g_df_mu;
 
-// Radices of a 2-3-5 length with the fewest double-float instructions a point: the butterfly, the twiddles (32 each, none
-// in the first stage), the stores' normalisation and a charge for a stage's passes over shared memory.
+// Radices of a 2-3-5 length with the fewest double-float instructions a point: the butterfly, the twiddles (32 each,
+// none in the first stage), the stores' normalisation and a charge for a stage's passes over shared memory.
 static std::vector<int> df_radices(int n) {
     static const struct { int R; double ops; } kR[] = {{2, 32}, {3, 108}, {4, 128}, {5, 320}, {6, 312}, {8, 432}};
     std::vector<int> best, cur;
@@ -687,7 +692,8 @@ static int line_stride(int N) {
     return (int)at<A>(N - 1) + 1 | 1;
 }
 
-// Lines (columns) to a block: up to 8 (whole 128-byte rows of the strided passes) within kDfSmem, fewer where the grid has too few lines to give every SM two blocks.
+// Lines (columns) to a block: up to 8 (whole 128-byte rows of the strided passes) within kDfSmem, fewer where the grid
+// has too few lines to give every SM two blocks.
 static int lines_per_block(size_t column, int64_t columns) {
     int L = 8;
     while (L > 1 && (column * L > kDfSmem || columns / L < 304)) L /= 2;

@@ -249,10 +249,11 @@ __device__ __forceinline__ void stage64_prime(double2 *in, double2 *out, int nl,
 }
 
 // Prime radix R with (R - 1) / 2 = 3 q, q prime to 3.  With r = g^T, k = g^S (g a generator), the sums over r of
-// a_r cos(2 pi k r / R) and d_r sin(2 pi k r / R) are correlations over the exponents, Z_3 x Z_2q: the coefficient depends
-// on (s1 + t1 mod 3, s2 + t2) only (and changes sign, the sine's, or not with s2 + t2 -> + q), t1 in Z_3, t2 < q standing
-// for the pairs r, R - r.  In the direction of 3, with c_u = c' + c~_u, c' their mean,
-//   y_s = c' (a_0 + a_1 + a_2) + z_s,  z_0 = alpha c~_0 + beta c~_1,  z_1 = alpha c~_1 + beta c~_2,  z_2 = -(z_0 + z_1),
+// a_r cos(2 pi k r / R) and d_r sin(2 pi k r / R) are correlations over the exponents, Z_3 x Z_2q: the coefficient
+// depends on (s1 + t1 mod 3, s2 + t2) only (and changes sign, the sine's, or not with s2 + t2 -> + q), t1 in Z_3, t2 <
+// q standing for the pairs r, R - r.  In the direction of 3, with c_u = c' + c~_u, c' their mean,
+//   y_s = c' (a_0 + a_1 + a_2) + z_s,
+//   z_0 = alpha c~_0 + beta c~_1,  z_1 = alpha c~_1 + beta c~_2,  z_2 = -(z_0 + z_1),
 // alpha = a_0 - a_2, beta = a_1 - a_2 (the c~ sum to zero): five multiplications instead of nine.
 //   1  sums and differences of the pairs, then sum, alpha and beta of each triple of them, in place
 //   2  a thread takes one part (cosine, sine), one component (re, im) and one s2 of a butterfly: three outputs
@@ -368,9 +369,10 @@ __device__ double2 *fft64_lines(double2 *a, double2 *b, int nl, int ld, const F6
 // well (128 registers, 4 blocks) 8.56, with none above 8 8.61.
 constexpr int kF64Threads = 128, kF64Blocks = 5;
 
-__global__ void __launch_bounds__(kF64Threads, kF64Blocks) k_f64_x_fwd(const double *__restrict__ grid,
-                                                           double2 *__restrict__ spec, int64_t npairs, RowPairs rp, F64Axis px,
-                                                           int L) {
+__global__ void __launch_bounds__(kF64Threads, kF64Blocks)
+    k_f64_x_fwd(const double *__restrict__ grid,
+                double2 *__restrict__ spec, int64_t npairs, RowPairs rp, F64Axis px,
+                int L) {
     extern __shared__ double2 sm64[];
     const int Nx = px.N, Nxh = Nx / 2 + 1, ld = Nx | 1;
     const int64_t ntiles = (npairs + L - 1) / L;
@@ -400,8 +402,9 @@ __global__ void __launch_bounds__(kF64Threads, kF64Blocks) k_f64_x_fwd(const dou
     }
 }
 
-__global__ void __launch_bounds__(kF64Threads, kF64Blocks) k_f64_x_inv(const double2 *__restrict__ spec, double *__restrict__ grid,
-                                                           int64_t npairs, RowPairs rp, F64Axis px, int L) {
+__global__ void __launch_bounds__(kF64Threads, kF64Blocks)
+    k_f64_x_inv(const double2 *__restrict__ spec, double *__restrict__ grid,
+                int64_t npairs, RowPairs rp, F64Axis px, int L) {
     extern __shared__ double2 sm64[];
     const int Nx = px.N, Nxh = Nx / 2 + 1, ld = Nx | 1;
     const int64_t ntiles = (npairs + L - 1) / L;
@@ -437,12 +440,13 @@ __global__ void __launch_bounds__(kF64Threads, kF64Blocks) k_f64_x_inv(const dou
 }
 
 // ---------------------------------------------------------------------------
-// y pass: L consecutive columns of the (component, z) planes, numbered through all planes: a tile of the one column that
-// 33 leave over beside four times eight would cost a warp's float64 instruction as much as a whole one (three vectors on
-// 64^3 54.9 -> 50.9 us a pass)
+// y pass: L consecutive columns of the (component, z) planes, numbered through all planes: a tile of the one column
+// that 33 leave over beside four times eight would cost a warp's float64 instruction as much as a whole one (three
+// vectors on 64^3 54.9 -> 50.9 us a pass)
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kF64Threads, kF64Blocks) k_f64_y(double2 *__restrict__ spec, int64_t nplanes, int Nxh, F64Axis py,
-                                                       int L, int inverse) {
+__global__ void __launch_bounds__(kF64Threads, kF64Blocks)
+    k_f64_y(double2 *__restrict__ spec, int64_t nplanes, int Nxh, F64Axis py,
+            int L, int inverse) {
     extern __shared__ double2 sm64[];
     const int Ny = py.N, ld = Ny | 1;
     const double sg = inverse ? -1.0 : 1.0;
@@ -480,8 +484,9 @@ __global__ void __launch_bounds__(kF64Threads, kF64Blocks) k_f64_y(double2 *__re
 // hs (a + kz b) and hs kz (a + kz b); where z is on the other side of the rule than x and y, of hs a and hs kz^2 b.
 // A block that holds one of the few other columns takes three lines a column.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kF64Threads, kF64Blocks) k_f64_z_scale(double2 *__restrict__ spec, int nrhs, GridParams gp,
-                                                             F64Axis pz, const double *__restrict__ hs, int L) {
+__global__ void __launch_bounds__(kF64Threads, kF64Blocks)
+    k_f64_z_scale(double2 *__restrict__ spec, int nrhs, GridParams gp,
+                  F64Axis pz, const double *__restrict__ hs, int L) {
     extern __shared__ double2 sm64[];
     const int Nx = gp.N[0], Ny = gp.N[1], Nz = gp.N[2], Nxh = Nx / 2 + 1, ld = Nz | 1, nblk = (Nxh + L - 1) / L;
     const int64_t zs = (int64_t)Ny * Nxh, Gc = zs * Nz;
@@ -744,12 +749,13 @@ int f64_plan(const GridParams &gp, F64Plan3 *out) {
     return MPS_OK;
 }
 
-// Both ways, cuFFT against these, us.  Fused, with the scale: rods behind a short x lose (12 x 12 x 400, 12 and 24 vectors 408
-// against 534 and 767 against 1012; 10 x 20 x 400, 3 vectors 177 against 221), wider ones and longer x do not (12 x 48 x 400,
-// 3 vectors 458 against 438; 14 x 14 x 500, 24 vectors 1519 against 1280; 400 x 12 x 12 1118 against 770).
-// Not fused: 24 grids on 16^3, 20^3, 25^3 78 against 100, 68 and 75, 99 and 116, 96 grids on 16^3, 20^3, 25^3, 28^3 78 and
-// 100, 123 and 188, 259 and 336, 326 and 328, on 24 x 24 x 48 363 and 430; on 30^3, 32^3, 36^3, 48^3 456 against 421, 415
-// and 385, 700 and 627, 1793 and 1250.
+// Both ways, cuFFT against these, us.  Fused, with the scale: rods behind a short x lose (12 x 12 x 400, 12 and 24
+// vectors 408 against 534 and 767 against 1012; 10 x 20 x 400, 3 vectors 177 against 221), wider ones and longer x do
+// not (12 x 48 x 400, 3 vectors 458 against 438; 14 x 14 x 500, 24 vectors 1519 against 1280; 400 x 12 x 12 1118
+// against 770).
+// Not fused: 24 grids on 16^3, 20^3, 25^3 78 against 100, 68 and 75, 99 and 116, 96 grids on 16^3, 20^3, 25^3, 28^3 78
+// and 100, 123 and 188, 259 and 336, 326 and 328, on 24 x 24 x 48 363 and 430; on 30^3, 32^3, 36^3, 48^3 456 against
+// 421, 415 and 385, 700 and 627, 1793 and 1250.
 bool f64_pays(const GridParams &gp, bool fused) {
     const int longest = std::max({gp.N[0], gp.N[1], gp.N[2]});
     if (fused) return gp.N[0] >= 14 || longest < 200 || std::min(gp.N[1], gp.N[2]) >= 40;

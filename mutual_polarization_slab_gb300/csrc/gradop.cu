@@ -89,12 +89,13 @@ constexpr int kGChunk = 96;
 // workload against 0.299 at 4 blocks (64 registers), 0.300 at 6 (spills) and 0.342 unbounded.
 // Depth 12 (36 accumulators for 3 vectors, 64 registers) at 4 blocks per SM, depth 16 (48) at 3.
 template <int TZ, int NR>
-__global__ void __launch_bounds__(256, TZ > 12 ? 3 : (TZ > 8 ? 4 : 5)) k_spread_grad_tiled(const double *__restrict__ m, int64_t n, int r0,
-                                                           const int32_t *__restrict__ start,
-                                                           const float *__restrict__ w, const float *__restrict__ g,
-                                                           GridParams gp, const int64_t *__restrict__ tstart,
-                                                           const int32_t *__restrict__ entries, int ntx, int nty,
-                                                           float *__restrict__ grid) {
+__global__ void __launch_bounds__(256, TZ > 12 ? 3 : (TZ > 8 ? 4 : 5))
+    k_spread_grad_tiled(const double *__restrict__ m, int64_t n, int r0,
+                        const int32_t *__restrict__ start,
+                        const float *__restrict__ w, const float *__restrict__ g,
+                        GridParams gp, const int64_t *__restrict__ tstart,
+                        const int32_t *__restrict__ entries, int ntx, int nty,
+                        float *__restrict__ grid) {
     constexpr int kPos = kTileX + kTileY + TZ + 1 - TZ % 2;   // aligned positions per particle (odd: no bank conflicts)
     constexpr int kMS = (3 * NR + 3) & ~3;       // moments, padded to a float4 multiple
     __shared__ float2 s_f[kGChunk][kPos];        // (w, dw/dr) at tile columns, rows, planes
@@ -326,10 +327,11 @@ __global__ void k_contract_grad_gather(const float *__restrict__ partial, int64_
     }
 }
 
-// The columns of a stencil by rounds of a warp, for the contractions below: lane's column (jx, jy) of a round, the planes
-// sub, sub + lpp, ... of it; false: none.  For the supports of the staged contraction (8 and 10) the columns that a round
-// reads together lie in different banks of its region, whose rows are 20 floats apart: 8 x 4 columns of every other row,
-// then the edge of 10 x 10, 24 columns and 12 with two lanes each.  Elsewhere 32 consecutive columns a round.
+// The columns of a stencil by rounds of a warp, for the contractions below: lane's column (jx, jy) of a round, the
+// planes sub, sub + lpp, ... of it; false: none.  For the supports of the staged contraction (8 and 10) the columns
+// that a round reads together lie in different banks of its region, whose rows are 20 floats apart: 8 x 4 columns of
+// every other row, then the edge of 10 x 10, 24 columns and 12 with two lanes each.  Elsewhere 32 consecutive columns a
+// round.
 __host__ __device__ constexpr int grad_rounds(int P) { return P == 8 ? 2 : (P == 10 ? 4 : (P * P + 31) / 32); }
 
 __device__ __forceinline__ bool grad_column(int P, int round, int lane, int *jx, int *jy, int *sub, int *lpp) {
@@ -427,20 +429,19 @@ __global__ void __launch_bounds__(256, 3) k_contract_grad_warp(const float *__re
 }
 
 // Contraction by home blocks (the default where the support is 8 or 10): one CTA per kHomeBlock^3 block of grid nodes
-// stages every node its particles' stencils can reach -- the block grown by P - 1 nodes per axis, one plane of nodes per
-// vector -- in shared memory, and its particles' offsets and per-axis factors (kHomeChunk particles at a time).  One warp
-// per particle then runs the sums of k_contract_grad_warp in the same order, from shared memory and registers instead of
-// L2: the results are bit-identical.  P is a template parameter, so the z runs unroll completely with the z factors in
-// registers and the shared-memory offsets are immediates.  A node is staged by about (1 + (P - 1) / 8)^3 blocks (9.6 at
-// P = 10), all from L2; with one vector a CTA takes three home blocks along y (6.2).
-// Shared memory bounds it (a node's read and its staging), so the rows lie 20 floats apart: the columns that a round of the
-// warp reads together then hit different banks (grad_column), and a row is staged by five 16-byte copies.  The sums end
-// one to a lane, converted and scaled together: lane 0's 3 NR conversions and multiplications had cost a warp 6 NR float64
-// instructions a particle.  Three vectors of N = 1e5 on 144^3 / one of N = 2e5 on 192^3: 0.209 / 0.155 ms with two-way bank
-// conflicts, staging by single floats and lane 0's epilogue; 0.168 / 0.136 with the sums one to a lane and asynchronous
-// copies; 0.118 / 0.109 so.
-// 78 KB of shared memory at P = 10 and 3 vectors, 3 blocks per SM (80 registers); float4 nodes (the 3 vectors interleaved,
-// 2 blocks per SM) were slower.
+// stages every node its particles' stencils can reach -- the block grown by P - 1 nodes per axis, one plane of nodes
+// per vector -- in shared memory, and its particles' offsets and per-axis factors (kHomeChunk particles at a time).
+// One warp per particle then runs the sums of k_contract_grad_warp in the same order, from shared memory and registers
+// instead of L2: the results are bit-identical.  P is a template parameter, so the z runs unroll completely with the z
+// factors in registers and the shared-memory offsets are immediates.  A node is staged by about (1 + (P - 1) / 8)^3
+// blocks (9.6 at P = 10), all from L2; with one vector a CTA takes three home blocks along y (6.2).  Shared memory
+// bounds it (a node's read and its staging), so the rows lie 20 floats apart: the columns that a round of the warp
+// reads together then hit different banks (grad_column), and a row is staged by five 16-byte copies.  The sums end one
+// to a lane, converted and scaled together: lane 0's 3 NR conversions and multiplications had cost a warp 6 NR float64
+// instructions a particle.  Three vectors of N = 1e5 on 144^3 / one of N = 2e5 on 192^3: 0.209 / 0.155 ms with two-way
+// bank conflicts, staging by single floats and lane 0's epilogue; 0.168 / 0.136 with the sums one to a lane and
+// asynchronous copies; 0.118 / 0.109 so.  78 KB of shared memory at P = 10 and 3 vectors, 3 blocks per SM (80
+// registers); float4 nodes (the 3 vectors interleaved, 2 blocks per SM) were slower.
 constexpr int kHomeChunk = 24;
 constexpr int kHomeRow = 20;   // floats from one row of the region to the next (grad_column), whole 16-byte pieces
 
@@ -613,8 +614,8 @@ static int home_launch(const float *grid, int64_t n, int r0, const int32_t *star
     return MPS_OK;
 }
 
-// One vector leaves room for three home blocks to a CTA: taken where every SM still gets four CTAs and the longer region
-// wraps at most twice.
+// One vector leaves room for three home blocks to a CTA: taken where every SM still gets four CTAs and the longer
+// region wraps at most twice.
 template <int P>
 static int home_dispatch(const float *grid, int64_t n, int nrhs, const int32_t *start, const float *w, const float *g,
                          const GridParams &gp, const TileBins &tb, double *out, cudaStream_t s) {

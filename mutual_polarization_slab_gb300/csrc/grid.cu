@@ -94,12 +94,12 @@ __global__ void __launch_bounds__(256) k_spread(const double *__restrict__ m, in
     }
 }
 
-// Contract: one warp per particle in the visiting order, gather + warp reduction; out = Hk (overwrites).  Lanes take the
-// stencil's (x, y) columns; a column's z sums are weighted by wx wy once, so a node costs one multiply-add per component
-// (in float64 the arithmetic bounds this kernel: three vectors, N = 100,000, P = 10 2.55 -> 1.92 ms, where 3.3
-// multiply-adds a node take 1.98 at the measured rate; one vector, N = 20,000, P = 8 100 -> 70 us; 36 vectors,
-// N = 2000, P = 5 202 -> 109 us).
-// Blocks of 4 warps and one warp per particle and vector (grid y): a few hundred particles still reach every SM.
+// Contract: one warp per particle in the visiting order, gather + warp reduction; out = Hk (overwrites).  Lanes take
+// the stencil's (x, y) columns; a column's z sums are weighted by wx wy once, so a node costs one multiply-add per
+// component (in float64 the arithmetic bounds this kernel: three vectors, N = 100,000, P = 10 2.55 -> 1.92 ms, where
+// 3.3 multiply-adds a node take 1.98 at the measured rate; one vector, N = 20,000, P = 8 100 -> 70 us; 36 vectors, N =
+// 2000, P = 5 202 -> 109 us).  Blocks of 4 warps and one warp per particle and vector (grid y): a few hundred particles
+// still reach every SM.
 template <typename T>
 __global__ void __launch_bounds__(128) k_contract(const T *__restrict__ grid, int64_t n,
                                                   const int32_t *__restrict__ start, const T *__restrict__ w,

@@ -111,14 +111,14 @@ __global__ void __launch_bounds__(256) k_contract_gen(const T *__restrict__ grid
     }
 }
 
-// Contraction of the eight float32 grids of a vector by home blocks: a block takes the particles whose stencils start in
-// one 8^3 block of nodes and four of the components; it stages the nodes that they reach, the block grown by P - 1 per
-// axis, as float4 (the four components side by side), then a warp per particle sums over its stencil from shared memory,
-// the lanes on the P^2 columns.  Rows of P + 8 nodes: consecutive columns of a warp then lie 16 bytes apart modulo the
-// banks, whatever P.  The gather from the grids (k_contract_gen) reads a line per row, plane and component of every
-// particle through L1, which bounds it; here the staging does (the blocks' chains of loads).  N = 50,320, 90 x 90 x 96,
-// P = 6: 96 us by the gather (with its sums converted by one lane), 60 so (with an interleaved copy of the grids, staged
-// 16 bytes at a time or gathered from, 63 and 68).
+// Contraction of the eight float32 grids of a vector by home blocks: a block takes the particles whose stencils start
+// in one 8^3 block of nodes and four of the components; it stages the nodes that they reach, the block grown by P - 1
+// per axis, as float4 (the four components side by side), then a warp per particle sums over its stencil from shared
+// memory, the lanes on the P^2 columns.  Rows of P + 8 nodes: consecutive columns of a warp then lie 16 bytes apart
+// modulo the banks, whatever P.  The gather from the grids (k_contract_gen) reads a line per row, plane and component
+// of every particle through L1, which bounds it; here the staging does (the blocks' chains of loads).  N = 50,320, 90 x
+// 90 x 96, P = 6: 96 us by the gather (with its sums converted by one lane), 60 so (with an interleaved copy of the
+// grids, staged 16 bytes at a time or gathered from, 63 and 68).
 constexpr int kHome8Chunk = 32;
 constexpr int kHome8Warps = 8;
 
@@ -223,8 +223,8 @@ __global__ void __launch_bounds__(kHome8Warps * 32, 5) k_contract_home8(
 // ---------------------------------------------------------------------------
 // The couplings depend on k only through its components' squares: worked out once for the quarter spectrum and written
 // for its mirror images.  The float32 table holds the unit wave vector too (the float64 square root and division of a
-// point cost the float32 scale kernel more than reading 16 bytes: 25 -> 12 us on 90 x 90 x 96); the float64 kernel works
-// it out.
+// point cost the float32 scale kernel more than reading 16 bytes: 25 -> 12 us on 90 x 90 x 96); the float64 kernel
+// works it out.
 __global__ void k_quad_kcoef(GridParams gp, double *__restrict__ c64, float4 *__restrict__ c32) {
     const HalfQuarter hq(gp.N);
     const double invG = 1.0 / (double)gp.G;
@@ -583,8 +583,8 @@ int contract_home8(const float *grid, int64_t n, int nrhs, const int32_t *start,
                    const TileBins &tb, double *out, cudaStream_t s) {
     if (!tb.has_home) return MPS_BAD_ARG;
     const size_t smem = home8_smem(gp.P);
-    // one limit for every launch (the largest support's): a thread that sets its own lower one between another's request
-    // and launch would make that launch fail
+    // one limit for every launch (the largest support's): a thread that sets its own lower one between another's
+    // request and launch would make that launch fail
     if (smem > 48 * 1024)
         MPS_CUDA_TRY(cudaFuncSetAttribute(k_contract_home8, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)home8_smem(kMaxP)));

@@ -278,9 +278,9 @@ int real_space_csr(const double *m, double *out, int64_t n, int nrhs, const int6
                    PairData<T> pd, const double *diag, const int32_t *diag_of_rhs, const double *slab, bool accumulate,
                    cudaStream_t s) {
     // Up to four vectors share a pass over the pair data, 8 lanes to a row.  Where that leaves most SMs without work, a
-    // warp takes one row of one vector, in blocks of 4 warps, and reads the pairs once a vector: N = 400, 62 neighbours,
-    // 1, 3, 12 and 24 vectors 1.6, 2.8, 1.6 and 1.0 times as fast, N = 1000, 18 neighbours, 1, 4, 12 vectors 1.1, 1.4, 0.7;
-    // N = 2000, 3 vectors with 5, 19, 73 neighbours 0.7, 0.9, 1.3.
+    // warp takes one row of one vector, in blocks of 4 warps, and reads the pairs once a vector: N = 400, 62
+    // neighbours, 1, 3, 12 and 24 vectors 1.6, 2.8, 1.6 and 1.0 times as fast, N = 1000, 18 neighbours, 1, 4, 12
+    // vectors 1.1, 1.4, 0.7; N = 2000, 3 vectors with 5, 19, 73 neighbours 0.7, 0.9, 1.3.
     if (n * std::max(nrhs, 4) <= (np >= 48 * n ? 10000 : 6000)) {
         for (int r0 = 0; r0 < nrhs; r0 += 32768) {
             k_rs_csr<T, 32, 1><<<dim3(grid_for(n * 32, 128, 152 * 64), min(32768, nrhs - r0)), 128, 0, s>>>(
@@ -323,8 +323,8 @@ int real_space_csr_df(const double *m, dfv *mdf, double *out, int64_t n, int nrh
                       bool accumulate, const int32_t *order, cudaStream_t s) {
     k_to_dfv<<<grid_for((int64_t)nrhs * n * 3, 256), 256, 0, s>>>(m, (int64_t)nrhs * n * 3, mdf);
     MPS_LAUNCH_CHECK();
-    // a warp per row and vector, as in float64 (3 vectors, N = 2000 and 4000, 20 neighbours 1.15 and 1.0 times as fast; N =
-    // 4000 and 7000, 65 neighbours 1.2 and 1.0)
+    // a warp per row and vector, as in float64 (3 vectors, N = 2000 and 4000, 20 neighbours 1.15 and 1.0 times as fast;
+    // N = 4000 and 7000, 65 neighbours 1.2 and 1.0)
     if (n <= (np >= 48 * n ? 6000 : 1500)) {
         for (int r0 = 0; r0 < nrhs; r0 += 32768) {
             k_rs_csr<dfv, 32, 1, dfv><<<dim3(grid_for(n * 32, 128, 152 * 64), min(32768, nrhs - r0)), 128, 0, s>>>(
@@ -368,10 +368,10 @@ size_t m32_floats(int64_t n, int nrhs) { return (size_t)n * (size_t)nrhs * 4; }
 // Float32 pair sum.  A warp takes a row and a lane one vector of one pair: RL vectors side by side, 32 / RL pairs at a
 // time.  The loads are what costs here (a warp's load takes the L1 a pass for every line it touches): 4 lanes to a row
 // and all vectors in a lane's registers touched 8 lines with each pair array and 32 with each 16 bytes of the gathered
-// moments; now a pair array's load touches one or two, and a gather one line a pair.  The row's sums end in float64 with
-// the diagonal, each component on a lane of its own.
-// Alone: one vector, N = 200,000, 60 neighbours 264 -> 122 us; 48 vectors, N = 3000 55 -> 25 us; three vectors, N = 100,000
-// 104 -> 115 us (a quarter of the lanes idle), but less in the way of the spread that runs beside it.
+// moments; now a pair array's load touches one or two, and a gather one line a pair.  The row's sums end in float64
+// with the diagonal, each component on a lane of its own.  Alone: one vector, N = 200,000, 60 neighbours 264 -> 122 us;
+// 48 vectors, N = 3000 55 -> 25 us; three vectors, N = 100,000 104 -> 115 us (a quarter of the lanes idle), but less in
+// the way of the spread that runs beside it.
 template <int RL>
 __global__ void __launch_bounds__(256) k_rs_csr_f32(const double *__restrict__ m, double *__restrict__ out, int64_t n,
                                                     int nrhs, int rfirst, const int64_t *__restrict__ row_ptr,
@@ -433,8 +433,8 @@ static int rs_f32_launch(const double *m, const float4 *mf, double *out, int64_t
     return MPS_OK;
 }
 
-// Eight vectors side by side (all such blocks in one launch: small systems fill the GPU with them), a rest of up to four
-// as 4, 2 or 1, a larger one as a block of eight with idle lanes.
+// Eight vectors side by side (all such blocks in one launch: small systems fill the GPU with them), a rest of up to
+// four as 4, 2 or 1, a larger one as a block of eight with idle lanes.
 int real_space_csr_f32(const double *m, float *m32, double *out, int64_t n, int nrhs, const int64_t *row_ptr,
                        PairData<float> pd, const double *diag, const int32_t *diag_of_rhs, const double *slab,
                        bool accumulate, const int32_t *order, cudaStream_t s) {

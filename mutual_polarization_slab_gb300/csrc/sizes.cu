@@ -161,8 +161,8 @@ __device__ __forceinline__ int64_t cs_search(const double *__restrict__ rv, int6
 }
 
 // Per-pair couplings of the CSR list: A (I - rr) and B - A, float64 and float32.  A warp takes a row and its lanes the
-// row's pairs: the loads and the search are chains of latencies, and with a thread a row 3,000 spheres filled 94 warps of
-// the chip (3,000 spheres, 60 pairs each: 1.58 ms, 0.25 with the lanes on the pairs).
+// row's pairs: the loads and the search are chains of latencies, and with a thread a row 3,000 spheres filled 94 warps
+// of the chip (3,000 spheres, 60 pairs each: 1.58 ms, 0.25 with the lanes on the pairs).
 __global__ void k_cs_pair_coefs(const int64_t *__restrict__ row_ptr, const int32_t *__restrict__ nbr,
                                 const double *__restrict__ dist, int64_t n, const double *__restrict__ radius,
                                 const int32_t *__restrict__ cls, int64_t M, const double *__restrict__ tab,
@@ -296,8 +296,9 @@ __global__ void __launch_bounds__(256, MB) k_spread_cs(const double *__restrict_
         const int r0 = (int)(t / n) * RB;
         const int cnt = min(RB, nrhs - r0);
         const int sx = start[3 * a], sy = start[3 * a + 1], sz = start[3 * a + 2];
-        // every lane loads all the vectors' moments: handed round by shuffles from a lane each, the kernel took up to twice as
-        // long (12 vectors, N = 4000, 64^3, P = 16 215 us so, 430 by shuffles; N = 20,000, 80^3, P = 8 171 and 269)
+        // every lane loads all the vectors' moments: handed round by shuffles from a lane each, the kernel took up to
+        // twice as long (12 vectors, N = 4000, 64^3, P = 16 215 us so, 430 by shuffles; N = 20,000, 80^3, P = 8 171 and
+        // 269)
         T px[RB], py[RB], pz[RB];
 #pragma unroll
         for (int q = 0; q < RB; ++q) {
@@ -349,9 +350,9 @@ struct CsCplx<double> {
     using type = double2;
 };
 
-// spec[r][k] *= coef[k]: a thread takes one spectrum point of a few vectors (blockIdx.y), with one complex (8 or 16 byte)
-// load and store per value; with all vectors to a thread a small grid's points filled the chip too thinly (48 vectors on
-// 40^3: 13.7 -> 4.0 us).
+// spec[r][k] *= coef[k]: a thread takes one spectrum point of a few vectors (blockIdx.y), with one complex (8 or 16
+// byte) load and store per value; with all vectors to a thread a small grid's points filled the chip too thinly (48
+// vectors on 40^3: 13.7 -> 4.0 us).
 constexpr int kScaleVec = 4;
 
 template <typename T>
@@ -448,18 +449,18 @@ __global__ void __launch_bounds__(256, MB) k_contract_cs(const T *__restrict__ g
 // ---------------------------------------------------------------------------
 // Many vectors (a spectrum or sweep batch).
 //
-// Spread: a block owns an 8 x 4 x 2 tile of nodes and walks the particles whose stencils reach it (TileBins), 32 at a time
-// with their moments in shared memory; a warp owns a row of 8 nodes, four lanes to a node, and takes the particles that
-// reach its row (a ballot) one after the other: one weight K(d)/d a node serves 16 vectors a group, V groups to a block.
-// Every node is written once, in the planes that the transforms read, in a fixed order of sums: no atomics, no zeroing.
-// 48 vectors, 3,000 spheres, 40^3, P = 8: 87 us with float atomics from a warp a particle (78 with four-vector atomics on
-// interleaved grids), 54 so; a lane keeps two nodes along z (one: 73), the moments read from shared
-// memory being what bounds it.
+// Spread: a block owns an 8 x 4 x 4 tile of nodes and walks the particles whose stencils reach it (TileBins), 32 at
+// a time with their moments in shared memory; a warp owns two rows of 8 nodes, one above the other, four lanes to a
+// pair of nodes, and takes the particles that reach its rows (a ballot), four at a time: one weight K(d)/d a node
+// serves 16 vectors a group, V groups to a block.  Every node is written once, in the planes that the transforms read,
+// in a fixed order of sums: no atomics, no zeroing.  48 vectors, 3,000 spheres, 40^3, P = 8: 87 us with float atomics
+// from a warp a particle (78 with four-vector atomics on interleaved grids), 54 so.  Reading the moments from shared
+// memory bounds it, so a lane keeps two nodes along z for each read (one: 73).
 //
-// Contraction: the grids lie side by side, node by node, four vectors to a float4.  From planes, a warp touched a line in
-// L1 for every vector and row of the stencil; here four lanes take a node's 16 vectors (64 contiguous bytes), eight nodes
-// of the stencil at a time, the weights are read once for all 16, and no sum crosses more than eight lanes.  103 -> 50 us,
-// the L2's bandwidth, and 7 us for the transposition.
+// Contraction: the grids lie side by side, node by node, four vectors to a float4.  From planes, a warp touched a line
+// in L1 for every vector and row of the stencil; here four lanes take a node's 16 vectors (64 contiguous bytes), eight
+// nodes of the stencil at a time, the weights are read once for all 16, and no sum crosses more than eight lanes.  103
+// -> 50 us, the L2's bandwidth, and 7 us for the transposition.
 // ---------------------------------------------------------------------------
 constexpr int kCsGroup = 16;
 constexpr int kCsTileX = 8, kCsTileY = 4, kCsTileZ = 4, kCsChunk = 32;
@@ -754,18 +755,18 @@ static bool cs_many(const GridParams &gp, int64_t n, int nrhs) {
     return true;
 }
 
-// Spread by tiles: with fewer than two tiles for every SM a tile's list is the time it takes, and on a large grid with few
-// particles every tile's own time is.  By warps a particle / by tiles, us: 16 vectors, P = 8, 40^3, 3000 and 216 particles
-// 39 / 34 and 21 / 14; 96^3, P = 6, 16 vectors, 1105 particles 27 / 45, 8847 66 / 76; 48 vectors, 500 particles, P = 8
-// 66 / 66.
+// Spread by tiles: with fewer than two tiles for every SM a tile's list is the time it takes, and on a large grid with
+// few particles every tile's own time is.  By warps a particle / by tiles, us: 16 vectors, P = 8, 40^3, 3000 and 216
+// particles 39 / 34 and 21 / 14; 96^3, P = 6, 16 vectors, 1105 particles 27 / 45, 8847 66 / 76; 48 vectors, 500
+// particles, P = 8 66 / 66.
 bool cs_many_spread(const GridParams &gp, int64_t n, int nrhs) {
     return cs_many(gp, n, nrhs) && gp.G >= 300 * kCsTileX * kCsTileY * kCsTileZ &&
            (gp.G < 150000 || (double)n * gp.P * gp.P * gp.P * nrhs >= 30.0 * gp.G);
 }
 
 // Contraction of interleaved grids: the transposition costs by nodes, the gather that it speeds up by particles, and a
-// group that is not full costs as much as a full one.  By planes / interleaved, us: 48 vectors, 40^3, 3000 spheres, P = 8
-// 85 / 60, 216 16 / 25; 16 vectors, 40^3, P = 8, 4000 43 / 37, 1600 23 / 25; 96^3, P = 6, 1105 27 / 69.
+// group that is not full costs as much as a full one.  By planes / interleaved, us: 48 vectors, 40^3, 3000 spheres, P =
+// 8 85 / 60, 216 16 / 25; 16 vectors, 40^3, P = 8, 4000 43 / 37, 1600 23 / 25; 96^3, P = 6, 1105 27 / 69.
 bool cs_many_contract(const GridParams &gp, int64_t n, int nrhs) {
     const int lanes = (nrhs + kCsGroup - 1) / kCsGroup * kCsGroup;
     return cs_many(gp, n, nrhs) && (double)n * gp.P * gp.P * (2 * nrhs - lanes) >= 20.0 * gp.G && n * nrhs >= 40000;

@@ -22,8 +22,8 @@ int scale_cs(void *spec, int nrhs, const GridParams &gp, const T *coef, cudaStre
 template <typename T>
 int contract_cs(const T *grid, int64_t n, int nrhs, const int32_t *start, const double *base, const T *g,
                 const GridParams &gp, double *out, cudaStream_t s);
-// The float32 spread and contraction of many vectors (scratch of cs_many_floats, 16-byte aligned; tb from cs_bins_build),
-// each where it is the faster one.
+// The float32 spread and contraction of many vectors (scratch of cs_many_floats, 16-byte aligned; tb from
+// cs_bins_build), each where it is the faster one.
 bool cs_many_spread(const GridParams &gp, int64_t n, int nrhs);
 bool cs_many_contract(const GridParams &gp, int64_t n, int nrhs);
 size_t cs_many_floats(int nrhs, int64_t G);

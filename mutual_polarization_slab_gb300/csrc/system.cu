@@ -712,9 +712,9 @@ static int ensure_nodes(mps_system *s, cudaStream_t st, bool *used) {
 
 static int df_usable(mps_system *s, bool *usable);
 
-// The float64 transforms of fft64.cu take every axis up to 1024 whose prime factors are at most 127; grids on which they do
-// not pay (f64_pays) and other grids keep cuFFT.  A failure to plan decides nothing: it is the
-// caller's status, and the next call plans again.
+// The float64 transforms of fft64.cu take every axis up to 1024 whose prime factors are at most 127; grids on which
+// they do not pay (f64_pays) and other grids keep cuFFT.  A failure to plan decides nothing: it is the caller's status,
+// and the next call plans again.
 static int f64_usable(mps_system *s, bool *usable) {
     if (s->f64_state == 0) {
         MPS_TRY(f64_plan(s->gp, &s->f64p));
@@ -774,8 +774,8 @@ static bool own_fft32() {
     return e && strcmp(e, "own") == 0;
 }
 
-// Wave-space field grids of nrhs moment vectors in float64 (spread, transforms, dipole scale), left in s->grid64.  Stage
-// marks 2..5 of the calling matvec (ev may be null).
+// Wave-space field grids of nrhs moment vectors in float64 (spread, transforms, dipole scale), left in s->grid64.
+// Stage marks 2..5 of the calling matvec (ev may be null).
 static int f64_field_grids(mps_system *s, const double *m, int nrhs, StageEvents *ev, cudaStream_t st) {
     bool own = false, nodes = false;
     MPS_TRY(f64_usable(s, &own));
@@ -980,9 +980,9 @@ static int df_usable(mps_system *s, bool *usable) {
 template <typename T>
 static int matvec_quad(mps_system *s, const double *m, double *out, int nrhs, cudaStream_t st) {
     const bool dbl = sizeof(T) == 8;
-    // float64 moments go up by atomics (spread_gen): by nodes, eight float64 sums a node and particle took about twice as
-    // long wherever the time counts (one vector, N = 3500, 64^3, P = 6 28 us against 54; three, N = 1041, 25^3, P = 12 121
-    // against 412)
+    // float64 moments go up by atomics (spread_gen): by nodes, eight float64 sums a node and particle took about twice
+    // as long wherever the time counts (one vector, N = 3500, 64^3, P = 6 28 us against 54; three, N = 1041, 25^3, P =
+    // 12 121 against 412)
     bool nodes = false;
     if (!dbl && spread_nodes8_pays(s->gp, s->n)) MPS_TRY(ensure_nodes(s, st, &nodes));
     const bool home = nodes && contract_home8_pays(s->gp, s->n);
@@ -1104,8 +1104,9 @@ static int matvec_cs(mps_system *s, const double *m, double *out, int nrhs, cuda
     StageEvents *ev = nullptr;
     MPS_TRY(stage_begin(s, dbl ? MPS_FP64 : MPS_FP32, &ev, st));
     const bool beside = !dbl && pair_sum_beside(ev);
-    // the spread of few vectors goes first: the pair sum's blocks kept it from the SMs (one vector, 4000 particles, 40^3,
-    // P = 8 a matvec of 77 -> 74 us; 7400, 48^3, P = 12 182 -> 166); that of many does not (a batch of 48 14.5 -> 15.1 ms)
+    // the spread of few vectors goes first: the pair sum's blocks kept it from the SMs (one vector, 4000 particles,
+    // 40^3, P = 8 a matvec of 77 -> 74 us; 7400, 48^3, P = 12 182 -> 166); that of many does not (a batch of 48 14.5 ->
+    // 15.1 ms)
     if (beside) MPS_TRY(pair_sum_ready(s, st, false));
     if (beside && many) MPS_TRY(pair_sum_start(s, m, nrhs, false));
     STAGE_MARK(1);
@@ -1622,8 +1623,8 @@ __device__ void loop_control(const GmresState &st, int restart, int j, int32_t *
     cudaGraphSetConditional(lc.handle, (active && j + 1 < restart) ? 1u : 0u);
 }
 
-// End of an Arnoldi step: w_r -= sum_c V_r[c] h_r[c] (h the last Gram-Schmidt pass's dots) and its norm in one pass; the
-// last block of each system does the column's rotations and the loop control.
+// End of an Arnoldi step: w_r -= sum_c V_r[c] h_r[c] (h the last Gram-Schmidt pass's dots) and its norm in one pass;
+// the last block of each system does the column's rotations and the loop control.
 __global__ void __launch_bounds__(kDotThreads) k_arnoldi_end(const double *__restrict__ V, int64_t ldv, int64_t n3,
                                                              double *__restrict__ w, const double *__restrict__ h,
                                                              GmresState st, int restart, int j,
@@ -1682,11 +1683,11 @@ __global__ void __launch_bounds__(kDotThreads) k_arnoldi_end(const double *__res
 }
 
 // A whole Arnoldi step after the matvec for systems of at most kSmallRows rows, one block a system with w in registers:
-// the Gram-Schmidt passes, the rotations, the next basis vector (also to vin when given) and the loop control.  One SM's
-// float64 rate bounds it, and every warp of the block pays its part of the reductions: eight rows a thread, so that the
-// block has no more warps than it needs (1500 rows, one to five columns, two passes: 28 us in seven launches -> 15 us).
-// Beyond 2048 rows more SMs are worth the launches (3000 rows, three systems, four columns: 27 us here, 25 there, and
-// the columns' work grows four times as fast here).
+// the Gram-Schmidt passes, the rotations, the next basis vector (also to vin when given) and the loop control.  One
+// SM's float64 rate bounds it, and every warp of the block pays its part of the reductions: eight rows a thread, so
+// that the block has no more warps than it needs (1500 rows, one to five columns, two passes: 28 us in seven launches
+// -> 15 us). Beyond 2048 rows more SMs are worth the launches (3000 rows, three systems, four columns: 27 us here, 25
+// there, and the columns' work grows four times as fast here).
 constexpr int kSmallThreads = 256;
 constexpr int kSmallRows = kSmallThreads * kDotItems;
 
@@ -1932,8 +1933,8 @@ static bool graphs_enabled(const mps_system *s) {
     return !(v && v[0] == '0');
 }
 
-// Everything of an Arnoldi step after its matvec (w = A V[j]): Gram-Schmidt (twice with reorth), the column's rotations,
-// V[j + 1], and, in the graph form (lc.jd set; j ignored), the copy to vin and the loop control.
+// Everything of an Arnoldi step after its matvec (w = A V[j]): Gram-Schmidt (twice with reorth), the column's
+// rotations, V[j + 1], and, in the graph form (lc.jd set; j ignored), the copy to vin and the loop control.
 static int arnoldi_step(const GmresWs &W, int64_t n3, int nrhs, int restart, int j, bool reorth, const LoopCtl &lc,
                         cudaStream_t st) {
     const int64_t ldv = (int64_t)nrhs * n3;

@@ -26,7 +26,8 @@
 
 namespace mps {
 
-constexpr int kMaxTileList = 8;  // distinct tiles per axis that a stencil may touch (axis_tile_bound: 6 for P = kMaxP, T = 4)
+// distinct tiles per axis that a stencil may touch (axis_tile_bound: 6 for P = kMaxP, T = 4)
+constexpr int kMaxTileList = 8;
 // particles staged per spread iteration (one barrier interval): 96 measured 1.42 ms for the double-float spread
 // at the bench workload against 1.57 for 32 and 1.46 for 64 (fewer barriers; the warps' shares even out)
 constexpr int kChunk = 96;
@@ -461,21 +462,20 @@ __global__ void __launch_bounds__(256) k_spread_tiled(const double *__restrict__
 // A float64 warp instruction costs GB300 the same whether one lane is active or thirty-two, so the tiled spread above,
 // whose lanes sit idle wherever a particle misses their column (about 60 % of them at P = 10), loses on every one.
 // Here a lane owns single nodes and walks the particles that cover each: the particles of an 8 x 8 x TZ tile are staged
-// up to kNodeChunk at a time with their factors aligned to the tile and, per tile column, row and plane, the bit mask of
-// the particles that reach it; the AND of a node's three masks lists its particles.  The lanes of a warp (a 4 x 4 x 2
-// patch) walk different particles at the same time, and what is lost is the difference between the patch's largest list
-// and its mean (14 particles a node and 18 in the largest list at P = 10 and one particle in 71 nodes).  The products
-// m wx are formed once per particle and column while staging, so a node's particle costs one product wy wz and one
-// multiply-add per component.  Lists run in the order of the particles' ids: the sums are deterministic, every node is
-// written once.  Measured against the tiled spread: three vectors, N = 100,000, 192^3, P = 10 3.82 -> 2.31 ms; one vector,
-// N = 20,000, 86^3, P = 8 277 -> 142 us; one vector, N = 500, 25^3 62 -> 12 us; 36 vectors, N = 2000, 31^3, P = 5 twelve
-// launches of 110 us -> one of 142 us.
-// In double-float a node's step is some 11 float instructions a component, and reading m wx of a lane's own particle
-// from shared memory costs as much; there a lane takes two nodes along z at once, with one list for both (11 of 10
-// planes) and one read.  Measured against the tiled double-float spread: one vector, N = 200,000, 240^3, P = 10
-// 1165 -> 646 us; one vector, N = 8228 in half of a 60 x 72 x 160 grid, P = 8 65 -> 28 us.
-// Float32 moments of eight components (dipole and quadrupole) take pairs of nodes too; against float atomics from a warp a
-// particle, N = 50,320, 90 x 90 x 96, P = 6: 118 us and the zeroing -> 54 us.
+// up to kNodeChunk at a time with their factors aligned to the tile and, per tile column, row and plane, the bit mask
+// of the particles that reach it; the AND of a node's three masks lists its particles.  The lanes of a warp (a 4 x 4 x
+// 2 patch) walk different particles at the same time, and what is lost is the difference between the patch's largest
+// list and its mean (14 particles a node and 18 in the largest list at P = 10 and one particle in 71 nodes).  The
+// products m wx are formed once per particle and column while staging, so a node's particle costs one product wy wz and
+// one multiply-add per component.  Lists run in the order of the particles' ids: the sums are deterministic, every node
+// is written once.  Measured against the tiled spread: three vectors, N = 100,000, 192^3, P = 10 3.82 -> 2.31 ms; one
+// vector, N = 20,000, 86^3, P = 8 277 -> 142 us; one vector, N = 500, 25^3 62 -> 12 us; 36 vectors, N = 2000, 31^3, P =
+// 5 twelve launches of 110 us -> one of 142 us. In double-float a node's step is some 11 float instructions a
+// component, and reading m wx of a lane's own particle from shared memory costs as much; there a lane takes two nodes
+// along z at once, with one list for both (11 of 10 planes) and one read.  Measured against the tiled double-float
+// spread: one vector, N = 200,000, 240^3, P = 10 1165 -> 646 us; one vector, N = 8228 in half of a 60 x 72 x 160 grid,
+// P = 8 65 -> 28 us. Float32 moments of eight components (dipole and quadrupole) take pairs of nodes too; against float
+// atomics from a warp a particle, N = 50,320, 90 x 90 x 96, P = 6: 118 us and the zeroing -> 54 us.
 constexpr int kNodeTile = 8;
 constexpr int kNodeChunk = 96;      // 3 mask words
 constexpr int kNodeWords = kNodeChunk / 32;
@@ -512,15 +512,17 @@ constexpr int kNodeThreads = 256;
 
 // NR vectors of NC components each to a block.
 template <typename T, int NR, int TZ, int NC>
-__global__ void __launch_bounds__(kNodeThreads, std::is_same<T, float>::value ? 4 : 1) k_spread_nodes(const double *__restrict__ m, int64_t n, int rfirst,
-                                                          const int32_t *__restrict__ start,
-                                                          const T *__restrict__ w, GridParams gp,
-                                                          const int64_t *__restrict__ tstart,
-                                                          const int32_t *__restrict__ entries, int ntx, int nty,
-                                                          T *__restrict__ grid) {
+__global__ void __launch_bounds__(kNodeThreads, std::is_same<T, float>::value ? 4 : 1)
+    k_spread_nodes(const double *__restrict__ m, int64_t n, int rfirst,
+                   const int32_t *__restrict__ start,
+                   const T *__restrict__ w, GridParams gp,
+                   const int64_t *__restrict__ tstart,
+                   const int32_t *__restrict__ entries, int ntx, int nty,
+                   T *__restrict__ grid) {
     constexpr int C = NC * NR, NQ = TZ / 4;
     constexpr bool PAIR = (std::is_same<T, dfv>::value || std::is_same<T, float>::value) && NQ == 2;   // a lane's two
-                                                                                                       // nodes share a list
+                                                                                                       // nodes share a
+                                                                                                       // list
     extern __shared__ __align__(16) unsigned char smem_nodes[];
     NodeStage<T, C, TZ> &st = *reinterpret_cast<NodeStage<T, C, TZ> *>(smem_nodes);
     const int r0 = rfirst + NR * (int)blockIdx.y;
@@ -676,9 +678,10 @@ int spread_nodes(const double *m, int64_t n, int nrhs, const int32_t *start, con
     return MPS_BAD_ARG;
 }
 
-// Every node of the grid costs, and the lists' set-up does: with stencils that cover less than half of the nodes, or on a
-// small grid, atomics from a warp a particle are no slower (three vectors, 96^3, P = 6, 884, 2949, 8847 particles 32 and 50,
-// 46 and 52, 86 and 65 us by atomics and by nodes; one vector, 16^3, 60 particles 11 and 8, after some 45 for the lists).
+// Every node of the grid costs, and the lists' set-up does: with stencils that cover less than half of the nodes, or on
+// a small grid, atomics from a warp a particle are no slower (three vectors, 96^3, P = 6, 884, 2949, 8847 particles 32
+// and 50, 46 and 52, 86 and 65 us by atomics and by nodes; one vector, 16^3, 60 particles 11 and 8, after some 45 for
+// the lists).
 bool spread_nodes8_pays(const GridParams &gp, int64_t n) {
     return gp.G >= 30000 && 2.0 * n * gp.P * gp.P * gp.P >= (double)gp.G;
 }
@@ -895,8 +898,8 @@ int contract_tiled_df(const dfv *grid, int64_t n, int nrhs, const int32_t *start
 // column), then the column sums are weighted by wx*wy in double-float.  Fixed
 // summation order: deterministic.  Bounds of 3 blocks per SM let ptxas keep more
 // loads in flight (72 registers for one vector; 1.19 ms per residual matvec at the
-// bench workload against 1.30 ms with 56 registers under the default heuristic).  The sums end one to a lane (N = 100,000,
-// P = 10 on 192^3: 393 -> 381 us a vector); deeper unrolling or other bounds were slower (399 to 451).
+// bench workload against 1.30 ms with 56 registers under the default heuristic).  The sums end one to a lane (N =
+// 100,000, P = 10 on 192^3: 393 -> 381 us a vector); deeper unrolling or other bounds were slower (399 to 451).
 template <int NR>
 __global__ void __launch_bounds__(256, 3) k_contract_df_warp(const dfv *__restrict__ grid, int64_t n, int r0,
                                                           const int32_t *__restrict__ order,

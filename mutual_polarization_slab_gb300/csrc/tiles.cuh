@@ -41,8 +41,8 @@ constexpr int kHomeBlock = 8;
 
 bool tiles_supported(const GridParams &gp, int tz);
 int tile_bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tz, TileBins &tb, cudaStream_t s);
-// Bins of tiles of tx x ty x tz nodes (4 or more an axis with P up to kMaxP; MPS_BAD_ARG where a stencil could touch more
-// tiles of an axis than the builder's lists hold), without a host round trip.
+// Bins of tiles of tx x ty x tz nodes (4 or more an axis with P up to kMaxP; MPS_BAD_ARG where a stencil could touch
+// more tiles of an axis than the builder's lists hold), without a host round trip.
 int bins_build(const int32_t *start, int64_t n, const GridParams &gp, int tx, int ty, int tz, TileBins &tb,
                cudaStream_t s);
 // Bins for spread_nodes and spread_nodes8: 8 x 8 tiles, of depth 8 or 4 by the number of blocks (groups to a tile).
