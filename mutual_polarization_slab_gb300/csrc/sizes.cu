@@ -160,43 +160,47 @@ __device__ __forceinline__ int64_t cs_search(const double *__restrict__ rv, int6
     return lo;
 }
 
-// Per-pair couplings of the CSR list: A (I - rr) and B - A, float64 and float32.  A warp takes a row and its lanes the
-// row's pairs: the loads and the search are chains of latencies, and with a thread a row 3,000 spheres filled 94 warps
-// of the chip (3,000 spheres, 60 pairs each: 1.58 ms, 0.25 with the lanes on the pairs).
+// Per-pair couplings of the CSR list: A (I - rr) and B - A, float64 and float32, a pair to a thread, its row by a search
+// in row_ptr: the couplings' float64 instructions bound it, and each costs a warp the same for one active lane as for
+// 32, however many pairs a row has.  With a thread a row 3,000 spheres filled 94 warps of the chip (60 pairs each:
+// 1.58 ms); with a warp a row (0.25 ms) rows of 8 pairs left three lanes of four idle.
 __global__ void k_cs_pair_coefs(const int64_t *__restrict__ row_ptr, const int32_t *__restrict__ nbr,
-                                const double *__restrict__ dist, int64_t n, const double *__restrict__ radius,
-                                const int32_t *__restrict__ cls, int64_t M, const double *__restrict__ tab,
-                                const double *__restrict__ rv, int64_t ntab, double xi, double *__restrict__ A64,
-                                double *__restrict__ BA64, float *__restrict__ A32, float *__restrict__ BA32,
-                                int *__restrict__ err) {
+                                const double *__restrict__ dist, int64_t n, int64_t np,
+                                const double *__restrict__ radius, const int32_t *__restrict__ cls, int64_t M,
+                                const double *__restrict__ tab, const double *__restrict__ rv, int64_t ntab, double xi,
+                                double *__restrict__ A64, double *__restrict__ BA64, float *__restrict__ A32,
+                                float *__restrict__ BA32, int *__restrict__ err) {
     const int64_t m = M * (M + 1) / 2;
-    const int lane = threadIdx.x & 31;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t a = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; a < n; a += nw) {
-        const int64_t end = row_ptr[a + 1];
-        for (int64_t e = row_ptr[a] + lane; e < end; e += 32) {
-            const int32_t b = nbr[e];
-            const double d = dist[e];
-            double A = 0.0, B = 0.0;
-            if (tab) {
-                const int64_t col = cs_column(cls[a], cls[b], M);
-                const int64_t i = cs_search(rv, ntab, d);
-                if (i <= 0 || i >= ntab) {
-                    atomicExch(err, 1);
-                } else {
-                    const double rl = rv[i - 1], rh = rv[i];
-                    const double *pp = tab + col * ntab, *pa = tab + (m + col) * ntab;
-                    A = pp[i - 1] * (rh - d) / (rh - rl) + pp[i] * (d - rl) / (rh - rl);
-                    B = pa[i - 1] * (rh - d) / (rh - rl) + pa[i] * (d - rl) / (rh - rl);
-                }
-            } else {
-                cs_couplings(d, radius[a], radius[b], xi, &A, &B);
-            }
-            A64[e] = A;
-            BA64[e] = B - A;
-            A32[e] = (float)A;
-            BA32[e] = (float)(B - A);
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < np; e += (int64_t)gridDim.x * blockDim.x) {
+        int64_t a = 0, hi = n - 1;   // the last row that starts at e or before
+        while (a < hi) {
+            const int64_t mid = (a + hi + 1) >> 1;
+            if (row_ptr[mid] <= e)
+                a = mid;
+            else
+                hi = mid - 1;
         }
+        const int32_t b = nbr[e];
+        const double d = dist[e];
+        double A = 0.0, B = 0.0;
+        if (tab) {
+            const int64_t col = cs_column(cls[a], cls[b], M);
+            const int64_t i = cs_search(rv, ntab, d);
+            if (i <= 0 || i >= ntab) {
+                atomicExch(err, 1);
+            } else {
+                const double rl = rv[i - 1], rh = rv[i];
+                const double *pp = tab + col * ntab, *pa = tab + (m + col) * ntab;
+                A = pp[i - 1] * (rh - d) / (rh - rl) + pp[i] * (d - rl) / (rh - rl);
+                B = pa[i - 1] * (rh - d) / (rh - rl) + pa[i] * (d - rl) / (rh - rl);
+            }
+        } else {
+            cs_couplings(d, radius[a], radius[b], xi, &A, &B);
+        }
+        A64[e] = A;
+        BA64[e] = B - A;
+        A32[e] = (float)A;
+        BA32[e] = (float)(B - A);
     }
 }
 
@@ -700,11 +704,11 @@ __global__ void __launch_bounds__(256) k_cs_interleave(const float *__restrict__
 // ---------------------------------------------------------------------------
 // Host wrappers
 // ---------------------------------------------------------------------------
-int cs_pair_coefs(const int64_t *row_ptr, const int32_t *nbr, const double *dist, int64_t n, const double *radius,
-                  const int32_t *cls, int64_t M, const double *tab, const double *rv, int64_t ntab, double xi,
-                  PairData<double> p64, PairData<float> p32, int *err, cudaStream_t s) {
-    k_cs_pair_coefs<<<grid_for(n * 32, 128), 128, 0, s>>>(row_ptr, nbr, dist, n, radius, cls, M, tab, rv, ntab, xi,
-                                                         p64.A, p64.BA, p32.A, p32.BA, err);
+int cs_pair_coefs(const int64_t *row_ptr, const int32_t *nbr, const double *dist, int64_t n, int64_t np,
+                  const double *radius, const int32_t *cls, int64_t M, const double *tab, const double *rv,
+                  int64_t ntab, double xi, PairData<double> p64, PairData<float> p32, int *err, cudaStream_t s) {
+    k_cs_pair_coefs<<<grid_for(np, 128), 128, 0, s>>>(row_ptr, nbr, dist, n, np, radius, cls, M, tab, rv, ntab, xi,
+                                                      p64.A, p64.BA, p32.A, p32.BA, err);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
 }

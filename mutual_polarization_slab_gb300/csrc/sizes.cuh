@@ -6,9 +6,9 @@
 
 namespace mps {
 
-int cs_pair_coefs(const int64_t *row_ptr, const int32_t *nbr, const double *dist, int64_t n, const double *radius,
-                  const int32_t *cls, int64_t M, const double *tab, const double *rv, int64_t ntab, double xi,
-                  PairData<double> p64, PairData<float> p32, int *err, cudaStream_t s);
+int cs_pair_coefs(const int64_t *row_ptr, const int32_t *nbr, const double *dist, int64_t n, int64_t np,
+                  const double *radius, const int32_t *cls, int64_t M, const double *tab, const double *rv,
+                  int64_t ntab, double xi, PairData<double> p64, PairData<float> p32, int *err, cudaStream_t s);
 int cs_diag(const double *lam, int64_t n, int64_t nsets, const double *radius, const int32_t *cls, int64_t M,
             const double *tab, int64_t ntab, double xi, double *diag, cudaStream_t s);
 int cs_geometry(const double *x, int64_t n, const GridParams &gp, const double *radius, double xi, double eta,

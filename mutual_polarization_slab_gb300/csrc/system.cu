@@ -2819,9 +2819,9 @@ extern "C" int mps_system_create(const mps_system_desc *d, mps_system **out, mps
         rc = dalloc(&perr, sizeof(int), st);
         if (!rc && cudaMemsetAsync(perr, 0, sizeof(int), st) != cudaSuccess) rc = MPS_CUDA_ERR;
         if (!rc)
-            rc = cs_pair_coefs(s->row_ptr, s->p64.nbr, s->p64.dist, n, d->radius, d->radius_class, d->n_class,
-                               d->radius_class ? d->sizes_tables : nullptr, d->rvals, d->n_tab, d->xi, s->p64, s->p32,
-                               perr, st);
+            rc = cs_pair_coefs(s->row_ptr, s->p64.nbr, s->p64.dist, n, s->n_pairs, d->radius, d->radius_class,
+                               d->n_class, d->radius_class ? d->sizes_tables : nullptr, d->rvals, d->n_tab, d->xi,
+                               s->p64, s->p32, perr, st);
         if (!rc && cudaMemcpyAsync(&herr, perr, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess)
             rc = MPS_CUDA_ERR;
         if (!rc && cudaStreamSynchronize(st) != cudaSuccess) rc = MPS_CUDA_ERR;
