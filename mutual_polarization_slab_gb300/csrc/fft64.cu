@@ -753,13 +753,14 @@ int f64_plan(const GridParams &gp, F64Plan3 *out) {
 // vectors 408 against 534 and 767 against 1012; 10 x 20 x 400, 3 vectors 177 against 221), wider ones and longer x do
 // not (12 x 48 x 400, 3 vectors 458 against 438; 14 x 14 x 500, 24 vectors 1519 against 1280; 400 x 12 x 12 1118
 // against 770).
-// Not fused: 24 grids on 16^3, 20^3, 25^3 78 against 100, 68 and 75, 99 and 116, 96 grids on 16^3, 20^3, 25^3, 28^3 78
-// and 100, 123 and 188, 259 and 336, 326 and 328, on 24 x 24 x 48 363 and 430; on 30^3, 32^3, 36^3, 48^3 456 against
-// 421, 415 and 385, 700 and 627, 1793 and 1250.
-bool f64_pays(const GridParams &gp, bool fused) {
+// Not fused, short axes: few grids leave cuFFT waiting for its launches, many leave these too few butterflies a block.
+// 4 grids on 18^3, 22^3, 24^3, 28^3 57 against 47, 78 and 50, 62 and 57, 75 and 53; 16 grids 57 and 53, 79 and 65, 71
+// and 75, 94 and 101; 24 grids 57 and 54, 82 and 85, 79 and 103, 117 and 115; 96 grids 103 and 123, 193 and 205, 188
+// and 260, 325 and 327.  On 30^3, 32^3, 36^3, 48^3 96 grids 456 against 421, 415 and 385, 700 and 627, 1793 and 1250.
+bool f64_pays(const GridParams &gp, bool fused, int ngrids) {
     const int longest = std::max({gp.N[0], gp.N[1], gp.N[2]});
     if (fused) return gp.N[0] >= 14 || longest < 200 || std::min(gp.N[1], gp.N[2]) >= 40;
-    return gp.N[0] >= 30 && gp.N[1] >= 30 && gp.N[2] >= 30;
+    return ngrids < 20 || std::min({gp.N[0], gp.N[1], gp.N[2]}) >= 30;
 }
 
 // Lines per block: up to 8 (full 128-byte rows of the strided passes) within about 56 KB of shared memory (4 blocks an

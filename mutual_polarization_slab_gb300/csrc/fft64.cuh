@@ -31,9 +31,9 @@ int f64_plan(const GridParams &gp, F64Plan3 *out);
 
 // Whether the transforms are the faster ones on a grid that they support; cuFFT keeps the others.  A pass deals the
 // butterflies of at most eight lines to a block, and short lines leave it few of them.  fused: f64_z_scale_dipole,
-// which saves a third of the z transforms and the scale's own pass; without it (f64_z) every axis has to be long
-// enough.
-bool f64_pays(const GridParams &gp, bool fused);
+// which saves a third of the z transforms and the scale's own pass; without it (f64_z) the axes have to be long enough
+// or the grids few.
+bool f64_pays(const GridParams &gp, bool fused, int ngrids);
 
 // 0.5 H / |k|^2 on the half spectrum (H includes 1/G; zero at k = 0): the factor 1/2 belongs to f64_forward_xy.
 int f64_scale_coef(const GridParams &gp, const double *H, double *hs, cudaStream_t s);

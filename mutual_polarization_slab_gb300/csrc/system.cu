@@ -715,12 +715,12 @@ static int df_usable(mps_system *s, bool *usable);
 // The float64 transforms of fft64.cu take every axis up to 1024 whose prime factors are at most 127; grids on which
 // they do not pay (f64_pays) and other grids keep cuFFT.  A failure to plan decides nothing: it is the caller's status,
 // and the next call plans again.
-static int f64_usable(mps_system *s, bool *usable) {
+static int f64_usable(mps_system *s, int ngrids, bool *usable) {
     if (s->f64_state == 0) {
         MPS_TRY(f64_plan(s->gp, &s->f64p));
-        s->f64_state = s->f64p.ok && f64_pays(s->gp, s->kind == MPS_DIPOLE) ? 1 : -1;
+        s->f64_state = s->f64p.ok ? 1 : -1;
     }
-    *usable = s->f64_state == 1;
+    *usable = s->f64_state == 1 && f64_pays(s->gp, s->kind == MPS_DIPOLE, ngrids);
     return MPS_OK;
 }
 
@@ -778,7 +778,7 @@ static bool own_fft32() {
 // Stage marks 2..5 of the calling matvec (ev may be null).
 static int f64_field_grids(mps_system *s, const double *m, int nrhs, StageEvents *ev, cudaStream_t st) {
     bool own = false, nodes = false;
-    MPS_TRY(f64_usable(s, &own));
+    MPS_TRY(f64_usable(s, 3 * nrhs, &own));
     if (own) MPS_TRY(f64_prepare(s, st));
     MPS_TRY(ensure_nodes(s, st, &nodes));
     MPS_TRY(ensure_grids(s, MPS_FP64, st));
@@ -1004,7 +1004,7 @@ static int matvec_quad(mps_system *s, const double *m, double *out, int nrhs, cu
         MPS_TRY(spread_gen<T>(m, s->n, nrhs, 8, s->start, w, s->gp, grid, st));
     STAGE_MARK(2);
     bool own = false;
-    if (dbl) MPS_TRY(f64_usable(s, &own));
+    if (dbl) MPS_TRY(f64_usable(s, 8 * nrhs, &own));
     if (own) {   // (twice the spectra: the scale takes on the factor)
         MPS_TRY(f64_forward_xy(s->grid64, spec, 8 * nrhs, s->gp, s->f64p, st));
         MPS_TRY(f64_z(spec, 8 * nrhs, s->gp, s->f64p, 0, st));
@@ -1118,7 +1118,7 @@ static int matvec_cs(mps_system *s, const double *m, double *out, int nrhs, cuda
     if (beside && !many) MPS_TRY(pair_sum_start(s, m, nrhs, false));
     STAGE_MARK(2);
     bool own = false;
-    if (dbl) MPS_TRY(f64_usable(s, &own));
+    if (dbl) MPS_TRY(f64_usable(s, nrhs, &own));
     if (own) {   // (twice the spectra: the scale takes on the factor)
         MPS_TRY(f64_forward_xy(s->grid64, spec, nrhs, s->gp, s->f64p, st));
         MPS_TRY(f64_z(spec, nrhs, s->gp, s->f64p, 0, st));
@@ -3148,7 +3148,7 @@ extern "C" int mps_field_map(const double *x_e, int64_t n_e, const double *x_p, 
     if (!rc_) rc_ = green_half(gp, H, nullptr, st);
     F64Plan3 f64;
     if (!rc_) rc_ = f64_plan(gp, &f64);
-    if (f64.ok && f64_pays(gp, true)) {   // the transforms of the float64 operator; cuFFT where they do not apply or pay
+    if (f64.ok && f64_pays(gp, true, 3)) {   // the transforms of the float64 operator; cuFFT where they do not apply or pay
         if (!rc_) rc_ = dalloc(&hs, sizeof(double) * (size_t)Gc, st);
         if (!rc_) rc_ = f64_scale_coef(gp, H, hs, st);
         if (!rc_) rc_ = f64_forward_xy(grid, spec, 3, gp, f64, st);
