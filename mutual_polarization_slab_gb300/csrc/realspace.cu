@@ -278,10 +278,13 @@ int real_space_csr(const double *m, double *out, int64_t n, int nrhs, const int6
                    PairData<T> pd, const double *diag, const int32_t *diag_of_rhs, const double *slab, bool accumulate,
                    cudaStream_t s) {
     // Up to four vectors share a pass over the pair data, 8 lanes to a row.  Where that leaves most SMs without work, a
-    // warp takes one row of one vector, in blocks of 4 warps, and reads the pairs once a vector: N = 400, 62
-    // neighbours, 1, 3, 12 and 24 vectors 1.6, 2.8, 1.6 and 1.0 times as fast, N = 1000, 18 neighbours, 1, 4, 12
-    // vectors 1.1, 1.4, 0.7; N = 2000, 3 vectors with 5, 19, 73 neighbours 0.7, 0.9, 1.3.
-    if (n * std::max(nrhs, 4) <= (np >= 48 * n ? 10000 : 6000)) {
+    // warp takes one row of one vector, in blocks of 4 warps, and reads the pairs once a vector: the more neighbours a
+    // row has, the longer its chain of loads, and the more rows that is worth (vectors beyond full groups of four don't
+    // count: they are a launch by themselves).  By 8 lanes / by warps, us: three vectors, N = 1728, 3375, 5832, 9261 with
+    // 18 neighbours - / 16, 16 / 25, 26 / 39, 27 / 60, with 58 - / 23, 29 / 37, 49 / 58, 50 / 88, with 122 - / 29, 45 / 47,
+    // 80 / 78, 80 / 119, with 199 - / 35, 64 / 59, 119 / 96, 120 / 150; N = 1728, six vectors with 18 and 199 31 / 27 and
+    // 125 / 62, twelve 31 / 46 and 156 / 115; N = 400, 62 neighbours, 24 vectors the same.
+    if ((n * std::max(nrhs & ~3, 4) - 6000) * n <= 100 * np) {
         for (int r0 = 0; r0 < nrhs; r0 += 32768) {
             k_rs_csr<T, 32, 1><<<dim3(grid_for(n * 32, 128, 152 * 64), min(32768, nrhs - r0)), 128, 0, s>>>(
                 m, out, n, nrhs, r0, row_ptr, pd, diag, diag_of_rhs, slab, accumulate, m, nullptr);
