@@ -368,23 +368,21 @@ __global__ void k_to_f32_rows(const double *__restrict__ m, int64_t n, int nrhs,
 
 size_t m32_floats(int64_t n, int nrhs) { return (size_t)n * (size_t)nrhs * 4; }
 
-// Float32 pair sum.  A warp takes a row and a lane one vector of one pair: RL vectors side by side, 32 / RL pairs at a
-// time.  The loads are what costs here (a warp's load takes the L1 a pass for every line it touches): 4 lanes to a row
+// Float32 pair sum.  A lane takes one vector of one pair: RL vectors side by side, PP pairs at a time, RL PP lanes to a
+// row.  The loads are what costs here (a warp's load takes the L1 a pass for every line it touches): 4 lanes to a row
 // and all vectors in a lane's registers touched 8 lines with each pair array and 32 with each 16 bytes of the gathered
-// moments; now a pair array's load touches one or two, and a gather one line a pair.  The row's sums end in float64
-// with the diagonal, each component on a lane of its own.  Alone: one vector, N = 200,000, 60 neighbours 264 -> 122 us;
-// 48 vectors, N = 3000 55 -> 25 us; three vectors, N = 100,000 104 -> 115 us (a quarter of the lanes idle), but less in
-// the way of the spread that runs beside it.
-template <int RL>
+// moments; now a pair array's load touches one to four, and a gather one line a pair.  The row's sums end in float64
+// with the diagonal, each component on a lane of its own.
+template <int RL, int PP>
 __global__ void __launch_bounds__(256) k_rs_csr_f32(const double *__restrict__ m, double *__restrict__ out, int64_t n,
                                                     int nrhs, int rfirst, const int64_t *__restrict__ row_ptr,
                                                     PairData<float> pd, const double *__restrict__ diag,
                                                     const int32_t *__restrict__ diag_of_rhs,
                                                     const double *__restrict__ slab, int accumulate,
                                                     const float4 *__restrict__ mf, const int32_t *__restrict__ order) {
-    constexpr int PP = 32 / RL;   // pairs at a time
-    static_assert(PP >= 4, "three lanes of a vector take its components");
-    const int lane = threadIdx.x & 31, q = lane / RL;
+    constexpr int G = RL * PP, ROWS = 32 / G;   // lanes to a row, rows to a warp
+    static_assert(PP >= 4 && G <= 32, "three lanes of a vector take its components");
+    const int lane = threadIdx.x & 31, q = lane % G / RL;
     const int r = rfirst + (int)blockIdx.y * RL + lane % RL;
     const bool live = r < nrhs;
     const int rc = live ? r : nrhs - 1;
@@ -392,13 +390,15 @@ __global__ void __launch_bounds__(256) k_rs_csr_f32(const double *__restrict__ m
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const double *dg = diag + (int64_t)(diag_of_rhs ? diag_of_rhs[rc] : 0) * n;
     const double sl = q == 2 ? slab[rc] : 0.0;
-    for (int64_t i = warp; i < n; i += nw) {
+    for (int64_t i0 = warp * ROWS; i0 < n; i0 += nw * ROWS) {
+        const int64_t i = i0 + lane / G;
+        const bool row = i < n;   // (lanes beyond the last row take no pairs)
         // rows in `order` (cell order): neighbouring warps read overlapping neighbour moments
-        const int64_t a = order ? (int64_t)order[i] : i;
+        const int64_t a = !row ? 0 : order ? (int64_t)order[i] : i;
         float ax = 0.f, ay = 0.f, az = 0.f;
-        const int64_t e1 = row_ptr[a + 1];
+        const int64_t e1 = row ? row_ptr[a + 1] : 0;
 #pragma unroll 4
-        for (int64_t e = row_ptr[a] + q; e < e1; e += PP) {
+        for (int64_t e = row ? row_ptr[a] + q : 0; e < e1; e += PP) {
             const int32_t b = pd.nbr[e];
             const float av = pd.A[e], ba = pd.BA[e];
             const float rx = pd.rx[e], ry = pd.ry[e], rz = pd.rz[e];
@@ -412,12 +412,12 @@ __global__ void __launch_bounds__(256) k_rs_csr_f32(const double *__restrict__ m
             az += s * rz;
         }
 #pragma unroll
-        for (int o = RL; o < 32; o <<= 1) {
+        for (int o = RL; o < G; o <<= 1) {
             ax += __shfl_xor_sync(0xffffffffu, ax, o);
             ay += __shfl_xor_sync(0xffffffffu, ay, o);
             az += __shfl_xor_sync(0xffffffffu, az, o);
         }
-        if (live && q < 3) {
+        if (live && row && q < 3) {
             const int64_t k = ((int64_t)r * n + a) * 3 + q;
             double v = dg[a] * m[k] + float_to_double(q == 0 ? ax : (q == 1 ? ay : az)) + sl;
             if (accumulate) v += out[k];
@@ -426,11 +426,11 @@ __global__ void __launch_bounds__(256) k_rs_csr_f32(const double *__restrict__ m
     }
 }
 
-template <int RL>
+template <int RL, int PP>
 static int rs_f32_launch(const double *m, const float4 *mf, double *out, int64_t n, int nrhs, int r0, int blocks,
                          const int64_t *row_ptr, PairData<float> pd, const double *diag, const int32_t *diag_of_rhs,
                          const double *slab, bool accumulate, const int32_t *order, cudaStream_t s) {
-    k_rs_csr_f32<RL><<<dim3(grid_for(n * 32, 256, 152 * 64), blocks), 256, 0, s>>>(
+    k_rs_csr_f32<RL, PP><<<dim3(grid_for(n * RL * PP, 256, 152 * 64), blocks), 256, 0, s>>>(
         m, out, n, nrhs, r0, row_ptr, pd, diag, diag_of_rhs, slab, accumulate, mf, order);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
@@ -438,31 +438,36 @@ static int rs_f32_launch(const double *m, const float4 *mf, double *out, int64_t
 
 // Eight vectors side by side (all such blocks in one launch: small systems fill the GPU with them), a rest of up to
 // four as 4, 2 or 1, a larger one as a block of eight with idle lanes.
+//
+// Lanes to a row: a warp; where there are rows enough for the GPU, 16 for three and four vectors, and 8 for one and two if
+// the rows are short.  A row of few pairs leaves most of a warp idle, and the end of a row costs a warp the same for one
+// row as for four.  A warp a row / so (4 lanes a row and all vectors to a lane), us: one vector, N = 50,653 with 6 and 27
+// neighbours 27 / 18 (18) and 29 / 25 (26), N = 97,336 with 6 41 / 23 (24); two 52 / 30 (34); three with 6 and 65 55 / 44
+// (45) and 121 / 109 (120).  Long rows of one vector are faster by 8 lanes too when the sum runs alone (N = 97,336, 65
+// neighbours 75 / 63), but they get in the way of the spread that runs beside it (energy and forces of 200,000 spheres
+// 25.3 ms a warp a row, 26.6 so).  Below some 5000 rows a row's chain of loads is the time it takes: 65 neighbours, N =
+// 2197 one vector 12.1 / 14.8, three 14.7 / 16.6, N = 8000 16.3 / 14.9 and 20.6 / 18.5.
+constexpr int64_t kF32WideRows = 5000;
+
 int real_space_csr_f32(const double *m, float *m32, double *out, int64_t n, int nrhs, const int64_t *row_ptr,
-                       PairData<float> pd, const double *diag, const int32_t *diag_of_rhs, const double *slab,
+                       int64_t np, PairData<float> pd, const double *diag, const int32_t *diag_of_rhs, const double *slab,
                        bool accumulate, const int32_t *order, cudaStream_t s) {
     float4 *mf = reinterpret_cast<float4 *>(m32);
     k_to_f32_rows<<<grid_for((int64_t)nrhs * n, 256), 256, 0, s>>>(m, n, nrhs, mf);
     MPS_LAUNCH_CHECK();
+    const bool wide = n <= kF32WideRows, long_rows = np >= 48 * n;
     int r0 = 0;
     while (r0 < nrhs) {
         const int left = nrhs - r0;
-        int rc;
-        if (left > 4) {
-            const int blocks = std::min(32768, left / 8 + (left % 8 > 4 ? 1 : 0));
-            rc = rs_f32_launch<8>(m, mf, out, n, nrhs, r0, blocks, row_ptr, pd, diag, diag_of_rhs, slab, accumulate,
-                                  order, s);
-            r0 += 8 * blocks;
-        } else {
-            rc = left > 2    ? rs_f32_launch<4>(m, mf, out, n, nrhs, r0, 1, row_ptr, pd, diag, diag_of_rhs, slab,
-                                                accumulate, order, s)
-                 : left == 2 ? rs_f32_launch<2>(m, mf, out, n, nrhs, r0, 1, row_ptr, pd, diag, diag_of_rhs, slab,
-                                                accumulate, order, s)
-                             : rs_f32_launch<1>(m, mf, out, n, nrhs, r0, 1, row_ptr, pd, diag, diag_of_rhs, slab,
-                                                accumulate, order, s);
-            r0 = nrhs;
-        }
+        const int blocks = left > 4 ? std::min(32768, left / 8 + (left % 8 > 4 ? 1 : 0)) : 1;
+        auto *launch = left > 4    ? rs_f32_launch<8, 4>
+                       : left > 2  ? (wide ? rs_f32_launch<4, 8> : rs_f32_launch<4, 4>)
+                       : left == 2 ? (wide || long_rows ? rs_f32_launch<2, 16> : rs_f32_launch<2, 4>)
+                                   : (wide || long_rows ? rs_f32_launch<1, 32> : rs_f32_launch<1, 8>);
+        const int rc = launch(m, mf, out, n, nrhs, r0, blocks, row_ptr, pd, diag, diag_of_rhs, slab, accumulate, order,
+                              s);
         if (rc) return rc;
+        r0 += left > 4 ? 8 * blocks : left;
     }
     return MPS_OK;
 }

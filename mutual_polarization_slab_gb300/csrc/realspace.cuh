@@ -18,7 +18,7 @@ int real_space_csr_df(const double *m, dfv *mdf, double *out, int64_t n, int nrh
 // aligned: per particle its nrhs vectors as float4).
 size_t m32_floats(int64_t n, int nrhs);
 int real_space_csr_f32(const double *m, float *m32, double *out, int64_t n, int nrhs, const int64_t *row_ptr,
-                       PairData<float> pd, const double *diag, const int32_t *diag_of_rhs, const double *slab,
+                       int64_t np, PairData<float> pd, const double *diag, const int32_t *diag_of_rhs, const double *slab,
                        bool accumulate, const int32_t *order, cudaStream_t s);
 int build_diag(const double *lam, int64_t total, const double *perp, double *diag, cudaStream_t s);
 // Real and imaginary parts of the diagonal for complex permittivities (lr + i li).

@@ -748,8 +748,8 @@ static int f64_prepare(mps_system *s, cudaStream_t st) {
 // Float32 pair sum (accumulates into out) on the system's float copy of the moments.
 static int real_space_f32(mps_system *s, const double *m, double *out, int nrhs, cudaStream_t st) {
     if (!s->m32) MPS_TRY(dalloc(&s->m32, sizeof(float) * m32_floats(s->n, s->max_rhs), st));
-    return real_space_csr_f32(m, s->m32, out, s->n, nrhs, s->row_ptr, s->p32, s->diag, s->diag_idx, s->slab, true,
-                              s->order, st);
+    return real_space_csr_f32(m, s->m32, out, s->n, nrhs, s->row_ptr, s->n_pairs, s->p32, s->diag, s->diag_idx,
+                              s->slab, true, s->order, st);
 }
 
 // Float64 pair data of the dipole operator, converted from the double-float list
@@ -1068,7 +1068,7 @@ static int pair_sum_start(mps_system *s, const double *m, int nrhs, bool df) {
         MPS_TRY(real_space_csr_df(m, s->mdf, s->rs_buf, s->n, nrhs, s->row_ptr, s->n_pairs, s->pdf, s->diag, s->diag_idx,
                                   s->slab, false, s->order, s->side));
     else
-        MPS_TRY(real_space_csr_f32(m, s->m32, s->rs_buf, s->n, nrhs, s->row_ptr, s->p32, s->diag, s->diag_idx,
+        MPS_TRY(real_space_csr_f32(m, s->m32, s->rs_buf, s->n, nrhs, s->row_ptr, s->n_pairs, s->p32, s->diag, s->diag_idx,
                                    s->slab, false, s->order, s->side));
     MPS_CUDA_TRY(cudaEventRecord(s->ev_join, s->side));
     return MPS_OK;
