@@ -984,7 +984,7 @@ static int matvec_quad(mps_system *s, const double *m, double *out, int nrhs, cu
     // as long wherever the time counts (one vector, N = 3500, 64^3, P = 6 28 us against 54; three, N = 1041, 25^3, P =
     // 12 121 against 412)
     bool nodes = false;
-    if (!dbl && spread_nodes8_pays(s->gp, s->n)) MPS_TRY(ensure_nodes(s, st, &nodes));
+    if (!dbl && spread_nodes8_pays(s->gp, s->n, nrhs)) MPS_TRY(ensure_nodes(s, st, &nodes));
     const bool home = nodes && contract_home8_pays(s->gp, s->n);
     if (home) MPS_TRY(tile_bins_home(s->start, s->n, s->gp, s->tbn, st));
     if (!dbl && !s->m32) MPS_TRY(dalloc(&s->m32, sizeof(float) * 8 * (size_t)s->n * s->max_rhs, st));

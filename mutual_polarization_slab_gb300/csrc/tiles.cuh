@@ -65,7 +65,7 @@ template <typename T>
 int spread_nodes(const double *m, int64_t n, int nrhs, const int32_t *start, const T *w, const GridParams &gp,
                  const TileBins &tb, T *grid, cudaStream_t s);
 
-bool spread_nodes8_pays(const GridParams &gp, int64_t n);
+bool spread_nodes8_pays(const GridParams &gp, int64_t n, int nrhs);
 // Eight float32 components a vector (m [r][a][8], grid[(r*8+c)][G]).
 int spread_nodes8(const double *m, int64_t n, int nrhs, const int32_t *start, const float *w, const GridParams &gp,
                   const TileBins &tb, float *grid, cudaStream_t s);
