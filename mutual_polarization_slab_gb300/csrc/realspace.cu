@@ -280,10 +280,10 @@ int real_space_csr(const double *m, double *out, int64_t n, int nrhs, const int6
     // Up to four vectors share a pass over the pair data, 8 lanes to a row.  Where that leaves most SMs without work, a
     // warp takes one row of one vector, in blocks of 4 warps, and reads the pairs once a vector: the more neighbours a
     // row has, the longer its chain of loads, and the more rows that is worth (vectors beyond full groups of four don't
-    // count: they are a launch by themselves).  By 8 lanes / by warps, us: three vectors, N = 1728, 3375, 5832, 9261 with
-    // 18 neighbours - / 16, 16 / 25, 26 / 39, 27 / 60, with 58 - / 23, 29 / 37, 49 / 58, 50 / 88, with 122 - / 29, 45 / 47,
-    // 80 / 78, 80 / 119, with 199 - / 35, 64 / 59, 119 / 96, 120 / 150; N = 1728, six vectors with 18 and 199 31 / 27 and
-    // 125 / 62, twelve 31 / 46 and 156 / 115; N = 400, 62 neighbours, 24 vectors the same.
+    // count: they are a launch by themselves).  By 8 lanes / by warps, us: three vectors, N = 1728, 3375, 5832, 9261
+    // with 18 neighbours - / 16, 16 / 25, 26 / 39, 27 / 60, with 58 - / 23, 29 / 37, 49 / 58, 50 / 88, with 122 - / 29,
+    // 45 / 47, 80 / 78, 80 / 119, with 199 - / 35, 64 / 59, 119 / 96, 120 / 150; N = 1728, six vectors with 18 and 199
+    // 31 / 27 and 125 / 62, twelve 31 / 46 and 156 / 115; N = 400, 62 neighbours, 24 vectors the same.
     if ((n * std::max(nrhs & ~3, 4) - 6000) * n <= 100 * np) {
         for (int r0 = 0; r0 < nrhs; r0 += 32768) {
             k_rs_csr<T, 32, 1><<<dim3(grid_for(n * 32, 128, 152 * 64), min(32768, nrhs - r0)), 128, 0, s>>>(
@@ -439,14 +439,14 @@ static int rs_f32_launch(const double *m, const float4 *mf, double *out, int64_t
 // Eight vectors side by side (all such blocks in one launch: small systems fill the GPU with them), a rest of up to
 // four as 4, 2 or 1, a larger one as a block of eight with idle lanes.
 //
-// Lanes to a row: a warp; where there are rows enough for the GPU, 16 for three and four vectors, and 8 for one and two if
-// the rows are short.  A row of few pairs leaves most of a warp idle, and the end of a row costs a warp the same for one
-// row as for four.  A warp a row / so (4 lanes a row and all vectors to a lane), us: one vector, N = 50,653 with 6 and 27
-// neighbours 27 / 18 (18) and 29 / 25 (26), N = 97,336 with 6 41 / 23 (24); two 52 / 30 (34); three with 6 and 65 55 / 44
-// (45) and 121 / 109 (120).  Long rows of one vector are faster by 8 lanes too when the sum runs alone (N = 97,336, 65
-// neighbours 75 / 63), but they get in the way of the spread that runs beside it (energy and forces of 200,000 spheres
-// 25.3 ms a warp a row, 26.6 so).  Below some 5000 rows a row's chain of loads is the time it takes: 65 neighbours, N =
-// 2197 one vector 12.1 / 14.8, three 14.7 / 16.6, N = 8000 16.3 / 14.9 and 20.6 / 18.5.
+// Lanes to a row: a warp; where there are rows enough for the GPU, 16 for three and four vectors, and 8 for one and two
+// if the rows are short.  A row of few pairs leaves most of a warp idle, and the end of a row costs a warp the same for
+// one row as for four.  A warp a row / so (4 lanes a row and all vectors to a lane), us: one vector, N = 50,653 with 6
+// and 27 neighbours 27 / 18 (18) and 29 / 25 (26), N = 97,336 with 6 41 / 23 (24); two 52 / 30 (34); three with 6 and
+// 65 55 / 44 (45) and 121 / 109 (120).  Long rows of one vector are faster by 8 lanes too when the sum runs alone (N =
+// 97,336, 65 neighbours 75 / 63), but they get in the way of the spread that runs beside it (energy and forces of
+// 200,000 spheres 25.3 ms a warp a row, 26.6 so).  Below some 5000 rows a row's chain of loads is the time it takes: 65
+// neighbours, N = 2197 one vector 12.1 / 14.8, three 14.7 / 16.6, N = 8000 16.3 / 14.9 and 20.6 / 18.5.
 constexpr int64_t kF32WideRows = 5000;
 
 int real_space_csr_f32(const double *m, float *m32, double *out, int64_t n, int nrhs, const int64_t *row_ptr,

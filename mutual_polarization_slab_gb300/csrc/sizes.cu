@@ -160,10 +160,11 @@ __device__ __forceinline__ int64_t cs_search(const double *__restrict__ rv, int6
     return lo;
 }
 
-// Per-pair couplings of the CSR list: A (I - rr) and B - A, float64 and float32, a pair to a thread, its row by a search
-// in row_ptr: the couplings' float64 instructions bound it, and each costs a warp the same for one active lane as for
-// 32, however many pairs a row has.  With a thread a row 3,000 spheres filled 94 warps of the chip (60 pairs each:
-// 1.58 ms); with a warp a row (0.25 ms) rows of 8 pairs left three lanes of four idle.
+// Per-pair couplings of the CSR list: A (I - rr) and B - A, float64 and float32, a pair to a thread, its row by a
+// search in row_ptr: the couplings' float64 instructions bound it, and each costs a warp the same for one active lane
+// as for 32, however many pairs a row has.  With a thread a row 3,000 spheres filled 94 warps of the chip (60 pairs
+// each: 1.58 ms); with a warp a row (0.25 ms) rows of few pairs left most lanes idle (a system of 29,791 spheres with 6
+// pairs a row 2.91 ms a thread a row, 3.61 a warp a row, 2.72 so, of 50,653 with 71 10.5, 10.0 and 8.5).
 __global__ void k_cs_pair_coefs(const int64_t *__restrict__ row_ptr, const int32_t *__restrict__ nbr,
                                 const double *__restrict__ dist, int64_t n, int64_t np,
                                 const double *__restrict__ radius, const int32_t *__restrict__ cls, int64_t M,

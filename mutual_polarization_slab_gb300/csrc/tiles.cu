@@ -678,14 +678,15 @@ int spread_nodes(const double *m, int64_t n, int nrhs, const int32_t *start, con
     return MPS_BAD_ARG;
 }
 
-// Every node of the grid costs: with stencils that cover less than half of the nodes, atomics from a warp a particle are
-// the faster form (three vectors, 96^3, P = 6, 884, 2949, 8847 particles 32 and 50, 46 and 52, 86 and 65 us by atomics
-// and by nodes).  Many particles on few nodes get in each other's way by atomics: 64 particles, 16^3, P = 4 one vector
-// 11.2 and 7.8, 729, 24^3, P = 10 eight vectors 77 and 29, 15,625, 30^3, P = 8 eight 752 and 256 us (with the contraction
-// by home blocks that the lists allow, whole matvecs 1114 and 511).  But the lists of a small grid's few tiles are long
-// where the particles are dense, and one vector gives them to few blocks: 1000 particles, 16^3, P = 14 whole matvecs of
-// one vector 152 and 244, 3375, 24^3, P = 8 99 and 120, 4096, 28^3, P = 6 75 and 87; 729, 24^3, P = 10 82 and 75, 1728,
-// 31^3, P = 12 128 and 105.  The lists cost a system some 45 us once, which the first ten steps of a solve give back.
+// Every node of the grid costs: with stencils that cover less than half of the nodes, atomics from a warp a particle
+// are the faster form (three vectors, 96^3, P = 6, 884, 2949, 8847 particles 32 and 50, 46 and 52, 86 and 65 us by
+// atomics and by nodes).  Many particles on few nodes get in each other's way by atomics: 64 particles, 16^3, P = 4 one
+// vector 11.2 and 7.8, 729, 24^3, P = 10 eight vectors 77 and 29, 15,625, 30^3, P = 8 eight 752 and 256 us (with the
+// contraction by home blocks that the lists allow, whole matvecs 1114 and 511).  But the lists of a small grid's few
+// tiles are long where the particles are dense, and one vector gives them to few blocks: 1000 particles, 16^3, P = 14
+// whole matvecs of one vector 152 and 244, 3375, 24^3, P = 8 99 and 120, 4096, 28^3, P = 6 75 and 87; 729, 24^3, P = 10
+// 82 and 75, 1728, 31^3, P = 12 128 and 105.  The lists cost a system some 45 us once, which the first ten steps of a
+// solve give back.
 bool spread_nodes8_pays(const GridParams &gp, int64_t n, int nrhs) {
     if (nrhs == 1 && gp.G < 30000 && 10 * n >= gp.G) return false;
     return 2.0 * n * gp.P * gp.P * gp.P >= (double)gp.G;
