@@ -16,6 +16,8 @@
 
 #include "quad.cuh"
 
+#include <algorithm>
+
 namespace mps {
 
 __device__ __forceinline__ double to_double(float v) { return float_to_double(v); }
@@ -24,17 +26,20 @@ __device__ __forceinline__ double to_double(double v) { return v; }
 // ---------------------------------------------------------------------------
 // Spread / contract for ncomp (<= 8) moment components per particle.
 // ---------------------------------------------------------------------------
+// Spread: a warp takes every parts-th pass over a particle's (x, y) rows, 32 rows at a time (spread_parts).
 template <typename T>
 __global__ void __launch_bounds__(256) k_spread_gen(const double *__restrict__ m, int64_t n, int nrhs, int ncomp,
-                                                    const int32_t *__restrict__ start, const T *__restrict__ w,
-                                                    GridParams gp, T *__restrict__ grid) {
+                                                    int parts, const int32_t *__restrict__ start,
+                                                    const T *__restrict__ w, GridParams gp, T *__restrict__ grid) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int P = gp.P;
     const int Nx = gp.N[0], Ny = gp.N[1], Nz = gp.N[2];
     const int64_t G = gp.G;
-    for (int64_t t = warp; t < n * nrhs; t += nw) {
+    for (int64_t u = warp; u < n * nrhs * parts; u += nw) {
+        const int64_t t = u / parts;
+        const int part = (int)(u - t * parts);
         const int64_t a = gp.order ? (int64_t)gp.order[t % n] : t % n;
         const int r = (int)(t / n);
         const int sx = start[3 * a], sy = start[3 * a + 1], sz = start[3 * a + 2];
@@ -43,7 +48,7 @@ __global__ void __launch_bounds__(256) k_spread_gen(const double *__restrict__ m
 #pragma unroll
         for (int c = 0; c < 8; ++c) mv[c] = c < ncomp ? (T)m[((int64_t)r * n + a) * ncomp + c] : (T)0;
         T *g0 = grid + (int64_t)r * ncomp * G;
-        for (int row0 = 0; row0 < P * P; row0 += 32) {
+        for (int row0 = 32 * part; row0 < P * P; row0 += 32 * parts) {
             int idx, sub, lpp;
             if (!stencil_row(row0, P, lane, &idx, &sub, &lpp)) continue;
             const int jx = idx % P, jy = idx / P;
@@ -545,11 +550,20 @@ __global__ void k_quad_diag(const double *__restrict__ lam, int64_t total, doubl
 // ---------------------------------------------------------------------------
 // Host wrappers
 // ---------------------------------------------------------------------------
+// Warps to a particle and vector: a stencil of many rows is a long chain of atomics, and few particles leave most SMs
+// without one; its passes over 32 rows go to warps of their own while the GPU has room for them (64 to an SM).
+static int spread_parts(int64_t items, int P) {
+    const int64_t room = 152 * 64 / std::max<int64_t>(items, 1);
+    return (int)std::max<int64_t>(1, std::min<int64_t>(room, (P * P + 31) / 32));
+}
+
 template <typename T>
 int spread_gen(const double *m, int64_t n, int nrhs, int ncomp, const int32_t *start, const T *w,
                const GridParams &gp, T *grid, cudaStream_t s) {
     MPS_CUDA_TRY(cudaMemsetAsync(grid, 0, sizeof(T) * (size_t)ncomp * nrhs * gp.G, s));
-    k_spread_gen<T><<<grid_for(n * nrhs * 32, 256, 152 * 64), 256, 0, s>>>(m, n, nrhs, ncomp, start, w, gp, grid);
+    const int parts = spread_parts(n * nrhs, gp.P);
+    k_spread_gen<T><<<grid_for(n * nrhs * parts * 32, 256, 152 * 64), 256, 0, s>>>(m, n, nrhs, ncomp, parts, start, w,
+                                                                                 gp, grid);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
 }
