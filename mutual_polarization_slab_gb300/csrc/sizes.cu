@@ -743,15 +743,16 @@ int spread_cs(const double *m, int64_t n, int nrhs, const int32_t *start, const 
     if (n == 0) return MPS_OK;
     // 8 vectors per warp pass (the node weights read once per 8 vectors); 4 and 16 measured slower.  Fewer vectors take
     // passes of their own width: the surplus vectors' loads and conversions cost a warp as much as the real ones' (one
-    // vector, 8000 particles, 54^3, P = 8 33 -> 22 us; in float64 1728, 31^3, P = 12 56 -> 46)
+    // vector, 8000 particles, 54^3, P = 8 33 -> 22 us; in float64 1728, 31^3, P = 12 56 -> 46;
+    // three and four in float64 were slower on larger grids, 64^3, P = 12 151 -> 181)
     const int64_t items = n * ((nrhs + 7) / 8);
     // float: bounds of 4 blocks per SM (72.8 ms over the 16-configuration batch's float32 matvecs against 75.8
     // unbounded); double: unbounded (a 64-register cap spills it)
     constexpr int MB = sizeof(T) == 4 ? 4 : 1;
     const auto kernel = nrhs == 1   ? k_spread_cs<T, 1, MB>
                         : nrhs == 2 ? k_spread_cs<T, 2, MB>
-                        : nrhs <= 4 ? k_spread_cs<T, 4, MB>
-                                    : k_spread_cs<T, 8, MB>;
+                        : nrhs <= 4 && sizeof(T) == 4 ? k_spread_cs<T, 4, MB>
+                                                      : k_spread_cs<T, 8, MB>;
     kernel<<<grid_for(items * 32, 256, 152 * 64), 256, 0, s>>>(m, n, nrhs, start, base, g, gp, grid);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
