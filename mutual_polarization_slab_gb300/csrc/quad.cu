@@ -26,8 +26,9 @@ __device__ __forceinline__ double to_double(double v) { return v; }
 // ---------------------------------------------------------------------------
 // Spread / contract for ncomp (<= 8) moment components per particle.
 // ---------------------------------------------------------------------------
-// Spread: a warp takes every parts-th pass over a particle's (x, y) rows, 32 rows at a time (spread_parts).
-template <typename T>
+// Spread: a warp to a particle and vector or, SPLIT, to every parts-th pass over its (x, y) rows, 32 rows at a time
+// (spread_parts).
+template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(256) k_spread_gen(const double *__restrict__ m, int64_t n, int nrhs, int ncomp,
                                                     int parts, const int32_t *__restrict__ start,
                                                     const T *__restrict__ w, GridParams gp, T *__restrict__ grid) {
@@ -37,8 +38,9 @@ __global__ void __launch_bounds__(256) k_spread_gen(const double *__restrict__ m
     const int P = gp.P;
     const int Nx = gp.N[0], Ny = gp.N[1], Nz = gp.N[2];
     const int64_t G = gp.G;
+    if (!SPLIT) parts = 1;
     for (int64_t u = warp; u < n * nrhs * parts; u += nw) {
-        const int64_t t = u / parts;
+        const int64_t t = SPLIT ? u / parts : u;
         const int part = (int)(u - t * parts);
         const int64_t a = gp.order ? (int64_t)gp.order[t % n] : t % n;
         const int r = (int)(t / n);
@@ -562,8 +564,8 @@ int spread_gen(const double *m, int64_t n, int nrhs, int ncomp, const int32_t *s
                const GridParams &gp, T *grid, cudaStream_t s) {
     MPS_CUDA_TRY(cudaMemsetAsync(grid, 0, sizeof(T) * (size_t)ncomp * nrhs * gp.G, s));
     const int parts = spread_parts(n * nrhs, gp.P);
-    k_spread_gen<T><<<grid_for(n * nrhs * parts * 32, 256, 152 * 64), 256, 0, s>>>(m, n, nrhs, ncomp, parts, start, w,
-                                                                                 gp, grid);
+    const auto kernel = parts > 1 ? k_spread_gen<T, true> : k_spread_gen<T, false>;
+    kernel<<<grid_for(n * nrhs * parts * 32, 256, 152 * 64), 256, 0, s>>>(m, n, nrhs, ncomp, parts, start, w, gp, grid);
     MPS_LAUNCH_CHECK();
     return MPS_OK;
 }
