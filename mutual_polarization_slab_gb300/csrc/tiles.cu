@@ -685,11 +685,12 @@ int spread_nodes(const double *m, int64_t n, int nrhs, const int32_t *start, con
 // contraction by home blocks that the lists allow, whole matvecs 1114 and 511).  But the lists of a small grid's few
 // tiles are long where the particles are dense, and one vector gives them to few blocks: 1000 particles, 16^3, P = 14
 // whole matvecs of one vector 152 and 244, 3375, 24^3, P = 8 99 and 120, 4096, 28^3, P = 6 75 and 87; 729, 24^3, P = 10
-// 82 and 75, 1728, 31^3, P = 12 128 and 105.  The lists cost a system some 45 us once, which the first ten steps of a
-// solve give back.
+// 82 and 75, 1728, 31^3, P = 12 128 and 105; beyond one particle to two nodes the nodes win again (solves of 39,304,
+// 30^3, P = 9 29.2 ms by atomics, 27.0 by nodes), and on the smallest grids always (64, 24^3, P = 4 56 and 52 us).  The
+// lists cost a system some 45 us once, which the first ten steps of a solve give back.
 bool spread_nodes8_pays(const GridParams &gp, int64_t n, int nrhs) {
-    if (nrhs == 1 && gp.G < 30000 && 10 * n >= gp.G) return false;
-    return 2.0 * n * gp.P * gp.P * gp.P >= (double)gp.G;
+    if (nrhs == 1 && gp.G < 30000 && 10 * n >= gp.G && 2 * n <= gp.G) return false;
+    return 2.0 * n * gp.P * gp.P * gp.P + 10000.0 >= (double)gp.G;
 }
 
 // Dipole and quadrupole moments: eight components to a vector, one vector to a block.

@@ -1,5 +1,5 @@
-"""Float32 quadrupole matvecs of many particles on small grids, which are spread by nodes whatever the grid's size (and
-contracted by home blocks where particles are many enough).  Tolerance: 2e-5 relative (max-norm), the bar of the operator's
+"""Float32 quadrupole matvecs of many particles on small grids, spread by nodes (and contracted by home blocks where particles
+are many enough), and both sides of the rule's lines: cover, and for one vector particles to a node.  Tolerance: 2e-5 relative (max-norm), the bar of the operator's
 other tests."""
 import numpy as np
 import pytest
@@ -8,7 +8,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("grid,P,n", [((16, 16, 16), 4, 64), ((16, 17, 19), 8, 287), ((16, 17, 19), 8, 288),
-                                      ((24, 8, 9), 6, 60), ((7, 24, 24), 5, 60)])
+                                      ((24, 8, 9), 6, 60), ((7, 24, 24), 5, 60), ((32, 33, 30), 6, 50),
+                                      ((32, 33, 30), 6, 51), ((16, 16, 16), 4, 409), ((16, 16, 16), 4, 410),
+                                      ((8, 8, 8), 4, 256), ((8, 8, 8), 4, 257)])
 @pytest.mark.parametrize("nrhs", [1, 3])
 def test_small_grids(grid, P, n, nrhs):
     from mutual_polarization_slab_gb300 import quadrupole as gq
